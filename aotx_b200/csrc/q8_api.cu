@@ -87,7 +87,7 @@ extern "C" int aotx_q8_init(aotx_q8_ctx **out, int device)
     ctx->scratch.blocks = 2u * ctx->sm_count; /* the decode kernel runs two blocks per SM */
     ctx->scratch.tile_floats = 128ull * kMaxTokenTile;
     size_t partial_bytes = 2u * (size_t)ctx->scratch.blocks * ctx->scratch.tile_floats * sizeof(float);
-    size_t flag_bytes = 2u * (size_t)ctx->scratch.blocks * 4u * sizeof(unsigned int);
+    size_t flag_bytes = 2u * (size_t)ctx->scratch.blocks * q8::kFlagWords * sizeof(unsigned int);
     err = cudaMalloc((void **)&ctx->scratch.partial, partial_bytes);
     if (err == cudaSuccess) {
         err = cudaMalloc((void **)&ctx->scratch.flags, flag_bytes + sizeof(unsigned int));
@@ -107,7 +107,7 @@ extern "C" int aotx_q8_init(aotx_q8_ctx **out, int device)
         delete ctx;
         return code;
     }
-    ctx->scratch.status = ctx->scratch.flags + 2u * (size_t)ctx->scratch.blocks * 4u;
+    ctx->scratch.status = ctx->scratch.flags + 2u * (size_t)ctx->scratch.blocks * q8::kFlagWords;
     *out = ctx;
     return AOTX_Q8_OK;
 }
@@ -177,7 +177,7 @@ extern "C" int aotx_q8_device_status(aotx_q8_ctx *ctx, uint32_t *status, int cle
         // was published and never taken); the next launch would misread them.  Nothing runs
         // now, so the flags of both sets go back to zero together with the status word, which
         // lies right behind them.
-        const size_t words = *status != 0u ? 2u * (size_t)ctx->scratch.blocks * 4u + 1u : 1u;
+        const size_t words = *status != 0u ? 2u * (size_t)ctx->scratch.blocks * q8::kFlagWords + 1u : 1u;
         err = cudaMemset(ctx->scratch.status + 1 - words, 0, words * sizeof(uint32_t));
     }
     if (err != cudaSuccess) {

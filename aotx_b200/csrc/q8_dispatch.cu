@@ -122,6 +122,14 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
         x_bf16 = 0;
     }
 
+#ifdef Q8_HOST_EMULATION
+    const bool warp_kernel = false; // cluster launches and warp-level MMA are not modelled
+#else
+    // Up to 16 rows, one copy of y: the register-fed kernel.  Stores into the peers' copies stay
+    // with the kernel they were measured on.
+    const bool warp_kernel = ntok <= 16u && out == nullptr;
+#endif
+
     CUtensorMap tw, tx;
     {
         cuuint64_t dims[2] = {row_b / 4ull, n};
@@ -135,7 +143,7 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
             return cudaErrorInvalidValue;
         }
     }
-    {
+    if (!warp_kernel) {
         cuuint64_t dims[2] = {k, m};
         cuuint64_t strides[1] = {(cuuint64_t)k * 2ull};
         cuuint32_t box[2] = {kSubK, ntok};
@@ -169,7 +177,7 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     // Two sets of slots and flags alternate between launches, so that a launch whose blocks
     // start early never meets the slots of the launch before it.
     args.partial = scratch.partial + (unsigned long long)(set & 1u) * scratch.blocks * scratch.tile_floats;
-    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * 4u;
+    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * kFlagWords;
     args.overlap = overlap ? 1u : 0u;
     args.group_tiles = nullptr;
     args.group_count = nullptr;
@@ -215,6 +223,11 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
         const unsigned int decode_blocks = decode_grid((unsigned int)row_tiles, k / kSegK, sm_count,
                                                        scratch.blocks, &cluster);
         args.split = cluster;
+#ifndef Q8_HOST_EMULATION
+        if (warp_kernel) {
+            return launch_decode_warp(stream, tw, x, args, decode_blocks, cluster, y_dtype);
+        }
+#endif
         return launch_decode_kernel(stream, tw, tx, args, decode_blocks, cluster, ntok, y_dtype);
     }
     if (ntok <= 128u) {
@@ -275,7 +288,7 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
     args.m_dev = nullptr;
     args.y = y;
     args.partial = scratch.partial + (unsigned long long)(set & 1u) * scratch.blocks * scratch.tile_floats;
-    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * 4u;
+    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * kFlagWords;
     args.status = scratch.status;
     args.tile_floats = scratch.tile_floats;
     args.b_bf16 = 0u;

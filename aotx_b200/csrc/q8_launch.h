@@ -133,8 +133,10 @@ cudaError_t launch_expert_sum_parts(cudaStream_t stream, const ProjParts &proj, 
                                     unsigned int used, void *out, int out_dtype);
 
 // The streaming tensor-core product.  Scratch, in two sets that alternate between launches:
-// `partial` holds one float tile of 128 x token_tile per block of the grid, `flags` four words
-// per block (zero between launches); `status` is one word that kernels only ever OR bits into.
+// `partial` holds one float tile of 128 x token_tile per block of the grid, `flags` kFlagWords
+// words per block (zero between launches); `status` is one word that kernels only ever OR bits into.
+constexpr unsigned int kFlagWords = 8u; // hand-over flags per block: one per warp that publishes
+
 struct UmmaScratch {
     float *partial;
     unsigned int *flags;

@@ -26,7 +26,8 @@
 #define Q8_STATIC_BLOCKS 160u                                     /* at least the SM count */
 #define Q8_STATIC_TILE_FLOATS (128u * Q8_STATIC_MAX_ROWS)         /* one 128 x 64 float tile per block */
 #define Q8_STATIC_PARTIAL_BYTES (Q8_STATIC_BLOCKS * Q8_STATIC_TILE_FLOATS * 4u)
-#define Q8_STATIC_FLAG_WORDS (Q8_STATIC_BLOCKS * 4u + 4u)         /* flags, then the status word */
+#define Q8_STATIC_FLAG_WORDS (Q8_STATIC_BLOCKS * 8u + 4u)         /* flags, then the status word */
+static_assert(q8::kFlagWords == 8u, "the fixed array's flags");
 #define Q8_STATIC_BYTES (Q8_STATIC_PARTIAL_BYTES + Q8_STATIC_FLAG_WORDS * 4u)
 #define Q8_STATIC_DEVICES 64
 
@@ -140,12 +141,12 @@ extern "C" int aotx_q8_matmul_static(void *stream, const void *w, uint32_t type,
     q8::UmmaScratch scratch = {};
     scratch.partial = reinterpret_cast<float *>(dev->base);
     scratch.flags = reinterpret_cast<unsigned int *>(dev->base + Q8_STATIC_PARTIAL_BYTES);
-    scratch.status = scratch.flags + Q8_STATIC_BLOCKS * 4u;
+    scratch.status = scratch.flags + Q8_STATIC_BLOCKS * q8::kFlagWords;
     scratch.blocks = Q8_STATIC_BLOCKS;
     scratch.tile_floats = Q8_STATIC_TILE_FLOATS;
     /* The flags must be zero when a launch starts, and the array keeps what the last call (or
      * a call that was cut short) left behind. */
-    cudaError_t err = cudaMemsetAsync(scratch.flags, 0, Q8_STATIC_BLOCKS * 4u * sizeof(unsigned int), s);
+    cudaError_t err = cudaMemsetAsync(scratch.flags, 0, Q8_STATIC_BLOCKS * q8::kFlagWords * sizeof(unsigned int), s);
     if (err == cudaSuccess) {
         err = q8::launch_umma(s, scratch, dev->sm_count, w, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y,
                               y_dtype, 0u, false);
@@ -164,7 +165,7 @@ extern "C" int aotx_q8_static_status(uint32_t *status, int clear)
         return AOTX_Q8_ERR_CUDA;
     }
     unsigned int *flags = reinterpret_cast<unsigned int *>(dev->base + Q8_STATIC_PARTIAL_BYTES);
-    unsigned int *word = flags + Q8_STATIC_BLOCKS * 4u;
+    unsigned int *word = flags + Q8_STATIC_BLOCKS * q8::kFlagWords;
     cudaError_t err = cudaDeviceSynchronize();
     if (err == cudaSuccess) {
         err = cudaMemcpy(status, word, sizeof(uint32_t), cudaMemcpyDeviceToHost);
@@ -172,7 +173,7 @@ extern "C" int aotx_q8_static_status(uint32_t *status, int clear)
     if (err == cudaSuccess && clear && *status != 0u) {
         /* a launch that was cut short may have left hand-over flags raised: nothing runs now,
          * so they go back to zero together with the word */
-        err = cudaMemset(flags, 0, (Q8_STATIC_BLOCKS * 4u + 1u) * sizeof(unsigned int));
+        err = cudaMemset(flags, 0, (Q8_STATIC_BLOCKS * q8::kFlagWords + 1u) * sizeof(unsigned int));
     }
     if (err != cudaSuccess) {
         return AOTX_Q8_ERR_CUDA;

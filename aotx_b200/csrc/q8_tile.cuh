@@ -639,6 +639,10 @@ cudaError_t launch_decode_kernel(cudaStream_t stream, const CUtensorMap &tw, con
                                  const UmmaArgs &args, unsigned int grid, unsigned int cluster, unsigned int ntok,
                                  int y_dtype);
 
+// Host launcher of the register-fed decode kernel (q8_decode_warp.cu), the same grids.
+cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const void *x, const UmmaArgs &args,
+                               unsigned int grid, unsigned int cluster, int y_dtype);
+
 // Host launcher of the second prefill-regime kernel (q8_wide.cu), token tiles of 256.
 cudaError_t launch_wide_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx,
                                const UmmaArgs &args, unsigned int grid, int y_dtype);
