@@ -93,6 +93,21 @@ __device__ __forceinline__ __half dequant_one(int q, __half d)
     return __float2half_rn((float)q * __half2float(d));
 }
 
+// One lane of a converged warp, the same one every time.  The issuing thread of bulk copies and MMAs is
+// chosen this way and not by its lane number: then the compiler knows that exactly one thread is
+// active and keeps descriptors and addresses in uniform registers.  Chosen by lane number, every
+// tcgen05.mma took 130 cycles whatever its width; chosen by election 23 (N = 16), 42 (N = 64), 74 (N = 128).
+__device__ __forceinline__ bool elect_one()
+{
+#ifdef Q8_HOST_EMULATION
+    return (threadIdx.x & 31u) == 0u;
+#else
+    uint32_t chosen;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+    return chosen != 0u;
+#endif
+}
+
 // ---------------------------------------------------------------------------------------
 // Shared-memory barriers.
 // ---------------------------------------------------------------------------------------

@@ -395,7 +395,7 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
     if (warp == kDecWeightWarp) {
         // ---------------------------------------------------------------- raw weight copies
-        if (lane == 0u) {
+        if (elect_one()) {
             uint32_t g = 0;
             uint32_t tile = tile_begin;
             uint32_t s = seg_begin;
@@ -426,7 +426,7 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const uint32_t total = u_end - u_begin;
         uint32_t next_seg = seg_begin;
         uint32_t issued = 0;
-        if (lane == 0u) {
+        if (elect_one()) {
             grid_dependency_wait();
             Q8_STAMP(2u, true)                     // the launches before this one have finished
             for (; issued < total; ++issued) {
@@ -471,7 +471,7 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             for (uint32_t s = s0; ok && s < s1; ++s, ++g) {
                 const uint32_t xst = g % S::x_depth;
                 const uint32_t xph = (g / S::x_depth) & 1u;
-                if (lane == 0u) {
+                if (elect_one()) {
                     // the x segment has landed and, where it was bfloat16, the converters have
                     // turned it into binary16
                     if (!mbar_wait((args.b_bf16 != 0u ? r.x_full : r.x_land) + 8u * xst, xph, abort_flag,
@@ -516,7 +516,7 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 // lane 0's waits may have run out: every lane leaves together
                 ok = __all_sync(0xFFFFFFFFu, ok) != 0;
             }
-            if (ok && lane == 0u) {
+            if (ok && elect_one()) {
                 umma_commit(r.acc_full);
             }
             u += (s1 - s0);

@@ -152,7 +152,7 @@ q8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
     if (warp == kWeightWarp) {
         // ---------------------------------------------------------------- raw weight copies
-        if (lane == 0u) {
+        if (elect_one()) {
             uint32_t g = 0;
             bool ok = true;
             // the table entry of a tile is fetched one tile ahead: a trip to memory at every
@@ -190,7 +190,7 @@ q8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
     } else if (warp == kInputWarp) {
         // ---------------------------------------------------------------- x copies
-        if (lane == 0u) {
+        if (elect_one()) {
             uint32_t g = 0;
             grid_dependency_wait();
             bool ok = true;
@@ -229,7 +229,7 @@ q8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
     } else if (warp == kMmaWarp) {
         // ---------------------------------------------------------------- MMA issue
-        if (lane == 0u) {
+        if (elect_one()) {
             // bfloat16 activations were turned into binary16 in shared memory by the converters
             uint32_t idesc = umma_idesc(kRows, (uint32_t)NTOK, 0u, 0u);
             uint32_t g = 0;

@@ -158,7 +158,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
     if (warp == kWeightWarp) {
         // ---------------------------------------------------------------- raw weight copies
-        if (lane == 0u) {
+        if (elect_one()) {
             uint32_t g = 0;
             bool ok = true;
             WorkIter work = first_work;
@@ -187,7 +187,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         }
     } else if (warp == kInputWarp) {
         // ---------------------------------------------------------------- x copies
-        if (lane == 0u) {
+        if (elect_one()) {
             uint32_t q = 0;
             grid_dependency_wait();
             bool ok = true;
@@ -217,7 +217,7 @@ q8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         }
     } else if (warp == kMmaWarp) {
         // ---------------------------------------------------------------- MMA issue
-        if (lane == 0u) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc(kRows, (uint32_t)NTOK, args.b_bf16, args.b_bf16);
             uint32_t g = 0;
             uint32_t q = 0;
