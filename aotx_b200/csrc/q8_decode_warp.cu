@@ -276,7 +276,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
     if (split) {
         // every block of the cluster has started (its shared memory may be written) before the exchange
         __syncwarp();
-        cluster_arrive_release();
+        cluster_arrive_relaxed();
     }
     __syncthreads();
 

@@ -18,6 +18,13 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Arrive on the cluster's barrier without ordering any memory access: tells the other blocks that
+// this one has started.  (The releasing form waits for what the thread has in flight.)
+__device__ __forceinline__ void cluster_arrive_relaxed()
+{
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b)
 {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
