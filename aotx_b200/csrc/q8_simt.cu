@@ -55,115 +55,308 @@ __global__ void q8_dequant_kernel(const unsigned char *__restrict__ w, unsigned 
 }
 
 // ---------------------------------------------------------------------------------------
-// Expert router.  One block per token (stepping by the grid), 256 threads.  Logits are float
-// dot products of the float router rows with the half activations, one warp per expert with
-// lanes 32 apart and a shuffle tree; the softmax takes the maximum away; the rank of an
-// expert is the count of experts with a larger probability, or an equal one and a lower
-// index.  The sums run in the same order as the reference kernel's, so the probabilities
-// are the same floats.
+// Expert router.  Logits are float dot products of the float router rows with the half
+// activations: lanes 32 apart along the row, then a shuffle tree; the softmax takes the maximum
+// away; the experts come out in order of probability, equal ones the lower index first.  Every
+// sum runs in the same order as the reference kernel's, so the probabilities are the same floats.
+//
+// A cluster of blocks shares TOKENS tokens: each block takes its share of the experts, a warp
+// EXPERTS of them at a time, and the logits of a token are gathered in the shared memory of the
+// block that finishes it.  What bounds it is the latency of the router rows (1 MB from L2 at 128
+// experts of 2048) as long as tokens are few, and the float additions (tokens * experts * hidden)
+// when they are many: so few tokens per cluster and many loads of a row in flight for a short
+// batch, many tokens per row value for a long one.  One block for all experts of four tokens,
+// one row of eight loads per warp at a time, took 78 us at any number of tokens up to
+// 512 (140 us with the router cold in L2); this takes 10 us for 8 tokens and 26 us for 512 (128 experts, hidden 2048).
 // ---------------------------------------------------------------------------------------
 #define Q8_ROUTE_THREADS 256u
-#define Q8_ROUTE_TOKENS 4u /* tokens that share one pass over the router rows */
+#define Q8_ROUTE_EXPERTS 256u
 
-// One block takes Q8_ROUTE_TOKENS tokens at a time: a warp reads a router row once and forms
-// the dot product of every token of the group with it.  Each (token, expert) sum still adds
-// the same products in the same order as one warp of the reference kernel does (lanes 32
-// apart, then the shuffle tree), so the probabilities are the same floats.
-__global__ void __launch_bounds__(Q8_ROUTE_THREADS)
-q8_route_kernel(const __half *__restrict__ x, const float *__restrict__ router, unsigned int tokens_max,
-                const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                unsigned int used, float *__restrict__ prob, unsigned int *__restrict__ ids)
+// Activations of a group in shared memory, [position along the row][token], rows padded so that
+// 16-byte reads of 8 neighbouring lanes meet 32 different banks.
+template <unsigned int TOKENS>
+struct RouteShape {
+    static constexpr unsigned int stride = TOKENS <= 4u ? TOKENS : TOKENS + 4u;
+};
+
+// One position of the rows: EXPERTS router values by TOKENS activations.
+template <unsigned int TOKENS, unsigned int EXPERTS>
+__device__ __forceinline__ void route_step(const float *at, const float (&r)[EXPERTS], float (&dot)[EXPERTS][TOKENS])
 {
-    // the group's activations as float: [Q8_ROUTE_TOKENS][hidden]
-#ifdef Q8_HOST_EMULATION
-    float *route_x = emulated_dynamic_shared;
-#else
-    extern __shared__ float route_x[];
-#endif
-    __shared__ float probability[Q8_ROUTE_TOKENS][Q8_ROUTE_THREADS];
-    __shared__ float reduce[Q8_ROUTE_THREADS];
+    constexpr unsigned int kTogether = TOKENS < 4u ? TOKENS : 4u;
+#pragma unroll
+    for (unsigned int g0 = 0; g0 < TOKENS; g0 += kTogether) {
+        float xv[kTogether];
+        if (TOKENS >= 4u) {
+            const float4 four = *reinterpret_cast<const float4 *>(at + g0);
+            xv[0] = four.x;
+            xv[1u % kTogether] = four.y;
+            xv[2u % kTogether] = four.z;
+            xv[3u % kTogether] = four.w;
+        } else {
+#pragma unroll
+            for (unsigned int g = 0; g < kTogether; ++g) {
+                xv[g] = at[g];
+            }
+        }
+#pragma unroll
+        for (unsigned int g = 0; g < kTogether; ++g) {
+#pragma unroll
+            for (unsigned int e = 0; e < EXPERTS; ++e) {
+                // the reference's own expression; both compile to one fused multiply-add
+                dot[e][g0 + g] += r[e] * xv[g];
+            }
+        }
+    }
+}
+
+template <unsigned int TOKENS, unsigned int EXPERTS, unsigned int AHEAD>
+__device__ __forceinline__ void route_body(const __half *__restrict__ x, const float *__restrict__ router,
+                                           unsigned int tokens_max, const unsigned int *tokens_dev,
+                                           unsigned int hidden, unsigned int experts, unsigned int used,
+                                           float *__restrict__ prob, unsigned int *__restrict__ ids, float *route_x,
+                                           float (&probability)[TOKENS][Q8_ROUTE_EXPERTS])
+{
+    constexpr unsigned int kStride = RouteShape<TOKENS>::stride;
+    constexpr unsigned int kPerLane = Q8_ROUTE_EXPERTS / 32u;
     unsigned int tokens = tokens_max;
     if (tokens_dev != nullptr) {
         unsigned int live = *tokens_dev;
         tokens = live < tokens_max ? live : tokens_max;
     }
-    unsigned int lane = threadIdx.x & 31u;
-    unsigned int warp = threadIdx.x >> 5;
-    unsigned int e = threadIdx.x;
-    for (unsigned int t0 = blockIdx.x * Q8_ROUTE_TOKENS; t0 < tokens; t0 += gridDim.x * Q8_ROUTE_TOKENS) {
-        unsigned int group = tokens - t0 < Q8_ROUTE_TOKENS ? tokens - t0 : Q8_ROUTE_TOKENS;
-        for (unsigned int at = threadIdx.x; at < Q8_ROUTE_TOKENS * hidden; at += Q8_ROUTE_THREADS) {
-            unsigned int g = at / hidden;
-            route_x[at] = g < group ? __half2float(x[(size_t)(t0 + g) * hidden + (at - g * hidden)]) : 0.0f;
-        }
-        __syncthreads();
-        for (unsigned int ex = warp; ex < experts; ex += Q8_ROUTE_THREADS / 32u) {
-            const float *row = router + (size_t)ex * hidden;
-            float dot[Q8_ROUTE_TOKENS];
+    const unsigned int lane = threadIdx.x & 31u;
+    const unsigned int warp = threadIdx.x >> 5;
+    const unsigned int warps = blockDim.x >> 5;
+    const unsigned int csize = cluster_nctarank();
+    const unsigned int crank = cluster_ctarank();
+    const unsigned int first_expert = crank * experts / csize;
+    const unsigned int last_expert = (crank + 1u) * experts / csize;
+    if (csize > 1u) {
+        // every block has started before another writes into its shared memory
+        cluster_arrive_release();
+        cluster_wait_acquire();
+    }
+    // the blocks of a cluster take the same groups, so they leave this loop together
+    for (unsigned int t0 = blockIdx.x / csize * TOKENS; t0 < tokens; t0 += gridDim.x / csize * TOKENS) {
+        const unsigned int group = tokens - t0 < TOKENS ? tokens - t0 : TOKENS;
+        // one value of every token at a time: the loads of several positions go out together, and the
+        // stores of a warp fill whole bank rows
+#pragma unroll 4
+        for (unsigned int d = threadIdx.x; d < hidden; d += blockDim.x) {
+            float in[TOKENS];
 #pragma unroll
-            for (unsigned int g = 0; g < Q8_ROUTE_TOKENS; ++g) {
-                dot[g] = 0.0f;
+            for (unsigned int g = 0; g < TOKENS; ++g) {
+                in[g] = g < group ? __half2float(x[(size_t)(t0 + g) * hidden + d]) : 0.0f;
             }
-#pragma unroll 8
-            for (unsigned int d = lane; d < hidden; d += 32u) {
-                float r = row[d];
+            if (TOKENS >= 4u) {
 #pragma unroll
-                for (unsigned int g = 0; g < Q8_ROUTE_TOKENS; ++g) {
-                    // the reference's own expression; both compile to one fused multiply-add
-                    dot[g] += r * route_x[g * hidden + d];
+                for (unsigned int g = 0; g < TOKENS; g += 4u) {
+                    *reinterpret_cast<float4 *>(route_x + d * kStride + g) =
+                        make_float4(in[g], in[(g + 1u) % TOKENS], in[(g + 2u) % TOKENS], in[(g + 3u) % TOKENS]);
+                }
+            } else {
+#pragma unroll
+                for (unsigned int g = 0; g < TOKENS; ++g) {
+                    route_x[d * kStride + g] = in[g];
                 }
             }
+        }
+        __syncthreads();
+        for (unsigned int ex = first_expert + warp * EXPERTS; ex < last_expert; ex += warps * EXPERTS) {
+            // rows past the end repeat the last one; their sums are not used
+            const float *row[EXPERTS];
 #pragma unroll
-            for (unsigned int g = 0; g < Q8_ROUTE_TOKENS; ++g) {
+            for (unsigned int e = 0; e < EXPERTS; ++e) {
+                row[e] = router + (size_t)(ex + e < last_expert ? ex + e : last_expert - 1u) * hidden;
+            }
+            float dot[EXPERTS][TOKENS];
+#pragma unroll
+            for (unsigned int e = 0; e < EXPERTS; ++e) {
+#pragma unroll
+                for (unsigned int g = 0; g < TOKENS; ++g) {
+                    dot[e][g] = 0.0f;
+                }
+            }
+            // Whole rounds of AHEAD positions per lane: the values of the next round are on their way
+            // while this one's are used, and every address is a register and a constant.
+            const unsigned int rounds = hidden / (32u * AHEAD);
+            float next[AHEAD][EXPERTS];
+            if (rounds != 0u) {
+#pragma unroll
+                for (unsigned int a = 0; a < AHEAD; ++a) {
+#pragma unroll
+                    for (unsigned int e = 0; e < EXPERTS; ++e) {
+                        next[a][e] = row[e][lane + 32u * a];
+                    }
+                }
+            }
+            const float *at = route_x + lane * kStride;
+            for (unsigned int round = 0; round < rounds; ++round) {
+                float here[AHEAD][EXPERTS];
+#pragma unroll
+                for (unsigned int a = 0; a < AHEAD; ++a) {
+#pragma unroll
+                    for (unsigned int e = 0; e < EXPERTS; ++e) {
+                        here[a][e] = next[a][e];
+                    }
+                }
+                if (round + 1u < rounds) {
+#pragma unroll
+                    for (unsigned int e = 0; e < EXPERTS; ++e) {
+                        row[e] += 32u * AHEAD;
+#pragma unroll
+                        for (unsigned int a = 0; a < AHEAD; ++a) {
+                            next[a][e] = row[e][lane + 32u * a];
+                        }
+                    }
+                }
+#pragma unroll
+                for (unsigned int a = 0; a < AHEAD; ++a) {
+                    route_step<TOKENS, EXPERTS>(at + 32u * a * kStride, here[a], dot);
+                }
+                at += 32u * AHEAD * kStride;
+            }
+            for (unsigned int d = rounds * 32u * AHEAD + lane; d < hidden; d += 32u) {
+                float here[EXPERTS];
+#pragma unroll
+                for (unsigned int e = 0; e < EXPERTS; ++e) {
+                    here[e] = router[(size_t)(ex + e < last_expert ? ex + e : last_expert - 1u) * hidden + d];
+                }
+                route_step<TOKENS, EXPERTS>(route_x + d * kStride, here, dot);
+            }
+#pragma unroll
+            for (unsigned int e = 0; e < EXPERTS; ++e) {
+#pragma unroll
+                for (unsigned int g = 0; g < TOKENS; ++g) {
+                    for (unsigned int step = 16u; step != 0u; step >>= 1) {
+                        dot[e][g] += __shfl_down_sync(0xFFFFFFFFu, dot[e][g], step);
+                    }
+                    if (lane == 0u && ex + e < last_expert) {
+                        if (csize == 1u) {
+                            probability[g][ex + e] = dot[e][g];
+                        } else {
+                            st_shared_cluster_f32(mapa_shared(smem_u32(&probability[g][ex + e]), g % csize), dot[e][g]);
+                        }
+                    }
+                }
+            }
+        }
+        // every logit of the group lies with the block that finishes its token
+        if (csize == 1u) {
+            __syncthreads();
+        } else {
+            __syncwarp();
+            cluster_arrive_release();
+            cluster_wait_acquire();
+        }
+        for (unsigned int g = crank + csize * warp; g < group; g += csize * warps) {
+            // one warp per token, lane holds experts lane, lane + 32, ..
+            const unsigned int t = t0 + g;
+            float value[kPerLane];
+            float sum[kPerLane];
+            float top = -CUDART_INF_F;
+#pragma unroll
+            for (unsigned int j = 0; j < kPerLane; ++j) {
+                const unsigned int e = lane + 32u * j;
+                value[j] = e < experts ? probability[g][e] : -CUDART_INF_F;
+                top = fmaxf(top, value[j]);
+            }
+            for (unsigned int step = 16u; step != 0u; step >>= 1) {
+                top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, step));
+            }
+#pragma unroll
+            for (unsigned int j = 0; j < kPerLane; ++j) {
+                value[j] = lane + 32u * j < experts ? expf(value[j] - top) : 0.0f;
+                sum[j] = value[j];
+            }
+            // the reference's tree over 256 places: halves 128 apart, 64, 32, then within the warp
+#pragma unroll
+            for (unsigned int half = kPerLane / 2u; half != 0u; half >>= 1) {
+#pragma unroll
+                for (unsigned int j = 0; j < half; ++j) {
+                    sum[j] += sum[j + half];
+                }
+            }
+            for (unsigned int step = 16u; step != 0u; step >>= 1) {
+                sum[0] += __shfl_down_sync(0xFFFFFFFFu, sum[0], step);
+            }
+            // lane 0 holds the whole sum: hand it round (every other lane puts in a zero)
+            float total = lane == 0u ? sum[0] : 0.0f;
+            for (unsigned int step = 16u; step != 0u; step >>= 1) {
+                total += __shfl_xor_sync(0xFFFFFFFFu, total, step);
+            }
+#pragma unroll
+            for (unsigned int j = 0; j < kPerLane; ++j) {
+                const unsigned int e = lane + 32u * j;
+                value[j] /= total;
+                if (e < experts) {
+                    prob[(size_t)t * experts + e] = value[j];
+                } else {
+                    value[j] = -1.0f; // below every probability
+                }
+            }
+            // the largest that is left, ties to the lower index, `used` times over
+            for (unsigned int rank = 0; rank < used; ++rank) {
+                float best = -1.0f;
+                float best_at = (float)rank;   // an index as a float: exact, at most 255
+#pragma unroll
+                for (unsigned int j = 0; j < kPerLane; ++j) {
+                    if (value[j] > best) {
+                        best = value[j];
+                        best_at = (float)(lane + 32u * j);
+                    }
+                }
                 for (unsigned int step = 16u; step != 0u; step >>= 1) {
-                    dot[g] += __shfl_down_sync(0xFFFFFFFFu, dot[g], step);
+                    const float other = __shfl_xor_sync(0xFFFFFFFFu, best, step);
+                    const float other_at = __shfl_xor_sync(0xFFFFFFFFu, best_at, step);
+                    if (other > best || (other == best && other_at < best_at)) {
+                        best = other;
+                        best_at = other_at;
+                    }
+                }
+                const unsigned int chosen = (unsigned int)best_at;
+#pragma unroll
+                for (unsigned int j = 0; j < kPerLane; ++j) {
+                    if (lane + 32u * j == chosen) {
+                        value[j] = -1.0f;
+                    }
                 }
                 if (lane == 0u) {
-                    probability[g][ex] = dot[g];
+                    ids[(size_t)t * used + rank] = chosen;
                 }
             }
         }
-        __syncthreads();
-        for (unsigned int g = 0; g < group; ++g) {
-            unsigned int t = t0 + g;
-            reduce[e] = e < experts ? probability[g][e] : -CUDART_INF_F;
+        // the next group's activations and logits come after everyone has read this one's
+        if (csize == 1u) {
             __syncthreads();
-            for (unsigned int step = Q8_ROUTE_THREADS / 2u; step != 0u; step >>= 1) {
-                if (e < step) {
-                    reduce[e] = fmaxf(reduce[e], reduce[e + step]);
-                }
-                __syncthreads();
-            }
-            float value = e < experts ? expf(probability[g][e] - reduce[0]) : 0.0f;
-            __syncthreads();
-            reduce[e] = value;
-            __syncthreads();
-            for (unsigned int step = Q8_ROUTE_THREADS / 2u; step != 0u; step >>= 1) {
-                if (e < step) {
-                    reduce[e] += reduce[e + step];
-                }
-                __syncthreads();
-            }
-            if (e < experts) {
-                value /= reduce[0];
-                probability[g][e] = value;
-                prob[(size_t)t * experts + e] = value;
-            }
-            __syncthreads();
-            if (e < experts) {
-                unsigned int rank = 0u;
-                for (unsigned int other = 0u; other < experts; ++other) {
-                    float candidate = probability[g][other];
-                    rank += (candidate > value || (candidate == value && other < e)) ? 1u : 0u;
-                }
-                if (rank < used) {
-                    ids[(size_t)t * used + rank] = e;
-                }
-            }
-            __syncthreads();
+        } else {
+            __syncwarp();
+            cluster_arrive_release();
+            cluster_wait_acquire();
         }
     }
 }
+
+#define Q8_ROUTE_KERNEL(NAME, TOKENS, EXPERTS, AHEAD)                                                                \
+    __global__ void __launch_bounds__(Q8_ROUTE_THREADS)                                                             \
+    NAME(const __half *__restrict__ x, const float *__restrict__ router, unsigned int tokens_max,                   \
+         const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts, unsigned int used,              \
+         float *__restrict__ prob, unsigned int *__restrict__ ids)                                                  \
+    {                                                                                                               \
+        Q8_ROUTE_DYNAMIC                                                                                            \
+        __shared__ float probability[TOKENS][Q8_ROUTE_EXPERTS];                                                     \
+        route_body<TOKENS, EXPERTS, AHEAD>(x, router, tokens_max, tokens_dev, hidden, experts, used, prob, ids,     \
+                                           route_x, probability);                                                   \
+    }
+#ifdef Q8_HOST_EMULATION
+#define Q8_ROUTE_DYNAMIC float *route_x = emulated_dynamic_shared;
+#else
+#define Q8_ROUTE_DYNAMIC extern __shared__ __align__(16) float route_x[];
+#endif
+// rows too long for eight tokens in shared memory; short batches; long ones
+Q8_ROUTE_KERNEL(q8_route_kernel, 4u, 2u, 4u)
+Q8_ROUTE_KERNEL(q8_route_kernel_few, 2u, 2u, 16u)
+Q8_ROUTE_KERNEL(q8_route_kernel_many, 8u, 4u, 4u)
 
 // ---------------------------------------------------------------------------------------
 // Per-pair expert products (pair = token t, rank r; index t * used + r).  These re-read an
@@ -398,19 +591,52 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     if (tokens == 0u) {
         return cudaSuccess;
     }
-    unsigned int groups = (tokens + Q8_ROUTE_TOKENS - 1u) / Q8_ROUTE_TOKENS;
-    unsigned int grid = groups < 148u * 8u ? groups : 148u * 8u;
-    size_t smem = (size_t)Q8_ROUTE_TOKENS * hidden * sizeof(float);
-    if (smem > 160u * 1024u) {
+#ifdef Q8_HOST_EMULATION
+    // a cluster of one block: it takes all experts
+    const size_t emulated = (size_t)RouteShape<4u>::stride * hidden * sizeof(float);
+    const unsigned int emulated_grid = (tokens + 3u) / 4u;
+    return launch_kernel(q8_route_kernel, emulated_grid, Q8_ROUTE_THREADS, emulated, stream, static_cast<const __half *>(x),
+                         router, tokens, tokens_dev, hidden, experts, used, prob, ids);
+#else
+    // Few tokens: two to a cluster of eight blocks, until the clusters fill the GPU (32 of them are
+    // 256 blocks).  More: eight tokens to a cluster of four, which quarters the reads of the router;
+    // eight tokens of a row longer than 4096 no longer leave room for two blocks on an SM.
+    const bool few = tokens <= 64u;
+    const bool many = !few && hidden <= 4096u;
+    const unsigned int group = few ? 2u : (many ? 8u : 4u);
+    const unsigned int cluster = many ? 4u : 8u;
+    const unsigned int stride = few ? RouteShape<2u>::stride : (many ? RouteShape<8u>::stride : RouteShape<4u>::stride);
+    const size_t smem = (size_t)stride * hidden * sizeof(float);
+    if (smem > 200u * 1024u) {
         return cudaErrorInvalidValue;
     }
-    static unsigned long long configured = 0ull;
-    cudaError_t err = allow_shared_memory(q8_route_kernel, 160u * 1024u, &configured);
+    unsigned int clusters = (tokens + group - 1u) / group;
+    const unsigned int most = 148u * 4u / cluster;
+    clusters = clusters < most ? clusters : most;
+    static unsigned long long configured[3] = {0ull, 0ull, 0ull};
+    void (*const kernels[3])(const __half *, const float *, unsigned int, const unsigned int *, unsigned int, unsigned int,
+                             unsigned int, float *, unsigned int *) = {q8_route_kernel, q8_route_kernel_few,
+                                                                       q8_route_kernel_many};
+    const unsigned int which = few ? 1u : (many ? 2u : 0u);
+    cudaError_t err = allow_shared_memory(kernels[which], 200u * 1024u, &configured[which]);
     if (err != cudaSuccess) {
         return err;
     }
-    return launch_kernel(q8_route_kernel, grid, Q8_ROUTE_THREADS, smem, stream, static_cast<const __half *>(x), router,
-                         tokens, tokens_dev, hidden, experts, used, prob, ids);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(clusters * cluster, 1, 1);
+    config.blockDim = dim3(Q8_ROUTE_THREADS, 1, 1);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = cluster;
+    attribute[0].val.clusterDim.y = 1;
+    attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernels[which], static_cast<const __half *>(x), router, tokens, tokens_dev, hidden,
+                              experts, used, prob, ids);
+#endif
 }
 
 cudaError_t launch_expert_pairs_simt(cudaStream_t stream, const void *w_gate, const void *w_up,
