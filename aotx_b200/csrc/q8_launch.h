@@ -94,6 +94,13 @@ cudaError_t launch_gemv_any(cudaStream_t stream, const void *w, unsigned int typ
                             unsigned int k, const void *x, int x_bf16, unsigned int m,
                             const unsigned int *m_dev, void *y, int y_dtype);
 
+// The same products on the warp-level tensor path (q_warp.cu): the types and alignments it takes
+// (Q8_0 among them, rows of any multiple of 32 weights), and the launch.
+bool warp_any_supports(const void *w, unsigned int type, unsigned int n, unsigned int k, const void *x, unsigned int m);
+cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int type, unsigned int n, unsigned int k,
+                            const void *x, int x_bf16, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
+                            unsigned int epilogue);
+
 cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
                          unsigned int used, float *prob, unsigned int *ids);

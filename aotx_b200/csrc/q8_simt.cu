@@ -567,6 +567,11 @@ cudaError_t launch_gemv_simt(cudaStream_t stream, const void *w, unsigned int n,
         || epilogue > kEpilogueSwiglu) {
         return cudaErrorInvalidValue;
     }
+#ifndef Q8_HOST_EMULATION
+    if (warp_any_supports(w, Q8_TYPE_Q8_0, n, k, x, m)) {
+        return launch_warp_any(stream, w, Q8_TYPE_Q8_0, n, k, x, x_bf16, m, m_dev, y, y_dtype, epilogue);
+    }
+#endif
 #define Q8_CASE(XT, YD, YT)                                                                      \
     if (y_dtype == (YD)) {                                                                       \
         return launch_gemv_simt_typed<XT, YT>(stream, w, n, k, x, m, m_dev, y, epilogue);        \

@@ -221,6 +221,11 @@ cudaError_t launch_gemv_any(cudaStream_t stream, const void *w, unsigned int typ
     if (n == 0u || m == 0u) {
         return cudaSuccess;
     }
+#ifndef Q8_HOST_EMULATION
+    if (warp_any_supports(w, type, n, k, x, m)) {
+        return launch_warp_any(stream, w, type, n, k, x, x_bf16, m, m_dev, y, y_dtype, kEpilogueStore);
+    }
+#endif
 #define QG_CASE(XT, YD, YT)                                                                       \
     if (y_dtype == (YD)) {                                                                       \
         return launch_gemv_any_typed<XT, YT>(stream, w, type, n, k, x, m, m_dev, y);             \
