@@ -96,21 +96,31 @@ __device__ __forceinline__ float half_bits(uint32_t bits)
     return __half2float(__ushort_as_half((unsigned short)bits));
 }
 
-// A word at an even shared-memory address (WORDS: a multiple of 4).
-template <bool WORDS>
-__device__ __forceinline__ uint32_t word_at(const unsigned char *at)
+// Where a row of a piece lies in the warp's ring: a word index, and whether its bytes start in the
+// middle of that word (rows start at any even address).  Every read below is then at a constant
+// distance from that index, and a word that straddles two is put together with a selector that is
+// one of two constants per row.
+struct RowAt {
+    const uint32_t *words;         // the word that holds (or precedes by two bytes) the first byte
+    const unsigned char *bytes;    // the first byte
+    uint32_t even, odd;            // selectors of a word at a distance of 4 i and 4 i + 2 bytes
+};
+
+// The word `C` + 4 * t bytes from the start of the row's piece (C even).
+template <bool WORDS, uint32_t C>
+__device__ __forceinline__ uint32_t word_at(const RowAt &row, uint32_t t)
 {
-    if (WORDS) {
-        return *reinterpret_cast<const uint32_t *>(at);
+    if constexpr (WORDS) {
+        return row.words[C / 4u + t];
+    } else {
+        return prmt(row.words[C / 4u + t], row.words[C / 4u + t + 1u], C % 4u == 0u ? row.even : row.odd);
     }
-    const uintptr_t address = reinterpret_cast<uintptr_t>(at);
-    const uint32_t *two = reinterpret_cast<const uint32_t *>(address & ~(uintptr_t)3);
-    return prmt(two[0], two[1], (address & 2u) != 0u ? 0x5432u : 0x3210u);
 }
 
-__device__ __forceinline__ uint32_t u16_at(const unsigned char *at)
+template <uint32_t C>
+__device__ __forceinline__ uint32_t u16_at(const RowAt &row)
 {
-    return *reinterpret_cast<const unsigned short *>(at);
+    return reinterpret_cast<const unsigned short *>(row.bytes)[C / 2u];
 }
 
 // Bits b0..b3 of `four` as bit 4 of the four bytes of a word.
@@ -120,62 +130,73 @@ __device__ __forceinline__ uint32_t fifth_bits(uint32_t four)
     return ((four | (four << 7) | (four << 14) | (four << 21)) & 0x01010101u) << 4;
 }
 
-// The codes of four runs of 32 weights (runs 4 * half .. + 3 of the piece at `at`) that lane t of a
-// row's four lanes holds: codes[run][step], weights 16 step + 4t .. + 3; and the runs' scales and
-// offsets (SIXTEENS: scales[2 * run + step]).
-template <uint32_t TYPE>
-__device__ __forceinline__ void four_runs(const unsigned char *at, uint32_t half, uint32_t t, uint32_t (&codes)[4][2],
-                                          float (&scale)[8], float (&off)[4])
+// One run of 32 weights of the formats whose block is a run (run R of the piece).
+template <uint32_t TYPE, uint32_t R>
+__device__ __forceinline__ void one_run(const RowAt &row, uint32_t t, uint32_t (&codes)[4][2], float (&scale)[8], float (&off)[4])
 {
     using S = AnyShape<TYPE>;
     constexpr bool W = S::words;
+    constexpr uint32_t at = R * S::block_bytes;
+    scale[R] = half_bits(u16_at<at>(row));
     if constexpr (TYPE == kTypeQ8_0) {
-#pragma unroll
-        for (uint32_t r = 0; r < 4u; ++r) {
-            const unsigned char *one = at + r * 34u;
-            scale[r] = half_bits(u16_at(one));
-            codes[r][0] = word_at<W>(one + 2u + 4u * t);
-            codes[r][1] = word_at<W>(one + 18u + 4u * t);
-        }
-    } else if constexpr (TYPE == kTypeQ4_0 || TYPE == kTypeQ4_1 || TYPE == kTypeQ5_0 || TYPE == kTypeQ5_1) {
+        codes[R][0] = word_at<W, at + 2u>(row, t);
+        codes[R][1] = word_at<W, at + 18u>(row, t);
+    } else {
         constexpr bool five = TYPE == kTypeQ5_0 || TYPE == kTypeQ5_1;
         constexpr uint32_t head = S::offset ? 4u : 2u;
-#pragma unroll
-        for (uint32_t r = 0; r < 4u; ++r) {
-            const unsigned char *one = at + r * S::block_bytes;
-            scale[r] = half_bits(u16_at(one));
-            off[r] = S::offset ? half_bits(u16_at(one + 2u)) : 0.0f;
-            const uint32_t pairs = word_at<W>(one + head + (five ? 4u : 0u) + 4u * t);
-            codes[r][0] = pairs & 0x0F0F0F0Fu;
-            codes[r][1] = (pairs >> 4) & 0x0F0F0F0Fu;
-            if (five) {
-                const uint32_t bits = word_at<W>(one + head);
-                codes[r][0] |= fifth_bits(bits >> (4u * t));
-                codes[r][1] |= fifth_bits(bits >> (16u + 4u * t));
-            }
+        if constexpr (S::offset) {
+            off[R] = half_bits(u16_at<at + 2u>(row));
         }
+        const uint32_t pairs = word_at<W, at + head + (five ? 4u : 0u)>(row, t);
+        codes[R][0] = pairs & 0x0F0F0F0Fu;
+        codes[R][1] = (pairs >> 4) & 0x0F0F0F0Fu;
+        if constexpr (five) {
+            const uint32_t bits = word_at<W, at + head>(row, 0u);
+            codes[R][0] |= fifth_bits(bits >> (4u * t));
+            codes[R][1] |= fifth_bits(bits >> (16u + 4u * t));
+        }
+    }
+}
+
+// The codes of four runs of 32 weights (runs 4 * HALF .. + 3 of the piece) that lane t of a
+// row's four lanes holds: codes[run][step], weights 16 step + 4t .. + 3; and the runs' scales and
+// offsets (Q6_K: scale[2 * run + step]).
+template <uint32_t TYPE, uint32_t HALF>
+__device__ __forceinline__ void four_runs(const RowAt &row, uint32_t t, uint32_t (&codes)[4][2], float (&scale)[8],
+                                          float (&off)[4])
+{
+    using S = AnyShape<TYPE>;
+    constexpr bool W = S::words;
+    if constexpr (!S::super) {
+        one_run<TYPE, 0>(row, t, codes, scale, off);
+        one_run<TYPE, 1>(row, t, codes, scale, off);
+        one_run<TYPE, 2>(row, t, codes, scale, off);
+        one_run<TYPE, 3>(row, t, codes, scale, off);
     } else if constexpr (TYPE == kTypeQ4_K || TYPE == kTypeQ5_K) {
-        const uint32_t both = *reinterpret_cast<const uint32_t *>(at);
-        const float d = half_bits(both & 0xFFFFu);
-        const float dmin = half_bits(both >> 16);
+        const float d = half_bits(row.words[0] & 0xFFFFu);
+        const float dmin = half_bits(row.words[0] >> 16);
         // twelve bytes of 6-bit scales and minima: words p0 (scales 0-3 and two bits of 4-7), p1
         // (minima likewise), p2 (four bits each of scales and minima 4-7)
-        const uint32_t p0 = *reinterpret_cast<const uint32_t *>(at + 4u);
-        const uint32_t p1 = *reinterpret_cast<const uint32_t *>(at + 8u);
-        const uint32_t p2 = *reinterpret_cast<const uint32_t *>(at + 12u);
-        const uint32_t sc = half == 0u ? p0 & 0x3F3F3F3Fu : (p2 & 0x0F0F0F0Fu) | ((p0 >> 2) & 0x30303030u);
-        const uint32_t mn = half == 0u ? p1 & 0x3F3F3F3Fu : ((p2 >> 4) & 0x0F0F0F0Fu) | ((p1 >> 2) & 0x30303030u);
+        const uint32_t p0 = row.words[1];
+        const uint32_t p1 = row.words[2];
+        uint32_t sc = p0 & 0x3F3F3F3Fu;
+        uint32_t mn = p1 & 0x3F3F3F3Fu;
+        if constexpr (HALF != 0u) {
+            const uint32_t p2 = row.words[3];
+            sc = (p2 & 0x0F0F0F0Fu) | ((p0 >> 2) & 0x30303030u);
+            mn = ((p2 >> 4) & 0x0F0F0F0Fu) | ((p1 >> 2) & 0x30303030u);
+        }
 #pragma unroll
         for (uint32_t r = 0; r < 4u; ++r) {
             scale[r] = d * (float)((sc >> (8u * r)) & 0xFFu);
             off[r] = -(dmin * (float)((mn >> (8u * r)) & 0xFFu));
         }
-        const unsigned char *nibbles = at + (TYPE == kTypeQ5_K ? 48u : 16u) + half * 64u + 4u * t;
+        constexpr uint32_t nibbles = (TYPE == kTypeQ5_K ? 48u : 16u) + HALF * 64u;
 #pragma unroll
         for (uint32_t c = 0; c < 2u; ++c) {
 #pragma unroll
             for (uint32_t step = 0; step < 2u; ++step) {
-                const uint32_t w = *reinterpret_cast<const uint32_t *>(nibbles + c * 32u + step * 16u);
+                const uint32_t w = row.words[nibbles / 4u + c * 8u + step * 4u + t];
                 codes[2u * c][step] = w & 0x0F0F0F0Fu;
                 codes[2u * c + 1u][step] = (w >> 4) & 0x0F0F0F0Fu;
             }
@@ -183,7 +204,7 @@ __device__ __forceinline__ void four_runs(const unsigned char *at, uint32_t half
         if constexpr (TYPE == kTypeQ5_K) {
 #pragma unroll
             for (uint32_t step = 0; step < 2u; ++step) {
-                const uint32_t w = *reinterpret_cast<const uint32_t *>(at + 16u + step * 16u + 4u * t) >> (4u * half);
+                const uint32_t w = row.words[4u + step * 4u + t] >> (4u * HALF);
 #pragma unroll
                 for (uint32_t r = 0; r < 4u; ++r) {
                     codes[r][step] |= ((w >> r) & 0x01010101u) << 4;
@@ -192,22 +213,23 @@ __device__ __forceinline__ void four_runs(const unsigned char *at, uint32_t half
         }
     } else {
         // Q6_K: the half's 128 weights are four quarters of 32
-        const float d = half_bits(u16_at(at + 208u));
+        const float d = half_bits(u16_at<208>(row));
 #pragma unroll
         for (uint32_t step = 0; step < 2u; ++step) {
-            const uint32_t n0 = word_at<W>(at + half * 64u + step * 16u + 4u * t);
-            const uint32_t n1 = word_at<W>(at + half * 64u + 32u + step * 16u + 4u * t);
-            const uint32_t up = word_at<W>(at + 128u + half * 32u + step * 16u + 4u * t);
-            codes[0][step] = (n0 & 0x0F0F0F0Fu) | ((up & 0x03030303u) << 4);
-            codes[1][step] = (n1 & 0x0F0F0F0Fu) | (((up >> 2) & 0x03030303u) << 4);
-            codes[2][step] = ((n0 >> 4) & 0x0F0F0F0Fu) | (((up >> 4) & 0x03030303u) << 4);
-            codes[3][step] = ((n1 >> 4) & 0x0F0F0F0Fu) | (((up >> 6) & 0x03030303u) << 4);
+            const uint32_t n0 = step == 0u ? word_at<W, HALF * 64u>(row, t) : word_at<W, HALF * 64u + 16u>(row, t);
+            const uint32_t n1 = step == 0u ? word_at<W, HALF * 64u + 32u>(row, t) : word_at<W, HALF * 64u + 48u>(row, t);
+            const uint32_t up = step == 0u ? word_at<W, 128u + HALF * 32u>(row, t) : word_at<W, 144u + HALF * 32u>(row, t);
+            codes[0][step] = (n0 & 0x0F0F0F0Fu) | ((up << 4) & 0x30303030u);
+            codes[1][step] = (n1 & 0x0F0F0F0Fu) | ((up << 2) & 0x30303030u);
+            codes[2][step] = ((n0 >> 4) & 0x0F0F0F0Fu) | (up & 0x30303030u);
+            codes[3][step] = ((n1 >> 4) & 0x0F0F0F0Fu) | ((up >> 2) & 0x30303030u);
         }
+        const uint32_t s0 = word_at<W, 192u + 8u * HALF>(row, 0u);
+        const uint32_t s1 = word_at<W, 196u + 8u * HALF>(row, 0u);
 #pragma unroll
-        for (uint32_t r = 0; r < 4u; ++r) {
-            const uint32_t two = u16_at(at + 192u + 8u * half + 2u * r);
-            scale[2u * r] = d * (float)(int)(signed char)(two & 0xFFu);
-            scale[2u * r + 1u] = d * (float)(int)(signed char)(two >> 8);
+        for (uint32_t i = 0; i < 4u; ++i) {
+            scale[i] = d * (float)(int)(signed char)(s0 >> (8u * i));
+            scale[4u + i] = d * (float)(int)(signed char)(s1 >> (8u * i));
         }
     }
 }
@@ -227,7 +249,7 @@ __global__ void __launch_bounds__(kAnyWarps * 32u, 2)
 q_gemv_any_kernel_warp(const AnyArgs args)
 {
     using S = AnyShape<TYPE>;
-    extern __shared__ unsigned char any_smem_[];
+    extern __shared__ __align__(16) unsigned char any_smem_[];
     __shared__ float parts[2][kAnyWarps][8u * TILES][kAnyRows];   // partial sums of the 8 warps, two row groups in turn
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
@@ -249,36 +271,47 @@ q_gemv_any_kernel_warp(const AnyArgs args)
     const uint32_t groups = (args.n + kAnyRows - 1u) / kAnyRows;
     const uint32_t my_groups = (groups - blockIdx.y + gridDim.y - 1u) / gridDim.y;
     const uint32_t items = my_groups * my_pieces;   // the host keeps this below 2^32
-    unsigned char *const ring = any_smem_ + warp * S::warp_bytes;
-    const uint32_t ring_at = smem_u32(ring);
+    const uint32_t ring_at = smem_u32(any_smem_) + warp * S::warp_bytes;
 
-    // item i of this warp: piece first_piece + i % my_pieces of the rows of group i / my_pieces
+    // Item i of this warp: piece first_piece + i % my_pieces of the rows of group i / my_pieces.
+    // Neighbouring lanes copy neighbouring 16-byte units of a row, then those of the next row.  (Two
+    // lanes to a row, every other unit each, saves the address arithmetic below and is slower: an
+    // instruction then touches 16 rows, and the copies queue up: 15.2 us against 12.9 at 5003 x 2912.)
+    constexpr uint32_t kLaneCopies = (kAnyRows * S::units + 31u) / 32u;
+    uint32_t copy_from[kLaneCopies];     // distance of this lane's rows from the group's first one
+#pragma unroll
+    for (uint32_t i = 0; i < kLaneCopies; ++i) {
+        copy_from[i] = (lane + 32u * i) / S::units * (uint32_t)args.row_bytes;
+    }
     uint32_t ahead_group = blockIdx.y;
     uint32_t ahead_piece = 0u;
+    const unsigned long long group_bytes = args.row_bytes * kAnyRows;
+    const unsigned char *ahead_rows = args.w + ahead_group * group_bytes + (unsigned long long)first_piece * S::piece_bytes;
     auto issue = [&](uint32_t item) {
         if (item < items) {
-            const unsigned char *base = args.w + (unsigned long long)ahead_group * kAnyRows * args.row_bytes
-                                      + (unsigned long long)(first_piece + ahead_piece) * S::piece_bytes;
-            const uint32_t rows = args.n - ahead_group * kAnyRows < kAnyRows ? args.n - ahead_group * kAnyRows : kAnyRows;
-            // the last piece of a row can be short
-            const uint32_t left = (runs - (first_piece + ahead_piece) * S::piece_runs) * 32u;
-            const uint32_t bytes = S::super || left >= 128u ? S::piece_bytes : left / 32u * S::block_bytes;
-            const uint32_t slot0 = ring_at + (item % kAnyDepth) * S::stage;
+            const unsigned char *base = ahead_rows + ahead_piece * S::piece_bytes;
+            // the last piece of a row can be short; rows past the last copy nothing
+            uint32_t bytes = S::piece_bytes;
+            if (!S::super && first_piece + ahead_piece + 1u == pieces) {
+                bytes = (runs - (pieces - 1u) * S::piece_runs) * S::block_bytes;
+            }
+            const uint32_t rows = args.n - ahead_group * kAnyRows;
+            const uint32_t to = ring_at + (item % kAnyDepth) * S::stage;
 #pragma unroll
-            for (uint32_t i = 0; i < (kAnyRows * S::units + 31u) / 32u; ++i) {
-                const uint32_t at = lane + 32u * i;
-                const uint32_t row = at / S::units;
-                const uint32_t unit = at - row * S::units;
-                const unsigned char *from = base + row * args.row_bytes;
+            for (uint32_t i = 0; i < kLaneCopies; ++i) {
+                const uint32_t row = (lane + 32u * i) / S::units;
+                const uint32_t unit = (lane + 32u * i) % S::units;
+                const unsigned char *from = base + copy_from[i];
                 const uint32_t shift = (uint32_t)reinterpret_cast<uintptr_t>(from) & 15u;
                 // only units that hold a byte of the piece: nothing past the tensor's own 16-byte units
-                if (row < rows && unit * 16u < shift + bytes) {
-                    copy_async_16(slot0 + row * S::slot + unit * 16u, from - shift + unit * 16u);
+                if (row < rows && row < kAnyRows && unit * 16u < shift + bytes) {
+                    copy_async_16(to + row * S::slot + unit * 16u, from - shift + unit * 16u);
                 }
             }
             if (++ahead_piece == my_pieces) {
                 ahead_piece = 0u;
                 ahead_group += gridDim.y;
+                ahead_rows += gridDim.y * group_bytes;
             }
         }
         copy_async_commit();
@@ -288,17 +321,23 @@ q_gemv_any_kernel_warp(const AnyArgs args)
         issue(i);
     }
 
-    const unsigned short *x = static_cast<const unsigned short *>(args.x);
-    // this lane's row of x per column of eight (past the batch: the last row; those sums are not stored)
+    // this lane's row of x per column of eight (past the batch: the last row; those sums are not
+    // stored), from the warp's first weight on
     const unsigned short *x_row[TILES];
 #pragma unroll
     for (uint32_t j = 0; j < TILES; ++j) {
         const uint32_t token = token0 + 8u * j + g;
-        x_row[j] = x + (size_t)(token < m ? token : m - 1u) * args.k + 4u * t;
+        x_row[j] = static_cast<const unsigned short *>(args.x) + (size_t)(token < m ? token : m - 1u) * args.k
+                 + first_piece * S::piece_runs * 32u + 4u * t;
     }
+    // where this lane's rows g and g + 8 start modulo 16 bytes, at the warp's first piece of a group
+    const uint32_t row_shift = (uint32_t)(reinterpret_cast<uintptr_t>(args.w) + g * args.row_bytes
+                                          + (unsigned long long)first_piece * S::piece_bytes);
+    const uint32_t eight_rows = (uint32_t)(8u * args.row_bytes);
     uint32_t item = 0u;
     for (uint32_t turn = 0; turn < my_groups; ++turn) {
         const uint32_t group = blockIdx.y + turn * gridDim.y;
+        const uint32_t group_shift = row_shift + group * (uint32_t)group_bytes;
         float acc[TILES][4];
 #pragma unroll
         for (uint32_t j = 0; j < TILES; ++j) {
@@ -307,19 +346,21 @@ q_gemv_any_kernel_warp(const AnyArgs args)
                 acc[j][i] = 0.0f;
             }
         }
+#pragma unroll 1
         for (uint32_t piece = 0; piece < my_pieces; ++piece, ++item) {
             const uint32_t run0 = (first_piece + piece) * S::piece_runs;
+            // a short last piece: its missing runs hold whatever the slot held before and are passed over
+            const uint32_t live_runs = S::super ? 8u : (runs - run0 < 4u ? runs - run0 : 4u);
             uint2 xv[TILES][4][2];
             auto fetch_x = [&](uint32_t half) {
 #pragma unroll
                 for (uint32_t j = 0; j < TILES; ++j) {
+                    const uint2 *from = reinterpret_cast<const uint2 *>(x_row[j] + piece * (S::piece_runs * 32u) + half * 128u);
 #pragma unroll
                     for (uint32_t r = 0; r < 4u; ++r) {
-                        const uint32_t run = run0 + 4u * half + r;
-#pragma unroll
-                        for (uint32_t step = 0; step < 2u; ++step) {
-                            xv[j][r][step] = run < runs ? __ldg(reinterpret_cast<const uint2 *>(x_row[j] + (size_t)run * 32u + 16u * step))
-                                                        : make_uint2(0u, 0u);
+                        if (S::super || r < live_runs) {
+                            xv[j][r][0] = __ldg(from + r * 8u);
+                            xv[j][r][1] = __ldg(from + r * 8u + 4u);
                         }
                     }
                 }
@@ -328,14 +369,15 @@ q_gemv_any_kernel_warp(const AnyArgs args)
             copy_async_wait<kAnyDepth - 2>();
             __syncwarp();
             issue(item + kAnyDepth - 1u);
-            const unsigned char *slot = ring + (item % kAnyDepth) * S::stage;
-            const unsigned char *at[2];
+            RowAt rows[2];
 #pragma unroll
             for (uint32_t r = 0; r < 2u; ++r) {
-                const uint32_t row = g + 8u * r;
-                const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(args.w) + ((unsigned long long)group * kAnyRows + row) * args.row_bytes
-                                                  + (unsigned long long)(first_piece + piece) * S::piece_bytes) & 15u;
-                at[r] = slot + row * S::slot + shift;
+                const uint32_t shift = (group_shift + r * eight_rows + piece * S::piece_bytes) & 15u;
+                const uint32_t at = warp * S::warp_bytes + (item % kAnyDepth) * S::stage + (g + 8u * r) * S::slot + shift;
+                rows[r].bytes = any_smem_ + at;
+                rows[r].words = reinterpret_cast<const uint32_t *>(any_smem_ + (at & ~3u));
+                rows[r].even = (at & 2u) != 0u ? 0x5432u : 0x3210u;
+                rows[r].odd = (at & 2u) != 0u ? 0x7654u : 0x5432u;
             }
 #pragma unroll
             for (uint32_t half = 0; half < S::piece_runs / 4u; ++half) {
@@ -345,13 +387,16 @@ q_gemv_any_kernel_warp(const AnyArgs args)
                 uint32_t codes[2][4][2];
                 float scale[2][8];
                 float off[2][4];
-                four_runs<TYPE>(at[0], half, t, codes[0], scale[0], off[0]);
-                four_runs<TYPE>(at[1], half, t, codes[1], scale[1], off[1]);
+                if (half == 0u) {
+                    four_runs<TYPE, 0>(rows[0], t, codes[0], scale[0], off[0]);
+                    four_runs<TYPE, 0>(rows[1], t, codes[1], scale[1], off[1]);
+                } else {
+                    four_runs<TYPE, 1>(rows[0], t, codes[0], scale[0], off[0]);
+                    four_runs<TYPE, 1>(rows[1], t, codes[1], scale[1], off[1]);
+                }
 #pragma unroll
                 for (uint32_t r = 0; r < 4u; ++r) {
-                    // a short last piece: its missing runs hold whatever the slot held before
-                    const bool live = S::super || run0 + r < runs;
-                    if (!live) {
+                    if (!S::super && r >= live_runs) {
                         continue;
                     }
                     uint32_t a[2][4];
