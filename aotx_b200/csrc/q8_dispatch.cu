@@ -69,6 +69,8 @@ unsigned int umma_token_tile(unsigned int m)
 // memory: exact between 2^-14 and 65504, saturating above).
 __global__ void q8_x_to_f16_kernel(const uint4 *__restrict__ x, unsigned long long chunks, uint4 *__restrict__ out)
 {
+    grid_launch_dependents();
+    grid_dependency_wait();   // x, and the products that still read the copy
     for (unsigned long long at = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; at < chunks;
          at += (unsigned long long)gridDim.x * blockDim.x) {
         uint4 v = x[at];
@@ -91,6 +93,35 @@ bool umma_supports(const void *w, unsigned int n, unsigned int k, const void *x,
     return true;
 }
 
+// The tensor map of a weight tensor's rows (boxes of box_rows rows by one segment) and of rows of x
+// (boxes of box_rows rows by 64 values, 128-byte swizzle).
+static bool map_weights(EncodeTiledFn encode, CUtensorMap *map, const void *w, unsigned int rows, unsigned int k,
+                        unsigned int box_rows)
+{
+    const cuuint64_t row_b = row_bytes(k);
+    const cuuint64_t dims[2] = {row_b / 4ull, rows};
+    const cuuint64_t strides[1] = {row_b};
+    const cuuint32_t box[2] = {kSegWords, box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(w), dims, strides, box, elem,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+        == CUDA_SUCCESS;
+}
+
+static bool map_rows(EncodeTiledFn encode, CUtensorMap *map, const void *x, unsigned int rows, unsigned int k,
+                     unsigned int box_rows, bool bf16)
+{
+    const cuuint64_t dims[2] = {k, rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)k * 2ull};
+    const cuuint32_t box[2] = {kSubK, box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    return encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(x),
+                  dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+        == CUDA_SUCCESS;
+}
+
 cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigned int sm_count,
                         const void *w, unsigned int n, unsigned int k, const void *x, int x_bf16,
                         unsigned int m, const unsigned int *m_dev, void *y, int y_dtype, unsigned int set,
@@ -104,16 +135,21 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
         return cudaErrorNotSupported;
     }
     const unsigned int ntok = umma_token_tile(m);
-    const unsigned long long row_b = row_bytes(k);
     // bfloat16 activations at 33 to 128 rows: the one-block-per-SM kernel would turn every x
     // tile into binary16 in shared memory, in every block and for every weight row tile, as many
     // bytes again as the weights; one pass over x into the context's copy does it once
-    if (x_bf16 && ntok >= 64u && ntok <= 128u && scratch.x16 != nullptr
-        && (unsigned long long)m * k * 2ull <= scratch.x16_bytes) {
+    const bool copy_fits = scratch.x16 != nullptr && (unsigned long long)m * k * 2ull <= scratch.x16_bytes;
+#ifdef Q8_HOST_EMULATION
+    const bool mid = false;
+#else
+    // the kernel for 17 to 128 rows takes binary16 x
+    const bool mid = ntok > 16u && ntok <= 128u && out == nullptr && (!x_bf16 || copy_fits);
+#endif
+    if (x_bf16 && (mid || ntok >= 64u) && ntok <= 128u && copy_fits) {
         const unsigned long long chunks = (unsigned long long)m * k / 8ull;
         const unsigned int blocks = (unsigned int)((chunks + 255ull) / 256ull < 4ull * sm_count
                                                        ? (chunks + 255ull) / 256ull : 4ull * sm_count);
-        cudaError_t turned = launch_kernel(q8_x_to_f16_kernel, blocks, 256, 0, stream,
+        cudaError_t turned = launch_kernel_early(overlap, q8_x_to_f16_kernel, blocks, 256, 0, stream,
                                            static_cast<const uint4 *>(x), chunks, static_cast<uint4 *>(scratch.x16));
         if (turned != cudaSuccess) {
             return turned;
@@ -125,36 +161,23 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
 #ifdef Q8_HOST_EMULATION
     const bool warp_kernel = false; // cluster launches and warp-level MMA are not modelled
 #else
-    // Up to 16 rows, one copy of y: the register-fed kernel.  Stores into the peers' copies stay
-    // with the kernel they were measured on.
+    // Up to 16 rows, one copy of y: the register-fed kernel; up to 128: q8_mid.cu.  Stores into the
+    // peers' copies stay with the kernels they were measured on.
     const bool warp_kernel = ntok <= 16u && out == nullptr;
+    if (mid) {
+        const MidPlan plan = mid_plan(n, k, m, sm_count, epilogue);
+        CUtensorMap tw, tx;
+        if (!map_weights(encode, &tw, w, n, k, plan.slab_rows) || !map_rows(encode, &tx, x, m, k, plan.ntok, false)) {
+            return cudaErrorInvalidValue;
+        }
+        return launch_mid_product(stream, tw, tx, plan, n, k, m, m_dev, y, y_dtype, epilogue == kEpilogueSwiglu ? n / 2u : n,
+                                  epilogue, scratch.status, overlap);
+    }
 #endif
 
     CUtensorMap tw, tx;
-    {
-        cuuint64_t dims[2] = {row_b / 4ull, n};
-        cuuint64_t strides[1] = {row_b};
-        cuuint32_t box[2] = {kSegWords, kRows};
-        cuuint32_t elem[2] = {1, 1};
-        CUresult r = encode(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(w), dims, strides, box,
-                            elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-            return cudaErrorInvalidValue;
-        }
-    }
-    if (!warp_kernel) {
-        cuuint64_t dims[2] = {k, m};
-        cuuint64_t strides[1] = {(cuuint64_t)k * 2ull};
-        cuuint32_t box[2] = {kSubK, ntok};
-        cuuint32_t elem[2] = {1, 1};
-        CUresult r = encode(&tx, x_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                            const_cast<void *>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-            return cudaErrorInvalidValue;
-        }
+    if (!map_weights(encode, &tw, w, n, k, kRows) || (!warp_kernel && !map_rows(encode, &tx, x, m, k, ntok, x_bf16 != 0))) {
+        return cudaErrorInvalidValue;
     }
 
     const unsigned long long row_tiles = (n + kRows - 1u) / kRows;
@@ -250,32 +273,20 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
     if (max_tiles == 0u || x_rows == 0u) {
         return cudaSuccess;
     }
-    const unsigned long long row_b = row_bytes(k);
     CUtensorMap tw, tx;
-    {
-        cuuint64_t dims[2] = {row_b / 4ull, total_rows};
-        cuuint64_t strides[1] = {row_b};
-        cuuint32_t box[2] = {kSegWords, kRows};
-        cuuint32_t elem[2] = {1, 1};
-        CUresult r = encode(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(w_stacked), dims, strides,
-                            box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-            return cudaErrorInvalidValue;
-        }
+    if (!map_weights(encode, &tw, w_stacked, total_rows, k, kRows) || !map_rows(encode, &tx, x_sorted, x_rows, k, ntok, false)) {
+        return cudaErrorInvalidValue;
     }
+#ifndef Q8_HOST_EMULATION
     {
-        cuuint64_t dims[2] = {k, x_rows};
-        cuuint64_t strides[1] = {(cuuint64_t)k * 2ull};
-        cuuint32_t box[2] = {kSubK, ntok};
-        cuuint32_t elem[2] = {1, 1};
-        CUresult r = encode(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(x_sorted), dims, strides,
-                            box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-            return cudaErrorInvalidValue;
-        }
+        // every expert has an even number of weight row tiles (hidden and ffn are multiples of 256), so
+        // the table's entries pair up
+        const unsigned int blocks = max_tiles / 2u < sm_count ? max_tiles / 2u : sm_count;
+        (void)set;
+        return launch_mid_grouped(stream, tw, tx, blocks, k, ntok, tiles, count_dev, row_map, y, ldy, y_dtype, epilogue,
+                                  scratch.status, overlap);
     }
+#endif
     const unsigned long long units = (unsigned long long)max_tiles * (k / kSegK);
     unsigned int grid = sm_count < scratch.blocks ? sm_count : scratch.blocks;
     if (units < grid) {

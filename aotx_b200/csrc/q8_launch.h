@@ -34,6 +34,31 @@ inline cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, unsigned 
 #endif
 }
 
+// The same for a kernel that starts early (programmatic dependent launch): its blocks may run beside
+// the end of the kernel before it on the stream and wait for it (griddepcontrol.wait) before
+// they touch anything that kernel writes.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_kernel_early(bool overlap, void (*kernel)(Params...), dim3 grid, unsigned int threads,
+                                       size_t shared_bytes, cudaStream_t stream, Args... args)
+{
+#ifdef Q8_HOST_EMULATION
+    (void)overlap;
+    return launch_kernel(kernel, grid, threads, shared_bytes, stream, args...);
+#else
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = dim3(threads, 1, 1);
+    config.dynamicSmemBytes = shared_bytes;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = overlap ? 1u : 0u;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+#endif
+}
+
 // Raise a kernel's dynamic shared-memory limit once per device (the attribute is per device).
 // `two_per_sm`: also ask for all of the SM's configurable memory as shared memory, so that two
 // blocks of the kernel fit on one SM.

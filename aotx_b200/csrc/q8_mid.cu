@@ -1,0 +1,811 @@
+// The Q8_0 product for 17 to 128 rows of x, and the grouped products of the routed experts:
+// y[i][j] = sum_c x[i][c] * half(q[j][c] * d[j][c / 32]), float sums.
+//
+// Between the two regimes: the weights cross HBM once (HBM-bound up to about 64 rows), but x,
+// read again for every piece of w, weighs as much as they do, and the arithmetic is too much for the
+// warp-level MMA of q8_decode_warp.cu.  Weights are dequantised into tensor memory and multiplied
+// by tcgen05.mma (128 x N x 16, N = the batch rounded up to 16), as in q8_stream.cu; what is
+// different there cost half the time of these products:
+//
+//   * No tile is cut between blocks that meet through global memory (the hand-over of partial
+//     tiles took 3 to 8 us at the end of a launch of 20).  The rows of w are dealt in SLABS of at
+//     most 128 rows, all of one size, so many of them that every block has the same number: with
+//     many rows a block takes its slabs over the whole depth and stores them, with fewer a CLUSTER
+//     of 2 or 4 blocks takes each slab, one run of its depth per block, and the parts are added
+//     through distributed shared memory.
+//   * A segment of x (256 deep) in shared memory meets two slabs, one after the other: half the x
+//     traffic, which at 64 rows was as many bytes as the weights.
+//   * 16 converter warps with a quarter of a segment each, four to a scheduler: eight with half a
+//     segment left the latencies of the chain (shared load, dequantisation, store to tensor
+//     memory and its wait) open, 1.1 us per segment against 0.8 that memory takes.
+//   * The first copies of weights go out before anything else is set up.
+//
+// 23 warps, one block per SM: 0-3 store, 4-19 convert (thread = row, warp / 4 = quarter of the
+// segment), 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
+// status bit when it runs out.  Reference kernels replaced: as q8_stream.cu.
+#include <cuda.h>
+
+#include "q8_launch.h"
+#include "q8_tile.cuh"
+#include "q8_warp_ptx.cuh"
+
+namespace q8 {
+
+constexpr uint32_t kMidThreads = 23 * 32;
+constexpr uint32_t kMidConvertWarps = 16;
+constexpr uint32_t kMidWeightWarp = 20;
+constexpr uint32_t kMidInputWarp = 21;
+constexpr uint32_t kMidMmaWarp = 22;
+constexpr uint32_t kMidMaxRaw = 12;        // stages of the rings, at most
+constexpr uint32_t kMidMaxX = 8;
+constexpr uint32_t kMidMaxA = 3;
+constexpr uint32_t kMidBars = 2 * kMidMaxRaw + 2 * kMidMaxX + 2 * kMidMaxA + 4 + 1;
+constexpr uint32_t kMidStageBytes = 4 * 2 * 2048;   // per storing warp: two turns of 16 rows of x by 32 columns, floats
+constexpr uint32_t kMidTail = kMidStageBytes + kMidBars * 8 + 16;
+constexpr uint32_t kMidSmem = 227u * 1024u;
+constexpr uint32_t kMidRings = (kMidSmem - 1024u - kMidTail) / 1024u * 1024u;   // both rings' shared memory
+
+struct MidArgs {
+    unsigned int n, k, m_max;
+    const unsigned int *m_dev;
+    void *y;
+    unsigned int *status;
+    unsigned int ldy;
+    unsigned int epilogue;
+    const GroupTile *group_tiles;      // grouped mode: the device's table, else null
+    const unsigned int *group_count;
+    const unsigned int *row_map;
+    unsigned int ntok;                 // columns of an accumulator: rows of x, a multiple of 16
+    unsigned int slab_rows;            // rows of w per slab (a multiple of 4)
+    unsigned int pair;                 // slabs that share a segment of x: 1 or 2
+    unsigned int turns;                // times `pair` slabs per block (not in grouped mode)
+    unsigned int x_stages, raw_stages, a_stages, acc_buffers;
+    unsigned int raw_offset, raw_stride;
+};
+
+// Two blocks of 32 weights of quarter Q of a segment: `raw` holds bytes [64 Q, 64 Q + 80) of the
+// thread's row segment, the quarter's blocks start at local byte 4 Q + 34 jb.  They become 32 words
+// in the thread's lane of tensor memory.
+template <int Q>
+__device__ __forceinline__ void convert_quarter(const uint32_t (&raw)[20], uint32_t taddr)
+{
+    uint32_t out[32];
+#pragma unroll
+    for (int jb = 0; jb < 2; ++jb) {
+        const int byte_off = 4 * Q + 34 * jb;
+        const int wi = byte_off / 4;
+        const bool odd = (byte_off % 4) == 2;
+        const uint32_t d_bits = prmt(raw[wi], raw[wi], odd ? 0x3232u : 0x1010u);
+        const __half2 d2 = *reinterpret_cast<const __half2 *>(&d_bits);
+#pragma unroll
+        for (int p = 0; p < 16; ++p) {
+            // odd: the payload starts at the next word boundary; else in the high half of the
+            // scale's word
+            const int word = odd ? wi + 1 + p / 2 : wi + (p + 1) / 2;
+            const bool high = odd ? (p % 2) != 0 : ((p + 1) % 2) != 0;
+            const uint32_t flipped = raw[word] ^ 0x80808080u;
+            out[16 * jb + p] = high ? dequant_pair<1>(flipped, d2) : dequant_pair<0>(flipped, d2);
+        }
+    }
+    tmem_st_32x32(taddr, out);
+}
+
+template <int Q>
+__device__ __forceinline__ void load_quarter(uint32_t raw_row, uint32_t (&raw)[20])
+{
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        ld_shared_v4(raw_row + (uint32_t)(Q * 64 + 16 * i), raw[4 * i], raw[4 * i + 1], raw[4 * i + 2], raw[4 * i + 3]);
+    }
+}
+
+// Every lane has the words of its row, not only asked for them, when the raw stage goes back
+// (raw_words_present in q8_tile.cuh says why); true about once in 2^64 loads.
+__device__ __forceinline__ void quarter_present(const uint32_t (&raw)[20], unsigned int *status)
+{
+    uint32_t all = raw[0];
+    uint32_t sum = raw[1];
+#pragma unroll
+    for (int i = 2; i < 20; i += 2) {
+        all ^= raw[i];
+        sum += raw[i + 1];
+    }
+    if (__any_sync(0xFFFFFFFFu, all == 0x5F3759DFu && sum == 0x9E3779B9u)) {
+        atomicOr(status, 0u);
+    }
+}
+
+// What one finished value becomes: stored, added to the float stream (cuda/model/norm.cu:78-89).
+template <typename YT>
+__device__ __forceinline__ void mid_store_one(const MidArgs &args, size_t at, float value)
+{
+    if (args.epilogue == kEpilogueAdd) {
+        float *sum = static_cast<float *>(args.y) + at;
+        *sum = *sum + value;
+    } else {
+        store_out<YT>(static_cast<YT *>(args.y), at, value);
+    }
+}
+
+// 16 rows of x by this warp's 32 columns of y, every lane one column: turned round in shared memory of
+// the warp's own and written four values per lane, 2 to 4 store instructions instead of 16 (the
+// number of store instructions is what a store costs here, see q8_tile.cuh).  GATED: neighbouring
+// lanes hold gate and up of one column (cuda/model/norm.cu:92-105); 16 columns then.
+// `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.
+template <typename YT, bool GATED>
+__device__ __forceinline__ void mid_store_staged(const MidArgs &args, uint32_t stage, uint32_t lane, uint32_t first_col,
+                                                 uint32_t columns, uint32_t first_row, uint32_t row_limit,
+                                                 const uint32_t (&v)[16])
+{
+    constexpr uint32_t kColumns = GATED ? 16u : 32u;
+    constexpr uint32_t kRowBytes = kColumns * sizeof(YT);
+    constexpr uint32_t kLanesPerRow = kColumns / 4u;
+    constexpr uint32_t kRowsPerStep = 32u / kLanesPerRow;      // 4 or 8
+    constexpr uint32_t kSteps = 16u / kRowsPerStep;
+    const uint32_t column = GATED ? lane / 2u : lane;
+#pragma unroll
+    for (uint32_t i = 0; i < 16u; ++i) {
+        float value = __uint_as_float(v[i]);
+        if (GATED) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
+            value = value / (1.0f + expf(-value)) * other;
+        }
+        if (!GATED || (lane & 1u) == 0u) {
+            if (sizeof(YT) == 4) {
+                st_shared_b32(stage + i * kRowBytes + column * 4u, __float_as_uint(value));
+            } else {
+                st_shared_b16(stage + i * kRowBytes + column * 2u, out_bits<YT>(value));
+            }
+        }
+    }
+    __syncwarp();
+    const uint32_t part = lane % kLanesPerRow;
+    const bool adds = !GATED && sizeof(YT) == 4 && args.epilogue == kEpilogueAdd;
+    YT *at[kSteps];
+#pragma unroll
+    for (uint32_t step = 0; step < kSteps; ++step) {
+        const uint32_t row_x = first_row + step * kRowsPerStep + lane / kLanesPerRow;
+        at[step] = nullptr;
+        if (row_x < row_limit && part * 4u < columns) {
+            const uint32_t row_y = args.row_map != nullptr ? __ldg(args.row_map + row_x) : row_x;
+            at[step] = static_cast<YT *>(args.y) + (size_t)row_y * args.ldy + first_col + part * 4u;
+        }
+    }
+    float4 before[kSteps];
+    if (adds) {
+        // one rounded add per value; the old values are fetched together, before the first store
+#pragma unroll
+        for (uint32_t step = 0; step < kSteps; ++step) {
+            before[step] = at[step] != nullptr ? *reinterpret_cast<const float4 *>(at[step]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+#pragma unroll
+    for (uint32_t step = 0; step < kSteps; ++step) {
+        const uint32_t from = stage + (step * kRowsPerStep + lane / kLanesPerRow) * kRowBytes + part * 4u * sizeof(YT);
+        if (sizeof(YT) == 4) {
+            uint32_t a, b, c, d;
+            ld_shared_v4(from, a, b, c, d);
+            float4 piece = make_float4(__uint_as_float(a), __uint_as_float(b), __uint_as_float(c), __uint_as_float(d));
+            if (adds) {
+                piece = make_float4(before[step].x + piece.x, before[step].y + piece.y, before[step].z + piece.z,
+                                    before[step].w + piece.w);
+            }
+            if (at[step] != nullptr) {
+                *reinterpret_cast<float4 *>(at[step]) = piece;
+            }
+        } else {
+            uint32_t a, b;
+            ld_shared_v2(from, a, b);
+            if (at[step] != nullptr) {
+                *reinterpret_cast<uint2 *>(at[step]) = make_uint2(a, b);
+            }
+        }
+    }
+}
+
+template <typename YT>
+__global__ void __launch_bounds__(kMidThreads, 1)
+q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const MidArgs args)
+{
+    extern __shared__ unsigned char smem_raw_[];
+    const uint32_t smem0 = (smem_u32(smem_raw_) + 1023u) & ~1023u;
+    unsigned char *const smem = smem_raw_ + (smem0 - smem_u32(smem_raw_));
+    const uint32_t raw_base = smem0 + args.raw_offset;
+    const uint32_t stage_base = smem0 + kMidRings;
+    const uint32_t raw_full = stage_base + kMidStageBytes;
+    const uint32_t raw_empty = raw_full + 8u * kMidMaxRaw;
+    const uint32_t x_full = raw_empty + 8u * kMidMaxRaw;
+    const uint32_t x_empty = x_full + 8u * kMidMaxX;
+    const uint32_t a_full = x_empty + 8u * kMidMaxX;
+    const uint32_t a_empty = a_full + 8u * kMidMaxA;
+    const uint32_t acc_full = a_empty + 8u * kMidMaxA;
+    const uint32_t acc_empty = acc_full + 16u;
+    const uint32_t drain_bar = acc_empty + 16u;
+    const uint32_t tmem_slot = drain_bar + 8u;
+    volatile uint32_t *tmem_slot_ptr = reinterpret_cast<volatile uint32_t *>(smem + (tmem_slot - smem0));
+    volatile uint32_t *abort_flag = tmem_slot_ptr + 1;
+
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool grouped = args.group_tiles != nullptr;
+    const uint32_t segs = args.k / kSegK;
+    const uint32_t pair = args.pair;
+    const uint32_t ntok = args.ntok;
+    const uint32_t x_seg_bytes = ntok * (kSegK * 2u);
+    const uint32_t raw_bytes = args.slab_rows * kSegBytes;
+    const uint32_t csize = cluster_nctarank();
+    const uint32_t crank = cluster_ctarank();
+    const uint32_t seg_begin = crank * segs / csize;
+    const uint32_t seg_end = (crank + 1u) * segs / csize;
+    const uint32_t slab0 = blockIdx.x / csize * args.turns * pair;   // the block's first slab (its cluster's)
+
+    grid_launch_dependents();
+
+    uint32_t early = 0u;
+    if (warp == kMidWeightWarp && elect_one()) {
+        tma_prefetch_desc(&tmap_w);
+        tma_prefetch_desc(&tmap_x);
+        for (uint32_t i = 0; i < args.raw_stages; ++i) {
+            mbar_init(raw_full + 8u * i, 1u);
+            mbar_init(raw_empty + 8u * i, kMidConvertWarps);
+        }
+        for (uint32_t i = 0; i < args.x_stages; ++i) {
+            mbar_init(x_full + 8u * i, 1u);
+            mbar_init(x_empty + 8u * i, 1u);
+        }
+        for (uint32_t i = 0; i < args.a_stages; ++i) {
+            mbar_init(a_full + 8u * i, kMidConvertWarps);
+            mbar_init(a_empty + 8u * i, 1u);
+        }
+        for (uint32_t i = 0; i < 2u; ++i) {
+            mbar_init(acc_full + 8u * i, 1u);
+            mbar_init(acc_empty + 8u * i, kEpilogueWarps);
+        }
+        mbar_init(drain_bar, 1u);
+        *abort_flag = 0u;
+        mbar_init_fence();
+        fence_proxy_async_smem();
+        if (!grouped) {
+            // the first weights: only the barriers they signal have to be there
+            const uint32_t total = args.turns * (seg_end - seg_begin) * pair;
+            const uint32_t per_turn = (seg_end - seg_begin) * pair;
+            for (; early < args.raw_stages && early < total; ++early) {
+                const uint32_t turn = early / per_turn;
+                const uint32_t in_turn = early - turn * per_turn;
+                const uint32_t s = seg_begin + in_turn / pair;
+                const uint32_t slab = slab0 + turn * pair + in_turn % pair;
+                mbar_expect_tx(raw_full + 8u * early, raw_bytes);
+                tma_load_2d(raw_base + early * args.raw_stride, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords),
+                            (int)(slab * args.slab_rows));
+            }
+        }
+    }
+    if (warp == kMidMmaWarp) {
+        tmem_alloc(tmem_slot, 512u);
+        tmem_relinquish();
+    }
+    if (csize > 1u) {
+        __syncwarp();
+        cluster_arrive_relaxed();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot_ptr;
+    const uint32_t a_column0 = args.acc_buffers * pair * ntok;
+
+    // how many pairs of slabs this block takes
+    uint32_t turns = args.turns;
+    if (grouped) {
+        // the table was built by the kernel before this one on the stream
+        grid_dependency_wait();
+        const uint32_t pairs = *args.group_count / pair;
+        turns = blockIdx.x < pairs ? (pairs - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+    }
+    unsigned int m_live = args.m_max;
+
+    if (warp == kMidWeightWarp) {
+        // ---------------------------------------------------------------- weight copies
+        if (elect_one()) {
+            uint32_t g = 0;
+            bool ok = true;
+            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
+                uint32_t w_row[2];
+                if (grouped) {
+                    const GroupTile *entry = args.group_tiles + (size_t)(blockIdx.x + turn * gridDim.x) * pair;
+                    w_row[0] = entry[0].w_row;
+                    w_row[1] = pair > 1u ? entry[1].w_row : 0u;
+                } else {
+                    w_row[0] = (slab0 + turn * pair) * args.slab_rows;
+                    w_row[1] = w_row[0] + args.slab_rows;
+                }
+                for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
+                    for (uint32_t p = 0; p < pair; ++p, ++g) {
+                        if (g < early) {
+                            continue;
+                        }
+                        const uint32_t st = g % args.raw_stages;
+                        const uint32_t ph = (g / args.raw_stages) & 1u;
+                        if (!mbar_wait(raw_empty + 8u * st, ph ^ 1u, abort_flag, args.status)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(raw_full + 8u * st, raw_bytes);
+                        tma_load_2d(raw_base + st * args.raw_stride, &tmap_w, raw_full + 8u * st, (int)(s * kSegWords),
+                                    (int)(p == 0u ? w_row[0] : w_row[1]));
+                    }
+                }
+            }
+            // Let every copy this thread started land before the block ends.
+            uint32_t local_abort = 0;
+            const uint32_t issued = g > early ? g : early;
+            const uint32_t first = issued > args.raw_stages ? issued - args.raw_stages : 0u;
+            for (uint32_t i = first; i < issued; ++i) {
+                mbar_wait(raw_full + 8u * (i % args.raw_stages), (i / args.raw_stages) & 1u, &local_abort, nullptr);
+            }
+        }
+    } else if (warp == kMidInputWarp) {
+        // ---------------------------------------------------------------- x copies
+        if (elect_one()) {
+            uint32_t g = 0;
+            grid_dependency_wait();
+            bool ok = true;
+            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
+                const uint32_t tok0 = grouped ? args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair].tok0 : 0u;
+                for (uint32_t s = seg_begin; s < seg_end; ++s, ++g) {
+                    const uint32_t st = g % args.x_stages;
+                    const uint32_t ph = (g / args.x_stages) & 1u;
+                    if (!mbar_wait(x_empty + 8u * st, ph ^ 1u, abort_flag, args.status)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(x_full + 8u * st, x_seg_bytes);
+#pragma unroll
+                    for (uint32_t j = 0; j < kSubs; ++j) {
+                        tma_load_2d(smem0 + st * x_seg_bytes + j * (x_seg_bytes / kSubs), &tmap_x, x_full + 8u * st,
+                                    (int)(s * kSegK + j * kSubK), (int)tok0);
+                    }
+                }
+            }
+            uint32_t local_abort = 0;
+            const uint32_t first = g > args.x_stages ? g - args.x_stages : 0u;
+            for (uint32_t i = first; i < g; ++i) {
+                mbar_wait(x_full + 8u * (i % args.x_stages), (i / args.x_stages) & 1u, &local_abort, nullptr);
+            }
+        }
+    } else if (warp == kMidMmaWarp) {
+        // ---------------------------------------------------------------- MMA issue
+        if (elect_one()) {
+            const uint32_t idesc = umma_idesc(kRows, ntok, 0u, 0u);
+            uint32_t g = 0;      // segments of x
+            uint32_t a = 0;      // segments of A
+            bool ok = true;
+            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
+                const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
+                const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
+                if (!mbar_wait(acc_empty + 8u * buf, (uses & 1u) ^ 1u, abort_flag, args.status)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                for (uint32_t s = seg_begin; ok && s < seg_end; ++s, ++g) {
+                    const uint32_t xst = g % args.x_stages;
+                    if (!mbar_wait(x_full + 8u * xst, (g / args.x_stages) & 1u, abort_flag, args.status)) {
+                        ok = false;
+                        break;
+                    }
+                    for (uint32_t p = 0; p < pair; ++p, ++a) {
+                        const uint32_t ast = a % args.a_stages;
+                        if (!mbar_wait(a_full + 8u * ast, (a / args.a_stages) & 1u, abort_flag, args.status)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        const uint32_t d_tmem = tmem_base + (buf * pair + p) * ntok;
+                        const uint32_t a_tmem = tmem_base + a_column0 + ast * (kSegK / 2u);
+                        const uint32_t x_seg = smem0 + xst * x_seg_bytes;
+#pragma unroll
+                        for (uint32_t j = 0; j < kSubs; ++j) {
+                            const uint64_t b_desc = umma_desc_sw128(x_seg + j * (x_seg_bytes / kSubs));
+#pragma unroll
+                            for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
+                                // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
+                                umma_f16_ts(d_tmem, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
+                                            s != seg_begin || j != 0u || kk != 0u ? 1u : 0u);
+                            }
+                        }
+                        umma_commit(a_empty + 8u * ast);
+                    }
+                    if (ok) {
+                        umma_commit(x_empty + 8u * xst);
+                    }
+                }
+                if (ok) {
+                    umma_commit(acc_full + 8u * buf);
+                }
+            }
+            if (!ok) {
+                // Outstanding MMAs must finish before the tensor memory goes back.
+                uint32_t local_abort = 0;
+                umma_commit(drain_bar);
+                mbar_wait(drain_bar, 0u, &local_abort, nullptr);
+            }
+        }
+    } else if (warp >= kConvertWarp0) {
+        // ---------------------------------------------------------------- dequantise
+        const uint32_t cw = warp - kConvertWarp0;
+        const uint32_t quarter = cw >> 2;
+        const uint32_t row = (cw & 3u) * 32u + lane;
+        // rows past the slab repeat its last one (their sums are not stored)
+        const uint32_t row_at = (row < args.slab_rows ? row : args.slab_rows - 1u) * kSegBytes;
+        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + quarter * (kSegK / 8u);
+        const uint32_t total = turns * (seg_end - seg_begin) * pair;
+        uint32_t rst = 0, rph = 0, ast = 0, aph = 0;
+        for (uint32_t g = 0; g < total; ++g) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * rst, rph, abort_flag, args.status))) {
+                break;
+            }
+            uint32_t raw[20];
+            const uint32_t raw_row = raw_base + rst * args.raw_stride + row_at;
+            switch (quarter) {
+            case 0u: load_quarter<0>(raw_row, raw); break;
+            case 1u: load_quarter<1>(raw_row, raw); break;
+            case 2u: load_quarter<2>(raw_row, raw); break;
+            default: load_quarter<3>(raw_row, raw); break;
+            }
+            quarter_present(raw, args.status);
+            if (lane == 0u) {
+                mbar_arrive(raw_empty + 8u * rst);
+            }
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(a_empty + 8u * ast, aph ^ 1u, abort_flag, args.status))) {
+                break;
+            }
+            const uint32_t taddr = lane_base + ast * (kSegK / 2u);
+            tc_fence_after_sync();
+            switch (quarter) {
+            case 0u: convert_quarter<0>(raw, taddr); break;
+            case 1u: convert_quarter<1>(raw, taddr); break;
+            case 2u: convert_quarter<2>(raw, taddr); break;
+            default: convert_quarter<3>(raw, taddr); break;
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0u) {
+                mbar_arrive(a_full + 8u * ast);
+            }
+            if (++rst == args.raw_stages) {
+                rst = 0u;
+                rph ^= 1u;
+            }
+            if (++ast == args.a_stages) {
+                ast = 0u;
+                aph ^= 1u;
+            }
+        }
+    } else if (csize == 1u) {
+        // ---------------------------------------------------------------- read sums, store
+        const uint32_t lane_taddr = tmem_base + ((warp * 32u) << 16);
+        const bool gated = args.epilogue == kEpilogueSwiglu;
+        const uint32_t buffers = stage_base + warp * (kMidStageBytes / 4u);
+        uint32_t flip = 0u;      // the two turns of the warp's staging buffer
+        grid_dependency_wait();
+        if (args.m_dev != nullptr) {
+            const unsigned int live = *args.m_dev;
+            m_live = live < m_live ? live : m_live;
+        }
+        // rows of y start on a boundary of four values, and so does every slab
+        const bool aligned = (args.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.y) % (4u * sizeof(YT))) == 0u
+                          && (args.slab_rows % (gated ? 8u : 4u)) == 0u;
+        for (uint32_t turn = 0; turn < turns; ++turn) {
+            const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
+            const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
+            // where the pair goes (table entries in grouped mode): asked for before the wait
+            GroupTile place[2];
+            for (uint32_t p = 0; p < pair; ++p) {
+                if (grouped) {
+                    place[p] = args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair + p];
+                } else {
+                    place[p].j0 = (slab0 + turn * pair + p) * args.slab_rows;
+                    place[p].j_limit = place[p].j0 + args.slab_rows < args.n ? place[p].j0 + args.slab_rows : args.n;
+                    place[p].tok0 = 0u;
+                    place[p].tok_limit = m_live;
+                }
+            }
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(acc_full + 8u * buf, uses & 1u, abort_flag, args.status))) {
+                break;
+            }
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t p = 0; p < pair; ++p) {
+                const GroupTile at = p == 0u ? place[0] : place[1];
+                const uint32_t rows = at.tok_limit > at.tok0 ? at.tok_limit - at.tok0 : 0u;
+                const uint32_t j = at.j0 + warp * 32u;                                   // this warp's first row of w
+                const uint32_t inside = at.j_limit > j ? at.j_limit - j : 0u;            // ... and how many are there
+                const uint32_t mine = inside < 32u ? inside : 32u;
+                const uint32_t columns = gated ? mine / 2u : mine;
+                const uint32_t col = gated ? j / 2u : j;
+                const bool staged = aligned && (columns % 4u) == 0u;
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < ntok && c0 < rows && mine != 0u; c0 += 16u) {
+                    uint32_t v[16];
+                    tmem_ld_32x16(lane_taddr + (buf * pair + p) * ntok + c0, v);
+                    tmem_ld_wait();
+                    if (staged) {
+                        const uint32_t buffer = buffers + flip;
+                        flip ^= kMidStageBytes / 8u;
+                        if (gated) {
+                            mid_store_staged<YT, true>(args, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
+                        } else {
+                            mid_store_staged<YT, false>(args, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < 16u; ++i) {
+                        float value = __uint_as_float(v[i]);
+                        if (gated) {
+                            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
+                            value = value / (1.0f + expf(-value)) * other;
+                        }
+                        const uint32_t row_x = at.tok0 + c0 + i;
+                        if (row_x < at.tok_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
+                            const uint32_t row_y = args.row_map != nullptr ? __ldg(args.row_map + row_x) : row_x;
+                            mid_store_one<YT>(args, (size_t)row_y * args.ldy + col + (gated ? lane / 2u : lane), value);
+                        }
+                    }
+                }
+            }
+            // The accumulators are free again.
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0u) {
+                mbar_arrive(acc_empty + 8u * buf);
+            }
+        }
+    }
+
+    if (csize > 1u) {
+        // ------------------------------------------------------------ sum of a cluster's parts
+        // One pair of slabs per cluster.  The rows of x are dealt to its blocks in runs of `share`;
+        // every block writes its part's sums into their owners' shared memory, over the rings, which are
+        // idle by then: [sender][slab][row of x][row of w].  The owner adds the parts in block order.
+        bool there = true;
+        if (warp < kMidWeightWarp) {
+            there = mbar_wait(acc_full, 0u, abort_flag, args.status);
+            tc_fence_after_sync();
+        }
+        const uint32_t share = ntok / csize;
+        __syncwarp();
+        cluster_wait_acquire();      // every block has started ...
+        cluster_arrive_release();    // ... and is done with its rings
+        cluster_wait_acquire();
+        if (warp < kMidWeightWarp) {
+            const uint32_t quarter_lanes = warp & 3u;
+            const uint32_t lane_taddr = tmem_base + ((quarter_lanes * 32u) << 16);
+            const uint32_t row = quarter_lanes * 32u + lane;
+            for (uint32_t c = warp >> 2; c < pair * ntok / 16u; c += kMidWeightWarp / 4u) {
+                const uint32_t p = c / (ntok / 16u);
+                const uint32_t c0 = (c - p * (ntok / 16u)) * 16u;
+                uint32_t v[16];
+                tmem_ld_32x16(lane_taddr + p * ntok + c0, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; ++i) {
+                    const uint32_t token = c0 + i;
+                    const uint32_t at = smem0 + (((crank * pair + p) * share + token % share) * kRows + row) * 4u;
+                    st_shared_cluster_f32(mapa_shared(at, token / share), __uint_as_float(v[i]));
+                }
+            }
+            tc_fence_before_sync();
+        }
+        __syncwarp();
+        cluster_arrive_release();
+        cluster_wait_acquire();
+        grid_dependency_wait();
+        if (args.m_dev != nullptr) {
+            const unsigned int live = *args.m_dev;
+            m_live = live < m_live ? live : m_live;
+        }
+        if (!there) {
+            m_live = 0u;
+        }
+        const float *recv = reinterpret_cast<const float *>(smem);
+        const bool gated = args.epilogue == kEpilogueSwiglu;
+        const uint32_t rows_of_x = pair * share;
+        // warp = 32 rows of w of one row of x
+        for (uint32_t at = warp; at < rows_of_x * (kRows / 32u); at += kMidThreads / 32u) {
+            const uint32_t local = at / (kRows / 32u);                  // slab * share + row of x within the share
+            const uint32_t row = (at % (kRows / 32u)) * 32u + lane;
+            const uint32_t p = local / share;
+            const uint32_t token = crank * share + (local - p * share);
+            float sum = recv[(size_t)local * kRows + row];
+            for (uint32_t src = 1; src < csize; ++src) {
+                sum += recv[((size_t)src * rows_of_x + local) * kRows + row];
+            }
+            const uint32_t j = (slab0 + p) * args.slab_rows + row;
+            if (gated) {
+                const float up = __shfl_xor_sync(0xFFFFFFFFu, sum, 1u);
+                sum = sum / (1.0f + expf(-sum)) * up;
+            }
+            if (token < m_live && row < args.slab_rows && j < args.n && (!gated || (row & 1u) == 0u)) {
+                mid_store_one<YT>(args, (size_t)token * args.ldy + (gated ? j / 2u : j), sum);
+            }
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kMidMmaWarp) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 512u);
+    }
+}
+
+template <typename YT>
+static cudaError_t launch_mid_typed(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidArgs &args,
+                                    unsigned int grid, unsigned int cluster, bool overlap)
+{
+    static unsigned long long configured = 0ull;
+    cudaError_t err = allow_shared_memory(q8_stream_kernel_mid<YT>, kMidSmem, &configured);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid, 1, 1);
+    config.blockDim = dim3(kMidThreads, 1, 1);
+    config.dynamicSmemBytes = kMidSmem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[2];
+    unsigned int count = 0;
+    if (overlap) {
+        attribute[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute[count].val.programmaticStreamSerializationAllowed = 1;
+        ++count;
+    }
+    if (cluster > 1u) {
+        attribute[count].id = cudaLaunchAttributeClusterDimension;
+        attribute[count].val.clusterDim.x = cluster;
+        attribute[count].val.clusterDim.y = 1;
+        attribute[count].val.clusterDim.z = 1;
+        ++count;
+    }
+    config.attrs = attribute;
+    config.numAttrs = count;
+    return cudaLaunchKernelEx(&config, q8_stream_kernel_mid<YT>, tw, tx, args);
+}
+
+static cudaError_t launch_mid(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, MidArgs &args,
+                              unsigned int grid, unsigned int cluster, bool overlap, int y_dtype)
+{
+    // Tensor memory: accumulators in two buffers where they leave room for two segments of A.
+    args.acc_buffers = 2u * args.pair * args.ntok <= 256u ? 2u : 1u;
+    const unsigned int a_stages = (512u - args.acc_buffers * args.pair * args.ntok) / (kSegK / 2u);
+    args.a_stages = a_stages < kMidMaxA ? a_stages : kMidMaxA;
+    // Shared memory: up to four segments of x, as far as they leave about 100 KB to the weights (three
+    // full slabs; 104 KB in flight per SM read memory at 6.8 TB/s), the rest to the weights.
+    const unsigned int x_seg = args.ntok * kSegK * 2u;
+    args.raw_stride = (args.slab_rows * kSegBytes + 127u) / 128u * 128u;
+    unsigned int x_stages = 4u;
+    while (x_stages > 2u && x_stages * x_seg + 3u * kRawStageBytes > kMidRings) {
+        --x_stages;
+    }
+    args.x_stages = x_stages;
+    args.raw_offset = x_stages * x_seg;
+    const unsigned int raw_stages = (kMidRings - args.raw_offset) / args.raw_stride;
+    args.raw_stages = raw_stages < kMidMaxRaw ? raw_stages : kMidMaxRaw;
+    switch (y_dtype) {
+    case 0:
+        return launch_mid_typed<float>(stream, tw, tx, args, grid, cluster, overlap);
+    case 1:
+        return launch_mid_typed<__half>(stream, tw, tx, args, grid, cluster, overlap);
+    case 2:
+        return launch_mid_typed<__nv_bfloat16>(stream, tw, tx, args, grid, cluster, overlap);
+    default:
+        return cudaErrorInvalidValue;
+    }
+}
+
+// How many clusters of four blocks run at once (clusters do not cross the boundaries of the GPU's
+// processing clusters, so it is fewer than a quarter of the SMs); once per device.
+static unsigned int clusters_of_four(unsigned int sm_count)
+{
+    static unsigned int known[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) {
+        return sm_count / 5u;
+    }
+    if (known[device] == 0u) {
+        static unsigned long long configured = 0ull;
+        int found = 0;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(4u * (sm_count / 4u), 1, 1);
+        config.blockDim = dim3(kMidThreads, 1, 1);
+        config.dynamicSmemBytes = kMidSmem;
+        cudaLaunchAttribute attribute[1];
+        attribute[0].id = cudaLaunchAttributeClusterDimension;
+        attribute[0].val.clusterDim.x = 4;
+        attribute[0].val.clusterDim.y = 1;
+        attribute[0].val.clusterDim.z = 1;
+        config.attrs = attribute;
+        config.numAttrs = 1;
+        if (allow_shared_memory(q8_stream_kernel_mid<float>, kMidSmem, &configured) != cudaSuccess
+            || cudaOccupancyMaxActiveClusters(&found, q8_stream_kernel_mid<float>, &config) != cudaSuccess || found <= 0) {
+            found = (int)(sm_count / 5u);
+        }
+        known[device] = (unsigned int)found;
+    }
+    return known[device];
+}
+
+MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue)
+{
+    MidPlan plan = {};
+    plan.ntok = (m + 15u) / 16u * 16u;
+    const unsigned int segs = k / kSegK;
+    const unsigned int step = epilogue == kEpilogueSwiglu ? 8u : 4u;
+    // The fewest blocks to a slab that leave every cluster at most two slabs; one block to a slab, and
+    // as many turns as it takes, beyond that.
+    const unsigned int fours = clusters_of_four(sm_count);
+    unsigned int clusters = sm_count;
+    plan.cluster = 1u;
+    if (segs >= 4u && n <= fours * 2u * kRows) {
+        plan.cluster = 4u;
+        clusters = fours;
+    } else if (segs >= 2u && n <= sm_count / 2u * 2u * kRows) {
+        plan.cluster = 2u;
+        clusters = sm_count / 2u;
+    }
+    unsigned int slabs = (n + clusters * kRows - 1u) / (clusters * kRows);     // per cluster
+    plan.pair = slabs > 1u ? 2u : 1u;
+    plan.turns = (slabs + plan.pair - 1u) / plan.pair;
+    const unsigned int all = clusters * plan.pair * plan.turns;
+    plan.slab_rows = ((n + all - 1u) / all + step - 1u) / step * step;
+    // rounding up can leave the last clusters without rows
+    const unsigned int used = (n + plan.slab_rows - 1u) / plan.slab_rows;
+    clusters = (used + plan.pair * plan.turns - 1u) / (plan.pair * plan.turns);
+    plan.grid = clusters * plan.cluster;
+    return plan;
+}
+
+cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
+                               unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
+                               unsigned int ldy, unsigned int epilogue, unsigned int *status, bool overlap)
+{
+    MidArgs args = {};
+    args.n = n;
+    args.k = k;
+    args.m_max = m;
+    args.m_dev = m_dev;
+    args.y = y;
+    args.status = status;
+    args.ldy = ldy;
+    args.epilogue = epilogue;
+    args.ntok = plan.ntok;
+    args.slab_rows = plan.slab_rows;
+    args.pair = plan.pair;
+    args.turns = plan.turns;
+    return launch_mid(stream, tw, tx, args, plan.grid, plan.cluster, overlap, y_dtype);
+}
+
+cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
+                               unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
+                               const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
+                               unsigned int *status, bool overlap)
+{
+    MidArgs args = {};
+    args.k = k;
+    args.y = y;
+    args.status = status;
+    args.ldy = ldy;
+    args.epilogue = epilogue;
+    args.group_tiles = tiles;
+    args.group_count = count_dev;
+    args.row_map = row_map;
+    args.ntok = ntok;
+    args.slab_rows = kRows;
+    args.pair = 2u;
+    return launch_mid(stream, tw, tx, args, grid, 1u, overlap, y_dtype);
+}
+
+} // namespace q8

@@ -7,6 +7,7 @@
 // (cuda/model/expert_matrix.cu:8-27, loop cuda/model/experts_host.cu:99-111), which re-reads an
 // expert's weights for every token routed to it.  The results are the same products; the
 // rank-ordered weighted sum (cuda/model/experts.cu:77-98) is kept as it is.
+#include <math.h>
 #include <stdlib.h>
 
 #include "q8_launch.h"
@@ -22,9 +23,21 @@ namespace q8 {
 #define Q8_GROUP_TOKENS 64u /* token tile of the grouped products */
 #endif
 
-static unsigned int group_tokens()
+// Token tile of the grouped products: the pairs an expert gets on average and two and a half standard
+// deviations more, so that all but a few experts need one tile (an expert with more takes another
+// tile, and its weights a second time), and no more columns than that.
+static unsigned int group_tokens(unsigned int pairs, unsigned int experts)
 {
+#ifdef Q8_HOST_EMULATION
+    (void)pairs;
+    (void)experts;
     return Q8_GROUP_TOKENS;
+#else
+    const float mean = (float)pairs / (float)experts;
+    const unsigned int want = (unsigned int)(mean + 2.5f * sqrtf(mean) + 1.0f);
+    const unsigned int tile = (want + 15u) / 16u * 16u;
+    return tile < 128u ? tile : 128u;
+#endif
 }
 
 // One block.  Counts the pairs of every expert, places each pair in its expert's run of
@@ -322,7 +335,8 @@ cudaError_t launch_moe_grouped(cudaStream_t stream, const UmmaScratch &scratch, 
                                const MoeWorkspace &ws, const RowParts *x_parts, float *proj_out)
 {
     const unsigned int pairs = tokens * used;
-    const unsigned int tile_tokens = group_tokens();
+    // (several GPUs: the pairs of all, of which this GPU's experts get their part)
+    const unsigned int tile_tokens = group_tokens(x_parts != nullptr ? pairs / x_parts->parts : pairs, experts);
     unsigned int *sorted_pair = reinterpret_cast<unsigned int *>(workspace + ws.sorted_pair);
     unsigned int *counts = reinterpret_cast<unsigned int *>(workspace + ws.counts);
     GroupTile *tiles_feed = reinterpret_cast<GroupTile *>(workspace + ws.tiles_feed);
@@ -384,7 +398,7 @@ cudaError_t launch_moe_grouped_fused(cudaStream_t stream, const UmmaScratch &scr
                                      unsigned char *workspace, const MoeWorkspace &ws)
 {
     const unsigned int pairs = tokens * used;
-    const unsigned int tile_tokens = group_tokens();
+    const unsigned int tile_tokens = group_tokens(pairs, experts);
     unsigned int *sorted_pair = reinterpret_cast<unsigned int *>(workspace + ws.sorted_pair);
     unsigned int *counts = reinterpret_cast<unsigned int *>(workspace + ws.counts);
     GroupTile *tiles_feed = reinterpret_cast<GroupTile *>(workspace + ws.tiles_feed);

@@ -643,6 +643,21 @@ cudaError_t launch_decode_kernel(cudaStream_t stream, const CUtensorMap &tw, con
 cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const void *x, const UmmaArgs &args,
                                unsigned int grid, unsigned int cluster, int y_dtype);
 
+// The product for 17 to 128 rows and the grouped products (q8_mid.cu): how a product's rows of w are
+// dealt (slabs of slab_rows rows, `pair` at a time, `turns` times per block; `cluster` blocks share a
+// slab's depth), and the launches.
+struct MidPlan {
+    unsigned int ntok, slab_rows, pair, turns, cluster, grid;
+};
+MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue);
+cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
+                               unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
+                               unsigned int ldy, unsigned int epilogue, unsigned int *status, bool overlap);
+cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
+                               unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
+                               const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
+                               unsigned int *status, bool overlap);
+
 // Host launcher of the second prefill-regime kernel (q8_wide.cu), token tiles of 256.
 cudaError_t launch_wide_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx,
                                const UmmaArgs &args, unsigned int grid, int y_dtype);

@@ -52,6 +52,11 @@ __device__ __forceinline__ void copy_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+__device__ __forceinline__ void ld_shared_v2(uint32_t addr, uint32_t &a, uint32_t &b)
+{
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
+}
+
 __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b)
 {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
