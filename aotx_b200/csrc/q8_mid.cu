@@ -15,13 +15,10 @@
 //     through distributed shared memory.
 //   * A segment of x (256 deep) in shared memory meets two slabs, one after the other: half the x
 //     traffic, which at 64 rows was as many bytes as the weights.
-//   * 16 converter warps with a quarter of a segment each, four to a scheduler: eight with half a
-//     segment left the latencies of the chain (shared load, dequantisation, store to tensor
-//     memory and its wait) open, 1.1 us per segment against 0.8 that memory takes.
+//   * 16 converter warps in two groups that take segments in turn (thread = row, half a segment).
 //   * The first copies of weights go out before anything else is set up.
 //
-// 23 warps, one block per SM: 0-3 store, 4-19 convert (thread = row, warp / 4 = quarter of the
-// segment), 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
+// 23 warps, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
 // status bit when it runs out.  Reference kernels replaced: as q8_stream.cu.
 #include <cuda.h>
 
@@ -32,14 +29,15 @@
 namespace q8 {
 
 constexpr uint32_t kMidThreads = 23 * 32;
-constexpr uint32_t kMidConvertWarps = 16;
+constexpr uint32_t kMidGroups = 2;         // of converter warps, which take segments in turn
+constexpr uint32_t kMidGroupWarps = 8;
 constexpr uint32_t kMidWeightWarp = 20;
 constexpr uint32_t kMidInputWarp = 21;
 constexpr uint32_t kMidMmaWarp = 22;
 constexpr uint32_t kMidMaxRaw = 12;        // stages of the rings, at most
 constexpr uint32_t kMidMaxX = 8;
 constexpr uint32_t kMidMaxA = 3;
-constexpr uint32_t kMidBars = 2 * kMidMaxRaw + 2 * kMidMaxX + 2 * kMidMaxA + 4 + 1;
+constexpr uint32_t kMidBars = 3 * kMidMaxRaw + 2 * kMidMaxX + 2 * kMidMaxA + 4 + 1;
 constexpr uint32_t kMidStageBytes = 4 * 2 * 2048;   // per storing warp: two turns of 16 rows of x by 32 columns, floats
 constexpr uint32_t kMidTail = kMidStageBytes + kMidBars * 8 + 16;
 constexpr uint32_t kMidSmem = 227u * 1024u;
@@ -63,54 +61,16 @@ struct MidArgs {
     unsigned int raw_offset, raw_stride;
 };
 
-// Two blocks of 32 weights of quarter Q of a segment: `raw` holds bytes [64 Q, 64 Q + 80) of the
-// thread's row segment, the quarter's blocks start at local byte 4 Q + 34 jb.  They become 32 words
-// in the thread's lane of tensor memory.
-template <int Q>
-__device__ __forceinline__ void convert_quarter(const uint32_t (&raw)[20], uint32_t taddr)
-{
-    uint32_t out[32];
-#pragma unroll
-    for (int jb = 0; jb < 2; ++jb) {
-        const int byte_off = 4 * Q + 34 * jb;
-        const int wi = byte_off / 4;
-        const bool odd = (byte_off % 4) == 2;
-        const uint32_t d_bits = prmt(raw[wi], raw[wi], odd ? 0x3232u : 0x1010u);
-        const __half2 d2 = *reinterpret_cast<const __half2 *>(&d_bits);
-#pragma unroll
-        for (int p = 0; p < 16; ++p) {
-            // odd: the payload starts at the next word boundary; else in the high half of the
-            // scale's word
-            const int word = odd ? wi + 1 + p / 2 : wi + (p + 1) / 2;
-            const bool high = odd ? (p % 2) != 0 : ((p + 1) % 2) != 0;
-            const uint32_t flipped = raw[word] ^ 0x80808080u;
-            out[16 * jb + p] = high ? dequant_pair<1>(flipped, d2) : dequant_pair<0>(flipped, d2);
-        }
-    }
-    tmem_st_32x32(taddr, out);
-}
-
-template <int Q>
-__device__ __forceinline__ void load_quarter(uint32_t raw_row, uint32_t (&raw)[20])
-{
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        ld_shared_v4(raw_row + (uint32_t)(Q * 64 + 16 * i), raw[4 * i], raw[4 * i + 1], raw[4 * i + 2], raw[4 * i + 3]);
-    }
-}
-
 // Every lane has the words of its row, not only asked for them, when the raw stage goes back
-// (raw_words_present in q8_tile.cuh says why); true about once in 2^64 loads.
-__device__ __forceinline__ void quarter_present(const uint32_t (&raw)[20], unsigned int *status)
+// (raw_words_present in q8_tile.cuh says why); true about once in 2^32 loads, and then does nothing.
+__device__ __forceinline__ void mid_words_present(const uint32_t (&raw)[36], unsigned int *status)
 {
-    uint32_t all = raw[0];
-    uint32_t sum = raw[1];
+    uint32_t all = 0x5F3759DFu;
 #pragma unroll
-    for (int i = 2; i < 20; i += 2) {
+    for (int i = 0; i < 36; ++i) {
         all ^= raw[i];
-        sum += raw[i + 1];
     }
-    if (__any_sync(0xFFFFFFFFu, all == 0x5F3759DFu && sum == 0x9E3779B9u)) {
+    if (__any_sync(0xFFFFFFFFu, all == 0u)) {
         atomicOr(status, 0u);
     }
 }
@@ -213,7 +173,12 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t raw_base = smem0 + args.raw_offset;
     const uint32_t stage_base = smem0 + kMidRings;
     const uint32_t raw_full = stage_base + kMidStageBytes;
-    const uint32_t raw_empty = raw_full + 8u * kMidMaxRaw;
+    // Two barriers per raw stage, for its uses in turn: a barrier then belongs to one group of
+    // converters.  (With one barrier and an odd number of stages the groups alternate on it, and a
+    // group that comes to a stage's second use while the first copy is still on its way - copies may
+    // land out of order - finds the parity it waits for: that of the use before the first.)
+    const uint32_t raw_empty = raw_full + 16u * kMidMaxRaw;
+    const uint32_t raw_turns = 2u * args.raw_stages;
     const uint32_t x_full = raw_empty + 8u * kMidMaxRaw;
     const uint32_t x_empty = x_full + 8u * kMidMaxX;
     const uint32_t a_full = x_empty + 8u * kMidMaxX;
@@ -247,14 +212,15 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         tma_prefetch_desc(&tmap_x);
         for (uint32_t i = 0; i < args.raw_stages; ++i) {
             mbar_init(raw_full + 8u * i, 1u);
-            mbar_init(raw_empty + 8u * i, kMidConvertWarps);
+            mbar_init(raw_full + 8u * (i + args.raw_stages), 1u);
+            mbar_init(raw_empty + 8u * i, kMidGroupWarps);
         }
         for (uint32_t i = 0; i < args.x_stages; ++i) {
             mbar_init(x_full + 8u * i, 1u);
             mbar_init(x_empty + 8u * i, 1u);
         }
         for (uint32_t i = 0; i < args.a_stages; ++i) {
-            mbar_init(a_full + 8u * i, kMidConvertWarps);
+            mbar_init(a_full + 8u * i, kMidGroupWarps);
             mbar_init(a_empty + 8u * i, 1u);
         }
         for (uint32_t i = 0; i < 2u; ++i) {
@@ -309,6 +275,8 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         if (elect_one()) {
             uint32_t g = 0;
             bool ok = true;
+            uint32_t full = 0u;                    // g modulo the full barriers
+            uint32_t st = 0u, ph = 1u;             // g modulo the stages, and the parity of the use before
             for (uint32_t turn = 0; ok && turn < turns; ++turn) {
                 uint32_t w_row[2];
                 if (grouped) {
@@ -321,18 +289,20 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 }
                 for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
                     for (uint32_t p = 0; p < pair; ++p, ++g) {
-                        if (g < early) {
-                            continue;
+                        if (g >= early) {
+                            if (!mbar_wait(raw_empty + 8u * st, ph, abort_flag, args.status)) {
+                                ok = false;
+                                break;
+                            }
+                            mbar_expect_tx(raw_full + 8u * full, raw_bytes);
+                            tma_load_2d(raw_base + st * args.raw_stride, &tmap_w, raw_full + 8u * full,
+                                        (int)(s * kSegWords), (int)(p == 0u ? w_row[0] : w_row[1]));
                         }
-                        const uint32_t st = g % args.raw_stages;
-                        const uint32_t ph = (g / args.raw_stages) & 1u;
-                        if (!mbar_wait(raw_empty + 8u * st, ph ^ 1u, abort_flag, args.status)) {
-                            ok = false;
-                            break;
+                        full = full + 1u == raw_turns ? 0u : full + 1u;
+                        if (++st == args.raw_stages) {
+                            st = 0u;
+                            ph ^= 1u;
                         }
-                        mbar_expect_tx(raw_full + 8u * st, raw_bytes);
-                        tma_load_2d(raw_base + st * args.raw_stride, &tmap_w, raw_full + 8u * st, (int)(s * kSegWords),
-                                    (int)(p == 0u ? w_row[0] : w_row[1]));
                     }
                 }
             }
@@ -341,7 +311,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const uint32_t issued = g > early ? g : early;
             const uint32_t first = issued > args.raw_stages ? issued - args.raw_stages : 0u;
             for (uint32_t i = first; i < issued; ++i) {
-                mbar_wait(raw_full + 8u * (i % args.raw_stages), (i / args.raw_stages) & 1u, &local_abort, nullptr);
+                mbar_wait(raw_full + 8u * (i % raw_turns), (i / raw_turns) & 1u, &local_abort, nullptr);
             }
         }
     } else if (warp == kMidInputWarp) {
@@ -350,12 +320,11 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             uint32_t g = 0;
             grid_dependency_wait();
             bool ok = true;
+            uint32_t st = 0u, ph = 1u;
             for (uint32_t turn = 0; ok && turn < turns; ++turn) {
                 const uint32_t tok0 = grouped ? args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair].tok0 : 0u;
                 for (uint32_t s = seg_begin; s < seg_end; ++s, ++g) {
-                    const uint32_t st = g % args.x_stages;
-                    const uint32_t ph = (g / args.x_stages) & 1u;
-                    if (!mbar_wait(x_empty + 8u * st, ph ^ 1u, abort_flag, args.status)) {
+                    if (!mbar_wait(x_empty + 8u * st, ph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
@@ -364,6 +333,10 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     for (uint32_t j = 0; j < kSubs; ++j) {
                         tma_load_2d(smem0 + st * x_seg_bytes + j * (x_seg_bytes / kSubs), &tmap_x, x_full + 8u * st,
                                     (int)(s * kSegK + j * kSubK), (int)tok0);
+                    }
+                    if (++st == args.x_stages) {
+                        st = 0u;
+                        ph ^= 1u;
                     }
                 }
             }
@@ -377,8 +350,10 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // ---------------------------------------------------------------- MMA issue
         if (elect_one()) {
             const uint32_t idesc = umma_idesc(kRows, ntok, 0u, 0u);
-            uint32_t g = 0;      // segments of x
-            uint32_t a = 0;      // segments of A
+            // (counted up, not divided: a division by a number that only the launch knows takes longer
+            // than the MMAs of a segment)
+            uint32_t xst = 0u, xph = 0u;
+            uint32_t ast = 0u, aph = 0u;
             bool ok = true;
             for (uint32_t turn = 0; ok && turn < turns; ++turn) {
                 const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
@@ -388,15 +363,13 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     break;
                 }
                 tc_fence_after_sync();
-                for (uint32_t s = seg_begin; ok && s < seg_end; ++s, ++g) {
-                    const uint32_t xst = g % args.x_stages;
-                    if (!mbar_wait(x_full + 8u * xst, (g / args.x_stages) & 1u, abort_flag, args.status)) {
+                for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
+                    if (!mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
-                    for (uint32_t p = 0; p < pair; ++p, ++a) {
-                        const uint32_t ast = a % args.a_stages;
-                        if (!mbar_wait(a_full + 8u * ast, (a / args.a_stages) & 1u, abort_flag, args.status)) {
+                    for (uint32_t p = 0; p < pair; ++p) {
+                        if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                             ok = false;
                             break;
                         }
@@ -415,9 +388,17 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                             }
                         }
                         umma_commit(a_empty + 8u * ast);
+                        if (++ast == args.a_stages) {
+                            ast = 0u;
+                            aph ^= 1u;
+                        }
                     }
                     if (ok) {
                         umma_commit(x_empty + 8u * xst);
+                        if (++xst == args.x_stages) {
+                            xst = 0u;
+                            xph ^= 1u;
+                        }
                     }
                 }
                 if (ok) {
@@ -433,27 +414,31 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
     } else if (warp >= kConvertWarp0) {
         // ---------------------------------------------------------------- dequantise
+        // Two groups of eight warps take segments in turn: while one group waits for its raw segment, for
+        // its stage of tensor memory or for its loads, the other has the arithmetic.  (Sixteen warps
+        // on one segment go through these phases together and leave the schedulers idle in between.)
         const uint32_t cw = warp - kConvertWarp0;
-        const uint32_t quarter = cw >> 2;
+        const uint32_t group = cw / kMidGroupWarps;
+        const uint32_t half = (cw >> 2) & 1u;
         const uint32_t row = (cw & 3u) * 32u + lane;
         // rows past the slab repeat its last one (their sums are not stored)
         const uint32_t row_at = (row < args.slab_rows ? row : args.slab_rows - 1u) * kSegBytes;
-        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + quarter * (kSegK / 8u);
+        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
         const uint32_t total = turns * (seg_end - seg_begin) * pair;
-        uint32_t rst = 0, rph = 0, ast = 0, aph = 0;
-        for (uint32_t g = 0; g < total; ++g) {
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * rst, rph, abort_flag, args.status))) {
+        uint32_t full = group, fph = 0, ast = group, aph = 0;
+        for (uint32_t g = group; g < total; g += kMidGroups) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
                 break;
             }
-            uint32_t raw[20];
+            const uint32_t rst = full < args.raw_stages ? full : full - args.raw_stages;
+            uint32_t raw[36];
             const uint32_t raw_row = raw_base + rst * args.raw_stride + row_at;
-            switch (quarter) {
-            case 0u: load_quarter<0>(raw_row, raw); break;
-            case 1u: load_quarter<1>(raw_row, raw); break;
-            case 2u: load_quarter<2>(raw_row, raw); break;
-            default: load_quarter<3>(raw_row, raw); break;
+            if (half == 0u) {
+                load_raw<0>(raw_row, raw);
+            } else {
+                load_raw<1>(raw_row, raw);
             }
-            quarter_present(raw, args.status);
+            mid_words_present(raw, args.status);
             if (lane == 0u) {
                 mbar_arrive(raw_empty + 8u * rst);
             }
@@ -462,11 +447,12 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             }
             const uint32_t taddr = lane_base + ast * (kSegK / 2u);
             tc_fence_after_sync();
-            switch (quarter) {
-            case 0u: convert_quarter<0>(raw, taddr); break;
-            case 1u: convert_quarter<1>(raw, taddr); break;
-            case 2u: convert_quarter<2>(raw, taddr); break;
-            default: convert_quarter<3>(raw, taddr); break;
+            if (half == 0u) {
+                convert_stage_tmem<0, 0>(raw, taddr);
+                convert_stage_tmem<0, 1>(raw, taddr + kSubK / 2u);
+            } else {
+                convert_stage_tmem<1, 0>(raw, taddr);
+                convert_stage_tmem<1, 1>(raw, taddr + kSubK / 2u);
             }
             tmem_st_wait();
             tc_fence_before_sync();
@@ -474,12 +460,14 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             if (lane == 0u) {
                 mbar_arrive(a_full + 8u * ast);
             }
-            if (++rst == args.raw_stages) {
-                rst = 0u;
-                rph ^= 1u;
+            full += kMidGroups;
+            if (full >= raw_turns) {
+                full -= raw_turns;
+                fph ^= 1u;
             }
-            if (++ast == args.a_stages) {
-                ast = 0u;
+            ast += kMidGroups;
+            if (ast >= args.a_stages) {
+                ast -= args.a_stages;
                 aph ^= 1u;
             }
         }
@@ -565,6 +553,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
     }
 
+    __syncwarp();
     if (csize > 1u) {
         // ------------------------------------------------------------ sum of a cluster's parts
         // One pair of slabs per cluster.  The rows of x are dealt to its blocks in runs of `share`;
