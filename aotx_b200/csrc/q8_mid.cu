@@ -56,7 +56,7 @@ struct MidArgs {
     unsigned int ntok;                 // columns of an accumulator: rows of x, a multiple of 16
     unsigned int slab_rows;            // rows of w per slab (a multiple of 4)
     unsigned int pair;                 // slabs that share a segment of x: 1 or 2
-    unsigned int turns;                // times `pair` slabs per block (not in grouped mode)
+    unsigned int slabs;                // ... and how many a block takes (not in grouped mode)
     unsigned int x_stages, raw_stages, a_stages, acc_buffers;
     unsigned int raw_offset, raw_stride;
 };
@@ -163,6 +163,13 @@ __device__ __forceinline__ void mid_store_staged(const MidArgs &args, uint32_t s
     }
 }
 
+// Slabs of turn `turn` out of `slabs` in turns of `pair`: the last turn can be one short.
+__device__ __forceinline__ uint32_t slabs_of_turn(uint32_t slabs, uint32_t pair, uint32_t turn)
+{
+    const uint32_t left = slabs - turn * pair;
+    return left < pair ? left : pair;
+}
+
 template <typename YT>
 __global__ void __launch_bounds__(kMidThreads, 1)
 q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const MidArgs args)
@@ -202,7 +209,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t crank = cluster_ctarank();
     const uint32_t seg_begin = crank * segs / csize;
     const uint32_t seg_end = (crank + 1u) * segs / csize;
-    const uint32_t slab0 = blockIdx.x / csize * args.turns * pair;   // the block's first slab (its cluster's)
+    const uint32_t slab0 = blockIdx.x / csize * args.slabs;   // the block's first slab (its cluster's)
 
     grid_launch_dependents();
 
@@ -233,16 +240,20 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         fence_proxy_async_smem();
         if (!grouped) {
             // the first weights: only the barriers they signal have to be there
-            const uint32_t total = args.turns * (seg_end - seg_begin) * pair;
-            const uint32_t per_turn = (seg_end - seg_begin) * pair;
+            const uint32_t total = args.slabs * (seg_end - seg_begin);
+            uint32_t s = seg_begin, p = 0u, turn = 0u;
             for (; early < args.raw_stages && early < total; ++early) {
-                const uint32_t turn = early / per_turn;
-                const uint32_t in_turn = early - turn * per_turn;
-                const uint32_t s = seg_begin + in_turn / pair;
-                const uint32_t slab = slab0 + turn * pair + in_turn % pair;
+                const uint32_t slab = slab0 + turn * pair + p;
                 mbar_expect_tx(raw_full + 8u * early, raw_bytes);
                 tma_load_2d(raw_base + early * args.raw_stride, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords),
                             (int)(slab * args.slab_rows));
+                if (++p == slabs_of_turn(args.slabs, pair, turn)) {
+                    p = 0u;
+                    if (++s == seg_end) {
+                        s = seg_begin;
+                        ++turn;
+                    }
+                }
             }
         }
     }
@@ -260,14 +271,15 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t tmem_base = *tmem_slot_ptr;
     const uint32_t a_column0 = args.acc_buffers * pair * ntok;
 
-    // how many pairs of slabs this block takes
-    uint32_t turns = args.turns;
+    // how many slabs this block takes, and in how many turns of at most `pair`
+    uint32_t slabs = args.slabs;
     if (grouped) {
         // the table was built by the kernel before this one on the stream
         grid_dependency_wait();
         const uint32_t pairs = *args.group_count / pair;
-        turns = blockIdx.x < pairs ? (pairs - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+        slabs = blockIdx.x < pairs ? (pairs - blockIdx.x + gridDim.x - 1u) / gridDim.x * pair : 0u;
     }
+    const uint32_t turns = pair > 1u ? (slabs + 1u) / 2u : slabs;
     unsigned int m_live = args.m_max;
 
     if (warp == kMidWeightWarp) {
@@ -288,7 +300,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     w_row[1] = w_row[0] + args.slab_rows;
                 }
                 for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
-                    for (uint32_t p = 0; p < pair; ++p, ++g) {
+                    for (uint32_t p = 0; p < slabs_of_turn(slabs, pair, turn); ++p, ++g) {
                         if (g >= early) {
                             if (!mbar_wait(raw_empty + 8u * st, ph, abort_flag, args.status)) {
                                 ok = false;
@@ -358,6 +370,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             for (uint32_t turn = 0; ok && turn < turns; ++turn) {
                 const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
                 const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
+                const uint32_t here = slabs_of_turn(slabs, pair, turn);
                 if (!mbar_wait(acc_empty + 8u * buf, (uses & 1u) ^ 1u, abort_flag, args.status)) {
                     ok = false;
                     break;
@@ -368,7 +381,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         ok = false;
                         break;
                     }
-                    for (uint32_t p = 0; p < pair; ++p) {
+                    for (uint32_t p = 0; p < here; ++p) {
                         if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                             ok = false;
                             break;
@@ -405,10 +418,10 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     umma_commit(acc_full + 8u * buf);
                 }
             }
+            umma_commit(drain_bar);     // every MMA has finished: what the helping warps wait for
             if (!ok) {
                 // Outstanding MMAs must finish before the tensor memory goes back.
                 uint32_t local_abort = 0;
-                umma_commit(drain_bar);
                 mbar_wait(drain_bar, 0u, &local_abort, nullptr);
             }
         }
@@ -424,7 +437,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // rows past the slab repeat its last one (their sums are not stored)
         const uint32_t row_at = (row < args.slab_rows ? row : args.slab_rows - 1u) * kSegBytes;
         const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
-        const uint32_t total = turns * (seg_end - seg_begin) * pair;
+        const uint32_t total = slabs * (seg_end - seg_begin);
         uint32_t full = group, fph = 0, ast = group, aph = 0;
         for (uint32_t g = group; g < total; g += kMidGroups) {
             if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
@@ -471,11 +484,20 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 aph ^= 1u;
             }
         }
-    } else if (csize == 1u) {
+    }
+
+    if (csize == 1u && warp < kMidWeightWarp && turns != 0u) {
         // ---------------------------------------------------------------- read sums, store
-        const uint32_t lane_taddr = tmem_base + ((warp * 32u) << 16);
+        // Warps 0-3 store every turn but the last beside the work of the next.  In the last one nothing
+        // is left to convert and the converters help: four warps alone took 4.6 us (64 rows) and 7 us
+        // (100 rows) at the end of launches of 30 and 40 us.  Their staging buffers lie over the
+        // rings, which are idle once the last sums are there.
+        const uint32_t lanes = warp & 3u;
+        const uint32_t helper = warp >> 2;                       // 0: the storing warps
+        const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
         const bool gated = args.epilogue == kEpilogueSwiglu;
-        const uint32_t buffers = stage_base + warp * (kMidStageBytes / 4u);
+        const uint32_t buffers = helper == 0u ? stage_base + warp * (kMidStageBytes / 4u)
+                                              : smem0 + (warp - kEpilogueWarps) * (kMidStageBytes / 4u);
         uint32_t flip = 0u;      // the two turns of the warp's staging buffer
         grid_dependency_wait();
         if (args.m_dev != nullptr) {
@@ -485,12 +507,14 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // rows of y start on a boundary of four values, and so does every slab
         const bool aligned = (args.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.y) % (4u * sizeof(YT))) == 0u
                           && (args.slab_rows % (gated ? 8u : 4u)) == 0u;
-        for (uint32_t turn = 0; turn < turns; ++turn) {
+        for (uint32_t turn = helper == 0u ? 0u : turns - 1u; turn < turns; ++turn) {
+            const bool last = turn + 1u == turns;
             const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
             const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
-            // where the pair goes (table entries in grouped mode): asked for before the wait
+            const uint32_t here = slabs_of_turn(slabs, pair, turn);
+            // where the slabs go (table entries in grouped mode): asked for before the wait
             GroupTile place[2];
-            for (uint32_t p = 0; p < pair; ++p) {
+            for (uint32_t p = 0; p < here; ++p) {
                 if (grouped) {
                     place[p] = args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair + p];
                 } else {
@@ -500,22 +524,32 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     place[p].tok_limit = m_live;
                 }
             }
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(acc_full + 8u * buf, uses & 1u, abort_flag, args.status))) {
+            // (a helper has seen none of the turns before, so it does not ask for a parity of their barrier)
+            if (!__all_sync(0xFFFFFFFFu, helper == 0u ? mbar_wait(acc_full + 8u * buf, uses & 1u, abort_flag, args.status)
+                                                      : mbar_wait(drain_bar, 0u, abort_flag, args.status))) {
                 break;
             }
             tc_fence_after_sync();
+            // pieces of 16 rows of x, dealt to the warps of the same lanes in the last turn
+            const uint32_t step = last ? kMidWeightWarp / 4u : 1u;
+            uint32_t piece = last ? helper : 0u;
 #pragma unroll 1
-            for (uint32_t p = 0; p < pair; ++p) {
+            for (uint32_t p = 0; p < here; ++p) {
                 const GroupTile at = p == 0u ? place[0] : place[1];
                 const uint32_t rows = at.tok_limit > at.tok0 ? at.tok_limit - at.tok0 : 0u;
-                const uint32_t j = at.j0 + warp * 32u;                                   // this warp's first row of w
+                const uint32_t live = (rows < ntok ? rows + 15u : ntok) / 16u;           // pieces with a row to store
+                const uint32_t j = at.j0 + lanes * 32u;                                  // this warp's first row of w
                 const uint32_t inside = at.j_limit > j ? at.j_limit - j : 0u;            // ... and how many are there
                 const uint32_t mine = inside < 32u ? inside : 32u;
                 const uint32_t columns = gated ? mine / 2u : mine;
                 const uint32_t col = gated ? j / 2u : j;
                 const bool staged = aligned && (columns % 4u) == 0u;
 #pragma unroll 1
-                for (uint32_t c0 = 0; c0 < ntok && c0 < rows && mine != 0u; c0 += 16u) {
+                for (; piece < live; piece += step) {
+                    if (mine == 0u) {
+                        continue;
+                    }
+                    const uint32_t c0 = piece * 16u;
                     uint32_t v[16];
                     tmem_ld_32x16(lane_taddr + (buf * pair + p) * ntok + c0, v);
                     tmem_ld_wait();
@@ -543,12 +577,15 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         }
                     }
                 }
+                piece -= live;
             }
-            // The accumulators are free again.
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0u) {
-                mbar_arrive(acc_empty + 8u * buf);
+            if (!last) {
+                // The accumulators are free again.
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0u) {
+                    mbar_arrive(acc_empty + 8u * buf);
+                }
             }
         }
     }
@@ -558,7 +595,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // ------------------------------------------------------------ sum of a cluster's parts
         // One pair of slabs per cluster.  The rows of x are dealt to its blocks in runs of `share`;
         // every block writes its part's sums into their owners' shared memory, over the rings, which are
-        // idle by then: [sender][slab][row of x][row of w].  The owner adds the parts in block order.
+        // idle by then: [sender][slab][run of four rows of x][row of w], 16 bytes at a time.  The owner adds the parts in block order.
         bool there = true;
         if (warp < kMidWeightWarp) {
             there = mbar_wait(acc_full, 0u, abort_flag, args.status);
@@ -580,10 +617,12 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 tmem_ld_32x16(lane_taddr + p * ntok + c0, v);
                 tmem_ld_wait();
 #pragma unroll
-                for (uint32_t i = 0; i < 16u; ++i) {
-                    const uint32_t token = c0 + i;
-                    const uint32_t at = smem0 + (((crank * pair + p) * share + token % share) * kRows + row) * 4u;
-                    st_shared_cluster_f32(mapa_shared(at, token / share), __uint_as_float(v[i]));
+                for (uint32_t i = 0; i < 16u; i += 4u) {
+                    const uint32_t owner = (c0 + i) / share;
+                    const uint32_t run = (c0 + i - owner * share) / 4u;
+                    const uint32_t at = smem0 + (((crank * pair + p) * (share / 4u) + run) * kRows + row) * 16u;
+                    st_shared_cluster_v4_f32(mapa_shared(at, owner), __uint_as_float(v[i]), __uint_as_float(v[i + 1u]),
+                                             __uint_as_float(v[i + 2u]), __uint_as_float(v[i + 3u]));
                 }
             }
             tc_fence_before_sync();
@@ -599,26 +638,32 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         if (!there) {
             m_live = 0u;
         }
-        const float *recv = reinterpret_cast<const float *>(smem);
+        const float4 *recv = reinterpret_cast<const float4 *>(smem);
         const bool gated = args.epilogue == kEpilogueSwiglu;
-        const uint32_t rows_of_x = pair * share;
-        // warp = 32 rows of w of one row of x
-        for (uint32_t at = warp; at < rows_of_x * (kRows / 32u); at += kMidThreads / 32u) {
-            const uint32_t local = at / (kRows / 32u);                  // slab * share + row of x within the share
+        const uint32_t runs = pair * (share / 4u);                      // runs of four rows of x per sender
+        // warp = 32 rows of w of one run
+        for (uint32_t at = warp; at < runs * (kRows / 32u); at += kMidThreads / 32u) {
+            const uint32_t local = at / (kRows / 32u);                  // slab * (share / 4) + run within the share
             const uint32_t row = (at % (kRows / 32u)) * 32u + lane;
-            const uint32_t p = local / share;
-            const uint32_t token = crank * share + (local - p * share);
-            float sum = recv[(size_t)local * kRows + row];
+            const uint32_t p = local / (share / 4u);
+            const uint32_t token = crank * share + (local - p * (share / 4u)) * 4u;
+            float4 four = recv[local * kRows + row];
             for (uint32_t src = 1; src < csize; ++src) {
-                sum += recv[((size_t)src * rows_of_x + local) * kRows + row];
+                const float4 more = recv[(src * runs + local) * kRows + row];
+                four = make_float4(four.x + more.x, four.y + more.y, four.z + more.z, four.w + more.w);
             }
             const uint32_t j = (slab0 + p) * args.slab_rows + row;
-            if (gated) {
-                const float up = __shfl_xor_sync(0xFFFFFFFFu, sum, 1u);
-                sum = sum / (1.0f + expf(-sum)) * up;
-            }
-            if (token < m_live && row < args.slab_rows && j < args.n && (!gated || (row & 1u) == 0u)) {
-                mid_store_one<YT>(args, (size_t)token * args.ldy + (gated ? j / 2u : j), sum);
+            const float sums[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) {
+                float sum = sums[i];
+                if (gated) {
+                    const float up = __shfl_xor_sync(0xFFFFFFFFu, sum, 1u);
+                    sum = sum / (1.0f + expf(-sum)) * up;
+                }
+                if (token + i < m_live && row < args.slab_rows && j < args.n && (!gated || (row & 1u) == 0u)) {
+                    mid_store_one<YT>(args, (size_t)(token + i) * args.ldy + (gated ? j / 2u : j), sum);
+                }
             }
         }
     }
@@ -745,14 +790,14 @@ MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm
         plan.cluster = 2u;
         clusters = sm_count / 2u;
     }
-    unsigned int slabs = (n + clusters * kRows - 1u) / (clusters * kRows);     // per cluster
+    const unsigned int slabs = (n + clusters * kRows - 1u) / (clusters * kRows);     // per cluster
     plan.pair = slabs > 1u ? 2u : 1u;
-    plan.turns = (slabs + plan.pair - 1u) / plan.pair;
-    const unsigned int all = clusters * plan.pair * plan.turns;
+    plan.slabs = slabs;
+    const unsigned int all = clusters * slabs;
     plan.slab_rows = ((n + all - 1u) / all + step - 1u) / step * step;
     // rounding up can leave the last clusters without rows
     const unsigned int used = (n + plan.slab_rows - 1u) / plan.slab_rows;
-    clusters = (used + plan.pair * plan.turns - 1u) / (plan.pair * plan.turns);
+    clusters = (used + slabs - 1u) / slabs;
     plan.grid = clusters * plan.cluster;
     return plan;
 }
@@ -773,7 +818,7 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
     args.ntok = plan.ntok;
     args.slab_rows = plan.slab_rows;
     args.pair = plan.pair;
-    args.turns = plan.turns;
+    args.slabs = plan.slabs;
     return launch_mid(stream, tw, tx, args, plan.grid, plan.cluster, overlap, y_dtype);
 }
 

@@ -644,10 +644,10 @@ cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const
                                unsigned int grid, unsigned int cluster, int y_dtype);
 
 // The product for 17 to 128 rows and the grouped products (q8_mid.cu): how a product's rows of w are
-// dealt (slabs of slab_rows rows, `pair` at a time, `turns` times per block; `cluster` blocks share a
+// dealt (slabs of slab_rows rows, `slabs` per block, `pair` at a time; `cluster` blocks share a
 // slab's depth), and the launches.
 struct MidPlan {
-    unsigned int ntok, slab_rows, pair, turns, cluster, grid;
+    unsigned int ntok, slab_rows, pair, slabs, cluster, grid;
 };
 MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue);
 cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
