@@ -122,6 +122,18 @@ static bool map_rows(EncodeTiledFn encode, CUtensorMap *map, const void *x, unsi
         == CUDA_SUCCESS;
 }
 
+// Two sets of slots and flags alternate between launches, so that a launch whose blocks start early
+// never meets the slots of the launch before it.
+static float *set_partial(const UmmaScratch &scratch, unsigned int set)
+{
+    return scratch.partial + (unsigned long long)(set & 1u) * scratch.blocks * scratch.tile_floats;
+}
+
+static unsigned int *set_flags(const UmmaScratch &scratch, unsigned int set)
+{
+    return scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * kFlagWords;
+}
+
 cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigned int sm_count,
                         const void *w, unsigned int n, unsigned int k, const void *x, int x_bf16,
                         unsigned int m, const unsigned int *m_dev, void *y, int y_dtype, unsigned int set,
@@ -143,7 +155,8 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     const bool mid = false;
 #else
     // the kernel for 17 to 128 rows takes binary16 x
-    const bool mid = ntok > 16u && ntok <= 128u && out == nullptr && (!x_bf16 || copy_fits);
+    const bool mid = ntok > 16u && ntok <= 128u && out == nullptr && (!x_bf16 || copy_fits)
+                  && (unsigned long long)(n / kRows + 1u) * (k / kSegK) < (1ull << 31);
 #endif
     if (x_bf16 && (mid || ntok >= 64u) && ntok <= 128u && copy_fits) {
         const unsigned long long chunks = (unsigned long long)m * k / 8ull;
@@ -165,13 +178,15 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     // peers' copies stay with the kernels they were measured on.
     const bool warp_kernel = ntok <= 16u && out == nullptr;
     if (mid) {
-        const MidPlan plan = mid_plan(n, k, m, sm_count, epilogue);
+        const MidPlan plan = mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats,
+                                      epilogue);
         CUtensorMap tw, tx;
         if (!map_weights(encode, &tw, w, n, k, plan.slab_rows) || !map_rows(encode, &tx, x, m, k, plan.ntok, false)) {
             return cudaErrorInvalidValue;
         }
         return launch_mid_product(stream, tw, tx, plan, n, k, m, m_dev, y, y_dtype, epilogue == kEpilogueSwiglu ? n / 2u : n,
-                                  epilogue, scratch.status, overlap);
+                                  epilogue, set_partial(scratch, set), set_flags(scratch, set), scratch.tile_floats,
+                                  scratch.status, overlap);
     }
 #endif
 
@@ -197,10 +212,8 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     args.m_max = m;
     args.m_dev = m_dev;
     args.y = y;
-    // Two sets of slots and flags alternate between launches, so that a launch whose blocks
-    // start early never meets the slots of the launch before it.
-    args.partial = scratch.partial + (unsigned long long)(set & 1u) * scratch.blocks * scratch.tile_floats;
-    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * kFlagWords;
+    args.partial = set_partial(scratch, set);
+    args.flags = set_flags(scratch, set);
     args.overlap = overlap ? 1u : 0u;
     args.group_tiles = nullptr;
     args.group_count = nullptr;
@@ -282,9 +295,9 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
         // every expert has an even number of weight row tiles (hidden and ffn are multiples of 256), so
         // the table's entries pair up
         const unsigned int blocks = max_tiles / 2u < sm_count ? max_tiles / 2u : sm_count;
-        (void)set;
         return launch_mid_grouped(stream, tw, tx, blocks, k, ntok, tiles, count_dev, row_map, y, ldy, y_dtype, epilogue,
-                                  scratch.status, overlap);
+                                  set_partial(scratch, set), set_flags(scratch, set), scratch.tile_floats, scratch.status,
+                                  overlap);
     }
 #endif
     const unsigned long long units = (unsigned long long)max_tiles * (k / kSegK);
@@ -298,8 +311,8 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
     args.m_max = x_rows;
     args.m_dev = nullptr;
     args.y = y;
-    args.partial = scratch.partial + (unsigned long long)(set & 1u) * scratch.blocks * scratch.tile_floats;
-    args.flags = scratch.flags + (unsigned long long)(set & 1u) * scratch.blocks * kFlagWords;
+    args.partial = set_partial(scratch, set);
+    args.flags = set_flags(scratch, set);
     args.status = scratch.status;
     args.tile_floats = scratch.tile_floats;
     args.b_bf16 = 0u;

@@ -7,12 +7,12 @@
 // by tcgen05.mma (128 x N x 16, N = the batch rounded up to 16), as in q8_stream.cu; what is
 // different there cost half the time of these products:
 //
-//   * No tile is cut between blocks that meet through global memory (the hand-over of partial
-//     tiles took 3 to 8 us at the end of a launch of 20).  The rows of w are dealt in SLABS of at
-//     most 128 rows, all of one size, so many of them that every block has the same number: with
-//     many rows a block takes its slabs over the whole depth and stores them, with fewer a CLUSTER
-//     of 2 or 4 blocks takes each slab, one run of its depth per block, and the parts are added
-//     through distributed shared memory.
+//   * Few rows of w (at most 256 per cluster of four): they are dealt in SLABS of at most 128 rows, all
+//     of one size, to clusters; each block takes a run of the depth, and the parts are added through
+//     distributed shared memory.  More rows: tiles of two slabs, as many to every block; or, where that
+//     would leave the last of the blocks' turns too empty (kMidCutUnits), tiles of 128-row slabs cut
+//     into (tile, segment) units that are dealt evenly, a cut tile finished by the block that holds
+//     its first segment.
 //   * A segment of x (256 deep) in shared memory meets two slabs, one after the other: half the x
 //     traffic, which at 64 rows was as many bytes as the weights.
 //   * 16 converter warps in two groups that take segments in turn (thread = row, half a segment).
@@ -43,6 +43,13 @@ constexpr uint32_t kMidTail = kMidStageBytes + kMidBars * 8 + 16;
 constexpr uint32_t kMidSmem = 227u * 1024u;
 constexpr uint32_t kMidRings = (kMidSmem - 1024u - kMidTail) / 1024u * 1024u;   // both rings' shared memory
 
+// Cutting tiles into units evens the blocks out and costs them the hand-over of the cut tiles, more
+// stores at the wrong moment and a longer end: about as long as five units (of two slabs) take.
+// Measured with and without: 28672 x 4096, 64 rows, 12.1 units against 16: 33.5 us against 30.6;
+// 151936 x 8192, 64 rows, 128.3 against 144: 249 us against 269; routed experts, 512 tokens, 21
+// against 24: 262 us against 217.
+constexpr uint32_t kMidCutUnits = 5;
+
 struct MidArgs {
     unsigned int n, k, m_max;
     const unsigned int *m_dev;
@@ -56,7 +63,12 @@ struct MidArgs {
     unsigned int ntok;                 // columns of an accumulator: rows of x, a multiple of 16
     unsigned int slab_rows;            // rows of w per slab (a multiple of 4)
     unsigned int pair;                 // slabs that share a segment of x: 1 or 2
-    unsigned int slabs;                // ... and how many a block takes (not in grouped mode)
+    unsigned int tiles;                // of `pair` slabs each (not in grouped mode)
+    unsigned int turns;                // whole tiles per block; 0: units (not in grouped mode)
+    // unit schedule: a block's partial tile, [slab][row of x][row of w], and its flags
+    float *partial;
+    unsigned int *flags;
+    unsigned long long tile_floats;
     unsigned int x_stages, raw_stages, a_stages, acc_buffers;
     unsigned int raw_offset, raw_stride;
 };
@@ -163,12 +175,26 @@ __device__ __forceinline__ void mid_store_staged(const MidArgs &args, uint32_t s
     }
 }
 
-// Slabs of turn `turn` out of `slabs` in turns of `pair`: the last turn can be one short.
-__device__ __forceinline__ uint32_t slabs_of_turn(uint32_t slabs, uint32_t pair, uint32_t turn)
-{
-    const uint32_t left = slabs - turn * pair;
-    return left < pair ? left : pair;
-}
+// A block's work: pieces of tiles, each the segments [s0, s1) of one tile.
+struct MidWork {
+    uint32_t tile, s0, s1;     // the piece
+    uint32_t next_tile, next_seg, left, segs;
+    uint32_t stride;           // from one tile of the block to the next
+
+    __device__ __forceinline__ bool next()
+    {
+        if (left == 0u) {
+            return false;
+        }
+        tile = next_tile;
+        s0 = next_seg;
+        s1 = segs - s0 < left ? segs : s0 + left;
+        left -= s1 - s0;
+        next_tile += stride;
+        next_seg = 0u;
+        return true;
+    }
+};
 
 template <typename YT>
 __global__ void __launch_bounds__(kMidThreads, 1)
@@ -207,9 +233,45 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t raw_bytes = args.slab_rows * kSegBytes;
     const uint32_t csize = cluster_nctarank();
     const uint32_t crank = cluster_ctarank();
-    const uint32_t seg_begin = crank * segs / csize;
-    const uint32_t seg_end = (crank + 1u) * segs / csize;
-    const uint32_t slab0 = blockIdx.x / csize * args.slabs;   // the block's first slab (its cluster's)
+    // Clusters: one tile each, a run of its segments per block.  Else (tile, segment) units dealt evenly,
+    // the same arithmetic as the decode kernel's.  (The table of the grouped products, and its length,
+    // were written two launches before the first of them, so they may be read here already.)
+    const uint32_t tiles = grouped ? *reinterpret_cast<const volatile unsigned int *>(args.group_count) / pair : args.tiles;
+    const uint32_t units = tiles * segs;      // the host refuses products with 2^31 units or more
+    const uint32_t blocks = units < gridDim.x ? units : gridDim.x;
+    MidWork work;
+    work.segs = segs;
+    work.stride = 1u;
+    if (csize > 1u) {
+        work.next_tile = blockIdx.x / csize;
+        work.next_seg = crank * segs / csize;
+        work.left = (crank + 1u) * segs / csize - work.next_seg;
+    } else {
+        uint32_t turns = args.turns;
+        if (grouped) {
+            turns = (tiles + gridDim.x - 1u) / gridDim.x;
+            if (turns * segs > units / gridDim.x + kMidCutUnits) {
+                turns = 0u;
+            }
+        }
+        if (turns != 0u) {
+            // neighbouring blocks take neighbouring tiles, and where the last turn is not full its
+            // blocks have memory to themselves
+            work.next_tile = blockIdx.x;
+            work.next_seg = 0u;
+            work.stride = gridDim.x;
+            work.left = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * segs : 0u;
+        } else {
+            uint32_t u_begin = 0u, u_end = 0u;
+            if (blockIdx.x < blocks) {
+                decode_range(blockIdx.x, blocks, units, &u_begin, &u_end);
+            }
+            work.next_tile = u_begin / segs;
+            work.next_seg = u_begin - work.next_tile * segs;
+            work.left = u_end - u_begin;
+        }
+    }
+    const uint32_t total = work.left * pair;   // segments of weights
 
     grid_launch_dependents();
 
@@ -238,21 +300,17 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         *abort_flag = 0u;
         mbar_init_fence();
         fence_proxy_async_smem();
-        if (!grouped) {
-            // the first weights: only the barriers they signal have to be there
-            const uint32_t total = args.slabs * (seg_end - seg_begin);
-            uint32_t s = seg_begin, p = 0u, turn = 0u;
-            for (; early < args.raw_stages && early < total; ++early) {
-                const uint32_t slab = slab0 + turn * pair + p;
-                mbar_expect_tx(raw_full + 8u * early, raw_bytes);
-                tma_load_2d(raw_base + early * args.raw_stride, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords),
-                            (int)(slab * args.slab_rows));
-                if (++p == slabs_of_turn(args.slabs, pair, turn)) {
-                    p = 0u;
-                    if (++s == seg_end) {
-                        s = seg_begin;
-                        ++turn;
-                    }
+        // the first weights: only the barriers they signal have to be there
+        uint32_t tile = work.next_tile, s = work.next_seg, p = 0u;
+        for (; early < args.raw_stages && early < total; ++early) {
+            const uint32_t w_row = grouped ? args.group_tiles[(size_t)tile * pair + p].w_row : (tile * pair + p) * args.slab_rows;
+            mbar_expect_tx(raw_full + 8u * early, raw_bytes);
+            tma_load_2d(raw_base + early * args.raw_stride, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords), (int)w_row);
+            if (++p == pair) {
+                p = 0u;
+                if (++s == segs) {
+                    s = 0u;
+                    tile += work.stride;
                 }
             }
         }
@@ -271,15 +329,6 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t tmem_base = *tmem_slot_ptr;
     const uint32_t a_column0 = args.acc_buffers * pair * ntok;
 
-    // how many slabs this block takes, and in how many turns of at most `pair`
-    uint32_t slabs = args.slabs;
-    if (grouped) {
-        // the table was built by the kernel before this one on the stream
-        grid_dependency_wait();
-        const uint32_t pairs = *args.group_count / pair;
-        slabs = blockIdx.x < pairs ? (pairs - blockIdx.x + gridDim.x - 1u) / gridDim.x * pair : 0u;
-    }
-    const uint32_t turns = pair > 1u ? (slabs + 1u) / 2u : slabs;
     unsigned int m_live = args.m_max;
 
     if (warp == kMidWeightWarp) {
@@ -289,18 +338,18 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             bool ok = true;
             uint32_t full = 0u;                    // g modulo the full barriers
             uint32_t st = 0u, ph = 1u;             // g modulo the stages, and the parity of the use before
-            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
+            while (ok && work.next()) {
                 uint32_t w_row[2];
                 if (grouped) {
-                    const GroupTile *entry = args.group_tiles + (size_t)(blockIdx.x + turn * gridDim.x) * pair;
+                    const GroupTile *entry = args.group_tiles + (size_t)work.tile * pair;
                     w_row[0] = entry[0].w_row;
                     w_row[1] = pair > 1u ? entry[1].w_row : 0u;
                 } else {
-                    w_row[0] = (slab0 + turn * pair) * args.slab_rows;
+                    w_row[0] = work.tile * pair * args.slab_rows;
                     w_row[1] = w_row[0] + args.slab_rows;
                 }
-                for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
-                    for (uint32_t p = 0; p < slabs_of_turn(slabs, pair, turn); ++p, ++g) {
+                for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
+                    for (uint32_t p = 0; p < pair; ++p, ++g) {
                         if (g >= early) {
                             if (!mbar_wait(raw_empty + 8u * st, ph, abort_flag, args.status)) {
                                 ok = false;
@@ -333,9 +382,9 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             grid_dependency_wait();
             bool ok = true;
             uint32_t st = 0u, ph = 1u;
-            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
-                const uint32_t tok0 = grouped ? args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair].tok0 : 0u;
-                for (uint32_t s = seg_begin; s < seg_end; ++s, ++g) {
+            while (ok && work.next()) {
+                const uint32_t tok0 = grouped ? args.group_tiles[(size_t)work.tile * pair].tok0 : 0u;
+                for (uint32_t s = work.s0; s < work.s1; ++s, ++g) {
                     if (!mbar_wait(x_empty + 8u * st, ph, abort_flag, args.status)) {
                         ok = false;
                         break;
@@ -367,21 +416,20 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             uint32_t xst = 0u, xph = 0u;
             uint32_t ast = 0u, aph = 0u;
             bool ok = true;
-            for (uint32_t turn = 0; ok && turn < turns; ++turn) {
+            for (uint32_t turn = 0; ok && work.next(); ++turn) {
                 const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
                 const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
-                const uint32_t here = slabs_of_turn(slabs, pair, turn);
                 if (!mbar_wait(acc_empty + 8u * buf, (uses & 1u) ^ 1u, abort_flag, args.status)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
-                for (uint32_t s = seg_begin; ok && s < seg_end; ++s) {
+                for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
                     if (!mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
-                    for (uint32_t p = 0; p < here; ++p) {
+                    for (uint32_t p = 0; p < pair; ++p) {
                         if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                             ok = false;
                             break;
@@ -397,7 +445,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                             for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
                                 // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
                                 umma_f16_ts(d_tmem, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
-                                            s != seg_begin || j != 0u || kk != 0u ? 1u : 0u);
+                                            s != work.s0 || j != 0u || kk != 0u ? 1u : 0u);
                             }
                         }
                         umma_commit(a_empty + 8u * ast);
@@ -437,7 +485,6 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // rows past the slab repeat its last one (their sums are not stored)
         const uint32_t row_at = (row < args.slab_rows ? row : args.slab_rows - 1u) * kSegBytes;
         const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
-        const uint32_t total = slabs * (seg_end - seg_begin);
         uint32_t full = group, fph = 0, ast = group, aph = 0;
         for (uint32_t g = group; g < total; g += kMidGroups) {
             if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
@@ -486,12 +533,18 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         }
     }
 
-    if (csize == 1u && warp < kMidWeightWarp && turns != 0u) {
+    uint32_t last_cc = blockIdx.x;      // the last block whose partial sums this one takes
+    if (csize == 1u && warp < kMidWeightWarp && total != 0u) {
         // ---------------------------------------------------------------- read sums, store
-        // Warps 0-3 store every turn but the last beside the work of the next.  In the last one nothing
+        // Warps 0-3 store every piece but the last beside the work of the next.  In the last one nothing
         // is left to convert and the converters help: four warps alone took 4.6 us (64 rows) and 7 us
         // (100 rows) at the end of launches of 30 and 40 us.  Their staging buffers lie over the
         // rings, which are idle once the last sums are there.
+        //
+        // A tile that is cut between blocks belongs to the block that holds its first segment: that
+        // block's last piece, while the other holders - the blocks right after it - meet the tile at the
+        // start of their ranges and have published their sums long before.  The owner adds them in
+        // block order.
         const uint32_t lanes = warp & 3u;
         const uint32_t helper = warp >> 2;                       // 0: the storing warps
         const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
@@ -504,37 +557,57 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const unsigned int live = *args.m_dev;
             m_live = live < m_live ? live : m_live;
         }
-        // rows of y start on a boundary of four values, and so does every slab
-        const bool aligned = (args.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.y) % (4u * sizeof(YT))) == 0u
-                          && (args.slab_rows % (gated ? 8u : 4u)) == 0u;
-        for (uint32_t turn = helper == 0u ? 0u : turns - 1u; turn < turns; ++turn) {
-            const bool last = turn + 1u == turns;
+        // rows of y start on a boundary of four values
+        const bool aligned = (args.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.y) % (4u * sizeof(YT))) == 0u;
+        for (uint32_t turn = 0; work.next(); ++turn) {
+            const bool last = work.left == 0u;
+            const bool owner = work.s0 == 0u;
+            const bool helped = last && owner;
+            if (helper != 0u && !helped) {
+                continue;
+            }
             const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
             const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
-            const uint32_t here = slabs_of_turn(slabs, pair, turn);
             // where the slabs go (table entries in grouped mode): asked for before the wait
             GroupTile place[2];
-            for (uint32_t p = 0; p < here; ++p) {
+            for (uint32_t p = 0; p < pair; ++p) {
                 if (grouped) {
-                    place[p] = args.group_tiles[(size_t)(blockIdx.x + turn * gridDim.x) * pair + p];
+                    place[p] = args.group_tiles[(size_t)work.tile * pair + p];
                 } else {
-                    place[p].j0 = (slab0 + turn * pair + p) * args.slab_rows;
+                    place[p].j0 = (work.tile * pair + p) * args.slab_rows;
                     place[p].j_limit = place[p].j0 + args.slab_rows < args.n ? place[p].j0 + args.slab_rows : args.n;
                     place[p].tok0 = 0u;
                     place[p].tok_limit = m_live;
                 }
             }
-            // (a helper has seen none of the turns before, so it does not ask for a parity of their barrier)
+            if (owner && work.s1 != segs) {
+                last_cc = decode_holder((work.tile + 1u) * segs - 1u, blocks, units);
+                for (uint32_t base = blockIdx.x + 1u; base <= last_cc; base += 32u) {
+                    const uint32_t cc = base + lane;
+                    if (cc <= last_cc) {
+                        const unsigned int *flag = args.flags + kFlagWords * cc + lanes;
+                        const long long begin = clock64();
+                        while (ld_acquire_gpu(flag) == 0u) {
+                            if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
+                                atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
+                                break;
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            // (a helper has seen none of the pieces before, so it does not ask for a parity of their barrier)
             if (!__all_sync(0xFFFFFFFFu, helper == 0u ? mbar_wait(acc_full + 8u * buf, uses & 1u, abort_flag, args.status)
                                                       : mbar_wait(drain_bar, 0u, abort_flag, args.status))) {
                 break;
             }
             tc_fence_after_sync();
-            // pieces of 16 rows of x, dealt to the warps of the same lanes in the last turn
-            const uint32_t step = last ? kMidWeightWarp / 4u : 1u;
-            uint32_t piece = last ? helper : 0u;
+            // pieces of 16 rows of x, dealt to the warps of the same lanes where they help
+            const uint32_t step = helped ? kMidWeightWarp / 4u : 1u;
+            uint32_t piece = helped ? helper : 0u;
 #pragma unroll 1
-            for (uint32_t p = 0; p < here; ++p) {
+            for (uint32_t p = 0; p < pair; ++p) {
                 const GroupTile at = p == 0u ? place[0] : place[1];
                 const uint32_t rows = at.tok_limit > at.tok0 ? at.tok_limit - at.tok0 : 0u;
                 const uint32_t live = (rows < ntok ? rows + 15u : ntok) / 16u;           // pieces with a row to store
@@ -550,9 +623,31 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         continue;
                     }
                     const uint32_t c0 = piece * 16u;
+                    const uint32_t slot = (p * ntok + c0) * kRows + lanes * 32u + lane;
                     uint32_t v[16];
                     tmem_ld_32x16(lane_taddr + (buf * pair + p) * ntok + c0, v);
                     tmem_ld_wait();
+                    if (!owner) {
+                        float *to = args.partial + (unsigned long long)blockIdx.x * args.tile_floats + slot;
+#pragma unroll
+                        for (uint32_t i = 0; i < 16u; ++i) {
+                            __stcg(to + i * kRows, __uint_as_float(v[i]));
+                        }
+                        continue;
+                    }
+#pragma unroll 1
+                    for (uint32_t cc = blockIdx.x + 1u; cc <= last_cc; ++cc) {
+                        const float *from = args.partial + (unsigned long long)cc * args.tile_floats + slot;
+                        float part[16];
+#pragma unroll
+                        for (uint32_t i = 0; i < 16u; ++i) {
+                            part[i] = __ldcg(from + i * kRows);
+                        }
+#pragma unroll
+                        for (uint32_t i = 0; i < 16u; ++i) {
+                            v[i] = __float_as_uint(__uint_as_float(v[i]) + part[i]);
+                        }
+                    }
                     if (staged) {
                         const uint32_t buffer = buffers + flip;
                         flip ^= kMidStageBytes / 8u;
@@ -578,6 +673,14 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     }
                 }
                 piece -= live;
+            }
+            if (!owner) {
+                // Publish this warp's quarter; every lane makes its own stores visible first.
+                __threadfence();
+                __syncwarp();
+                if (lane == 0u) {
+                    st_release_gpu(args.flags + kFlagWords * blockIdx.x + lanes, 1u);
+                }
             }
             if (!last) {
                 // The accumulators are free again.
@@ -652,7 +755,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 const float4 more = recv[(src * runs + local) * kRows + row];
                 four = make_float4(four.x + more.x, four.y + more.y, four.z + more.z, four.w + more.w);
             }
-            const uint32_t j = (slab0 + p) * args.slab_rows + row;
+            const uint32_t j = (blockIdx.x / csize * pair + p) * args.slab_rows + row;
             const float sums[4] = {four.x, four.y, four.z, four.w};
 #pragma unroll
             for (uint32_t i = 0; i < 4u; ++i) {
@@ -670,6 +773,13 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 
     tc_fence_before_sync();
     __syncthreads();
+    if (warp < kEpilogueWarps) {
+        // Hand the consumed slots back for the next launch that uses this set (every warp has passed its
+        // waits; ordered by the end of the kernel).
+        for (uint32_t cc = blockIdx.x + 1u + lane; cc <= last_cc; cc += 32u) {
+            *reinterpret_cast<volatile unsigned int *>(args.flags + kFlagWords * cc + warp) = 0u;
+        }
+    }
     if (warp == kMidMmaWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512u);
@@ -772,39 +882,53 @@ static unsigned int clusters_of_four(unsigned int sm_count)
     return known[device];
 }
 
-MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue)
+MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
+                 unsigned int epilogue)
 {
     MidPlan plan = {};
     plan.ntok = (m + 15u) / 16u * 16u;
     const unsigned int segs = k / kSegK;
     const unsigned int step = epilogue == kEpilogueSwiglu ? 8u : 4u;
-    // The fewest blocks to a slab that leave every cluster at most two slabs; one block to a slab, and
-    // as many turns as it takes, beyond that.
-    const unsigned int fours = clusters_of_four(sm_count);
-    unsigned int clusters = sm_count;
-    plan.cluster = 1u;
-    if (segs >= 4u && n <= fours * 2u * kRows) {
-        plan.cluster = 4u;
-        clusters = fours;
-    } else if (segs >= 2u && n <= sm_count / 2u * 2u * kRows) {
-        plan.cluster = 2u;
-        clusters = sm_count / 2u;
+    // Few rows: clusters of four or two, at most two slabs to a cluster, all of one size so that every
+    // cluster has work.  (Cutting them into units instead leaves pieces of a few segments and as many
+    // hand-overs through memory: 16384 x 4096, 100 rows, 28.9 us against 24.5.)
+    for (unsigned int size = 4u; size >= 2u; size /= 2u) {
+        const unsigned int clusters = size == 4u ? clusters_of_four(sm_count) : sm_count / 2u;
+        if (segs < size || n > clusters * 2u * kRows) {
+            continue;
+        }
+        plan.cluster = size;
+        plan.pair = n > clusters * kRows ? 2u : 1u;
+        const unsigned int all = clusters * plan.pair;
+        plan.slab_rows = ((n + all - 1u) / all + step - 1u) / step * step;
+        const unsigned int used = (n + plan.slab_rows - 1u) / plan.slab_rows;
+        plan.tiles = (used + plan.pair - 1u) / plan.pair;
+        plan.grid = plan.tiles * plan.cluster;
+        return plan;
     }
-    const unsigned int slabs = (n + clusters * kRows - 1u) / (clusters * kRows);     // per cluster
-    plan.pair = slabs > 1u ? 2u : 1u;
-    plan.slabs = slabs;
-    const unsigned int all = clusters * slabs;
-    plan.slab_rows = ((n + all - 1u) / all + step - 1u) / step * step;
-    // rounding up can leave the last clusters without rows
-    const unsigned int used = (n + plan.slab_rows - 1u) / plan.slab_rows;
-    clusters = (used + slabs - 1u) / slabs;
-    plan.grid = clusters * plan.cluster;
+    plan.cluster = 1u;
+    // (the fixed scratch of aotx_q8_matmul_static holds one slab)
+    plan.pair = n > kRows && 2ull * kRows * plan.ntok <= tile_floats ? 2u : 1u;
+    plan.slab_rows = kRows;
+    plan.tiles = (n + plan.pair * kRows - 1u) / (plan.pair * kRows);
+    const unsigned long long units = (unsigned long long)plan.tiles * segs;
+    plan.grid = units < sm_count ? (unsigned int)units : sm_count;
+    // Whole tiles, all of one size and as many to every block, unless cutting them is cheaper.
+    const unsigned int turns = (plan.tiles + sm_count - 1u) / sm_count;
+    if ((unsigned long long)turns * segs <= units / plan.grid + kMidCutUnits) {
+        const unsigned int all = sm_count * turns * plan.pair;
+        plan.turns = turns;
+        plan.slab_rows = ((n + all - 1u) / all + step - 1u) / step * step;
+        plan.tiles = (n + plan.pair * plan.slab_rows - 1u) / (plan.pair * plan.slab_rows);
+        plan.grid = plan.tiles < sm_count ? plan.tiles : sm_count;
+    }
     return plan;
 }
 
 cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
                                unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
-                               unsigned int ldy, unsigned int epilogue, unsigned int *status, bool overlap)
+                               unsigned int ldy, unsigned int epilogue, float *partial, unsigned int *flags,
+                               unsigned long long tile_floats, unsigned int *status, bool overlap)
 {
     MidArgs args = {};
     args.n = n;
@@ -818,17 +942,25 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
     args.ntok = plan.ntok;
     args.slab_rows = plan.slab_rows;
     args.pair = plan.pair;
-    args.slabs = plan.slabs;
+    args.tiles = plan.tiles;
+    args.turns = plan.turns;
+    args.partial = partial;
+    args.flags = flags;
+    args.tile_floats = tile_floats;
     return launch_mid(stream, tw, tx, args, plan.grid, plan.cluster, overlap, y_dtype);
 }
 
 cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
                                unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
                                const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
-                               unsigned int *status, bool overlap)
+                               float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
+                               bool overlap)
 {
     MidArgs args = {};
     args.k = k;
+    args.partial = partial;
+    args.flags = flags;
+    args.tile_floats = tile_floats;
     args.y = y;
     args.status = status;
     args.ldy = ldy;

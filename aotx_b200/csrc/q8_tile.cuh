@@ -644,19 +644,22 @@ cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const
                                unsigned int grid, unsigned int cluster, int y_dtype);
 
 // The product for 17 to 128 rows and the grouped products (q8_mid.cu): how a product's rows of w are
-// dealt (slabs of slab_rows rows, `slabs` per block, `pair` at a time; `cluster` blocks share a
-// slab's depth), and the launches.
+// dealt (tiles of `pair` slabs of slab_rows rows; `cluster` blocks share a tile's depth, or
+// 1: `turns` whole tiles per block, 0: units), and the launches.
 struct MidPlan {
-    unsigned int ntok, slab_rows, pair, slabs, cluster, grid;
+    unsigned int ntok, slab_rows, pair, tiles, turns, cluster, grid;
 };
-MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue);
+MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
+                 unsigned int epilogue);
 cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
                                unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
-                               unsigned int ldy, unsigned int epilogue, unsigned int *status, bool overlap);
+                               unsigned int ldy, unsigned int epilogue, float *partial, unsigned int *flags,
+                               unsigned long long tile_floats, unsigned int *status, bool overlap);
 cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
                                unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
                                const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
-                               unsigned int *status, bool overlap);
+                               float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
+                               bool overlap);
 
 // Host launcher of the second prefill-regime kernel (q8_wide.cu), token tiles of 256.
 cudaError_t launch_wide_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx,
