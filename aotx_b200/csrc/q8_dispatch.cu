@@ -177,6 +177,17 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     // Up to 16 rows, one copy of y: the register-fed kernel; up to 128: q8_mid.cu.  Stores into the
     // peers' copies stay with the kernels they were measured on.
     const bool warp_kernel = ntok <= 16u && out == nullptr;
+    if (ntok > 128u && out == nullptr && scratch.blocks >= sm_count && scratch.tile_floats >= 256ull * kRows
+        && (unsigned long long)(n / (2u * kRows) + 1u) * (m / 128u + 1u) * (k / kSegK) < (1ull << 31)) {
+        const unsigned int rows = pair_token_tile(m);
+        CUtensorMap tw, tx;
+        if (!map_weights(encode, &tw, w, n, k, kRows) || !map_rows(encode, &tx, x, m, k, rows / 2u, x_bf16 != 0)) {
+            return cudaErrorInvalidValue;
+        }
+        return launch_pair_kernel(stream, tw, tx, rows, sm_count, n, k, x_bf16 != 0, m, m_dev, y, y_dtype,
+                                  epilogue == kEpilogueSwiglu ? n / 2u : n, epilogue, set_partial(scratch, set),
+                                  set_flags(scratch, set), scratch.tile_floats, scratch.status, overlap);
+    }
     if (mid) {
         const MidPlan plan = mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats,
                                       epilogue);

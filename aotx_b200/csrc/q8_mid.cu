@@ -23,8 +23,7 @@
 #include <cuda.h>
 
 #include "q8_launch.h"
-#include "q8_tile.cuh"
-#include "q8_warp_ptx.cuh"
+#include "q8_rows.cuh"
 
 namespace q8 {
 
@@ -53,13 +52,10 @@ constexpr uint32_t kMidCutUnits = 5;
 struct MidArgs {
     unsigned int n, k, m_max;
     const unsigned int *m_dev;
-    void *y;
+    RowStore to;
     unsigned int *status;
-    unsigned int ldy;
-    unsigned int epilogue;
     const GroupTile *group_tiles;      // grouped mode: the device's table, else null
     const unsigned int *group_count;
-    const unsigned int *row_map;
     unsigned int ntok;                 // columns of an accumulator: rows of x, a multiple of 16
     unsigned int slab_rows;            // rows of w per slab (a multiple of 4)
     unsigned int pair;                 // slabs that share a segment of x: 1 or 2
@@ -72,108 +68,6 @@ struct MidArgs {
     unsigned int x_stages, raw_stages, a_stages, acc_buffers;
     unsigned int raw_offset, raw_stride;
 };
-
-// Every lane has the words of its row, not only asked for them, when the raw stage goes back
-// (raw_words_present in q8_tile.cuh says why); true about once in 2^32 loads, and then does nothing.
-__device__ __forceinline__ void mid_words_present(const uint32_t (&raw)[36], unsigned int *status)
-{
-    uint32_t all = 0x5F3759DFu;
-#pragma unroll
-    for (int i = 0; i < 36; ++i) {
-        all ^= raw[i];
-    }
-    if (__any_sync(0xFFFFFFFFu, all == 0u)) {
-        atomicOr(status, 0u);
-    }
-}
-
-// What one finished value becomes: stored, added to the float stream (cuda/model/norm.cu:78-89).
-template <typename YT>
-__device__ __forceinline__ void mid_store_one(const MidArgs &args, size_t at, float value)
-{
-    if (args.epilogue == kEpilogueAdd) {
-        float *sum = static_cast<float *>(args.y) + at;
-        *sum = *sum + value;
-    } else {
-        store_out<YT>(static_cast<YT *>(args.y), at, value);
-    }
-}
-
-// 16 rows of x by this warp's 32 columns of y, every lane one column: turned round in shared memory of
-// the warp's own and written four values per lane, 2 to 4 store instructions instead of 16 (the
-// number of store instructions is what a store costs here, see q8_tile.cuh).  GATED: neighbouring
-// lanes hold gate and up of one column (cuda/model/norm.cu:92-105); 16 columns then.
-// `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.
-template <typename YT, bool GATED>
-__device__ __forceinline__ void mid_store_staged(const MidArgs &args, uint32_t stage, uint32_t lane, uint32_t first_col,
-                                                 uint32_t columns, uint32_t first_row, uint32_t row_limit,
-                                                 const uint32_t (&v)[16])
-{
-    constexpr uint32_t kColumns = GATED ? 16u : 32u;
-    constexpr uint32_t kRowBytes = kColumns * sizeof(YT);
-    constexpr uint32_t kLanesPerRow = kColumns / 4u;
-    constexpr uint32_t kRowsPerStep = 32u / kLanesPerRow;      // 4 or 8
-    constexpr uint32_t kSteps = 16u / kRowsPerStep;
-    const uint32_t column = GATED ? lane / 2u : lane;
-#pragma unroll
-    for (uint32_t i = 0; i < 16u; ++i) {
-        float value = __uint_as_float(v[i]);
-        if (GATED) {
-            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-            value = value / (1.0f + expf(-value)) * other;
-        }
-        if (!GATED || (lane & 1u) == 0u) {
-            if (sizeof(YT) == 4) {
-                st_shared_b32(stage + i * kRowBytes + column * 4u, __float_as_uint(value));
-            } else {
-                st_shared_b16(stage + i * kRowBytes + column * 2u, out_bits<YT>(value));
-            }
-        }
-    }
-    __syncwarp();
-    const uint32_t part = lane % kLanesPerRow;
-    const bool adds = !GATED && sizeof(YT) == 4 && args.epilogue == kEpilogueAdd;
-    YT *at[kSteps];
-#pragma unroll
-    for (uint32_t step = 0; step < kSteps; ++step) {
-        const uint32_t row_x = first_row + step * kRowsPerStep + lane / kLanesPerRow;
-        at[step] = nullptr;
-        if (row_x < row_limit && part * 4u < columns) {
-            const uint32_t row_y = args.row_map != nullptr ? __ldg(args.row_map + row_x) : row_x;
-            at[step] = static_cast<YT *>(args.y) + (size_t)row_y * args.ldy + first_col + part * 4u;
-        }
-    }
-    float4 before[kSteps];
-    if (adds) {
-        // one rounded add per value; the old values are fetched together, before the first store
-#pragma unroll
-        for (uint32_t step = 0; step < kSteps; ++step) {
-            before[step] = at[step] != nullptr ? *reinterpret_cast<const float4 *>(at[step]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-    }
-#pragma unroll
-    for (uint32_t step = 0; step < kSteps; ++step) {
-        const uint32_t from = stage + (step * kRowsPerStep + lane / kLanesPerRow) * kRowBytes + part * 4u * sizeof(YT);
-        if (sizeof(YT) == 4) {
-            uint32_t a, b, c, d;
-            ld_shared_v4(from, a, b, c, d);
-            float4 piece = make_float4(__uint_as_float(a), __uint_as_float(b), __uint_as_float(c), __uint_as_float(d));
-            if (adds) {
-                piece = make_float4(before[step].x + piece.x, before[step].y + piece.y, before[step].z + piece.z,
-                                    before[step].w + piece.w);
-            }
-            if (at[step] != nullptr) {
-                *reinterpret_cast<float4 *>(at[step]) = piece;
-            }
-        } else {
-            uint32_t a, b;
-            ld_shared_v2(from, a, b);
-            if (at[step] != nullptr) {
-                *reinterpret_cast<uint2 *>(at[step]) = make_uint2(a, b);
-            }
-        }
-    }
-}
 
 // A block's work: pieces of tiles, each the segments [s0, s1) of one tile.
 struct MidWork {
@@ -498,7 +392,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             } else {
                 load_raw<1>(raw_row, raw);
             }
-            mid_words_present(raw, args.status);
+            row_words_present(raw, args.status);
             if (lane == 0u) {
                 mbar_arrive(raw_empty + 8u * rst);
             }
@@ -548,7 +442,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         const uint32_t lanes = warp & 3u;
         const uint32_t helper = warp >> 2;                       // 0: the storing warps
         const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
-        const bool gated = args.epilogue == kEpilogueSwiglu;
+        const bool gated = args.to.epilogue == kEpilogueSwiglu;
         const uint32_t buffers = helper == 0u ? stage_base + warp * (kMidStageBytes / 4u)
                                               : smem0 + (warp - kEpilogueWarps) * (kMidStageBytes / 4u);
         uint32_t flip = 0u;      // the two turns of the warp's staging buffer
@@ -558,7 +452,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             m_live = live < m_live ? live : m_live;
         }
         // rows of y start on a boundary of four values
-        const bool aligned = (args.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.y) % (4u * sizeof(YT))) == 0u;
+        const bool aligned = (args.to.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.to.y) % (4u * sizeof(YT))) == 0u;
         for (uint32_t turn = 0; work.next(); ++turn) {
             const bool last = work.left == 0u;
             const bool owner = work.s0 == 0u;
@@ -570,8 +464,11 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const uint32_t uses = args.acc_buffers > 1u ? turn >> 1 : turn;
             // where the slabs go (table entries in grouped mode): asked for before the wait
             GroupTile place[2];
-            for (uint32_t p = 0; p < pair; ++p) {
-                if (grouped) {
+#pragma unroll
+            for (uint32_t p = 0; p < 2u; ++p) {
+                if (p >= pair) {
+                    place[p] = place[0];
+                } else if (grouped) {
                     place[p] = args.group_tiles[(size_t)work.tile * pair + p];
                 } else {
                     place[p].j0 = (work.tile * pair + p) * args.slab_rows;
@@ -652,9 +549,9 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         const uint32_t buffer = buffers + flip;
                         flip ^= kMidStageBytes / 8u;
                         if (gated) {
-                            mid_store_staged<YT, true>(args, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
+                            store_rows_staged<YT, true>(args.to, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
                         } else {
-                            mid_store_staged<YT, false>(args, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
+                            store_rows_staged<YT, false>(args.to, buffer, lane, col, columns, at.tok0 + c0, at.tok_limit, v);
                         }
                         continue;
                     }
@@ -667,8 +564,8 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         }
                         const uint32_t row_x = at.tok0 + c0 + i;
                         if (row_x < at.tok_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
-                            const uint32_t row_y = args.row_map != nullptr ? __ldg(args.row_map + row_x) : row_x;
-                            mid_store_one<YT>(args, (size_t)row_y * args.ldy + col + (gated ? lane / 2u : lane), value);
+                            const uint32_t row_y = args.to.row_map != nullptr ? __ldg(args.to.row_map + row_x) : row_x;
+                            store_value<YT>(args.to, (size_t)row_y * args.to.ldy + col + (gated ? lane / 2u : lane), value);
                         }
                     }
                 }
@@ -742,7 +639,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             m_live = 0u;
         }
         const float4 *recv = reinterpret_cast<const float4 *>(smem);
-        const bool gated = args.epilogue == kEpilogueSwiglu;
+        const bool gated = args.to.epilogue == kEpilogueSwiglu;
         const uint32_t runs = pair * (share / 4u);                      // runs of four rows of x per sender
         // warp = 32 rows of w of one run
         for (uint32_t at = warp; at < runs * (kRows / 32u); at += kMidThreads / 32u) {
@@ -765,7 +662,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     sum = sum / (1.0f + expf(-sum)) * up;
                 }
                 if (token + i < m_live && row < args.slab_rows && j < args.n && (!gated || (row & 1u) == 0u)) {
-                    mid_store_one<YT>(args, (size_t)(token + i) * args.ldy + (gated ? j / 2u : j), sum);
+                    store_value<YT>(args.to, (size_t)(token + i) * args.to.ldy + (gated ? j / 2u : j), sum);
                 }
             }
         }
@@ -935,10 +832,10 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
     args.k = k;
     args.m_max = m;
     args.m_dev = m_dev;
-    args.y = y;
+    args.to.y = y;
     args.status = status;
-    args.ldy = ldy;
-    args.epilogue = epilogue;
+    args.to.ldy = ldy;
+    args.to.epilogue = epilogue;
     args.ntok = plan.ntok;
     args.slab_rows = plan.slab_rows;
     args.pair = plan.pair;
@@ -961,13 +858,13 @@ cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const
     args.partial = partial;
     args.flags = flags;
     args.tile_floats = tile_floats;
-    args.y = y;
+    args.to.y = y;
     args.status = status;
-    args.ldy = ldy;
-    args.epilogue = epilogue;
+    args.to.ldy = ldy;
+    args.to.epilogue = epilogue;
     args.group_tiles = tiles;
     args.group_count = count_dev;
-    args.row_map = row_map;
+    args.to.row_map = row_map;
     args.ntok = ntok;
     args.slab_rows = kRows;
     args.pair = 2u;

@@ -1,0 +1,736 @@
+// The prefill-regime kernel: batches above 128 rows of x.  y[i][j] = sum_c x[i][c] * w[j][c], float sums, w
+// dequantised to binary16, or (bfloat16 x) rounded once to bfloat16.
+//
+// Tensor-bound.  A tile is 256 rows of w by up to 256 rows of x, and two blocks on neighbouring SMs
+// (cta_group::2) work on it together: each dequantises 128 rows of w into its own tensor memory and
+// brings half of the tile's rows of x into its own shared memory, which the MMA reads in both.  What
+// bounds the one-block form of this tile (128 x 256, q8_wide.cu) is shared memory: 256 deep, a block
+// writes and reads 34 KB of weights twice over (544 cycles of its 128 bytes) and writes and reads 128 KB of
+// x (2048 cycles) under 2048 cycles of MMAs.  Sharing x halves the second part.
+//
+//   * Weights: converter warps in two groups of eight that take segments in turn, as in q8_mid.cu.
+//   * One accumulator (256 columns; the other 256 are two segments of A), so the MMAs of a tile wait until
+//     the sums of the one before are out of tensor memory: the storing warps first turn all of them
+//     into rows in shared memory (64 KB for the four warps), give the accumulator back and store
+//     from there beside the next tile.
+//   * The first tiles are dealt whole, one after the other to every pair; what is left for less than a turn of
+//     all pairs is cut into (tile, segment) units.  A cut tile is finished by the pair that holds its
+//     first segment, each block its own rows; that is a pair's last piece and all its warps store.
+//   * The tile's rows of x are the batch in equal parts of at most 256, rounded up to 32.
+//
+// 23 warps per block, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 of the
+// first block issues the MMAs.  Every wait is bounded and raises a status bit when it runs out.
+// Measured against q8_wide.cu (gate+up 28672 x 4096, 2048 rows, bfloat16): see the dispatch
+// (q8_dispatch.cu).  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
+#include <cuda.h>
+
+#include "q8_launch.h"
+#include "q8_rows.cuh"
+
+namespace q8 {
+
+constexpr uint32_t kPairThreads = 23 * 32;
+constexpr uint32_t kPairGroups = 2;
+constexpr uint32_t kPairGroupWarps = 8;
+constexpr uint32_t kPairWeightWarp = 20;
+constexpr uint32_t kPairInputWarp = 21;
+constexpr uint32_t kPairMmaWarp = 22;
+constexpr uint32_t kPairTok = 256;          // rows of x per tile, at most
+constexpr uint32_t kPairMaxRaw = 4;
+constexpr uint32_t kPairMaxX = 8;
+constexpr uint32_t kPairAStages = 2;
+constexpr uint32_t kPairAColumns = kSegK / 2;
+constexpr uint32_t kPairBars = 3 * kPairMaxRaw + 2 * kPairMaxX + 2 * kPairAStages + 2 + 1;
+constexpr uint32_t kPairWarpStage = 16384;  // per storing warp: its 32 columns of the tile's rows of x
+constexpr uint32_t kPairTail = kEpilogueWarps * kPairWarpStage + kPairBars * 8 + 16;
+constexpr uint32_t kPairSmem = 227u * 1024u;
+constexpr uint32_t kPairRings = (kPairSmem - 1024u - kPairTail) / 1024u * 1024u;
+// What cutting a tile costs, in units (256 weights deep): the hand-over of the partial sums and the
+// stores at the end.
+constexpr uint32_t kPairCutUnits = 5;
+
+struct PairArgs {
+    unsigned int n, k, m_max;
+    const unsigned int *m_dev;
+    RowStore to;
+    unsigned int *status;
+    unsigned int ntok;                 // rows of x per tile
+    unsigned int b_bf16;
+    float *partial;                    // per block: [row of x][row of w], and its flags
+    unsigned int *flags;
+    unsigned long long tile_floats;
+    unsigned int x_stages, raw_stages;
+};
+
+__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, unsigned int *status)
+{
+#pragma unroll 1
+    for (uint32_t spin = 0; spin < 64u; ++spin) {
+        if (mbar_try_wait_cluster(bar, parity)) {
+            return true;
+        }
+    }
+    if (!mbar_wait(bar, parity, abort_flag, status)) {
+        return false;
+    }
+    return mbar_try_wait_cluster(bar, parity) != 0u; // complete by now; with the other block's writes
+}
+
+// A pair's work: whole tiles `stride` apart, then a run of units.
+struct PairWork {
+    uint32_t tile, s0, s1;
+    uint32_t next_whole, whole_left, stride, segs;
+    uint32_t next_tile, next_seg, left;
+
+    __device__ __forceinline__ bool next()
+    {
+        if (whole_left != 0u) {
+            tile = next_whole;
+            s0 = 0u;
+            s1 = segs;
+            next_whole += stride;
+            whole_left -= 1u;
+            return true;
+        }
+        if (left == 0u) {
+            return false;
+        }
+        tile = next_tile;
+        s0 = next_seg;
+        s1 = segs - s0 < left ? segs : s0 + left;
+        left -= s1 - s0;
+        next_tile += 1u;
+        next_seg = 0u;
+        return true;
+    }
+    __device__ __forceinline__ bool last() const
+    {
+        return whole_left == 0u && left == 0u;
+    }
+};
+
+// The sums of a whole tile's `rows` rows of x (accumulator columns) and this warp's 32 rows of w: into rows in the
+// warp's own shared memory, then - `release` is called in between - 16 bytes per lane to y.  Everything
+// is inside the tensor and on 16-byte boundaries (pair_drain_fits).  GATED: rows of w in pairs, gate and up of one
+// column (arithmetic of cuda/model/norm.cu:92-105); of two rows of x the even lane forms the first's
+// value and the odd lane the second's.
+template <typename YT, bool GATED, typename Release>
+__device__ __forceinline__ void pair_drain(const RowStore &to, uint32_t stage, uint32_t lane_taddr, uint32_t lane,
+                                           uint32_t first_col, uint32_t first_row, uint32_t rows, Release release)
+{
+    constexpr uint32_t kRowBytes = (GATED ? 16u : 32u) * sizeof(YT);
+    constexpr uint32_t kRound = kPairWarpStage / kRowBytes < kPairTok ? kPairWarpStage / kRowBytes : kPairTok;
+    constexpr uint32_t kLanesPerRow = kRowBytes / 16u;
+    constexpr uint32_t kRowsPerStep = 32u / kLanesPerRow;
+    constexpr uint32_t kTogether = 4u;
+    const bool odd = (lane & 1u) != 0u;
+    for (uint32_t base = 0; base < rows; base += kRound) {
+        const uint32_t here = rows - base < kRound ? rows - base : kRound;
+#pragma unroll 1
+        for (uint32_t c0 = 0; c0 < here; c0 += 16u) {
+            uint32_t v[16];
+            tmem_ld_32x16(lane_taddr + base + c0, v);
+            tmem_ld_wait();
+            const uint32_t at = stage + c0 * kRowBytes;
+            if (GATED) {
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; i += 2u) {
+                    const float give = __uint_as_float(odd ? v[i] : v[i + 1u]);
+                    const float keep = __uint_as_float(odd ? v[i + 1u] : v[i]);
+                    const float got = __shfl_xor_sync(0xFFFFFFFFu, give, 1u);
+                    const float gate = odd ? got : keep;
+                    const float up = odd ? keep : got;
+                    const float value = gate / (1.0f + expf(-gate)) * up;
+                    const uint32_t cell = at + (i + (odd ? 1u : 0u)) * kRowBytes + lane / 2u * sizeof(YT);
+                    if (sizeof(YT) == 4) {
+                        st_shared_b32(cell, __float_as_uint(value));
+                    } else {
+                        st_shared_b16(cell, out_bits<YT>(value));
+                    }
+                }
+            } else {
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; ++i) {
+                    if (sizeof(YT) == 4) {
+                        st_shared_b32(at + i * kRowBytes + lane * 4u, v[i]);
+                    } else {
+                        st_shared_b16(at + i * kRowBytes + lane * 2u, out_bits<YT>(__uint_as_float(v[i])));
+                    }
+                }
+            }
+        }
+        if (base + kRound >= rows) {
+            release();
+        }
+        __syncwarp();
+        const uint32_t part = lane % kLanesPerRow;
+        const bool adds = !GATED && sizeof(YT) == 4 && to.epilogue == kEpilogueAdd;
+        for (uint32_t r0 = lane / kLanesPerRow; r0 < here; r0 += kRowsPerStep * kTogether) {
+            float4 before[kTogether];
+            YT *y[kTogether];
+#pragma unroll
+            for (uint32_t i = 0; i < kTogether; ++i) {
+                const uint32_t r = r0 + i * kRowsPerStep;
+                y[i] = r < here ? static_cast<YT *>(to.y) + (size_t)(first_row + base + r) * to.ldy + first_col + part * (16u / sizeof(YT))
+                                : nullptr;
+                before[i] = adds && y[i] != nullptr ? *reinterpret_cast<const float4 *>(y[i]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < kTogether; ++i) {
+                uint4 piece;
+                const uint32_t r = r0 + i * kRowsPerStep;
+                ld_shared_v4(stage + (r < here ? r : 0u) * kRowBytes + part * 16u, piece.x, piece.y, piece.z, piece.w);
+                if (adds) {
+                    // one rounded add per value (cuda/model/norm.cu:78-89)
+                    piece.x = __float_as_uint(before[i].x + __uint_as_float(piece.x));
+                    piece.y = __float_as_uint(before[i].y + __uint_as_float(piece.y));
+                    piece.z = __float_as_uint(before[i].z + __uint_as_float(piece.z));
+                    piece.w = __float_as_uint(before[i].w + __uint_as_float(piece.w));
+                }
+                if (y[i] != nullptr) {
+                    *reinterpret_cast<uint4 *>(y[i]) = piece;
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <bool BF>
+__device__ __forceinline__ void pair_convert(uint32_t half, const uint32_t (&raw)[36], uint32_t taddr)
+{
+    if (half == 0u) {
+        convert_stage_tmem<0, 0, BF>(raw, taddr);
+        convert_stage_tmem<0, 1, BF>(raw, taddr + kSubK / 2u);
+    } else {
+        convert_stage_tmem<1, 0, BF>(raw, taddr);
+        convert_stage_tmem<1, 1, BF>(raw, taddr + kSubK / 2u);
+    }
+}
+
+template <typename YT>
+__global__ void __launch_bounds__(kPairThreads, 1)
+q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const PairArgs args)
+{
+    extern __shared__ unsigned char smem_raw_[];
+    const uint32_t smem0 = (smem_u32(smem_raw_) + 1023u) & ~1023u;
+    unsigned char *const smem = smem_raw_ + (smem0 - smem_u32(smem_raw_));
+    const uint32_t ntok = args.ntok;
+    const uint32_t x_stage_bytes = ntok * (kSubK * 2u) / 2u;      // this block's half of the rows, 64 deep
+    const uint32_t raw_base = smem0 + args.x_stages * x_stage_bytes;
+    const uint32_t stage_base = smem0 + kPairRings;
+    const uint32_t raw_full = stage_base + kEpilogueWarps * kPairWarpStage;
+    const uint32_t raw_empty = raw_full + 16u * kPairMaxRaw;      // two full barriers per stage (q8_mid.cu says why)
+    const uint32_t raw_turns = 2u * args.raw_stages;
+    const uint32_t x_full = raw_empty + 8u * kPairMaxRaw;         // the first block's: both halves have landed
+    const uint32_t x_empty = x_full + 8u * kPairMaxX;
+    const uint32_t a_full = x_empty + 8u * kPairMaxX;             // the first block's: both blocks' weights are there
+    const uint32_t a_empty = a_full + 8u * kPairAStages;
+    const uint32_t acc_full = a_empty + 8u * kPairAStages;
+    const uint32_t acc_empty = acc_full + 8u;                     // the first block's: both blocks' sums are out
+    const uint32_t drain_bar = acc_empty + 8u;
+    const uint32_t tmem_slot = drain_bar + 8u;
+    volatile uint32_t *tmem_slot_ptr = reinterpret_cast<volatile uint32_t *>(smem + (tmem_slot - smem0));
+    volatile uint32_t *abort_flag = tmem_slot_ptr + 1;
+
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t rank = cluster_ctarank();
+
+    grid_launch_dependents();
+    unsigned int m = args.m_max;
+    if (args.m_dev != nullptr) {
+        // the live batch decides how many tiles there are
+        grid_dependency_wait();
+        const unsigned int live = *args.m_dev;
+        m = live < m ? live : m;
+    }
+    if (m == 0u) {
+        return;
+    }
+    const uint32_t segs = args.k / kSegK;
+    const uint32_t tok_tiles = (m + ntok - 1u) / ntok;
+    const uint32_t pairs = gridDim.x / 2u;
+    const uint32_t tiles = (args.n + 2u * kRows - 1u) / (2u * kRows) * tok_tiles;   // below 2^31 units: the host checks
+    uint32_t turns = tiles / pairs;
+    uint32_t cut = tiles - turns * pairs;
+    const uint32_t units = cut * segs;
+    const uint32_t pair_id = blockIdx.x / 2u;
+    const uint32_t sharers = units < pairs ? units : pairs;
+    PairWork work;
+    work.segs = segs;
+    work.stride = pairs;
+    work.next_whole = pair_id;
+    work.whole_left = turns;
+    work.next_tile = work.next_seg = work.left = 0u;
+    if (units != 0u && segs <= units / pairs + kPairCutUnits) {
+        work.whole_left += pair_id < cut ? 1u : 0u;               // cutting would cost more than it evens out
+    } else if (pair_id < sharers) {
+        uint32_t u_begin, u_end;
+        decode_range(pair_id, sharers, units, &u_begin, &u_end);
+        work.next_tile = turns * pairs + u_begin / segs;
+        work.next_seg = u_begin % segs;
+        work.left = u_end - u_begin;
+    }
+    const uint32_t first_cut = turns * pairs;
+    const uint32_t total = work.whole_left * segs + work.left;    // segments of weights
+
+    uint32_t early = 0u;
+    if (warp == kPairWeightWarp && elect_one()) {
+        tma_prefetch_desc(&tmap_w);
+        tma_prefetch_desc(&tmap_x);
+        for (uint32_t i = 0; i < args.raw_stages; ++i) {
+            mbar_init(raw_full + 8u * i, 1u);
+            mbar_init(raw_full + 8u * (i + args.raw_stages), 1u);
+            mbar_init(raw_empty + 8u * i, kPairGroupWarps);
+        }
+        for (uint32_t i = 0; i < args.x_stages; ++i) {
+            mbar_init(x_full + 8u * i, 1u);
+            mbar_init(x_empty + 8u * i, 1u);
+        }
+        for (uint32_t i = 0; i < kPairAStages; ++i) {
+            mbar_init(a_full + 8u * i, 2u * kPairGroupWarps);
+            mbar_init(a_empty + 8u * i, 1u);
+        }
+        mbar_init(acc_full, 1u);
+        mbar_init(acc_empty, 2u * kEpilogueWarps);
+        mbar_init(drain_bar, 1u);
+        *abort_flag = 0u;
+        mbar_init_fence();
+        fence_proxy_async_smem();
+        // the first weights: only this block's own barriers have to be there
+        PairWork ahead = work;
+        uint32_t s = 0u;
+        ahead.s1 = 0u;
+        for (; early < args.raw_stages && early < total; ++early, ++s) {
+            if (s == ahead.s1) {
+                ahead.next();
+                s = ahead.s0;
+            }
+            mbar_expect_tx(raw_full + 8u * early, kRawStageBytes);
+            tma_load_2d(raw_base + early * kRawStageBytes, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords),
+                        (int)((ahead.tile / tok_tiles * 2u + rank) * kRows));
+        }
+    }
+    if (warp == kPairMmaWarp) {
+        pair_tmem_alloc(tmem_slot, 512u);
+        pair_tmem_relinquish();
+    }
+    // both blocks' barriers are there before either signals the other's
+    __syncwarp();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot_ptr;
+    const uint32_t a_column0 = kPairTok;
+
+    if (warp == kPairWeightWarp) {
+        // ---------------------------------------------------------------- weight copies
+        if (elect_one()) {
+            uint32_t g = 0;
+            bool ok = true;
+            uint32_t full = 0u;
+            uint32_t st = 0u, ph = 1u;
+            while (ok && work.next()) {
+                const uint32_t w_row = (work.tile / tok_tiles * 2u + rank) * kRows;
+                for (uint32_t s = work.s0; s < work.s1; ++s, ++g) {
+                    if (g >= early) {
+                        if (!mbar_wait(raw_empty + 8u * st, ph, abort_flag, args.status)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(raw_full + 8u * full, kRawStageBytes);
+                        tma_load_2d(raw_base + st * kRawStageBytes, &tmap_w, raw_full + 8u * full, (int)(s * kSegWords),
+                                    (int)w_row);
+                    }
+                    full = full + 1u == raw_turns ? 0u : full + 1u;
+                    if (++st == args.raw_stages) {
+                        st = 0u;
+                        ph ^= 1u;
+                    }
+                }
+            }
+            // Let every copy this thread started land before the block ends.
+            uint32_t local_abort = 0;
+            const uint32_t issued = g > early ? g : early;
+            const uint32_t first = issued > args.raw_stages ? issued - args.raw_stages : 0u;
+            for (uint32_t i = first; i < issued; ++i) {
+                mbar_wait(raw_full + 8u * (i % raw_turns), (i / raw_turns) & 1u, &local_abort, nullptr);
+            }
+        }
+    } else if (warp == kPairInputWarp) {
+        // ---------------------------------------------------------------- x copies
+        // each block its half of the tile's rows, both signalling the first block's barrier
+        if (elect_one()) {
+            uint32_t q = 0;
+            grid_dependency_wait();
+            bool ok = true;
+            uint32_t st = 0u, ph = 1u;
+            const uint32_t signal = mapa_shared(x_full, 0u);
+            while (ok && work.next()) {
+                const uint32_t row = work.tile % tok_tiles * ntok + rank * (ntok / 2u);
+                for (uint32_t sub = work.s0 * kSubs; sub < work.s1 * kSubs; ++sub, ++q) {
+                    if (!pair_wait(x_empty + 8u * st, ph, abort_flag, args.status)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0u) {
+                        mbar_expect_tx(x_full + 8u * st, 2u * x_stage_bytes);
+                    }
+                    pair_tma_load_2d(smem0 + st * x_stage_bytes, &tmap_x, signal + 8u * st, (int)(sub * kSubK), (int)row);
+                    if (++st == args.x_stages) {
+                        st = 0u;
+                        ph ^= 1u;
+                    }
+                }
+            }
+            if (rank == 0u) {
+                // both blocks' copies (the second block stays until the first has seen this)
+                uint32_t local_abort = 0;
+                const uint32_t first = q > args.x_stages ? q - args.x_stages : 0u;
+                for (uint32_t i = first; i < q; ++i) {
+                    mbar_wait(x_full + 8u * (i % args.x_stages), (i / args.x_stages) & 1u, &local_abort, nullptr);
+                }
+            }
+        }
+    } else if (warp == kPairMmaWarp) {
+        // ---------------------------------------------------------------- MMA issue, for both blocks
+        if (rank == 0u && elect_one()) {
+            const uint32_t idesc = umma_idesc(2u * kRows, ntok, args.b_bf16, args.b_bf16);
+            uint32_t xst = 0u, xph = 0u;
+            uint32_t ast = 0u, aph = 0u;
+            bool ok = true;
+            for (uint32_t turn = 0; ok && work.next(); ++turn) {
+                if (!pair_wait(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
+                    if (!pair_wait(a_full + 8u * ast, aph, abort_flag, args.status)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t a_tmem = tmem_base + a_column0 + ast * kPairAColumns;
+#pragma unroll 1
+                    for (uint32_t j = 0; j < kSubs; ++j) {
+                        if (!pair_wait(x_full + 8u * xst, xph, abort_flag, args.status)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        const uint64_t b_desc = umma_desc_sw128(smem0 + xst * x_stage_bytes);
+#pragma unroll
+                        for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
+                            // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
+                            pair_mma_f16_ts(tmem_base, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
+                                            s != work.s0 || j != 0u || kk != 0u ? 1u : 0u);
+                        }
+                        pair_commit(x_empty + 8u * xst);
+                        if (++xst == args.x_stages) {
+                            xst = 0u;
+                            xph ^= 1u;
+                        }
+                    }
+                    if (ok) {
+                        pair_commit(a_empty + 8u * ast);
+                        if (++ast == kPairAStages) {
+                            ast = 0u;
+                            aph ^= 1u;
+                        }
+                    }
+                }
+                if (ok) {
+                    pair_commit(acc_full);
+                }
+            }
+            pair_commit(drain_bar);     // every MMA has finished: what the helping warps wait for
+            if (!ok) {
+                uint32_t local_abort = 0;
+                mbar_wait(drain_bar, 0u, &local_abort, nullptr);
+            }
+        }
+    } else if (warp >= kConvertWarp0) {
+        // ---------------------------------------------------------------- dequantise
+        const uint32_t cw = warp - kConvertWarp0;
+        const uint32_t group = cw / kPairGroupWarps;
+        const uint32_t half = (cw >> 2) & 1u;
+        const uint32_t row_at = ((cw & 3u) * 32u + lane) * kSegBytes;
+        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
+        const uint32_t signal = mapa_shared(a_full, 0u);
+        uint32_t full = group, fph = 0, ast = group, aph = 0;
+        for (uint32_t g = group; g < total; g += kPairGroups) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
+                break;
+            }
+            const uint32_t rst = full < args.raw_stages ? full : full - args.raw_stages;
+            uint32_t raw[36];
+            const uint32_t raw_row = raw_base + rst * kRawStageBytes + row_at;
+            if (half == 0u) {
+                load_raw<0>(raw_row, raw);
+            } else {
+                load_raw<1>(raw_row, raw);
+            }
+            row_words_present(raw, args.status);
+            if (lane == 0u) {
+                mbar_arrive(raw_empty + 8u * rst);
+            }
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(a_empty + 8u * ast, aph ^ 1u, abort_flag, args.status))) {
+                break;
+            }
+            const uint32_t taddr = lane_base + ast * kPairAColumns;
+            tc_fence_after_sync();
+            if (args.b_bf16 != 0u) {
+                pair_convert<true>(half, raw, taddr);
+            } else {
+                pair_convert<false>(half, raw, taddr);
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0u) {
+                mbar_arrive_cluster(signal + 8u * ast);
+            }
+            full += kPairGroups;
+            if (full >= raw_turns) {
+                full -= raw_turns;
+                fph ^= 1u;
+            }
+            // two stages, two groups: each group keeps its own
+            aph ^= 1u;
+        }
+    }
+
+    uint32_t last_cc = pair_id;         // the last pair whose partial sums this one takes
+    if (warp < kPairWeightWarp && total != 0u) {
+        // ---------------------------------------------------------------- read sums, store
+        const uint32_t lanes = warp & 3u;
+        const uint32_t helper = warp >> 2;                       // 0: the storing warps
+        const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
+        const bool gated = args.to.epilogue == kEpilogueSwiglu;
+        const uint32_t stage = helper == 0u ? stage_base + warp * kPairWarpStage : smem0 + (warp - kEpilogueWarps) * 4096u;
+        const uint32_t release_bar = mapa_shared(acc_empty, 0u);
+        uint32_t flip = 0u;      // the two turns of a helper's staging buffer
+        grid_dependency_wait();
+        // rows of y on a boundary of 16 bytes (the drain of a whole tile) or of four values (the others)
+        const bool aligned16 = ((size_t)args.to.ldy * sizeof(YT)) % 16u == 0u && (reinterpret_cast<uintptr_t>(args.to.y) % 16u) == 0u;
+        const bool aligned4 = (args.to.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.to.y) % (4u * sizeof(YT))) == 0u;
+        for (uint32_t turn = 0; work.next(); ++turn) {
+            const bool last = work.last();
+            const bool owner = work.s0 == 0u;
+            const bool helped = last && owner;
+            if (helper != 0u && !helped) {
+                continue;
+            }
+            const uint32_t row_tile = work.tile / tok_tiles;
+            const uint32_t tok0 = (work.tile - row_tile * tok_tiles) * ntok;
+            const uint32_t rows = m - tok0 < ntok ? m - tok0 : ntok;                     // live rows of x of the tile
+            const uint32_t j = (row_tile * 2u + rank) * kRows + lanes * 32u;             // this warp's first row of w
+            const uint32_t inside = args.n > j ? args.n - j : 0u;                        // ... and how many are there
+            const uint32_t mine = inside < 32u ? inside : 32u;
+            const uint32_t columns = gated ? mine / 2u : mine;
+            const uint32_t col = gated ? j / 2u : j;
+            if (owner && work.s1 != segs) {
+                // The other holders of this tile are the pairs right after this one; they met it at the start of
+                // their runs of units.
+                last_cc = decode_holder((work.tile - first_cut + 1u) * segs - 1u, sharers, units);
+                for (uint32_t base = pair_id + 1u; base <= last_cc; base += 32u) {
+                    const uint32_t cc = base + lane;
+                    if (cc <= last_cc) {
+                        const unsigned int *flag = args.flags + kFlagWords * (2u * cc + rank) + lanes;
+                        const long long begin = clock64();
+                        while (ld_acquire_gpu(flag) == 0u) {
+                            if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
+                                atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
+                                break;
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            // (a helper has seen none of the pieces before, so it does not ask for a parity of their barrier)
+            if (!__all_sync(0xFFFFFFFFu, helper == 0u ? pair_wait(acc_full, turn & 1u, abort_flag, args.status)
+                                                      : pair_wait(drain_bar, 0u, abort_flag, args.status))) {
+                break;
+            }
+            tc_fence_after_sync();
+            auto release = [&]() {
+                // The accumulator is free again.
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0u) {
+                    mbar_arrive_cluster(release_bar);
+                }
+            };
+            if (!last && owner && aligned16 && mine == 32u) {
+                if (gated) {
+                    pair_drain<YT, true>(args.to, stage, lane_taddr, lane, col, tok0, rows, release);
+                } else {
+                    pair_drain<YT, false>(args.to, stage, lane_taddr, lane, col, tok0, rows, release);
+                }
+                continue;
+            }
+            const bool staged = aligned4 && (columns % 4u) == 0u;
+            const uint32_t step = helped ? kPairWeightWarp / 4u : 1u;
+#pragma unroll 1
+            for (uint32_t c0 = helped ? helper * 16u : 0u; c0 < rows && mine != 0u; c0 += 16u * step) {
+                const uint32_t slot = c0 * kRows + lanes * 32u + lane;
+                uint32_t v[16];
+                tmem_ld_32x16(lane_taddr + c0, v);
+                tmem_ld_wait();
+                if (!owner) {
+                    float *to = args.partial + (unsigned long long)blockIdx.x * args.tile_floats + slot;
+#pragma unroll
+                    for (uint32_t i = 0; i < 16u; ++i) {
+                        __stcg(to + i * kRows, __uint_as_float(v[i]));
+                    }
+                    continue;
+                }
+#pragma unroll 1
+                for (uint32_t cc = pair_id + 1u; cc <= last_cc; ++cc) {
+                    const float *from = args.partial + (unsigned long long)(2u * cc + rank) * args.tile_floats + slot;
+                    float part[16];
+#pragma unroll
+                    for (uint32_t i = 0; i < 16u; ++i) {
+                        part[i] = __ldcg(from + i * kRows);
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < 16u; ++i) {
+                        v[i] = __float_as_uint(__uint_as_float(v[i]) + part[i]);
+                    }
+                }
+                if (staged) {
+                    const uint32_t buffer = stage + flip;
+                    flip ^= 2048u;
+                    if (gated) {
+                        store_rows_staged<YT, true>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                    } else {
+                        store_rows_staged<YT, false>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                    }
+                    continue;
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; ++i) {
+                    float value = __uint_as_float(v[i]);
+                    if (gated) {
+                        const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
+                        value = value / (1.0f + expf(-value)) * other;
+                    }
+                    if (c0 + i < rows && lane < mine && (!gated || (lane & 1u) == 0u)) {
+                        store_value<YT>(args.to, (size_t)(tok0 + c0 + i) * args.to.ldy + col + (gated ? lane / 2u : lane), value);
+                    }
+                }
+            }
+            if (!owner) {
+                // Publish this warp's quarter; every lane makes its own stores visible first.
+                __threadfence();
+                __syncwarp();
+                if (lane == 0u) {
+                    st_release_gpu(args.flags + kFlagWords * blockIdx.x + lanes, 1u);
+                }
+            }
+            if (!last) {
+                release();
+            }
+        }
+    }
+
+    // Neither block leaves while the other may still signal its barriers or read its shared memory.
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    if (warp < kEpilogueWarps) {
+        // Hand the consumed slots back for the next launch that uses this set (ordered by the end of the kernel).
+        for (uint32_t cc = pair_id + 1u + lane; cc <= last_cc; cc += 32u) {
+            *reinterpret_cast<volatile unsigned int *>(args.flags + kFlagWords * (2u * cc + rank) + warp) = 0u;
+        }
+    }
+    if (warp == kPairMmaWarp) {
+        tc_fence_after_sync();
+        pair_tmem_dealloc(tmem_base, 512u);
+    }
+}
+
+template <typename YT>
+static cudaError_t launch_pair_typed(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const PairArgs &args,
+                                     unsigned int grid, bool overlap)
+{
+    static unsigned long long configured = 0ull;
+    cudaError_t err = allow_shared_memory(q8_wide_kernel_pair<YT>, kPairSmem, &configured);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid, 1, 1);
+    config.blockDim = dim3(kPairThreads, 1, 1);
+    config.dynamicSmemBytes = kPairSmem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[2];
+    unsigned int count = 0;
+    attribute[count].id = cudaLaunchAttributeClusterDimension;
+    attribute[count].val.clusterDim.x = 2;
+    attribute[count].val.clusterDim.y = 1;
+    attribute[count].val.clusterDim.z = 1;
+    ++count;
+    if (overlap) {
+        attribute[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute[count].val.programmaticStreamSerializationAllowed = 1;
+        ++count;
+    }
+    config.attrs = attribute;
+    config.numAttrs = count;
+    return cudaLaunchKernelEx(&config, q8_wide_kernel_pair<YT>, tw, tx, args);
+}
+
+// Rows of x per tile: the batch in equal parts of at most 256, a multiple of 32 (what an MMA of two blocks
+// takes).
+unsigned int pair_token_tile(unsigned int m)
+{
+    const unsigned int parts = (m + kPairTok - 1u) / kPairTok;
+    return ((m + parts - 1u) / parts + 31u) / 32u * 32u;
+}
+
+cudaError_t launch_pair_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int ntok,
+                               unsigned int sm_count, unsigned int n, unsigned int k, bool x_bf16, unsigned int m,
+                               const unsigned int *m_dev, void *y, int y_dtype, unsigned int ldy, unsigned int epilogue,
+                               float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
+                               bool overlap)
+{
+    PairArgs args = {};
+    args.n = n;
+    args.k = k;
+    args.m_max = m;
+    args.m_dev = m_dev;
+    args.to.y = y;
+    args.to.ldy = ldy;
+    args.to.epilogue = epilogue;
+    args.status = status;
+    args.ntok = ntok;
+    args.b_bf16 = x_bf16 ? 1u : 0u;
+    args.partial = partial;
+    args.flags = flags;
+    args.tile_floats = tile_floats;
+    // Shared memory: two raw segments and as many pieces of x as fit, three where that leaves five pieces.
+    const unsigned int x_stage = ntok * kSubK;                    // bytes: half of the rows, 64 halves each
+    args.raw_stages = 3u * kRawStageBytes + 5u * x_stage <= kPairRings ? 3u : 2u;
+    const unsigned int x_stages = (kPairRings - args.raw_stages * kRawStageBytes) / x_stage;
+    args.x_stages = x_stages < kPairMaxX ? x_stages : kPairMaxX;
+    const unsigned long long units = (unsigned long long)((n + 2u * kRows - 1u) / (2u * kRows)) * ((m + ntok - 1u) / ntok) * (k / kSegK);
+    const unsigned int pairs = units < sm_count / 2u ? (unsigned int)units : sm_count / 2u;
+    switch (y_dtype) {
+    case 0:
+        return launch_pair_typed<float>(stream, tw, tx, args, 2u * pairs, overlap);
+    case 1:
+        return launch_pair_typed<__half>(stream, tw, tx, args, 2u * pairs, overlap);
+    case 2:
+        return launch_pair_typed<__nv_bfloat16>(stream, tw, tx, args, 2u * pairs, overlap);
+    default:
+        return cudaErrorInvalidValue;
+    }
+}
+
+} // namespace q8

@@ -1,0 +1,120 @@
+// What the one-block-per-SM kernels with converter groups (q8_mid.cu, q8_pair.cu) share: the hand-back
+// check of a raw stage and the stores of finished sums.
+#pragma once
+
+#include "q8_tile.cuh"
+#include "q8_warp_ptx.cuh"
+
+namespace q8 {
+
+// Where finished sums go, and what becomes of them (the epilogue codes of q8_launch.h).
+struct RowStore {
+    void *y;
+    const unsigned int *row_map;       // rows of y of the rows of x, or null
+    unsigned int ldy;
+    unsigned int epilogue;
+};
+
+// Every lane has the words of its row, not only asked for them, when the raw stage goes back
+// (raw_words_present in q8_tile.cuh says why); true about once in 2^32 loads, and then does nothing.
+__device__ __forceinline__ void row_words_present(const uint32_t (&raw)[36], unsigned int *status)
+{
+    uint32_t all = 0x5F3759DFu;
+#pragma unroll
+    for (int i = 0; i < 36; ++i) {
+        all ^= raw[i];
+    }
+    if (__any_sync(0xFFFFFFFFu, all == 0u)) {
+        atomicOr(status, 0u);
+    }
+}
+
+// What one finished value becomes: stored, added to the float stream (cuda/model/norm.cu:78-89).
+template <typename YT>
+__device__ __forceinline__ void store_value(const RowStore &to, size_t at, float value)
+{
+    if (to.epilogue == kEpilogueAdd) {
+        float *sum = static_cast<float *>(to.y) + at;
+        *sum = *sum + value;
+    } else {
+        store_out<YT>(static_cast<YT *>(to.y), at, value);
+    }
+}
+
+// 16 rows of x by this warp's 32 columns of y, every lane one column: turned round in shared memory of
+// the warp's own and written four values per lane, 2 to 4 store instructions instead of 16 (the
+// number of store instructions is what a store costs here, see q8_tile.cuh).  GATED: neighbouring
+// lanes hold gate and up of one column (cuda/model/norm.cu:92-105); 16 columns then.
+// `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.
+template <typename YT, bool GATED>
+__device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t stage, uint32_t lane, uint32_t first_col,
+                                                 uint32_t columns, uint32_t first_row, uint32_t row_limit,
+                                                 const uint32_t (&v)[16])
+{
+    constexpr uint32_t kColumns = GATED ? 16u : 32u;
+    constexpr uint32_t kRowBytes = kColumns * sizeof(YT);
+    constexpr uint32_t kLanesPerRow = kColumns / 4u;
+    constexpr uint32_t kRowsPerStep = 32u / kLanesPerRow;      // 4 or 8
+    constexpr uint32_t kSteps = 16u / kRowsPerStep;
+    const uint32_t column = GATED ? lane / 2u : lane;
+#pragma unroll
+    for (uint32_t i = 0; i < 16u; ++i) {
+        float value = __uint_as_float(v[i]);
+        if (GATED) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
+            value = value / (1.0f + expf(-value)) * other;
+        }
+        if (!GATED || (lane & 1u) == 0u) {
+            if (sizeof(YT) == 4) {
+                st_shared_b32(stage + i * kRowBytes + column * 4u, __float_as_uint(value));
+            } else {
+                st_shared_b16(stage + i * kRowBytes + column * 2u, out_bits<YT>(value));
+            }
+        }
+    }
+    __syncwarp();
+    const uint32_t part = lane % kLanesPerRow;
+    const bool adds = !GATED && sizeof(YT) == 4 && to.epilogue == kEpilogueAdd;
+    YT *at[kSteps];
+#pragma unroll
+    for (uint32_t step = 0; step < kSteps; ++step) {
+        const uint32_t row_x = first_row + step * kRowsPerStep + lane / kLanesPerRow;
+        at[step] = nullptr;
+        if (row_x < row_limit && part * 4u < columns) {
+            const uint32_t row_y = to.row_map != nullptr ? __ldg(to.row_map + row_x) : row_x;
+            at[step] = static_cast<YT *>(to.y) + (size_t)row_y * to.ldy + first_col + part * 4u;
+        }
+    }
+    float4 before[kSteps];
+    if (adds) {
+        // one rounded add per value; the old values are fetched together, before the first store
+#pragma unroll
+        for (uint32_t step = 0; step < kSteps; ++step) {
+            before[step] = at[step] != nullptr ? *reinterpret_cast<const float4 *>(at[step]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+#pragma unroll
+    for (uint32_t step = 0; step < kSteps; ++step) {
+        const uint32_t from = stage + (step * kRowsPerStep + lane / kLanesPerRow) * kRowBytes + part * 4u * sizeof(YT);
+        if (sizeof(YT) == 4) {
+            uint32_t a, b, c, d;
+            ld_shared_v4(from, a, b, c, d);
+            float4 piece = make_float4(__uint_as_float(a), __uint_as_float(b), __uint_as_float(c), __uint_as_float(d));
+            if (adds) {
+                piece = make_float4(before[step].x + piece.x, before[step].y + piece.y, before[step].z + piece.z,
+                                    before[step].w + piece.w);
+            }
+            if (at[step] != nullptr) {
+                *reinterpret_cast<float4 *>(at[step]) = piece;
+            }
+        } else {
+            uint32_t a, b;
+            ld_shared_v2(from, a, b);
+            if (at[step] != nullptr) {
+                *reinterpret_cast<uint2 *>(at[step]) = make_uint2(a, b);
+            }
+        }
+    }
+}
+
+} // namespace q8

@@ -661,6 +661,14 @@ cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const
                                float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
                                bool overlap);
 
+// The product for more than 128 rows on pairs of SMs (q8_pair.cu): rows of x per tile, and the launch.
+unsigned int pair_token_tile(unsigned int m);
+cudaError_t launch_pair_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int ntok,
+                               unsigned int sm_count, unsigned int n, unsigned int k, bool x_bf16, unsigned int m,
+                               const unsigned int *m_dev, void *y, int y_dtype, unsigned int ldy, unsigned int epilogue,
+                               float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
+                               bool overlap);
+
 // Host launcher of the second prefill-regime kernel (q8_wide.cu), token tiles of 256.
 cudaError_t launch_wide_kernel(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx,
                                const UmmaArgs &args, unsigned int grid, int y_dtype);
