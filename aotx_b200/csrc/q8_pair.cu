@@ -62,20 +62,6 @@ struct PairArgs {
     unsigned int x_stages, raw_stages;
 };
 
-__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, unsigned int *status)
-{
-#pragma unroll 1
-    for (uint32_t spin = 0; spin < 64u; ++spin) {
-        if (mbar_try_wait_cluster(bar, parity)) {
-            return true;
-        }
-    }
-    if (!mbar_wait(bar, parity, abort_flag, status)) {
-        return false;
-    }
-    return mbar_try_wait_cluster(bar, parity) != 0u; // complete by now; with the other block's writes
-}
-
 // A pair's work: whole tiles `stride` apart, then a run of units.
 struct PairWork {
     uint32_t tile, s0, s1;
@@ -372,7 +358,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             while (ok && work.next()) {
                 const uint32_t row = work.tile % tok_tiles * ntok + rank * (ntok / 2u);
                 for (uint32_t sub = work.s0 * kSubs; sub < work.s1 * kSubs; ++sub, ++q) {
-                    if (!pair_wait(x_empty + 8u * st, ph, abort_flag, args.status)) {
+                    if (!mbar_wait_hot(x_empty + 8u * st, ph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
@@ -403,20 +389,20 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             uint32_t ast = 0u, aph = 0u;
             bool ok = true;
             for (uint32_t turn = 0; ok && work.next(); ++turn) {
-                if (!pair_wait(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
+                if (!mbar_wait_hot(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
-                    if (!pair_wait(a_full + 8u * ast, aph, abort_flag, args.status)) {
+                    if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
                     const uint32_t a_tmem = tmem_base + a_column0 + ast * kPairAColumns;
 #pragma unroll 1
                     for (uint32_t j = 0; j < kSubs; ++j) {
-                        if (!pair_wait(x_full + 8u * xst, xph, abort_flag, args.status)) {
+                        if (!mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
                             ok = false;
                             break;
                         }
@@ -552,8 +538,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 __syncwarp();
             }
             // (a helper has seen none of the pieces before, so it does not ask for a parity of their barrier)
-            if (!__all_sync(0xFFFFFFFFu, helper == 0u ? pair_wait(acc_full, turn & 1u, abort_flag, args.status)
-                                                      : pair_wait(drain_bar, 0u, abort_flag, args.status))) {
+            if (!__all_sync(0xFFFFFFFFu, helper == 0u ? mbar_wait_hot(acc_full, turn & 1u, abort_flag, args.status)
+                                                      : mbar_wait_hot(drain_bar, 0u, abort_flag, args.status))) {
                 break;
             }
             tc_fence_after_sync();

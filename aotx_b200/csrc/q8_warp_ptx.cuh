@@ -115,24 +115,12 @@ __device__ __forceinline__ void pair_tma_load_2d(uint32_t dst, const void *tmap,
         : "memory");
 }
 
-// Arrive on a barrier of either block (an address of mapa_shared); what this thread did before is visible to
-// who waits there with cluster scope.
+// Arrive on a barrier of either block (an address of mapa_shared).  Without cluster-scope release on purpose:
+// what changes hands here is tensor memory, which tcgen05.wait and the tcgen05 fences order; a release
+// at cluster scope holds the warp for 2400 cycles until its other memory operations are done.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ uint32_t mbar_try_wait_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done;
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 } // namespace q8
