@@ -309,6 +309,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             // than the MMAs of a segment)
             uint32_t xst = 0u, xph = 0u;
             uint32_t ast = 0u, aph = 0u;
+            uint32_t x_there = 0u, a_there = 0u;   // the next segment of x, of A, is known to be there
             bool ok = true;
             for (uint32_t turn = 0; ok && work.next(); ++turn) {
                 const uint32_t buf = args.acc_buffers > 1u ? turn & 1u : 0u;
@@ -319,16 +320,25 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 }
                 tc_fence_after_sync();
                 for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
-                    if (!mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
+                    if (!x_there && !mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
                     for (uint32_t p = 0; p < pair; ++p) {
-                        if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
+                        if (!a_there && !mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                             ok = false;
                             break;
                         }
                         tc_fence_after_sync();
+                        // ask for the next segments before the MMAs of this one are issued, so that the answer
+                        // is there when they are
+                        const uint32_t anext = ast + 1u == args.a_stages ? 0u : ast + 1u;
+                        const uint32_t anext_ph = ast + 1u == args.a_stages ? aph ^ 1u : aph;
+                        a_there = mbar_test_wait(a_full + 8u * anext, anext_ph);
+                        if (p + 1u == pair) {
+                            const bool wraps = xst + 1u == args.x_stages;
+                            x_there = mbar_test_wait(x_full + 8u * (wraps ? 0u : xst + 1u), wraps ? xph ^ 1u : xph);
+                        }
                         const uint32_t d_tmem = tmem_base + (buf * pair + p) * ntok;
                         const uint32_t a_tmem = tmem_base + a_column0 + ast * (kSegK / 2u);
                         const uint32_t x_seg = smem0 + xst * x_seg_bytes;
@@ -343,10 +353,8 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                             }
                         }
                         umma_commit(a_empty + 8u * ast);
-                        if (++ast == args.a_stages) {
-                            ast = 0u;
-                            aph ^= 1u;
-                        }
+                        ast = anext;
+                        aph = anext_ph;
                     }
                     if (ok) {
                         umma_commit(x_empty + 8u * xst);
@@ -456,7 +464,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         for (uint32_t turn = 0; work.next(); ++turn) {
             const bool last = work.left == 0u;
             const bool owner = work.s0 == 0u;
-            const bool helped = last && owner;
+            const bool helped = last;
             if (helper != 0u && !helped) {
                 continue;
             }
@@ -484,7 +492,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     if (cc <= last_cc) {
                         const unsigned int *flag = args.flags + kFlagWords * cc + lanes;
                         const long long begin = clock64();
-                        while (ld_acquire_gpu(flag) == 0u) {
+                        while (ld_acquire_gpu(flag) < kPublishers) {
                             if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
                                 atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
                                 break;
@@ -576,7 +584,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 __threadfence();
                 __syncwarp();
                 if (lane == 0u) {
-                    st_release_gpu(args.flags + kFlagWords * blockIdx.x + lanes, 1u);
+                    red_release_gpu_add(args.flags + kFlagWords * blockIdx.x + lanes, helped ? 1u : kPublishers);
                 }
             }
             if (!last) {
@@ -604,7 +612,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         const uint32_t share = ntok / csize;
         __syncwarp();
         cluster_wait_acquire();      // every block has started ...
-        cluster_arrive_release();    // ... and is done with its rings
+        cluster_arrive_relaxed();    // ... and is done with its rings
         cluster_wait_acquire();
         if (warp < kMidWeightWarp) {
             const uint32_t quarter_lanes = warp & 3u;

@@ -126,7 +126,7 @@ __device__ __forceinline__ void pair_drain(const RowStore &to, uint32_t stage, u
                     const float got = __shfl_xor_sync(0xFFFFFFFFu, give, 1u);
                     const float gate = odd ? got : keep;
                     const float up = odd ? keep : got;
-                    const float value = gate / (1.0f + expf(-gate)) * up;
+                    const float value = gated_unit(gate, up);
                     const uint32_t cell = at + (i + (odd ? 1u : 0u)) * kRowBytes + lane / 2u * sizeof(YT);
                     if (sizeof(YT) == 4) {
                         st_shared_b32(cell, __float_as_uint(value));
@@ -302,9 +302,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         pair_tmem_alloc(tmem_slot, 512u);
         pair_tmem_relinquish();
     }
-    // both blocks' barriers are there before either signals the other's
+    // both blocks' barriers are there before either signals the other's (the fence after their
+    // initialisation orders it)
     __syncwarp();
-    cluster_arrive_release();
+    cluster_arrive_relaxed();
     cluster_wait_acquire();
     tc_fence_before_sync();
     __syncthreads();
@@ -387,6 +388,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t idesc = umma_idesc(2u * kRows, ntok, args.b_bf16, args.b_bf16);
             uint32_t xst = 0u, xph = 0u;
             uint32_t ast = 0u, aph = 0u;
+            uint32_t x_there = 0u, a_there = 0u;   // the next piece of x, the next segment of A, are known to be there
             bool ok = true;
             for (uint32_t turn = 0; ok && work.next(); ++turn) {
                 if (!mbar_wait_hot(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
@@ -395,18 +397,27 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
                 tc_fence_after_sync();
                 for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
-                    if (!mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
+                    if (!a_there && !mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
                     const uint32_t a_tmem = tmem_base + a_column0 + ast * kPairAColumns;
 #pragma unroll 1
                     for (uint32_t j = 0; j < kSubs; ++j) {
-                        if (!mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
+                        if (!x_there && !mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
                             ok = false;
                             break;
                         }
                         tc_fence_after_sync();
+                        // ask for the next piece (and segment) before the MMAs of this one are issued: an answer
+                        // takes as long as two MMAs, and with every wait in the way of the issue a piece took 350
+                        // cycles whatever its width
+                        const uint32_t xnext = xst + 1u == args.x_stages ? 0u : xst + 1u;
+                        const uint32_t xnext_ph = xst + 1u == args.x_stages ? xph ^ 1u : xph;
+                        x_there = mbar_test_wait(x_full + 8u * xnext, xnext_ph);
+                        if (j + 1u == kSubs) {
+                            a_there = mbar_test_wait(a_full + 8u * (ast ^ 1u), ast == 0u ? aph : aph ^ 1u);
+                        }
                         const uint64_t b_desc = umma_desc_sw128(smem0 + xst * x_stage_bytes);
 #pragma unroll
                         for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
@@ -415,10 +426,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                                             s != work.s0 || j != 0u || kk != 0u ? 1u : 0u);
                         }
                         pair_commit(x_empty + 8u * xst);
-                        if (++xst == args.x_stages) {
-                            xst = 0u;
-                            xph ^= 1u;
-                        }
+                        xst = xnext;
+                        xph = xnext_ph;
                     }
                     if (ok) {
                         pair_commit(a_empty + 8u * ast);
@@ -506,7 +515,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         for (uint32_t turn = 0; work.next(); ++turn) {
             const bool last = work.last();
             const bool owner = work.s0 == 0u;
-            const bool helped = last && owner;
+            const bool helped = last;
             if (helper != 0u && !helped) {
                 continue;
             }
@@ -527,7 +536,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     if (cc <= last_cc) {
                         const unsigned int *flag = args.flags + kFlagWords * (2u * cc + rank) + lanes;
                         const long long begin = clock64();
-                        while (ld_acquire_gpu(flag) == 0u) {
+                        while (ld_acquire_gpu(flag) < kPublishers) {
                             if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
                                 atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
                                 break;
@@ -575,18 +584,9 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     }
                     continue;
                 }
-#pragma unroll 1
-                for (uint32_t cc = pair_id + 1u; cc <= last_cc; ++cc) {
-                    const float *from = args.partial + (unsigned long long)(2u * cc + rank) * args.tile_floats + slot;
-                    float part[16];
-#pragma unroll
-                    for (uint32_t i = 0; i < 16u; ++i) {
-                        part[i] = __ldcg(from + i * kRows);
-                    }
-#pragma unroll
-                    for (uint32_t i = 0; i < 16u; ++i) {
-                        v[i] = __float_as_uint(__uint_as_float(v[i]) + part[i]);
-                    }
+                if (last_cc != pair_id) {
+                    add_partial_sums(v, args.partial + (2ull * pair_id + 2u + rank) * args.tile_floats + slot, 2u * args.tile_floats,
+                                     last_cc - pair_id);
                 }
                 if (staged) {
                     const uint32_t buffer = stage + flip;
@@ -603,7 +603,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     float value = __uint_as_float(v[i]);
                     if (gated) {
                         const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-                        value = value / (1.0f + expf(-value)) * other;
+                        value = gated_unit(value, other);
                     }
                     if (c0 + i < rows && lane < mine && (!gated || (lane & 1u) == 0u)) {
                         store_value<YT>(args.to, (size_t)(tok0 + c0 + i) * args.to.ldy + col + (gated ? lane / 2u : lane), value);
@@ -615,7 +615,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 __threadfence();
                 __syncwarp();
                 if (lane == 0u) {
-                    st_release_gpu(args.flags + kFlagWords * blockIdx.x + lanes, 1u);
+                    red_release_gpu_add(args.flags + kFlagWords * blockIdx.x + lanes, helped ? 1u : kPublishers);
                 }
             }
             if (!last) {
@@ -625,9 +625,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
 
     // Neither block leaves while the other may still signal its barriers or read its shared memory.
+    // (Nothing is handed over here, so the arrival need not wait for what a thread has in flight.)
     __syncwarp();
     tc_fence_before_sync();
-    cluster_arrive_release();
+    cluster_arrive_relaxed();
     cluster_wait_acquire();
     if (warp < kEpilogueWarps) {
         // Hand the consumed slots back for the next launch that uses this set (ordered by the end of the kernel).

@@ -29,6 +29,49 @@ __device__ __forceinline__ void row_words_present(const uint32_t (&raw)[36], uns
     }
 }
 
+// silu(gate) * up (cuda/model/norm.cu:92-105).  The quotient gate / (1 + e^-gate) by a reciprocal and one
+// correction of the quotient by its remainder (Markstein's division step) in place of the division
+// operator, whose branches kept a storing warp from working on several values at a time: 1300 cycles per
+// 8 values a lane, 16 x 32 sums, against 280 for a plain store.  The divisor is at least 1; where e^-gate
+// would overflow (gate below -88) it stays finite and its reciprocal is zero or tiny: the value is
+// then zero to within 1e-36.
+__device__ __forceinline__ float gated_unit(float gate, float up)
+{
+    const float divisor = 1.0f + expf(-fmaxf(gate, -88.0f));
+    const float r = rcp_approx(divisor);
+    const float quotient = gate * r;
+    return fmaf(fmaf(-quotient, divisor, gate), r, quotient) * up;
+}
+
+// The partial sums of one piece (16 rows of x by 32 rows of w) that other blocks have left in `slots` (one slot
+// every `stride` floats, `count` of them) added to v in order; two slots' loads are on their way at a time.
+__device__ __forceinline__ void add_partial_sums(uint32_t (&v)[16], const float *slots, unsigned long long stride, uint32_t count)
+{
+#pragma unroll 1
+    for (uint32_t c = 0; c < count; c += 2u) {
+        const bool two = c + 1u < count;
+        const float *first = slots + c * stride;
+        const float *second = two ? first + stride : first;
+#pragma unroll
+        for (uint32_t h = 0; h < 16u; h += 8u) {
+            float a[8], b[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i) {
+                a[i] = __ldcg(first + (h + i) * kRows);
+                b[i] = two ? __ldcg(second + (h + i) * kRows) : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i) {
+                v[h + i] = __float_as_uint(__uint_as_float(v[h + i]) + a[i] + b[i]);
+            }
+        }
+    }
+}
+
+// A flag counts the warps that have published their part of a quarter of a partial tile; this many make it whole
+// (one warp alone counts for all).
+constexpr uint32_t kPublishers = 5;
+
 // What one finished value becomes: stored, added to the float stream (cuda/model/norm.cu:78-89).
 template <typename YT>
 __device__ __forceinline__ void store_value(const RowStore &to, size_t at, float value)
@@ -62,7 +105,7 @@ __device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t s
         float value = __uint_as_float(v[i]);
         if (GATED) {
             const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-            value = value / (1.0f + expf(-value)) * other;
+            value = gated_unit(value, other);
         }
         if (!GATED || (lane & 1u) == 0u) {
             if (sizeof(YT) == 4) {

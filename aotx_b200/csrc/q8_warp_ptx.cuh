@@ -52,6 +52,21 @@ __device__ __forceinline__ void copy_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+// An approximate reciprocal (within an ulp).
+__device__ __forceinline__ float rcp_approx(float v)
+{
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Add to a word with release at GPU scope: what this thread (and those it synchronised with) wrote before is there
+// for who reads the word with acquire.
+__device__ __forceinline__ void red_release_gpu_add(unsigned int *p, uint32_t v)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void ld_shared_v2(uint32_t addr, uint32_t &a, uint32_t &b)
 {
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
