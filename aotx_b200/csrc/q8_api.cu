@@ -317,7 +317,7 @@ extern "C" int aotx_q8_moe_route(aotx_q8_ctx *ctx, void *stream, const void *x_f
         return AOTX_Q8_ERR_UNSUPPORTED; /* four rows of x as floats must fit in shared memory */
     }
     cudaError_t err = q8::launch_route((cudaStream_t)stream, x_f16, router, tokens, tokens_dev, hidden,
-                                       experts, used, prob, ids);
+                                       experts, used, prob, ids, ctx->overlap != 0);
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }
 
@@ -371,7 +371,7 @@ extern "C" int aotx_q8_moe_ffn(aotx_q8_ctx *ctx, void *stream, const void *w_gat
     }
     if (err == cudaSuccess) {
         err = q8::launch_expert_sum(s, proj, prob, ids, tokens, tokens_dev, hidden, experts, used, out,
-                                    out_dtype);
+                                    out_dtype, ctx->overlap != 0);
     }
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }
@@ -416,7 +416,7 @@ extern "C" int aotx_q8_moe_ffn_fused(aotx_q8_ctx *ctx, void *stream, const void 
                                                    x_f16, ids, tokens, tokens_dev, used, base, ws);
     if (err == cudaSuccess) {
         err = q8::launch_expert_sum(s, proj, prob, ids, tokens, tokens_dev, hidden, experts, used, out,
-                                    out_dtype);
+                                    out_dtype, ctx->overlap != 0);
     }
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }

@@ -288,7 +288,8 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
                                 const void *x_sorted, unsigned int x_rows, unsigned int ntok,
                                 const GroupTile *tiles, const unsigned int *count_dev, unsigned int max_tiles,
                                 const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype,
-                                unsigned int set, bool overlap, unsigned int epilogue)
+                                unsigned int set, bool overlap, unsigned int epilogue, const void *w_second,
+                                bool table_late)
 {
     EncodeTiledFn encode = encode_tiled();
     if (encode == nullptr || (k % kSegK) != 0u || ntok > 128u) {
@@ -304,13 +305,22 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
 #ifndef Q8_HOST_EMULATION
     {
         // every expert has an even number of weight row tiles (hidden and ffn are multiples of 256), so
-        // the table's entries pair up
-        const unsigned int blocks = max_tiles / 2u < sm_count ? max_tiles / 2u : sm_count;
-        return launch_mid_grouped(stream, tw, tx, blocks, k, ntok, tiles, count_dev, row_map, y, ldy, y_dtype, epilogue,
+        // the table's entries pair up (with a second tensor, an entry is a tile by itself)
+        const unsigned int most = w_second != nullptr ? max_tiles : max_tiles / 2u;
+        const unsigned int blocks = most < sm_count ? most : sm_count;
+        CUtensorMap tw2;
+        if (w_second != nullptr && !map_weights(encode, &tw2, w_second, total_rows, k, kRows)) {
+            return cudaErrorInvalidValue;
+        }
+        return launch_mid_grouped(stream, tw, w_second != nullptr ? &tw2 : nullptr, tx, table_late, blocks, k, ntok, tiles, count_dev, row_map, y, ldy, y_dtype, epilogue,
                                   set_partial(scratch, set), set_flags(scratch, set), scratch.tile_floats, scratch.status,
                                   overlap);
     }
 #endif
+    if (w_second != nullptr) {
+        return cudaErrorNotSupported;
+    }
+    (void)table_late;
     const unsigned long long units = (unsigned long long)max_tiles * (k / kSegK);
     unsigned int grid = sm_count < scratch.blocks ? sm_count : scratch.blocks;
     if (units < grid) {

@@ -128,7 +128,7 @@ cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int typ
 
 cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                         unsigned int used, float *prob, unsigned int *ids);
+                         unsigned int used, float *prob, unsigned int *ids, bool overlap = false);
 
 // Expert parallel (several GPUs, each holding a run of the experts; q8_api.cu aotx_q8_moe_ep).
 // Where the rows of x of all GPUs' tokens lie: rows_per_part rows in each of `parts` arrays
@@ -158,11 +158,11 @@ cudaError_t launch_expert_pairs_simt(cudaStream_t stream, const void *w_gate, co
 cudaError_t launch_expert_sum(cudaStream_t stream, const float *proj, const float *prob,
                               const unsigned int *ids, unsigned int tokens,
                               const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                              unsigned int used, void *out, int out_dtype);
+                              unsigned int used, void *out, int out_dtype, bool overlap = false);
 cudaError_t launch_expert_sum_parts(cudaStream_t stream, const ProjParts &proj, const float *prob,
                                     const unsigned int *ids, unsigned int tokens,
                                     const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                                    unsigned int used, void *out, int out_dtype);
+                                    unsigned int used, void *out, int out_dtype, bool overlap = false);
 
 // The streaming tensor-core product.  Scratch, in two sets that alternate between launches:
 // `partial` holds one float tile of 128 x token_tile per block of the grid, `flags` kFlagWords
@@ -203,14 +203,17 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
                         unsigned int m, const unsigned int *m_dev, void *y, int y_dtype, unsigned int set,
                         bool overlap, const PeerOut *out = nullptr, unsigned int epilogue = 0u);
 
-// Grouped mode of the decode-regime kernel: tiles from a device table (see q8_tile.cuh).
+// Grouped products: tiles from a device table (see q8_tile.cuh).  `w_second`: a second tensor of the same
+// shape; the product of both with the gated unit in the store (w_stacked gives the gate, w_second the
+// value it gates).  `table_late`: the launch before this one writes the table.
 struct GroupTile;
 cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch, unsigned int sm_count,
                                 const void *w_stacked, unsigned int total_rows, unsigned int k,
                                 const void *x_sorted, unsigned int x_rows, unsigned int ntok,
                                 const GroupTile *tiles, const unsigned int *count_dev, unsigned int max_tiles,
                                 const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype,
-                                unsigned int set, bool overlap, unsigned int epilogue = 0u);
+                                unsigned int set, bool overlap, unsigned int epilogue = 0u,
+                                const void *w_second = nullptr, bool table_late = false);
 
 // Routed experts as grouped products (q8_moe.cu).  Offsets are bytes into the workspace.
 struct MoeWorkspace {

@@ -59,6 +59,7 @@ struct MidArgs {
     unsigned int ntok;                 // columns of an accumulator: rows of x, a multiple of 16
     unsigned int slab_rows;            // rows of w per slab (a multiple of 4)
     unsigned int pair;                 // slabs that share a segment of x: 1 or 2
+    unsigned int table_late;           // grouped: the launch before this one writes the table
     unsigned int tiles;                // of `pair` slabs each (not in grouped mode)
     unsigned int turns;                // whole tiles per block; 0: units (not in grouped mode)
     // unit schedule: a block's partial tile, [slab][row of x][row of w], and its flags
@@ -90,9 +91,12 @@ struct MidWork {
     }
 };
 
-template <typename YT>
+// TWIN (grouped, pair 2): the second slab of a tile is the same rows of a second tensor, and what is stored is
+// the gated unit of the two.
+template <typename YT, bool TWIN>
 __global__ void __launch_bounds__(kMidThreads, 1)
-q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const MidArgs args)
+q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_second,
+                     const __grid_constant__ CUtensorMap tmap_x, const MidArgs args)
 {
     extern __shared__ unsigned char smem_raw_[];
     const uint32_t smem0 = (smem_u32(smem_raw_) + 1023u) & ~1023u;
@@ -128,9 +132,16 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t csize = cluster_nctarank();
     const uint32_t crank = cluster_ctarank();
     // Clusters: one tile each, a run of its segments per block.  Else (tile, segment) units dealt evenly,
-    // the same arithmetic as the decode kernel's.  (The table of the grouped products, and its length,
-    // were written two launches before the first of them, so they may be read here already.)
-    const uint32_t tiles = grouped ? *reinterpret_cast<const volatile unsigned int *>(args.group_count) / pair : args.tiles;
+    // the same arithmetic as the decode kernel's.  (The table of the grouped products, and its length, are
+    // there already unless the launch before this one writes them.  That launch is then waited for before
+    // the next one may start, so that the next one finds the table, too.)
+    if (args.table_late != 0u) {
+        grid_dependency_wait();
+    }
+    // table entries per tile, and from the first slab's to the second's
+    const uint32_t entries = TWIN ? 1u : pair;
+    constexpr uint32_t second = TWIN ? 0u : 1u;
+    const uint32_t tiles = grouped ? *reinterpret_cast<const volatile unsigned int *>(args.group_count) / entries : args.tiles;
     const uint32_t units = tiles * segs;      // the host refuses products with 2^31 units or more
     const uint32_t blocks = units < gridDim.x ? units : gridDim.x;
     MidWork work;
@@ -172,6 +183,9 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     uint32_t early = 0u;
     if (warp == kMidWeightWarp && elect_one()) {
         tma_prefetch_desc(&tmap_w);
+        if (TWIN) {
+            tma_prefetch_desc(&tmap_second);
+        }
         tma_prefetch_desc(&tmap_x);
         for (uint32_t i = 0; i < args.raw_stages; ++i) {
             mbar_init(raw_full + 8u * i, 1u);
@@ -197,9 +211,11 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // the first weights: only the barriers they signal have to be there
         uint32_t tile = work.next_tile, s = work.next_seg, p = 0u;
         for (; early < args.raw_stages && early < total; ++early) {
-            const uint32_t w_row = grouped ? args.group_tiles[(size_t)tile * pair + p].w_row : (tile * pair + p) * args.slab_rows;
+            const uint32_t w_row = grouped ? args.group_tiles[(size_t)tile * entries + p * second].w_row
+                                           : (tile * pair + p) * args.slab_rows;
             mbar_expect_tx(raw_full + 8u * early, raw_bytes);
-            tma_load_2d(raw_base + early * args.raw_stride, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords), (int)w_row);
+            tma_load_2d(raw_base + early * args.raw_stride, TWIN && p != 0u ? &tmap_second : &tmap_w,
+                        raw_full + 8u * early, (int)(s * kSegWords), (int)w_row);
             if (++p == pair) {
                 p = 0u;
                 if (++s == segs) {
@@ -235,9 +251,9 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             while (ok && work.next()) {
                 uint32_t w_row[2];
                 if (grouped) {
-                    const GroupTile *entry = args.group_tiles + (size_t)work.tile * pair;
+                    const GroupTile *entry = args.group_tiles + (size_t)work.tile * entries;
                     w_row[0] = entry[0].w_row;
-                    w_row[1] = pair > 1u ? entry[1].w_row : 0u;
+                    w_row[1] = pair > 1u ? entry[second].w_row : 0u;
                 } else {
                     w_row[0] = work.tile * pair * args.slab_rows;
                     w_row[1] = w_row[0] + args.slab_rows;
@@ -250,8 +266,8 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                                 break;
                             }
                             mbar_expect_tx(raw_full + 8u * full, raw_bytes);
-                            tma_load_2d(raw_base + st * args.raw_stride, &tmap_w, raw_full + 8u * full,
-                                        (int)(s * kSegWords), (int)(p == 0u ? w_row[0] : w_row[1]));
+                            tma_load_2d(raw_base + st * args.raw_stride, TWIN && p != 0u ? &tmap_second : &tmap_w,
+                                        raw_full + 8u * full, (int)(s * kSegWords), (int)(p == 0u ? w_row[0] : w_row[1]));
                         }
                         full = full + 1u == raw_turns ? 0u : full + 1u;
                         if (++st == args.raw_stages) {
@@ -277,7 +293,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             bool ok = true;
             uint32_t st = 0u, ph = 1u;
             while (ok && work.next()) {
-                const uint32_t tok0 = grouped ? args.group_tiles[(size_t)work.tile * pair].tok0 : 0u;
+                const uint32_t tok0 = grouped ? args.group_tiles[(size_t)work.tile * entries].tok0 : 0u;
                 for (uint32_t s = work.s0; s < work.s1; ++s, ++g) {
                     if (!mbar_wait(x_empty + 8u * st, ph, abort_flag, args.status)) {
                         ok = false;
@@ -450,7 +466,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         const uint32_t lanes = warp & 3u;
         const uint32_t helper = warp >> 2;                       // 0: the storing warps
         const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
-        const bool gated = args.to.epilogue == kEpilogueSwiglu;
+        const bool gated = args.to.epilogue == kEpilogueSwiglu && !TWIN;
         const uint32_t buffers = helper == 0u ? stage_base + warp * (kMidStageBytes / 4u)
                                               : smem0 + (warp - kEpilogueWarps) * (kMidStageBytes / 4u);
         uint32_t flip = 0u;      // the two turns of the warp's staging buffer
@@ -477,7 +493,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 if (p >= pair) {
                     place[p] = place[0];
                 } else if (grouped) {
-                    place[p] = args.group_tiles[(size_t)work.tile * pair + p];
+                    place[p] = args.group_tiles[(size_t)work.tile * entries + p * second];
                 } else {
                     place[p].j0 = (work.tile * pair + p) * args.slab_rows;
                     place[p].j_limit = place[p].j0 + args.slab_rows < args.n ? place[p].j0 + args.slab_rows : args.n;
@@ -512,7 +528,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const uint32_t step = helped ? kMidWeightWarp / 4u : 1u;
             uint32_t piece = helped ? helper : 0u;
 #pragma unroll 1
-            for (uint32_t p = 0; p < pair; ++p) {
+            for (uint32_t p = 0; p < (TWIN && owner ? 1u : pair); ++p) {
                 const GroupTile at = p == 0u ? place[0] : place[1];
                 const uint32_t rows = at.tok_limit > at.tok0 ? at.tok_limit - at.tok0 : 0u;
                 const uint32_t live = (rows < ntok ? rows + 15u : ntok) / 16u;           // pieces with a row to store
@@ -540,17 +556,18 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         }
                         continue;
                     }
-#pragma unroll 1
-                    for (uint32_t cc = blockIdx.x + 1u; cc <= last_cc; ++cc) {
-                        const float *from = args.partial + (unsigned long long)cc * args.tile_floats + slot;
-                        float part[16];
+                    const uint32_t holders = last_cc - blockIdx.x;   // none for a whole tile
+                    const float *others = args.partial + (unsigned long long)(blockIdx.x + 1u) * args.tile_floats + slot;
+                    add_partial_sums(v, others, args.tile_floats, holders);
+                    if (TWIN) {
+                        // gate and up of the same columns lie in the two slabs' sums
+                        uint32_t up[16];
+                        tmem_ld_32x16(lane_taddr + (buf * pair + 1u) * ntok + c0, up);
+                        tmem_ld_wait();
+                        add_partial_sums(up, others + ntok * kRows, args.tile_floats, holders);
 #pragma unroll
                         for (uint32_t i = 0; i < 16u; ++i) {
-                            part[i] = __ldcg(from + i * kRows);
-                        }
-#pragma unroll
-                        for (uint32_t i = 0; i < 16u; ++i) {
-                            v[i] = __float_as_uint(__uint_as_float(v[i]) + part[i]);
+                            v[i] = __float_as_uint(gated_unit(__uint_as_float(v[i]), __uint_as_float(up[i])));
                         }
                     }
                     if (staged) {
@@ -691,12 +708,12 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
 }
 
-template <typename YT>
-static cudaError_t launch_mid_typed(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidArgs &args,
+template <typename YT, bool TWIN>
+static cudaError_t launch_mid_typed(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tw2, const CUtensorMap &tx, const MidArgs &args,
                                     unsigned int grid, unsigned int cluster, bool overlap)
 {
     static unsigned long long configured = 0ull;
-    cudaError_t err = allow_shared_memory(q8_stream_kernel_mid<YT>, kMidSmem, &configured);
+    cudaError_t err = allow_shared_memory(q8_stream_kernel_mid<YT, TWIN>, kMidSmem, &configured);
     if (err != cudaSuccess) {
         return err;
     }
@@ -721,11 +738,11 @@ static cudaError_t launch_mid_typed(cudaStream_t stream, const CUtensorMap &tw, 
     }
     config.attrs = attribute;
     config.numAttrs = count;
-    return cudaLaunchKernelEx(&config, q8_stream_kernel_mid<YT>, tw, tx, args);
+    return cudaLaunchKernelEx(&config, q8_stream_kernel_mid<YT, TWIN>, tw, tw2, tx, args);
 }
 
-static cudaError_t launch_mid(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, MidArgs &args,
-                              unsigned int grid, unsigned int cluster, bool overlap, int y_dtype)
+static cudaError_t launch_mid(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap *tw_second,
+                              const CUtensorMap &tx, MidArgs &args, unsigned int grid, unsigned int cluster, bool overlap, int y_dtype)
 {
     // Tensor memory: accumulators in two buffers where they leave room for two segments of A.
     args.acc_buffers = 2u * args.pair * args.ntok <= 256u ? 2u : 1u;
@@ -743,13 +760,17 @@ static cudaError_t launch_mid(cudaStream_t stream, const CUtensorMap &tw, const 
     args.raw_offset = x_stages * x_seg;
     const unsigned int raw_stages = (kMidRings - args.raw_offset) / args.raw_stride;
     args.raw_stages = raw_stages < kMidMaxRaw ? raw_stages : kMidMaxRaw;
+    if (tw_second != nullptr) {
+        return y_dtype == 1 ? launch_mid_typed<__half, true>(stream, tw, *tw_second, tx, args, grid, cluster, overlap)
+                            : cudaErrorInvalidValue;
+    }
     switch (y_dtype) {
     case 0:
-        return launch_mid_typed<float>(stream, tw, tx, args, grid, cluster, overlap);
+        return launch_mid_typed<float, false>(stream, tw, tw, tx, args, grid, cluster, overlap);
     case 1:
-        return launch_mid_typed<__half>(stream, tw, tx, args, grid, cluster, overlap);
+        return launch_mid_typed<__half, false>(stream, tw, tw, tx, args, grid, cluster, overlap);
     case 2:
-        return launch_mid_typed<__nv_bfloat16>(stream, tw, tx, args, grid, cluster, overlap);
+        return launch_mid_typed<__nv_bfloat16, false>(stream, tw, tw, tx, args, grid, cluster, overlap);
     default:
         return cudaErrorInvalidValue;
     }
@@ -778,8 +799,8 @@ static unsigned int clusters_of_four(unsigned int sm_count)
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        if (allow_shared_memory(q8_stream_kernel_mid<float>, kMidSmem, &configured) != cudaSuccess
-            || cudaOccupancyMaxActiveClusters(&found, q8_stream_kernel_mid<float>, &config) != cudaSuccess || found <= 0) {
+        if (allow_shared_memory(q8_stream_kernel_mid<float, false>, kMidSmem, &configured) != cudaSuccess
+            || cudaOccupancyMaxActiveClusters(&found, q8_stream_kernel_mid<float, false>, &config) != cudaSuccess || found <= 0) {
             found = (int)(sm_count / 5u);
         }
         known[device] = (unsigned int)found;
@@ -852,11 +873,11 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
     args.partial = partial;
     args.flags = flags;
     args.tile_floats = tile_floats;
-    return launch_mid(stream, tw, tx, args, plan.grid, plan.cluster, overlap, y_dtype);
+    return launch_mid(stream, tw, nullptr, tx, args, plan.grid, plan.cluster, overlap, y_dtype);
 }
 
-cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
-                               unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
+cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap *tw_second,
+                               const CUtensorMap &tx, bool table_late, unsigned int grid, unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
                                const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
                                float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
                                bool overlap)
@@ -871,12 +892,13 @@ cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const
     args.to.ldy = ldy;
     args.to.epilogue = epilogue;
     args.group_tiles = tiles;
+    args.table_late = table_late ? 1u : 0u;
     args.group_count = count_dev;
     args.to.row_map = row_map;
     args.ntok = ntok;
     args.slab_rows = kRows;
     args.pair = 2u;
-    return launch_mid(stream, tw, tx, args, grid, 1u, overlap, y_dtype);
+    return launch_mid(stream, tw, tw_second, tx, args, grid, 1u, overlap, y_dtype);
 }
 
 } // namespace q8

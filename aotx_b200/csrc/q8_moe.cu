@@ -1,7 +1,8 @@
 // Routed experts as grouped products: the (token, rank) pairs are sorted by expert on the
-// device, each expert's rows then form token tiles of 64, and the decode-regime tensor-core
-// kernel runs over a table of (expert, token tile, weight row tile) entries, reading every
-// expert's weights once for all of its tokens.
+// device, each expert's rows then form token tiles of up to 128, and the tensor-core kernel
+// of q8_mid.cu runs over a table of (expert, token tile, weight row tile) entries, reading every
+// expert's weights once for all of its tokens.  Five launches with the router and the sum, each of
+// which starts while the one before it ends.
 //
 // The reference runs one single-row product per token and rank on the token's expert slice
 // (cuda/model/expert_matrix.cu:8-27, loop cuda/model/experts_host.cu:99-111), which re-reads an
@@ -263,6 +264,220 @@ cudaError_t launch_collect_ids(cudaStream_t stream, const unsigned int *const *i
     return launch_kernel(q8_collect_ids_kernel, grid, 256, 0, stream, ids, parts, count, first_expert, ids_all);
 }
 
+#ifndef Q8_HOST_EMULATION
+// The same table, sort and gather as one launch over many blocks; what the routed-expert step runs on the
+// GPU.  (The two kernels above are the serial form, which the host emulation steps through.)
+//
+// Latency bounds this step, not bytes: one block, with a launch of its own for the gather behind it, took
+// 16 + 6 us for 512 tokens of 8 experts and 7 + 3.5 us for 8 tokens.  So every block counts all pairs by
+// itself (a few steps per warp, their loads issued together), which leaves nothing to hand over between
+// blocks; then the places of the sorted order are dealt to the blocks in equal runs - not by
+// expert: one expert may hold most of the pairs - and a block writes and gathers its own run.
+// The tile tables are dealt to all warps of the grid by expert.
+constexpr unsigned int kGroupAhead = 4;   // pairs per lane whose loads are issued together
+
+__device__ __forceinline__ void group_load_ids(const unsigned int *__restrict__ ids, unsigned int first, unsigned int end,
+                                               unsigned int experts, unsigned int lane, unsigned int (&e)[kGroupAhead])
+{
+#pragma unroll
+    for (unsigned int a = 0; a < kGroupAhead; ++a) {
+        const unsigned int p = first + 32u * a + lane;
+        e[a] = p < end ? __ldg(ids + p) : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (unsigned int a = 0; a < kGroupAhead; ++a) {
+        e[a] = e[a] < experts ? e[a] : 0xFFFFFFFFu;    // a selection outside the table is left out
+    }
+}
+
+// The rows of one expert in a tile table: token tiles by 128-row tiles of its weights.
+__device__ __forceinline__ void group_write_tiles(GroupTile *__restrict__ tiles, unsigned int expert, unsigned int rows,
+                                                  unsigned int first_place, unsigned int pairs, unsigned int tile_tokens,
+                                                  unsigned int lane)
+{
+    const unsigned int row_tiles = (rows + kRows - 1u) / kRows;
+    const unsigned int entries = (pairs + tile_tokens - 1u) / tile_tokens * row_tiles;
+    for (unsigned int i = lane; i < entries; i += 32u) {
+        const unsigned int tt = i / row_tiles;
+        const unsigned int r = i - tt * row_tiles;
+        const unsigned int left = pairs - tt * tile_tokens;
+        GroupTile t;
+        t.w_row = expert * rows + r * kRows;
+        t.j0 = r * kRows;
+        t.j_limit = rows;
+        t.tok0 = first_place + tt * tile_tokens;
+        t.tok_limit = t.tok0 + (left < tile_tokens ? left : tile_tokens);
+        tiles[i] = t;
+    }
+}
+
+__global__ void __launch_bounds__(Q8_GROUP_THREADS, 1)
+q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned int *__restrict__ ids, unsigned int tokens_max,
+                       const unsigned int *tokens_dev, unsigned int used, unsigned int experts, unsigned int feed,
+                       unsigned int hidden, unsigned int *sorted_pair, GroupTile *__restrict__ tiles_feed,
+                       GroupTile *__restrict__ tiles_down, unsigned int *__restrict__ counts, unsigned int tile_tokens,
+                       uint4 *__restrict__ x_sorted)
+{
+    constexpr unsigned int kWarps = Q8_GROUP_THREADS / 32u;
+    // per warp and expert: the number of the warp's pairs, then the next free place of the warp in the order
+    __shared__ unsigned int warp_place[kWarps][Q8_GROUP_MAX_EXPERTS];
+    __shared__ unsigned int scan_pairs[Q8_GROUP_MAX_EXPERTS];       // up to and with the expert
+    __shared__ unsigned int scan_tiles[Q8_GROUP_MAX_EXPERTS];
+    __shared__ unsigned int warp_pairs[kWarps];
+    __shared__ unsigned int warp_tiles[kWarps];
+    const unsigned int warp = threadIdx.x >> 5;
+    const unsigned int lane = threadIdx.x & 31u;
+    for (unsigned int e = lane; e < experts; e += 32u) {
+        warp_place[warp][e] = 0u;
+    }
+    __syncwarp();
+    grid_launch_dependents();
+    grid_dependency_wait();
+    unsigned int tokens = tokens_max;
+    if (tokens_dev != nullptr) {
+        const unsigned int live = *tokens_dev;
+        tokens = live < tokens_max ? live : tokens_max;
+    }
+    const unsigned int pairs = tokens * used;
+    // the warp's run of pairs, a whole number of steps of 32
+    const unsigned int per_warp = ((pairs + kWarps - 1u) / kWarps + 31u) / 32u * 32u;
+    const unsigned int run_begin = warp * per_warp < pairs ? warp * per_warp : pairs;
+    const unsigned int run_end = run_begin + per_warp < pairs ? run_begin + per_warp : pairs;
+
+    unsigned int e[kGroupAhead];
+    for (unsigned int first = run_begin; first < run_end; first += 32u * kGroupAhead) {
+        group_load_ids(ids, first, run_end, experts, lane, e);
+#pragma unroll
+        for (unsigned int a = 0; a < kGroupAhead; ++a) {
+            const unsigned int same = __match_any_sync(0xFFFFFFFFu, e[a]);
+            if (e[a] != 0xFFFFFFFFu && (same & ((1u << lane) - 1u)) == 0u) {
+                warp_place[warp][e[a]] += (unsigned int)__popc(same);   // the lowest lane speaks for the expert
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // One thread per expert: its pairs, and the running totals over the experts of pairs and token tiles.
+    {
+        const unsigned int ex = threadIdx.x;
+        unsigned int mine = 0u;
+        if (ex < experts) {
+#pragma unroll 8
+            for (unsigned int w = 0u; w < kWarps; ++w) {
+                const unsigned int here = warp_place[w][ex];
+                warp_place[w][ex] = mine;
+                mine += here;
+            }
+        }
+        const unsigned int mine_tiles = (mine + tile_tokens - 1u) / tile_tokens;
+        unsigned int run_pairs = mine;
+        unsigned int run_tiles = mine_tiles;
+#pragma unroll
+        for (unsigned int step = 1u; step < 32u; step <<= 1) {
+            const unsigned int below_pairs = __shfl_up_sync(0xFFFFFFFFu, run_pairs, step);
+            const unsigned int below_tiles = __shfl_up_sync(0xFFFFFFFFu, run_tiles, step);
+            if (lane >= step) {
+                run_pairs += below_pairs;
+                run_tiles += below_tiles;
+            }
+        }
+        if (lane == 31u) {
+            warp_pairs[warp] = run_pairs;
+            warp_tiles[warp] = run_tiles;
+        }
+        __syncthreads();
+        if (ex < Q8_GROUP_MAX_EXPERTS) {
+            for (unsigned int w = 0u; w < warp; ++w) {
+                run_pairs += warp_pairs[w];
+                run_tiles += warp_tiles[w];
+            }
+            scan_pairs[ex] = run_pairs;
+            scan_tiles[ex] = run_tiles;
+        }
+        __syncthreads();
+    }
+    const unsigned int placed = scan_pairs[experts - 1u];
+    const unsigned int feed_rows = (feed + kRows - 1u) / kRows;
+    const unsigned int down_rows = (hidden + kRows - 1u) / kRows;
+    if (blockIdx.x == 0u && threadIdx.x == 0u) {
+        counts[0] = scan_tiles[experts - 1u] * feed_rows;
+        counts[1] = scan_tiles[experts - 1u] * down_rows;
+    }
+    for (unsigned int ex = blockIdx.x + gridDim.x * warp; ex < experts; ex += gridDim.x * kWarps) {
+        const unsigned int place = ex != 0u ? scan_pairs[ex - 1u] : 0u;
+        const unsigned int tile = ex != 0u ? scan_tiles[ex - 1u] : 0u;
+        const unsigned int mine = scan_pairs[ex] - place;
+        group_write_tiles(tiles_feed + (size_t)tile * feed_rows, ex, feed, place, mine, tile_tokens, lane);
+        group_write_tiles(tiles_down + (size_t)tile * down_rows, ex, hidden, place, mine, tile_tokens, lane);
+    }
+    // the block's run of places
+    const unsigned int per_block = (pairs + gridDim.x - 1u) / gridDim.x;
+    const unsigned int place_begin = blockIdx.x * per_block < pairs ? blockIdx.x * per_block : pairs;
+    const unsigned int place_end = place_begin + per_block < pairs ? place_begin + per_block : pairs;
+    for (unsigned int first = run_begin; first < run_end; first += 32u * kGroupAhead) {
+        if (per_warp > 32u * kGroupAhead) {
+            group_load_ids(ids, first, run_end, experts, lane, e);     // else they are still there
+        }
+#pragma unroll
+        for (unsigned int a = 0; a < kGroupAhead; ++a) {
+            const unsigned int same = __match_any_sync(0xFFFFFFFFu, e[a]);
+            const unsigned int below = (unsigned int)__popc(same & ((1u << lane) - 1u));
+            const bool there = e[a] != 0xFFFFFFFFu;
+            const unsigned int base = there ? warp_place[warp][e[a]] : 0u;
+            __syncwarp();
+            if (there) {
+                const unsigned int place = (e[a] != 0u ? scan_pairs[e[a] - 1u] : 0u) + base + below;
+                if (place >= place_begin && place < place_end) {
+                    sorted_pair[place] = first + 32u * a + lane;
+                }
+                if (below == 0u) {
+                    warp_place[warp][e[a]] = base + (unsigned int)__popc(same);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    // the places that pairs left out would have taken name no pair
+    for (unsigned int at = (placed > place_begin ? placed : place_begin) + threadIdx.x; at < place_end; at += blockDim.x) {
+        sorted_pair[at] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    // the rows of x of the block's places, 16 bytes per thread step
+    const unsigned int row_chunks = hidden / 8u;
+    const unsigned int last = placed < place_end ? placed : place_end;
+    const unsigned int total = last > place_begin ? (last - place_begin) * row_chunks : 0u;
+#pragma unroll 4
+    for (unsigned int i = threadIdx.x; i < total; i += Q8_GROUP_THREADS) {
+        const unsigned int at = i / row_chunks;
+        const unsigned int c = i - at * row_chunks;
+        unsigned int t = sorted_pair[place_begin + at] / used;
+        const uint4 *from = static_cast<const uint4 *>(x.base[0]);
+        if (x.parts > 1u) {
+            const unsigned int part = t / x.rows_per_part;
+            from = static_cast<const uint4 *>(x.base[part]);
+            t -= part * x.rows_per_part;
+        }
+        x_sorted[(size_t)(place_begin + at) * row_chunks + c] = from[(size_t)t * row_chunks + c];
+    }
+}
+
+static cudaError_t launch_group_gather(cudaStream_t stream, bool overlap, unsigned int sm_count, const RowParts &rows,
+                                       const unsigned int *ids, unsigned int tokens, const unsigned int *tokens_dev,
+                                       unsigned int used, unsigned int experts, unsigned int feed, unsigned int hidden,
+                                       unsigned char *workspace, const MoeWorkspace &ws, unsigned int tile_tokens)
+{
+    const unsigned int pairs = tokens * used;
+    const unsigned int blocks = pairs < sm_count ? pairs : sm_count;
+    return launch_kernel_early(overlap, q8_group_build_kernel_many, blocks, Q8_GROUP_THREADS, 0, stream, rows, ids, tokens,
+                               tokens_dev, used, experts, feed, hidden,
+                               reinterpret_cast<unsigned int *>(workspace + ws.sorted_pair),
+                               reinterpret_cast<GroupTile *>(workspace + ws.tiles_feed),
+                               reinterpret_cast<GroupTile *>(workspace + ws.tiles_down),
+                               reinterpret_cast<unsigned int *>(workspace + ws.counts), tile_tokens,
+                               reinterpret_cast<uint4 *>(workspace + ws.x_sorted));
+}
+#endif
+
 // act = half(silu(gate) * up), silu(g) = g / (1 + exp(-g))  (cuda/model/norm.cu:92-105)
 __global__ void q8_swiglu_kernel(const float *__restrict__ gate, const float *__restrict__ up,
                                  unsigned int tokens_max, const unsigned int *tokens_dev, unsigned int used,
@@ -353,6 +568,24 @@ cudaError_t launch_moe_grouped(cudaStream_t stream, const UmmaScratch &scratch, 
         rows = *x_parts;
     }
 
+#ifndef Q8_HOST_EMULATION
+    cudaError_t err = launch_group_gather(stream, overlap, sm_count, rows, ids, tokens, tokens_dev, used, experts, ffn,
+                                          hidden, workspace, ws, tile_tokens);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    // Gate and up in one launch: a tile's two slabs are the same rows of the two tensors, and the store
+    // applies the gated unit.  (Two products, their sums through memory as floats and an elementwise
+    // kernel took 2 x 50 + 14 us for 512 tokens of 8 of 128 experts, 2048 x 768.)
+    err = launch_umma_grouped(stream, scratch, sm_count, w_gate, experts * ffn, hidden, x_sorted, pairs, tile_tokens,
+                              tiles_feed, counts + 0, ws.max_feed, nullptr, act, ffn, 1, (*launches)++, overlap,
+                              kEpilogueSwiglu, w_up, true);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    (void)gate;
+    (void)up;
+#else
     cudaError_t err = launch_kernel(q8_group_build_kernel, 1, Q8_GROUP_THREADS, 0, stream, ids, tokens, tokens_dev,
                                     used, experts, ffn, hidden, sorted_pair, tiles_feed, tiles_down, counts,
                                     tile_tokens);
@@ -381,6 +614,7 @@ cudaError_t launch_moe_grouped(cudaStream_t stream, const UmmaScratch &scratch, 
     if (err != cudaSuccess) {
         return err;
     }
+#endif
     return launch_umma_grouped(stream, scratch, sm_count, w_down, experts * hidden, ffn, act, pairs,
                                tile_tokens, tiles_down, counts + 1, ws.max_down, sorted_pair, proj, hidden,
                                0, (*launches)++, overlap);
@@ -407,7 +641,15 @@ cudaError_t launch_moe_grouped_fused(cudaStream_t stream, const UmmaScratch &scr
     __half *act = reinterpret_cast<__half *>(workspace + ws.act);
     float *proj = reinterpret_cast<float *>(workspace + ws.proj);
 
+    RowParts rows = {};
+    rows.base[0] = x;
+    rows.parts = 1u;
     // the feed table is built over the 2 * ffn interleaved rows of every expert
+#ifndef Q8_HOST_EMULATION
+    cudaError_t err = launch_group_gather(stream, overlap, sm_count, rows, ids, tokens, tokens_dev, used, experts, 2u * ffn,
+                                          hidden, workspace, ws, tile_tokens);
+    const bool table_late = true;
+#else
     cudaError_t err = launch_kernel(q8_group_build_kernel, 1, Q8_GROUP_THREADS, 0, stream, ids, tokens, tokens_dev,
                                     used, experts, 2u * ffn, hidden, sorted_pair, tiles_feed, tiles_down, counts,
                                     tile_tokens);
@@ -415,17 +657,16 @@ cudaError_t launch_moe_grouped_fused(cudaStream_t stream, const UmmaScratch &scr
         return err;
     }
     const unsigned int wave = pairs < 148u * 16u ? pairs : 148u * 16u;
-    RowParts rows = {};
-    rows.base[0] = x;
-    rows.parts = 1u;
     err = launch_kernel(q8_gather_rows_kernel, wave, 128, 0, stream, rows, sorted_pair, tokens,
                         tokens_dev, used, hidden / 8u, reinterpret_cast<uint4 *>(x_sorted));
+    const bool table_late = false;
+#endif
     if (err != cudaSuccess) {
         return err;
     }
     err = launch_umma_grouped(stream, scratch, sm_count, w_gate_up, experts * 2u * ffn, hidden, x_sorted, pairs,
                               tile_tokens, tiles_feed, counts + 0, ws.max_feed, nullptr, act, ffn, 1,
-                              (*launches)++, overlap, kEpilogueSwiglu);
+                              (*launches)++, overlap, kEpilogueSwiglu, nullptr, table_late);
     if (err != cudaSuccess) {
         return err;
     }

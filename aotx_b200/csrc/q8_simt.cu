@@ -13,6 +13,9 @@
 #include "q8_common.cuh"
 #include "q8_launch.h"
 #include "q8_simt_gemv.cuh"
+#ifndef Q8_HOST_EMULATION
+#include "q8_warp_ptx.cuh"
+#endif
 
 #include <math_constants.h>
 
@@ -67,9 +70,11 @@ __global__ void q8_dequant_kernel(const unsigned char *__restrict__ w, unsigned 
 // when they are many: so few tokens per cluster and many loads of a row in flight for a short
 // batch, many tokens per row value for a long one.  One block for all experts of four tokens,
 // one row of eight loads per warp at a time, took 78 us at any number of tokens up to
-// 512 (140 us with the router cold in L2); this takes 10 us for 8 tokens and 26 us for 512 (128 experts, hidden 2048).
+// 512 (140 us with the router cold in L2); this takes 7 us for 8 tokens and
+// 23 us for 512 (128 experts, hidden 2048).
 // ---------------------------------------------------------------------------------------
-#define Q8_ROUTE_THREADS 256u
+#define Q8_ROUTE_THREADS 256u     // of the emulated launch
+#define Q8_ROUTE_GPU_THREADS 512u
 #define Q8_ROUTE_EXPERTS 256u
 
 // Activations of a group in shared memory, [position along the row][token], rows padded so that
@@ -110,6 +115,36 @@ __device__ __forceinline__ void route_step(const float *at, const float (&r)[EXP
     }
 }
 
+// The largest value over the warp and the lowest index that has it.  Every value is a probability or -1, so
+// their bits order them as signed integers do: two reductions in place of ten shuffles.
+__device__ __forceinline__ void largest_first(float *best, float *best_at)
+{
+#ifdef Q8_HOST_EMULATION
+    for (unsigned int step = 16u; step != 0u; step >>= 1) {
+        const float other = __shfl_xor_sync(0xFFFFFFFFu, *best, step);
+        const float other_at = __shfl_xor_sync(0xFFFFFFFFu, *best_at, step);
+        if (other > *best || (other == *best && other_at < *best_at)) {
+            *best = other;
+            *best_at = other_at;
+        }
+    }
+#else
+    const int most = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(*best));
+    const unsigned int mine = __float_as_int(*best) == most ? (unsigned int)*best_at : 0xFFFFFFFFu;
+    *best_at = (float)__reduce_min_sync(0xFFFFFFFFu, mine);
+    *best = __int_as_float(most);
+#endif
+}
+
+__device__ __forceinline__ void route_arrive()
+{
+#ifdef Q8_HOST_EMULATION
+    cluster_arrive_release();
+#else
+    cluster_arrive_relaxed();
+#endif
+}
+
 template <unsigned int TOKENS, unsigned int EXPERTS, unsigned int AHEAD>
 __device__ __forceinline__ void route_body(const __half *__restrict__ x, const float *__restrict__ router,
                                            unsigned int tokens_max, const unsigned int *tokens_dev,
@@ -132,10 +167,11 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
     const unsigned int first_expert = crank * experts / csize;
     const unsigned int last_expert = (crank + 1u) * experts / csize;
     if (csize > 1u) {
-        // every block has started before another writes into its shared memory
-        cluster_arrive_release();
-        cluster_wait_acquire();
+        // every block has started before another writes into its shared memory (nothing is handed over:
+        // a relaxed arrival, which spares the 2400 cycles of a cluster-scope release); waited for below
+        route_arrive();
     }
+    bool others_started = csize == 1u;
     // the blocks of a cluster take the same groups, so they leave this loop together
     for (unsigned int t0 = blockIdx.x / csize * TOKENS; t0 < tokens; t0 += gridDim.x / csize * TOKENS) {
         const unsigned int group = tokens - t0 < TOKENS ? tokens - t0 : TOKENS;
@@ -162,6 +198,10 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
             }
         }
         __syncthreads();
+        if (!others_started) {
+            cluster_wait_acquire();
+            others_started = true;
+        }
         for (unsigned int ex = first_expert + warp * EXPERTS; ex < last_expert; ex += warps * EXPERTS) {
             // rows past the end repeat the last one; their sums are not used
             const float *row[EXPERTS];
@@ -306,14 +346,7 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
                         best_at = (float)(lane + 32u * j);
                     }
                 }
-                for (unsigned int step = 16u; step != 0u; step >>= 1) {
-                    const float other = __shfl_xor_sync(0xFFFFFFFFu, best, step);
-                    const float other_at = __shfl_xor_sync(0xFFFFFFFFu, best_at, step);
-                    if (other > best || (other == best && other_at < best_at)) {
-                        best = other;
-                        best_at = other_at;
-                    }
-                }
+                largest_first(&best, &best_at);
                 const unsigned int chosen = (unsigned int)best_at;
 #pragma unroll
                 for (unsigned int j = 0; j < kPerLane; ++j) {
@@ -327,6 +360,9 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
             }
         }
         // the next group's activations and logits come after everyone has read this one's
+        if (t0 + gridDim.x / csize * TOKENS >= tokens) {
+            break;
+        }
         if (csize == 1u) {
             __syncthreads();
         } else {
@@ -335,16 +371,21 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
             cluster_wait_acquire();
         }
     }
+    if (!others_started) {
+        cluster_wait_acquire();
+    }
 }
 
-#define Q8_ROUTE_KERNEL(NAME, TOKENS, EXPERTS, AHEAD)                                                                \
-    __global__ void __launch_bounds__(Q8_ROUTE_THREADS)                                                             \
+#define Q8_ROUTE_KERNEL(NAME, TOKENS, EXPERTS, AHEAD)                                                               \
+    __global__ void __launch_bounds__(Q8_ROUTE_GPU_THREADS, 2)                                                      \
     NAME(const __half *__restrict__ x, const float *__restrict__ router, unsigned int tokens_max,                   \
          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts, unsigned int used,              \
          float *__restrict__ prob, unsigned int *__restrict__ ids)                                                  \
     {                                                                                                               \
         Q8_ROUTE_DYNAMIC                                                                                            \
         __shared__ float probability[TOKENS][Q8_ROUTE_EXPERTS];                                                     \
+        grid_launch_dependents();                                                                                   \
+        grid_dependency_wait();                                                                                     \
         route_body<TOKENS, EXPERTS, AHEAD>(x, router, tokens_max, tokens_dev, hidden, experts, used, prob, ids,     \
                                            route_x, probability);                                                   \
     }
@@ -353,10 +394,10 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
 #else
 #define Q8_ROUTE_DYNAMIC extern __shared__ __align__(16) float route_x[];
 #endif
-// rows too long for eight tokens in shared memory; short batches; long ones
-Q8_ROUTE_KERNEL(q8_route_kernel, 4u, 2u, 4u)
-Q8_ROUTE_KERNEL(q8_route_kernel_few, 2u, 2u, 16u)
-Q8_ROUTE_KERNEL(q8_route_kernel_many, 8u, 4u, 4u)
+// middling batches, and rows too long for eight tokens in shared memory; short batches; long ones
+Q8_ROUTE_KERNEL(q8_route_kernel, 4u, 1u, 8u)
+Q8_ROUTE_KERNEL(q8_route_kernel_few, 2u, 1u, 16u)
+Q8_ROUTE_KERNEL(q8_route_kernel_many, 8u, 2u, 4u)
 
 // ---------------------------------------------------------------------------------------
 // Per-pair expert products (pair = token t, rank r; index t * used + r).  These re-read an
@@ -452,13 +493,19 @@ __global__ void q8_expert_sum_kernel(const __grid_constant__ ProjParts from, con
                                      unsigned int experts, unsigned int used, YT *__restrict__ out)
 {
     constexpr unsigned int kTogether = 8u;
+    grid_launch_dependents();
+    grid_dependency_wait();
     unsigned int tokens = tokens_max;
     if (tokens_dev != nullptr) {
         unsigned int live = *tokens_dev;
         tokens = live < tokens_max ? live : tokens_max;
     }
-    for (unsigned int t = blockIdx.x; t < tokens; t += gridDim.x) {
-        for (unsigned int d = threadIdx.x * WIDTH; d < hidden; d += blockDim.x * WIDTH) {
+    // a block takes a part of a token's row, one step of its threads wide
+    const unsigned int parts = (hidden + blockDim.x * WIDTH - 1u) / (blockDim.x * WIDTH);
+    for (unsigned int item = blockIdx.x; item < tokens * parts; item += gridDim.x) {
+        const unsigned int t = item / parts;
+        const unsigned int d = ((item - t * parts) * blockDim.x + threadIdx.x) * WIDTH;
+        if (d < hidden) {
             float sum[WIDTH];
 #pragma unroll
             for (unsigned int i = 0; i < WIDTH; ++i) {
@@ -591,7 +638,7 @@ cudaError_t launch_gemv_simt(cudaStream_t stream, const void *w, unsigned int n,
 
 cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                         unsigned int used, float *prob, unsigned int *ids)
+                         unsigned int used, float *prob, unsigned int *ids, bool overlap)
 {
     if (tokens == 0u) {
         return cudaSuccess;
@@ -603,11 +650,14 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     return launch_kernel(q8_route_kernel, emulated_grid, Q8_ROUTE_THREADS, emulated, stream, static_cast<const __half *>(x),
                          router, tokens, tokens_dev, hidden, experts, used, prob, ids);
 #else
-    // Few tokens: two to a cluster of eight blocks, until the clusters fill the GPU (32 of them are
-    // 256 blocks).  More: eight tokens to a cluster of four, which quarters the reads of the router;
-    // eight tokens of a row longer than 4096 no longer leave room for two blocks on an SM.
-    const bool few = tokens <= 64u;
-    const bool many = !few && hidden <= 4096u;
+    // Few tokens: two to a cluster of eight blocks, as long as the clusters have an SM per block (18 of them
+    // are 144 blocks).  More: four to a cluster of eight, two blocks per SM (37 of them); then eight to a
+    // cluster of four, which quarters the reads of the router and of the activations; eight tokens of a
+    // row longer than 4096 no longer leave room for two blocks on an SM.  Latency bounds all three, so a
+    // block has 16 warps of one or two experts each (measured against 8 warps of two or four; 128
+    // experts, 2048 wide: 8 tokens 9.5 -> 7.2 us, 128 tokens 20.8 -> 13.0, 512 tokens 25.0 -> 22.6).
+    const bool few = tokens <= 36u;
+    const bool many = !few && tokens > 148u && hidden <= 4096u;
     const unsigned int group = few ? 2u : (many ? 8u : 4u);
     const unsigned int cluster = many ? 4u : 8u;
     const unsigned int stride = few ? RouteShape<2u>::stride : (many ? RouteShape<8u>::stride : RouteShape<4u>::stride);
@@ -629,16 +679,18 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(clusters * cluster, 1, 1);
-    config.blockDim = dim3(Q8_ROUTE_THREADS, 1, 1);
+    config.blockDim = dim3(Q8_ROUTE_GPU_THREADS, 1, 1);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
     attribute[0].val.clusterDim.x = cluster;
     attribute[0].val.clusterDim.y = 1;
     attribute[0].val.clusterDim.z = 1;
+    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
-    config.numAttrs = 1;
+    config.numAttrs = overlap ? 2u : 1u;
     return cudaLaunchKernelEx(&config, kernels[which], static_cast<const __half *>(x), router, tokens, tokens_dev, hidden,
                               experts, used, prob, ids);
 #endif
@@ -671,43 +723,46 @@ cudaError_t launch_expert_pairs_simt(cudaStream_t stream, const void *w_gate, co
 }
 
 template <typename YT>
-static cudaError_t expert_sum_launch(bool wide, unsigned int grid, cudaStream_t stream, const ProjParts &proj,
+static cudaError_t expert_sum_launch(bool overlap, bool wide, cudaStream_t stream, const ProjParts &proj,
                                      const float *prob, const unsigned int *ids, unsigned int tokens,
                                      const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
                                      unsigned int used, void *out)
 {
+    // a block per part of a token's row (see the kernel), eight blocks per SM at most
+    const unsigned int step = 256u * (wide ? 4u : 1u);
+    const unsigned long long items = (unsigned long long)tokens * ((hidden + step - 1u) / step);
+    const unsigned int grid = items < 148u * 8u ? (unsigned int)items : 148u * 8u;
     if (wide) {
-        return launch_kernel(q8_expert_sum_kernel<YT, 4u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
+        return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 4u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
                              hidden, experts, used, static_cast<YT *>(out));
     }
-    return launch_kernel(q8_expert_sum_kernel<YT, 1u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
+    return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 1u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
                          hidden, experts, used, static_cast<YT *>(out));
 }
 
 cudaError_t launch_expert_sum_parts(cudaStream_t stream, const ProjParts &proj, const float *prob,
                                     const unsigned int *ids, unsigned int tokens,
                                     const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                                    unsigned int used, void *out, int out_dtype)
+                                    unsigned int used, void *out, int out_dtype, bool overlap)
 {
     if (tokens == 0u) {
         return cudaSuccess;
     }
-    unsigned int grid = tokens < 148u * 8u ? tokens : 148u * 8u;
     // 16-byte loads of proj need rows of a multiple of four floats on a 16-byte boundary
     bool wide = (hidden % 4u) == 0u;
     for (unsigned int i = 0; i < (proj.parts > 1u ? proj.parts : 1u); ++i) {
         wide = wide && (reinterpret_cast<uintptr_t>(proj.base[i]) & 15u) == 0u;
     }
     if (out_dtype == 0) {
-        return expert_sum_launch<float>(wide, grid, stream, proj, prob, ids, tokens, tokens_dev, hidden, experts,
+        return expert_sum_launch<float>(overlap, wide, stream, proj, prob, ids, tokens, tokens_dev, hidden, experts,
                                         used, out);
     }
     if (out_dtype == 1) {
-        return expert_sum_launch<__half>(wide, grid, stream, proj, prob, ids, tokens, tokens_dev, hidden, experts,
+        return expert_sum_launch<__half>(overlap, wide, stream, proj, prob, ids, tokens, tokens_dev, hidden, experts,
                                          used, out);
     }
     if (out_dtype == 2) {
-        return expert_sum_launch<__nv_bfloat16>(wide, grid, stream, proj, prob, ids, tokens, tokens_dev, hidden,
+        return expert_sum_launch<__nv_bfloat16>(overlap, wide, stream, proj, prob, ids, tokens, tokens_dev, hidden,
                                                 experts, used, out);
     }
     return cudaErrorInvalidValue;
@@ -716,13 +771,13 @@ cudaError_t launch_expert_sum_parts(cudaStream_t stream, const ProjParts &proj, 
 cudaError_t launch_expert_sum(cudaStream_t stream, const float *proj, const float *prob,
                               const unsigned int *ids, unsigned int tokens,
                               const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                              unsigned int used, void *out, int out_dtype)
+                              unsigned int used, void *out, int out_dtype, bool overlap)
 {
     ProjParts one = {};
     one.base[0] = proj;
     one.parts = 1u;
     return launch_expert_sum_parts(stream, one, prob, ids, tokens, tokens_dev, hidden, experts, used, out,
-                                   out_dtype);
+                                   out_dtype, overlap);
 }
 
 } // namespace q8

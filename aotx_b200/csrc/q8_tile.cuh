@@ -655,8 +655,8 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
                                unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
                                unsigned int ldy, unsigned int epilogue, float *partial, unsigned int *flags,
                                unsigned long long tile_floats, unsigned int *status, bool overlap);
-cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, unsigned int grid,
-                               unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
+cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap *tw_second,
+                               const CUtensorMap &tx, bool table_late, unsigned int grid, unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
                                const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
                                float *partial, unsigned int *flags, unsigned long long tile_floats, unsigned int *status,
                                bool overlap);

@@ -77,3 +77,43 @@ def test_every_store(ctx, n, k, m):
             slack = 2.2 * (bound[:, 0:even:2] * up.abs() + bound[:, 1:even:2] * (gate.abs() + 1.0)) + eps * unit.abs() + 2.0 ** -24
             assert bool(((g[:m].double() - unit).abs() <= slack).all())
             assert bool((g[m] == torch.tensor(GUARD, dtype=kind)).all())
+
+
+# pairs: fewer than blocks; one step of a warp and one more; more than a warp keeps in registers (4096)
+@pytest.mark.parametrize("tokens,experts,used,hidden,ffn", [(1, 16, 2, 256, 256), (33, 8, 4, 512, 256),
+                                                            (700, 16, 6, 1024, 512), (1100, 128, 4, 256, 256)])
+def test_routed_experts_sorted_by_many_blocks(ctx, tokens, experts, used, hidden, ffn):
+    """The sort and gather over many blocks and the product of gate and up in one launch, with a live batch,
+    selections outside the table and an expert that most tokens choose."""
+    import aotx_b200
+    torch = torch_mod()
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    wg = aotx_b200.synth_q8_0_device(experts * ffn, hidden, 1)
+    wu = aotx_b200.synth_q8_0_device(experts * ffn, hidden, 2)
+    wd = aotx_b200.synth_q8_0_device(experts * hidden, ffn, 3)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).half()
+    ids = torch.stack([torch.randperm(experts, device="cuda", generator=gen)[:used] for _ in range(tokens)]).int()
+    ids[: tokens * 3 // 4, 0] = 0                 # (a pair twice is a pair like any other)
+    ids[tokens // 2, used - 1] = experts + 5      # outside the table: adds nothing
+    prob = torch.rand(tokens, experts, device="cuda", generator=gen)
+    live = tokens - tokens // 3
+    out = torch.full((tokens, hidden), GUARD, device="cuda")
+    ctx.moe_ffn(wg, wu, wd, experts, hidden, ffn, x, prob, ids, tokens_dev=torch.tensor([live], dtype=torch.int32, device="cuda"),
+                out=out)
+    gate_w, up_w = (ctx.dequant(w, hidden, 0, experts * ffn).double().view(experts, ffn, hidden) for w in (wg, wu))
+    down_w = ctx.dequant(wd, ffn, 0, experts * hidden).double().view(experts, hidden, ffn)
+    want = torch.zeros(tokens, hidden, device="cuda", dtype=torch.float64)
+    bound = torch.zeros_like(want)
+    for e in range(experts):
+        for t, r in (ids[:live] == e).nonzero().tolist():
+            xd = x[t].double()
+            gate, up = gate_w[e] @ xd, up_w[e] @ xd
+            unit = gate / (1.0 + torch.exp(-gate)) * up
+            # act: the float sums' errors through the unit (slope at most 1.1), and one rounding to binary16
+            eg, eu = (hidden * 2.0 ** -23 * (w[e].abs() @ xd.abs()) for w in (gate_w, up_w))
+            err = 2.2 * (eg * up.abs() + eu * (gate.abs() + 1.0)) + 2.0 ** -10 * unit.abs() + 2.0 ** -24
+            p = prob[t, e].double()
+            want[t] += p * (down_w[e] @ unit)
+            bound[t] += p * (down_w[e].abs() @ (err + (ffn + used + 2) * 2.0 ** -23 * unit.abs()))
+    assert bool(((out[:live].double() - want[:live]).abs() <= bound[:live] * 1.001 + 1e-30).all())
+    assert bool((out[live:] == GUARD).all())
