@@ -397,7 +397,7 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
 // middling batches, and rows too long for eight tokens in shared memory; short batches; long ones
 Q8_ROUTE_KERNEL(q8_route_kernel, 4u, 1u, 8u)
 Q8_ROUTE_KERNEL(q8_route_kernel_few, 2u, 1u, 16u)
-Q8_ROUTE_KERNEL(q8_route_kernel_many, 8u, 2u, 4u)
+Q8_ROUTE_KERNEL(q8_route_kernel_many, 8u, 2u, 3u)
 
 // ---------------------------------------------------------------------------------------
 // Per-pair expert products (pair = token t, rank r; index t * used + r).  These re-read an
