@@ -203,7 +203,7 @@ extern "C" int aotx_q8_dequant(aotx_q8_ctx *ctx, void *stream, const void *w, ui
         return AOTX_Q8_ERR_ARGUMENT;
     }
     cudaError_t err = type == AOTX_Q8_TYPE_Q8_0
-        ? q8::launch_dequant((cudaStream_t)stream, w, k, first_row, rows, out_f16)
+        ? q8::launch_dequant((cudaStream_t)stream, w, k, first_row, rows, out_f16, ctx->overlap != 0)
         : q8::launch_dequant_any((cudaStream_t)stream, w, type, k, first_row, rows, out_f16);
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }
@@ -234,7 +234,8 @@ extern "C" int aotx_q8_matmul(aotx_q8_ctx *ctx, void *stream, const void *w, uin
         if (ctx->path == AOTX_Q8_PATH_TENSOR) {
             return AOTX_Q8_ERR_UNSUPPORTED;
         }
-        cudaError_t any = q8::launch_gemv_any(s, w, type, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y, y_dtype);
+        cudaError_t any = q8::launch_gemv_any(s, w, type, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y, y_dtype,
+                                              ctx->overlap != 0);
         return any == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, any);
     }
     /* One MMA takes both operands in one 16-bit format (binary16 weights against bfloat16
@@ -250,7 +251,8 @@ extern "C" int aotx_q8_matmul(aotx_q8_ctx *ctx, void *stream, const void *w, uin
         err = q8::launch_umma(s, ctx->scratch, ctx->sm_count, w, n, k, x, x_dtype == AOTX_Q8_BF16, m,
                               m_dev, y, y_dtype, ctx->launches++, ctx->overlap != 0, nullptr, 0u);
     } else {
-        err = q8::launch_gemv_simt(s, w, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y, y_dtype);
+        err = q8::launch_gemv_simt(s, w, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y, y_dtype, q8::kEpilogueStore,
+                                   ctx->overlap != 0);
     }
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }
@@ -294,7 +296,7 @@ extern "C" int aotx_q8_matmul_fused(aotx_q8_ctx *ctx, void *stream, const void *
                               y_dtype, ctx->launches++, ctx->overlap != 0, nullptr, (unsigned int)epilogue);
     } else {
         err = q8::launch_gemv_simt(s, w, n, k, x, x_dtype == AOTX_Q8_BF16, m, m_dev, y, y_dtype,
-                                   (unsigned int)epilogue);
+                                   (unsigned int)epilogue, ctx->overlap != 0);
     }
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }

@@ -102,13 +102,13 @@ constexpr unsigned int kEpilogueAdd = 1u;    // y is float and the sum is added 
 constexpr unsigned int kEpilogueSwiglu = 2u; // rows 2p, 2p+1 of w are gate and up of column p
 
 cudaError_t launch_dequant(cudaStream_t stream, const void *w, unsigned int k, unsigned int first_row,
-                           unsigned int rows, void *out);
+                           unsigned int rows, void *out, bool overlap = false);
 
 // `epilogue`: 0 store, 1 add into a float y, 2 silu(gate) * up over row pairs of w into a y of
 // n / 2 columns (the same three modes as the tensor-core kernel, see q8_tile.cuh).
 cudaError_t launch_gemv_simt(cudaStream_t stream, const void *w, unsigned int n, unsigned int k,
                              const void *x, int x_bf16, unsigned int m, const unsigned int *m_dev,
-                             void *y, int y_dtype, unsigned int epilogue = 0u);
+                             void *y, int y_dtype, unsigned int epilogue = 0u, bool overlap = false);
 
 // Every other block type of the model file (q_generic.cu, decoder in q_blocks.cuh).
 bool block_type_known(unsigned int type);
@@ -117,14 +117,14 @@ cudaError_t launch_dequant_any(cudaStream_t stream, const void *w, unsigned int 
                                unsigned int first_row, unsigned int rows, void *out);
 cudaError_t launch_gemv_any(cudaStream_t stream, const void *w, unsigned int type, unsigned int n,
                             unsigned int k, const void *x, int x_bf16, unsigned int m,
-                            const unsigned int *m_dev, void *y, int y_dtype);
+                            const unsigned int *m_dev, void *y, int y_dtype, bool overlap = false);
 
 // The same products on the warp-level tensor path (q_warp.cu): the types and alignments it takes
 // (Q8_0 among them, rows of any multiple of 32 weights), and the launch.
 bool warp_any_supports(const void *w, unsigned int type, unsigned int n, unsigned int k, const void *x, unsigned int m);
 cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int type, unsigned int n, unsigned int k,
                             const void *x, int x_bf16, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
-                            unsigned int epilogue);
+                            unsigned int epilogue, bool overlap);
 
 cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,

@@ -216,14 +216,15 @@ static cudaError_t launch_gemv_any_typed(cudaStream_t stream, const void *w, uns
 
 cudaError_t launch_gemv_any(cudaStream_t stream, const void *w, unsigned int type, unsigned int n,
                             unsigned int k, const void *x, int x_bf16, unsigned int m,
-                            const unsigned int *m_dev, void *y, int y_dtype)
+                            const unsigned int *m_dev, void *y, int y_dtype, bool overlap)
 {
+    (void)overlap;
     if (n == 0u || m == 0u) {
         return cudaSuccess;
     }
 #ifndef Q8_HOST_EMULATION
     if (warp_any_supports(w, type, n, k, x, m)) {
-        return launch_warp_any(stream, w, type, n, k, x, x_bf16, m, m_dev, y, y_dtype, kEpilogueStore);
+        return launch_warp_any(stream, w, type, n, k, x, x_bf16, m, m_dev, y, y_dtype, kEpilogueStore, overlap);
     }
 #endif
 #define QG_CASE(XT, YD, YT)                                                                       \

@@ -188,8 +188,10 @@ __device__ __forceinline__ void four_runs(const RowAt &row, uint32_t t, uint32_t
         }
 #pragma unroll
         for (uint32_t r = 0; r < 4u; ++r) {
-            scale[r] = d * (float)((sc >> (8u * r)) & 0xFFu);
-            off[r] = -(dmin * (float)((mn >> (8u * r)) & 0xFFu));
+            // 0x4B000000 is 2^23, one unit per step of the mantissa: a whole number by a byte permute and an
+            // exact subtraction; the conversion instruction runs at a quarter of their rate
+            scale[r] = d * (__uint_as_float(prmt(sc, 0x4B000000u, 0x7650u + r)) - 8388608.0f);
+            off[r] = dmin * (8388608.0f - __uint_as_float(prmt(mn, 0x4B000000u, 0x7650u + r)));
         }
         constexpr uint32_t nibbles = (TYPE == kTypeQ5_K ? 48u : 16u) + HALF * 64u;
 #pragma unroll
@@ -255,15 +257,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t g = lane >> 2;
     const uint32_t t = lane & 3u;
-    uint32_t m = args.m_max;
-    if (args.m_dev != nullptr) {
-        const uint32_t live = *args.m_dev;
-        m = live < m ? live : m;
-    }
-    const uint32_t token0 = blockIdx.x * 8u * TILES;
-    if (token0 >= m) {
-        return;
-    }
+    grid_launch_dependents();
     const uint32_t runs = args.k / 32u;
     const uint32_t pieces = (runs + S::piece_runs - 1u) / S::piece_runs;
     const uint32_t first_piece = pieces * warp / kAnyWarps;
@@ -319,6 +313,19 @@ q_gemv_any_kernel_warp(const AnyArgs args)
 #pragma unroll
     for (uint32_t i = 0; i < kAnyDepth - 1u; ++i) {
         issue(i);
+    }
+
+    // everything but the weights may come from the launch before this one
+    grid_dependency_wait();
+    uint32_t m = args.m_max;
+    if (args.m_dev != nullptr) {
+        const uint32_t live = *args.m_dev;
+        m = live < m ? live : m;
+    }
+    const uint32_t token0 = blockIdx.x * 8u * TILES;
+    if (token0 >= m) {
+        copy_async_wait<0>();
+        return;
     }
 
     // this lane's row of x per column of eight (past the batch: the last row; those sums are not
@@ -492,7 +499,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
 }
 
 template <uint32_t TYPE, bool BF, uint32_t TILES>
-static cudaError_t launch_any_tiles(cudaStream_t stream, const AnyArgs &args)
+static cudaError_t launch_any_tiles(cudaStream_t stream, bool overlap, const AnyArgs &args)
 {
     using S = AnyShape<TYPE>;
     static unsigned long long configured = 0ull;
@@ -502,22 +509,23 @@ static cudaError_t launch_any_tiles(cudaStream_t stream, const AnyArgs &args)
     }
     const uint32_t passes = (args.m_max + 8u * TILES - 1u) / (8u * TILES);
     const uint32_t groups = (args.n + kAnyRows - 1u) / kAnyRows;
-    // a wave of two blocks per SM where the rows are enough for it, dealt evenly
+    // Two blocks per SM where the rows are enough for it, some with a group more than others.  (As few blocks as
+    // give all the same number of groups leave half of the SMs with one block: 14336 rows, 896 groups: 224
+    // blocks of four against 296 of three or four.)
     const uint32_t wave = (2u * 148u + passes - 1u) / passes;
-    const uint32_t turns = (groups + wave - 1u) / wave;
-    const uint32_t blocks = (groups + turns - 1u) / turns;
-    return launch_kernel(q_gemv_any_kernel_warp<TYPE, BF, TILES>, dim3(passes, blocks), kAnyWarps * 32u, S::smem_bytes,
+    const uint32_t blocks = groups < wave ? groups : wave;
+    return launch_kernel_early(overlap, q_gemv_any_kernel_warp<TYPE, BF, TILES>, dim3(passes, blocks), kAnyWarps * 32u, S::smem_bytes,
                          stream, args);
 }
 
 template <uint32_t TYPE>
-static cudaError_t launch_any_type(cudaStream_t stream, const AnyArgs &args, bool bf)
+static cudaError_t launch_any_type(cudaStream_t stream, bool overlap, const AnyArgs &args, bool bf)
 {
     // 8 rows of x to a pass, or 16
     if (args.m_max <= 8u) {
-        return bf ? launch_any_tiles<TYPE, true, 1u>(stream, args) : launch_any_tiles<TYPE, false, 1u>(stream, args);
+        return bf ? launch_any_tiles<TYPE, true, 1u>(stream, overlap, args) : launch_any_tiles<TYPE, false, 1u>(stream, overlap, args);
     }
-    return bf ? launch_any_tiles<TYPE, true, 2u>(stream, args) : launch_any_tiles<TYPE, false, 2u>(stream, args);
+    return bf ? launch_any_tiles<TYPE, true, 2u>(stream, overlap, args) : launch_any_tiles<TYPE, false, 2u>(stream, overlap, args);
 }
 
 bool warp_any_supports(const void *w, unsigned int type, unsigned int n, unsigned int k, const void *x, unsigned int m)
@@ -532,7 +540,7 @@ bool warp_any_supports(const void *w, unsigned int type, unsigned int n, unsigne
 
 cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int type, unsigned int n, unsigned int k,
                             const void *x, int x_bf16, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
-                            unsigned int epilogue)
+                            unsigned int epilogue, bool overlap)
 {
     if (y_dtype < 0 || y_dtype > 2 || (epilogue == kEpilogueAdd && y_dtype != 0)
         || (epilogue == kEpilogueSwiglu && (n & 1u) != 0u) || epilogue > kEpilogueSwiglu) {
@@ -551,14 +559,14 @@ cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int typ
     args.epilogue = epilogue;
     const bool bf = x_bf16 != 0;
     switch (type) {
-    case kTypeQ8_0: return launch_any_type<kTypeQ8_0>(stream, args, bf);
-    case kTypeQ4_0: return launch_any_type<kTypeQ4_0>(stream, args, bf);
-    case kTypeQ4_1: return launch_any_type<kTypeQ4_1>(stream, args, bf);
-    case kTypeQ5_0: return launch_any_type<kTypeQ5_0>(stream, args, bf);
-    case kTypeQ5_1: return launch_any_type<kTypeQ5_1>(stream, args, bf);
-    case kTypeQ4_K: return launch_any_type<kTypeQ4_K>(stream, args, bf);
-    case kTypeQ5_K: return launch_any_type<kTypeQ5_K>(stream, args, bf);
-    case kTypeQ6_K: return launch_any_type<kTypeQ6_K>(stream, args, bf);
+    case kTypeQ8_0: return launch_any_type<kTypeQ8_0>(stream, overlap, args, bf);
+    case kTypeQ4_0: return launch_any_type<kTypeQ4_0>(stream, overlap, args, bf);
+    case kTypeQ4_1: return launch_any_type<kTypeQ4_1>(stream, overlap, args, bf);
+    case kTypeQ5_0: return launch_any_type<kTypeQ5_0>(stream, overlap, args, bf);
+    case kTypeQ5_1: return launch_any_type<kTypeQ5_1>(stream, overlap, args, bf);
+    case kTypeQ4_K: return launch_any_type<kTypeQ4_K>(stream, overlap, args, bf);
+    case kTypeQ5_K: return launch_any_type<kTypeQ5_K>(stream, overlap, args, bf);
+    case kTypeQ6_K: return launch_any_type<kTypeQ6_K>(stream, overlap, args, bf);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -83,3 +83,20 @@ def test_fused_stores(ctx, n, k, m):
     gate, up = y[:, 0::2].double(), y[:, 1::2].double()
     unit = gate / (1.0 + torch.exp(-gate)) * up
     assert bool(((g - unit).abs() <= 2.0 ** -20 * unit.abs() + 1e-12).all())   # expf and three float roundings
+
+
+# one piece per thread up to 591 * 1024 pieces of 8 weights, four from there on; a last block that is full, and not
+@pytest.mark.parametrize("rows,k", [(1, 32), (2327, 2080), (2332, 2080), (592, 8192), (593, 8192), (1999, 4064)])
+def test_dequant_exact_on_both_sides_of_the_line(ctx, rows, k):
+    import aotx_b200
+    torch = torch_mod()
+    w = aotx_b200.synth_q8_0_device(rows, k, rows)
+    raw = w.view(-1, 34)
+    d = raw[:, :2].contiguous().view(torch.float16)
+    want = (raw[:, 2:].contiguous().view(torch.int8).half() * d).view(rows, k)    # rounded once, like the kernel
+    assert torch.equal(ctx.dequant(w, k, 0, rows), want)
+    # a result that starts between 16-byte boundaries, and nothing written around it
+    store = torch.full((rows * k + 4,), GUARD, device="cuda", dtype=torch.float16)
+    ctx.dequant(w, k, 0, rows, out=store[2:2 + rows * k].view(rows, k))
+    assert torch.equal(store[2:2 + rows * k].view(rows, k), want)
+    assert bool((store[:2] == store[-1]).all()) and bool((store[-2:] == GUARD).all())
