@@ -177,7 +177,13 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     // Up to 16 rows, one copy of y: the register-fed kernel; up to 128: q8_mid.cu.  Stores into the
     // peers' copies stay with the kernels they were measured on.
     const bool warp_kernel = ntok <= 16u && out == nullptr;
-    if (ntok > 128u && out == nullptr && scratch.blocks >= sm_count && scratch.tile_floats >= 256ull * kRows
+    // Above 112 rows q8_mid.cu has accumulators as wide as a pair's; with rows of w enough for every block a
+    // pair of SMs, which reads half of x each, is then faster: 28672 x 4096, 128 rows, 42.0 -> 38.6 us,
+    // 151936 x 8192 359 -> 341 (100 rows: the same time; few rows of w: clusters, 24.1 against 26.1).
+    const bool wide = ntok > 128u
+                   || (mid && m > 112u
+                       && mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats, epilogue).cluster == 1u);
+    if (wide && out == nullptr && scratch.blocks >= sm_count && scratch.tile_floats >= 256ull * kRows
         && (unsigned long long)(n / (2u * kRows) + 1u) * (m / 128u + 1u) * (k / kSegK) < (1ull << 31)) {
         const unsigned int rows = pair_token_tile(m);
         CUtensorMap tw, tx;

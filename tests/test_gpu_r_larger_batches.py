@@ -31,7 +31,7 @@ def sums(ctx, w, n, k, x, extra=0.0):
 
 # rows of w: a partial tile; one tile; a cluster of four's, of two's; two turns; cut into units; and deep
 # enough that one tile has several holders
-SHAPES = [(1, 256, 17), (130, 1024, 33), (1023, 2048, 128), (9990, 512, 40), (20004, 768, 64), (60001, 256, 100),
+SHAPES = [(20004, 512, 113), (1, 256, 17), (130, 1024, 33), (1023, 2048, 128), (9990, 512, 40), (20004, 768, 64), (60001, 256, 100),
           (77, 1536, 129), (300, 5120, 257), (2049, 1024, 300), (19456, 512, 512), (40962, 256, 700)]
 
 
