@@ -275,6 +275,7 @@ cudaError_t launch_collect_ids(cudaStream_t stream, const unsigned int *const *i
 // expert: one expert may hold most of the pairs - and a block writes and gathers its own run.
 // The tile tables are dealt to all warps of the grid by expert.
 constexpr unsigned int kGroupAhead = 4;   // pairs per lane whose loads are issued together
+constexpr unsigned int kGroupRun = 1024;  // places of a block that are kept in shared memory as well
 
 __device__ __forceinline__ void group_load_ids(const unsigned int *__restrict__ ids, unsigned int first, unsigned int end,
                                                unsigned int experts, unsigned int lane, unsigned int (&e)[kGroupAhead])
@@ -323,12 +324,18 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
     __shared__ unsigned int warp_place[kWarps][Q8_GROUP_MAX_EXPERTS];
     __shared__ unsigned int scan_pairs[Q8_GROUP_MAX_EXPERTS];       // up to and with the expert
     __shared__ unsigned int scan_tiles[Q8_GROUP_MAX_EXPERTS];
+    __shared__ unsigned int edge[2];
+    __shared__ unsigned int run[kGroupRun];
     __shared__ unsigned int warp_pairs[kWarps];
     __shared__ unsigned int warp_tiles[kWarps];
     const unsigned int warp = threadIdx.x >> 5;
     const unsigned int lane = threadIdx.x & 31u;
     for (unsigned int e = lane; e < experts; e += 32u) {
         warp_place[warp][e] = 0u;
+    }
+    if (threadIdx.x == 0u) {
+        edge[0] = 1u;     // none: the first is after the last
+        edge[1] = 0u;
     }
     __syncwarp();
     grid_launch_dependents();
@@ -344,16 +351,18 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
     const unsigned int run_begin = warp * per_warp < pairs ? warp * per_warp : pairs;
     const unsigned int run_end = run_begin + per_warp < pairs ? run_begin + per_warp : pairs;
 
+    // the block's run of places
+    const unsigned int per_block = (pairs + gridDim.x - 1u) / gridDim.x;
+    const unsigned int place_begin = blockIdx.x * per_block < pairs ? blockIdx.x * per_block : pairs;
+    const unsigned int place_end = place_begin + per_block < pairs ? place_begin + per_block : pairs;
     unsigned int e[kGroupAhead];
     for (unsigned int first = run_begin; first < run_end; first += 32u * kGroupAhead) {
         group_load_ids(ids, first, run_end, experts, lane, e);
 #pragma unroll
         for (unsigned int a = 0; a < kGroupAhead; ++a) {
-            const unsigned int same = __match_any_sync(0xFFFFFFFFu, e[a]);
-            if (e[a] != 0xFFFFFFFFu && (same & ((1u << lane) - 1u)) == 0u) {
-                warp_place[warp][e[a]] += (unsigned int)__popc(same);   // the lowest lane speaks for the expert
+            if (e[a] != 0xFFFFFFFFu) {
+                atomicAdd(&warp_place[warp][e[a]], 1u);
             }
-            __syncwarp();
         }
     }
     __syncthreads();
@@ -393,6 +402,14 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
             }
             scan_pairs[ex] = run_pairs;
             scan_tiles[ex] = run_tiles;
+            // the experts that hold the first and the last of the block's places
+            const unsigned int begin = run_pairs - mine;
+            if (begin <= place_begin && place_begin < run_pairs) {
+                edge[0] = ex;
+            }
+            if (begin < place_end && place_begin < run_pairs) {
+                atomicMax(&edge[1], ex);
+            }
         }
         __syncthreads();
     }
@@ -410,28 +427,34 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
         group_write_tiles(tiles_feed + (size_t)tile * feed_rows, ex, feed, place, mine, tile_tokens, lane);
         group_write_tiles(tiles_down + (size_t)tile * down_rows, ex, hidden, place, mine, tile_tokens, lane);
     }
-    // the block's run of places
-    const unsigned int per_block = (pairs + gridDim.x - 1u) / gridDim.x;
-    const unsigned int place_begin = blockIdx.x * per_block < pairs ? blockIdx.x * per_block : pairs;
-    const unsigned int place_end = place_begin + per_block < pairs ? place_begin + per_block : pairs;
-    for (unsigned int first = run_begin; first < run_end; first += 32u * kGroupAhead) {
-        if (per_warp > 32u * kGroupAhead) {
-            group_load_ids(ids, first, run_end, experts, lane, e);     // else they are still there
-        }
+    // Only the few experts of the block's run matter here: a ballot per expert and step tells the pairs'
+    // places, steps in order within the warp, warps in order within the expert.
+    const unsigned int edge_first = edge[0];
+    const unsigned int edge_last = edge[1];
+    if (edge_first <= edge_last && place_begin < placed) {
+        for (unsigned int first = run_begin; first < run_end; first += 32u * kGroupAhead) {
+            if (per_warp > 32u * kGroupAhead) {
+                group_load_ids(ids, first, run_end, experts, lane, e);     // else they are still there
+            }
+            for (unsigned int ex = edge_first; ex <= edge_last; ++ex) {
+                const unsigned int in_expert = warp_place[warp][ex];
+                unsigned int place = (ex != 0u ? scan_pairs[ex - 1u] : 0u) + in_expert;
+                unsigned int seen = 0u;
 #pragma unroll
-        for (unsigned int a = 0; a < kGroupAhead; ++a) {
-            const unsigned int same = __match_any_sync(0xFFFFFFFFu, e[a]);
-            const unsigned int below = (unsigned int)__popc(same & ((1u << lane) - 1u));
-            const bool there = e[a] != 0xFFFFFFFFu;
-            const unsigned int base = there ? warp_place[warp][e[a]] : 0u;
-            __syncwarp();
-            if (there) {
-                const unsigned int place = (e[a] != 0u ? scan_pairs[e[a] - 1u] : 0u) + base + below;
-                if (place >= place_begin && place < place_end) {
-                    sorted_pair[place] = first + 32u * a + lane;
+                for (unsigned int a = 0; a < kGroupAhead; ++a) {
+                    const unsigned int same = __ballot_sync(0xFFFFFFFFu, e[a] == ex);
+                    const unsigned int at = place + seen + (unsigned int)__popc(same & ((1u << lane) - 1u));
+                    if (e[a] == ex && at >= place_begin && at < place_end) {
+                        sorted_pair[at] = first + 32u * a + lane;
+                        if (at - place_begin < kGroupRun) {
+                            run[at - place_begin] = first + 32u * a + lane;
+                        }
+                    }
+                    seen += (unsigned int)__popc(same);
                 }
-                if (below == 0u) {
-                    warp_place[warp][e[a]] = base + (unsigned int)__popc(same);
+                __syncwarp();
+                if (lane == 0u) {
+                    warp_place[warp][ex] = in_expert + seen;
                 }
             }
             __syncwarp();
@@ -450,7 +473,7 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
     for (unsigned int i = threadIdx.x; i < total; i += Q8_GROUP_THREADS) {
         const unsigned int at = i / row_chunks;
         const unsigned int c = i - at * row_chunks;
-        unsigned int t = sorted_pair[place_begin + at] / used;
+        unsigned int t = (at < kGroupRun ? run[at] : sorted_pair[place_begin + at]) / used;
         const uint4 *from = static_cast<const uint4 *>(x.base[0]);
         if (x.parts > 1u) {
             const unsigned int part = t / x.rows_per_part;
