@@ -1,10 +1,10 @@
-// The decode-regime kernel of the Q8_0 product for batches of up to 32 rows of x:
+// The decode-regime kernel of the Q8_0 product for batches of up to 16 rows of x:
 // y[i][j] = sum_c x[i][c] * half(q[j][c] * d[j][c / 32]), float sums.
 //
 // HBM-bound: a launch moves n * (k / 32) * 34 bytes of weights once, and an SM has to turn about
 // 21 weights per cycle into products to keep up with memory.  The weights therefore go from
 // shared memory straight into the registers of the warp that multiplies them (mma.sync
-// m16n8k16, 951 products per cycle and SM measured, 21 x 32 needed at 32 rows): one hand-over
+// m16n8k16, 951 products per cycle and SM measured, 21 x 16 needed at 16 rows): one hand-over
 // per segment (copy lands -> warps read) where a kernel on tensor memory has five, each a
 // fraction of a microsecond long.
 //
@@ -22,13 +22,16 @@
 //   * x (half, or bfloat16 turned into half once per block and segment) is stored so that a lane
 //     reads its four words of a block's two MMA steps as 16 bytes: row stride 528 bytes, lane t
 //     of a pair of blocks at 32 t.
-//   * Up to 16 rows of x a warp takes 16 rows of w over the whole segment; from 17 on it takes 32
-//     rows over half of it, because each warp reads every x row it multiplies with (8 warps
-//     would read the x segment 8 times, more than the banks carry at this rate), and the two
-//     halves are added at the end of a tile.
+//   * A warp takes 16 rows of w over the whole segment.  (At 32 rows of x, warps of 32 rows over half a segment
+//     each, this kernel is bound by its instructions: q8_mid.cu is as fast there and needs no second form.)
 //   * Schedule as in q8_decode.cu: few row tiles run as a cluster per tile, each block one run of
 //     its segments, pieces added through distributed shared memory in block order; larger
 //     tensors run (tile, segment) units dealt evenly, the first holder of a cut tile owns it.
+//
+// Against the kernel on tensor memory that these batches ran on before (q8_decode.cu): 4096 x 4096, one row,
+// 7.9 -> 6.5 us in a graph; the four products of a layer of 4096 by 14336, 8 rows, 95 -> 60 us; 151936 x 8192,
+// 8 rows, 328 -> 246 us (5.4 TB/s with a cold L2 full of changed lines, 6.3 without).  What is left of a
+// small product is its start and end: the first copy's latency, the exchange in the cluster.
 //
 // Every wait is bounded and raises a status bit when it runs out.  Reference kernels replaced:
 // ptx/gemv_q8.ptx:18-223, cuda/model/gemv.cuh:33-145 (and the three-node switch of
@@ -49,26 +52,18 @@ constexpr uint32_t kWarpXRow = 528;        // bytes of a row of x in a stage: 25
 template <int NTOK>
 struct WarpShape {
     static constexpr uint32_t tiles = NTOK / 8;                   // MMA columns of 8 rows of x
-    static constexpr uint32_t k_groups = NTOK > 16 ? 2 : 1;
-    static constexpr uint32_t row_groups = kWarpCompute / k_groups;
-    static constexpr uint32_t m_tiles = kRows / row_groups / 16;  // 16-row pieces of w per warp
-    static constexpr uint32_t chains = tiles * m_tiles >= 4 ? 1 : 2; // sums that successive steps take in turn
+    static constexpr uint32_t chains = 2;                         // sums that successive steps take in turn
     static constexpr uint32_t stages = 2;
-    static constexpr uint32_t held = m_tiles * tiles * 4 / k_groups; // finished sums per thread
+    static constexpr uint32_t held = tiles * 4;                   // finished sums per thread
     static constexpr uint32_t x_stage_bytes = NTOK * kWarpXRow;
     static constexpr uint32_t raw_offset = 0;
     static constexpr uint32_t x_offset = stages * kRawStageBytes;
-    // the halves of a tile change hands here, 1 KB per warp at a time
-    static constexpr uint32_t swap_offset = x_offset + stages * x_stage_bytes;
-    static constexpr uint32_t swap_bytes = k_groups == 2 ? kWarpCompute * 1024 : 0;
-    // what the blocks of a cluster send: a tile of floats; beside the rings where there is room (a
-    // block may then receive while it still multiplies), else over the x ring's place and the raw
-    // ring, which are idle by then
+    // what the blocks of a cluster send: a tile of floats, beside the rings, so that a block may receive
+    // while it still multiplies
     static constexpr uint32_t recv_bytes = kRows * NTOK * 4;
-    static constexpr bool recv_apart = NTOK <= 16;
-    static constexpr uint32_t recv_offset = recv_apart ? swap_offset + swap_bytes : 0;
-    static constexpr uint32_t bar_offset = swap_offset + swap_bytes + (recv_apart ? recv_bytes : 0);
-    static constexpr uint32_t bar_count = 3 * stages + 8;
+    static constexpr uint32_t recv_offset = x_offset + stages * x_stage_bytes;
+    static constexpr uint32_t bar_offset = recv_offset + recv_bytes;
+    static constexpr uint32_t bar_count = 3 * stages;
     static constexpr uint32_t smem_bytes = bar_offset + bar_count * 8 + 16 + 1024;
     static_assert(2u * (smem_bytes + 1024u) <= 228u * 1024u, "two blocks' shared memory on one SM");
 };
@@ -112,30 +107,23 @@ __device__ __forceinline__ void block_operands(const uint32_t (&first)[2], const
     }
 }
 
-// Finished sums: value `i` of a thread belongs to row row_of(i) of the tile and row token_of(i)
-// of x.  After the halves were added a warp of k group q holds the tiles [q * tiles / 2, ..).
-template <int NTOK>
-struct WarpPlace {
-    using S = WarpShape<NTOK>;
-    static __device__ __forceinline__ uint32_t row_of(uint32_t i, uint32_t row_group, uint32_t g)
-    {
-        const uint32_t mt = i / (S::held / S::m_tiles);
-        return row_group * (16u * S::m_tiles) + mt * 16u + g + ((i >> 1) & 1u) * 8u;
-    }
-    static __device__ __forceinline__ uint32_t token_of(uint32_t i, uint32_t k_group, uint32_t t)
-    {
-        const uint32_t j = (i / 4u) % (S::tiles / S::k_groups) + k_group * (S::tiles / S::k_groups);
-        return j * 8u + 2u * t + (i & 1u);
-    }
-};
+// Finished sums: value `i` of a thread belongs to row row_of(i) of the tile and row token_of(i) of x.
+static __device__ __forceinline__ uint32_t row_of(uint32_t i, uint32_t warp, uint32_t g)
+{
+    return warp * 16u + g + ((i >> 1) & 1u) * 8u;
+}
+
+static __device__ __forceinline__ uint32_t token_of(uint32_t i, uint32_t t)
+{
+    return i / 4u * 8u + 2u * t + (i & 1u);
+}
 
 // Store the sums of a tile that lie in fragment order (pairs of rows of x in d0, d1 and d2, d3).
 template <int NTOK, typename YT>
-__device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t tile, uint32_t m_live, uint32_t row_group,
-                                                uint32_t k_group, uint32_t lane, float (&v)[WarpShape<NTOK>::held])
+__device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t tile, uint32_t m_live, uint32_t warp,
+                                                uint32_t lane, float (&v)[WarpShape<NTOK>::held])
 {
     using S = WarpShape<NTOK>;
-    using P = WarpPlace<NTOK>;
     const uint32_t g = lane >> 2;
     const uint32_t t = lane & 3u;
     const uint32_t n = args.n;
@@ -153,8 +141,8 @@ __device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t t
             const float got = __shfl_xor_sync(0xFFFFFFFFu, give, 4u);
             const float low = odd ? got : keep;
             const float high = odd ? keep : got;
-            const uint32_t token = P::token_of(i, k_group, t) + (odd ? 1u : 0u);
-            const uint32_t row = tile * kRows + (P::row_of(i, row_group, g) & ~1u);
+            const uint32_t token = token_of(i, t) + (odd ? 1u : 0u);
+            const uint32_t row = tile * kRows + (row_of(i, warp, g) & ~1u);
             if (token < m_live && row < n) {
                 if (args.epilogue == kEpilogueSwiglu) {
                     // gate and up rows of one column (the arithmetic of cuda/model/norm.cu:92-105)
@@ -176,14 +164,14 @@ __device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t t
         float before[S::held];
 #pragma unroll
         for (uint32_t i = 0; i < S::held; ++i) {
-            const uint32_t token = P::token_of(i, k_group, t);
-            const uint32_t row = tile * kRows + P::row_of(i, row_group, g);
+            const uint32_t token = token_of(i, t);
+            const uint32_t row = tile * kRows + row_of(i, warp, g);
             before[i] = token < m_live && row < n ? sums[(size_t)token * ldy + row] : 0.0f;
         }
 #pragma unroll
         for (uint32_t i = 0; i < S::held; ++i) {
-            const uint32_t token = P::token_of(i, k_group, t);
-            const uint32_t row = tile * kRows + P::row_of(i, row_group, g);
+            const uint32_t token = token_of(i, t);
+            const uint32_t row = tile * kRows + row_of(i, warp, g);
             if (token < m_live && row < n) {
                 sums[(size_t)token * ldy + row] = before[i] + v[i];
             }
@@ -192,8 +180,8 @@ __device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t t
     }
 #pragma unroll
     for (uint32_t i = 0; i < S::held; ++i) {
-        const uint32_t token = P::token_of(i, k_group, t);
-        const uint32_t row = tile * kRows + P::row_of(i, row_group, g);
+        const uint32_t token = token_of(i, t);
+        const uint32_t row = tile * kRows + row_of(i, warp, g);
         if (token < m_live && row < n) {
             store_out<YT>(y, (size_t)token * ldy + row, v[i]);
         }
@@ -213,7 +201,6 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
     const uint32_t raw_full = smem0 + S::bar_offset;
     const uint32_t x_full = raw_full + 8u * S::stages;
     const uint32_t empty = x_full + 8u * S::stages;
-    const uint32_t swap_bar = empty + 8u * S::stages;        // two per pair of warps
     volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + S::bar_offset + 8u * S::bar_count);
 
     const uint32_t warp = threadIdx.x >> 5;
@@ -254,9 +241,6 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
             mbar_init(x_full + 8u * i, kWarpLoaders);
             mbar_init(empty + 8u * i, kWarpCompute);
         }
-        for (uint32_t i = 0; i < 8u; ++i) {
-            mbar_init(swap_bar + 8u * i, 2u);
-        }
         *abort_flag = 0u;
         mbar_init_fence();
         fence_proxy_async_smem();
@@ -282,9 +266,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
 
     unsigned int m_live = 0u;
     bool ok = true;
-    float acc[S::chains][S::m_tiles][S::tiles][4];
-    const uint32_t row_group = warp / S::k_groups;
-    const uint32_t k_group = warp % S::k_groups;
+    float acc[S::chains][S::tiles][4];
 
     if (warp >= kWarpCompute) {
         // ---------------------------------------------------------------- x, and the weight copies
@@ -358,28 +340,23 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
         const uint32_t g8 = lane >> 2;
         const uint32_t t = lane & 3u;
         const uint32_t turn = t == 3u ? 0x7610u : 0x3210u;     // lane 3's second word of an even block
-        constexpr uint32_t kPairs = kSegK / 64u / S::k_groups; // pairs of blocks of a segment per warp
         // this lane's first row and first pair of blocks, and its x
-        const unsigned char *w_lane = smem + S::raw_offset + (row_group * (16u * S::m_tiles) + g8) * kSegBytes
-                                    + k_group * kPairs * 68u + 4u * t;
-        const unsigned char *x_lane = smem + S::x_offset + g8 * kWarpXRow + k_group * kPairs * 128u + 32u * t;
+        const unsigned char *w_lane = smem + S::raw_offset + (warp * 16u + g8) * kSegBytes + 4u * t;
+        const unsigned char *x_lane = smem + S::x_offset + g8 * kWarpXRow + 32u * t;
         uint32_t g = 0;
         uint32_t tile = tile_begin;
         uint32_t s0 = seg_begin;
-        uint32_t pieces = 0;
-        for (uint32_t u = u_begin; ok && u < u_end; ++pieces) {
+        bool first_piece = true;
+        for (uint32_t u = u_begin; ok && u < u_end;) {
             const uint32_t left = u_end - u;
             const uint32_t s1 = (segs - s0) < left ? segs : s0 + left;
 #pragma unroll
             for (uint32_t c = 0; c < S::chains; ++c) {
 #pragma unroll
-                for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
+                for (uint32_t j = 0; j < S::tiles; ++j) {
 #pragma unroll
-                    for (uint32_t j = 0; j < S::tiles; ++j) {
-#pragma unroll
-                        for (uint32_t i = 0; i < 4u; ++i) {
-                            acc[c][mt][j][i] = 0.0f;
-                        }
+                    for (uint32_t i = 0; i < 4u; ++i) {
+                        acc[c][j][i] = 0.0f;
                     }
                 }
             }
@@ -396,66 +373,48 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
                 const unsigned char *w_at = w_lane + st * kRawStageBytes;
                 const unsigned char *x_at = x_lane + st * S::x_stage_bytes;
 #pragma unroll
-                for (uint32_t b = 0; b < 2u * kPairs; ++b) {
+                for (uint32_t b = 0; b < kSegK / 32u; ++b) {
                     // block b: its scale in word 0 (low half) or 8 (high half) of the pair
                     const uint32_t word0 = (b / 2u) * 68u + (b & 1u) * 32u;
-                    uint32_t a[S::m_tiles][2][4];
+                    uint32_t a[2][4];
+                    uint32_t first[2], second[2], d_bits[2];
 #pragma unroll
-                    for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-                        uint32_t first[2], second[2], d_bits[2];
-#pragma unroll
-                        for (uint32_t r = 0; r < 2u; ++r) {
-                            const unsigned char *row = w_at + (mt * 16u + r * 8u) * kSegBytes + word0;
-                            const uint32_t scale = *reinterpret_cast<const uint32_t *>(row - 4u * t);
-                            first[r] = *reinterpret_cast<const uint32_t *>(row + 4u);
-                            second[r] = *reinterpret_cast<const uint32_t *>(row + 20u);
-                            if ((b & 1u) == 0u) {
-                                second[r] = prmt(second[r], scale, turn);
-                                d_bits[r] = prmt(scale, scale, 0x1010u);
-                            } else {
-                                d_bits[r] = prmt(scale, scale, 0x3232u);
-                            }
+                    for (uint32_t r = 0; r < 2u; ++r) {
+                        const unsigned char *row = w_at + r * 8u * kSegBytes + word0;
+                        const uint32_t scale = *reinterpret_cast<const uint32_t *>(row - 4u * t);
+                        first[r] = *reinterpret_cast<const uint32_t *>(row + 4u);
+                        second[r] = *reinterpret_cast<const uint32_t *>(row + 20u);
+                        if ((b & 1u) == 0u) {
+                            second[r] = prmt(second[r], scale, turn);
+                            d_bits[r] = prmt(scale, scale, 0x1010u);
+                        } else {
+                            d_bits[r] = prmt(scale, scale, 0x3232u);
                         }
-                        block_operands(first, second, d_bits, a[mt]);
                     }
-                    // two columns of tiles at a time, one step of both before the next: an MMA that
-                    // adds to the sums of the one before it waits for them, about four MMAs' time
-                    constexpr uint32_t kTogether = S::tiles < 2u ? 1u : 2u;
+                    block_operands(first, second, d_bits, a);
+                    // one step of all columns before the next: an MMA that adds to the sums of the one
+                    // before it waits for them, about four MMAs' time
+                    uint4 xv[S::tiles];
 #pragma unroll
-                    for (uint32_t j0 = 0; j0 < S::tiles; j0 += kTogether) {
-                        uint4 xv[kTogether];
+                    for (uint32_t j = 0; j < S::tiles; ++j) {
+                        xv[j] = *reinterpret_cast<const uint4 *>(x_at + j * 8u * kWarpXRow + (b / 2u) * 128u + (b & 1u) * 16u);
+                    }
 #pragma unroll
-                        for (uint32_t j = 0; j < kTogether; ++j) {
-                            xv[j] = *reinterpret_cast<const uint4 *>(x_at + (j0 + j) * 8u * kWarpXRow + (b / 2u) * 128u
-                                                                     + (b & 1u) * 16u);
-                        }
+                    for (uint32_t j = 0; j < S::tiles; ++j) {
+                        mma_16816(acc[0][j], a[0], xv[j].x, xv[j].y);
+                    }
 #pragma unroll
-                        for (uint32_t j = 0; j < kTogether; ++j) {
-#pragma unroll
-                            for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-                                mma_16816(acc[0][mt][j0 + j], a[mt][0], xv[j].x, xv[j].y);
-                            }
-                        }
-#pragma unroll
-                        for (uint32_t j = 0; j < kTogether; ++j) {
-#pragma unroll
-                            for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-                                mma_16816(acc[S::chains - 1u][mt][j0 + j], a[mt][1], xv[j].z, xv[j].w);
-                            }
-                        }
+                    for (uint32_t j = 0; j < S::tiles; ++j) {
+                        mma_16816(acc[1][j], a[1], xv[j].z, xv[j].w);
                     }
                 }
                 // The stage goes back when the words of every lane have arrived, not only been asked
                 // for (the next copy overwrites it): the vote needs sums that every load of the
                 // segment went into.  It is true about once in 2^32 segments, and then does nothing.
-                uint32_t seen = __float_as_uint(acc[0][0][0][0]);
+                uint32_t seen = __float_as_uint(acc[0][0][0]) ^ __float_as_uint(acc[1][0][2]);
 #pragma unroll
                 for (uint32_t j = 0; j < S::tiles; ++j) {
-                    seen ^= __float_as_uint(acc[S::chains - 1u][0][j][1]);
-                }
-#pragma unroll
-                for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-                    seen ^= __float_as_uint(acc[S::chains - 1u][mt][0][2]);
+                    seen ^= __float_as_uint(acc[1][j][1]);
                 }
                 if (__any_sync(0xFFFFFFFFu, seen == 0x7FB1A5C3u)) {
                     atomicOr(args.status, 0u);
@@ -467,75 +426,13 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
             if (!ok) {
                 break;
             }
-            if (S::chains == 2u) {
-#pragma unroll
-                for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-#pragma unroll
-                    for (uint32_t j = 0; j < S::tiles; ++j) {
-#pragma unroll
-                        for (uint32_t i = 0; i < 4u; ++i) {
-                            acc[0][mt][j][i] += acc[S::chains - 1u][mt][j][i];
-                        }
-                    }
-                }
-            }
             float v[S::held];
-            if constexpr (S::k_groups == 1u) {
 #pragma unroll
-                for (uint32_t i = 0; i < S::held; ++i) {
-                    v[i] = acc[0][i / (4u * S::tiles)][(i / 4u) % S::tiles][i % 4u];
-                }
-            } else {
-                // The two warps of a pair trade halves of their sums: k group 0 keeps the first
-                // half of the columns, k group 1 the second; one 16-row piece at a time.
-                constexpr uint32_t kHalf = S::tiles / 2u;
-                const uint32_t pair_bar = swap_bar + 16u * row_group;
-                float4 *mine = reinterpret_cast<float4 *>(smem + S::swap_offset + warp * 1024u) + lane;
-                const float4 *other = reinterpret_cast<const float4 *>(smem + S::swap_offset + (warp ^ 1u) * 1024u) + lane;
-#pragma unroll
-                for (uint32_t mt = 0; mt < S::m_tiles; ++mt) {
-                    if (mt != 0u || pieces != 0u) {
-                        // the other warp has read what lies there: its read came before its
-                        // arrival on the second barrier
-                        const uint32_t turns = pieces * S::m_tiles + mt - 1u;
-                        ok = mbar_wait_hot(pair_bar + 8u, turns & 1u, abort_flag, args.status) && ok;
-                    }
-#pragma unroll
-                    for (uint32_t j = 0; j < kHalf; ++j) {
-                        float give[4];
-#pragma unroll
-                        for (uint32_t i = 0; i < 4u; ++i) {
-                            give[i] = k_group == 0u ? acc[0][mt][kHalf + j][i] : acc[0][mt][j][i];
-                        }
-                        mine[32u * j] = make_float4(give[0], give[1], give[2], give[3]);
-                    }
-                    __syncwarp();
-                    if (lane == 0u) {
-                        mbar_arrive(pair_bar);
-                    }
-                    const uint32_t turn_now = pieces * S::m_tiles + mt;
-                    ok = mbar_wait_hot(pair_bar, turn_now & 1u, abort_flag, args.status) && ok;
-#pragma unroll
-                    for (uint32_t j = 0; j < kHalf; ++j) {
-                        const float4 got = other[32u * j];
-                        const float from[4] = {got.x, got.y, got.z, got.w};
-#pragma unroll
-                        for (uint32_t i = 0; i < 4u; ++i) {
-                            // one addition of two values: the same whichever warp of the pair does it
-                            v[(mt * kHalf + j) * 4u + i] = (k_group == 0u ? acc[0][mt][j][i] : acc[0][mt][kHalf + j][i]) + from[i];
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0u) {
-                        mbar_arrive(pair_bar + 8u);
-                    }
-                }
-                ok = __all_sync(0xFFFFFFFFu, ok) != 0;
-                if (!ok) {
-                    break;
-                }
+            for (uint32_t i = 0; i < S::held; ++i) {
+                v[i] = acc[0][i / 4u][i % 4u] + acc[1][i / 4u][i % 4u];
             }
-            if (pieces == 0u) {
+            if (first_piece) {
+                first_piece = false;
                 grid_dependency_wait();
                 m_live = args.m_max;
                 if (args.m_dev != nullptr) {
@@ -546,7 +443,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
             if (split) {
 #pragma unroll
                 for (uint32_t i = 0; i < S::held; ++i) {
-                    acc[0][i / (4u * S::tiles)][(i / 4u) % S::tiles][i % 4u] = v[i];
+                    acc[0][i / 4u][i % 4u] = v[i];
                 }
                 break;
             }
@@ -606,7 +503,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
                         }
                     }
                 }
-                store_fragments<NTOK, YT>(args, tile, m_live, row_group, k_group, lane, v);
+                store_fragments<NTOK, YT>(args, tile, m_live, warp, lane, v);
             }
             u += s1 - s0;
             s0 = 0u;
@@ -623,22 +520,16 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
     // owner adds the pieces in block order and stores.
     __syncwarp();
     cluster_wait_acquire();
-    if (!S::recv_apart) {
-        // the received tile lies over the rings: every block is done with its own
-        __syncwarp();
-        cluster_arrive_release();
-        cluster_wait_acquire();
-    }
-    const uint32_t share = (uint32_t)NTOK / csize;   // 1 to 32: the cluster size is a power of two up to 8
+    const uint32_t share = (uint32_t)NTOK / csize;   // 1 to 16: the cluster size is a power of two up to 8
     if (warp < kWarpCompute) {
         const uint32_t g8 = lane >> 2;
         const uint32_t t = lane & 3u;
 #pragma unroll
         for (uint32_t i = 0; i < S::held; ++i) {
-            const uint32_t token = WarpPlace<NTOK>::token_of(i, k_group, t);
-            const uint32_t row = WarpPlace<NTOK>::row_of(i, row_group, g8);
+            const uint32_t token = token_of(i, t);
+            const uint32_t row = row_of(i, warp, g8);
             const uint32_t at = smem0 + S::recv_offset + ((crank * share + token % share) * kRows + row) * 4u;
-            st_shared_cluster_f32(mapa_shared(at, token / share), acc[0][i / (4u * S::tiles)][(i / 4u) % S::tiles][i % 4u]);
+            st_shared_cluster_f32(mapa_shared(at, token / share), acc[0][i / 4u][i % 4u]);
         }
     }
     __syncwarp();

@@ -1,11 +1,18 @@
 // Host side of the tensor-core products: which kernel serves a product, its tensor maps, its
 // grid and its scratch.
 //
-//   rows of x     kernel                                                        file
-//   1 .. 32       decode kernel, two blocks per SM, cluster split along k       q8_decode.cu
-//   33 .. 128     decode-regime kernel, one block per SM (also the grouped      q8_stream.cu
-//                 products of the routed experts, token tiles of 64)
-//   129 ..        prefill kernel, token tiles of 256, weights in tensor memory  q8_wide.cu
+//   rows of x     kernel                                                          file
+//   1 .. 16       weights through registers into mma.sync, two blocks per SM      q8_decode_warp.cu
+//   17 .. 128     weights through tensor memory, one block per SM; also the       q8_mid.cu
+//                 grouped products of the routed experts
+//   129 ..        pairs of SMs, tiles of 256 rows of w by up to 256 of x; from    q8_pair.cu
+//                 113 rows on where w has rows for every block
+//
+// Where the lines lie: at 17 rows mma.sync would need a third column of eight and is bound by its
+// instructions at 32 (q8_decode_warp.cu); above 128 an accumulator of q8_mid.cu no longer fits
+// beside two segments of A.  Products stored into several GPUs' copies of y, bfloat16 x without room for
+// its binary16 copy, and the host emulation run on the kernels these replaced (q8_decode.cu up to 32 rows,
+// q8_stream.cu up to 128, q8_wide.cu above).
 //
 // Shapes none of them takes (k not a multiple of 256, unaligned pointers) return
 // cudaErrorNotSupported and the caller uses the general kernel (q8_simt.cu).  Reference: the
