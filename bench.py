@@ -62,8 +62,8 @@ EPILOGUE_OF = {"o": 1, "down": 1, "gate_up": 2}  # AOTX_Q8_EPILOGUE_ADD / _SWIGL
 
 # DRAM bytes (read + write) per algorithmic byte of the dominant kernel: one ncu capture of the
 # gate+up projection at 32 rows, scaled to the average launch by bytes (source named in the line).
-TRAFFIC_RATIO = {"decode_m32_llama3_8b_layer": 1.2168, "decode_m32_gate_up": 1.2168}
-TRAFFIC_SOURCE = "profiles/q8_decode_kernel_gate_up_m32.md (28672 x 4096, 32 rows, one launch)"
+TRAFFIC_RATIO = {"decode_m32_llama3_8b_layer": 0.9973, "decode_m32_gate_up": 0.9973}
+TRAFFIC_SOURCE = "profiles/q8_products_by_regime.md (28672 x 4096, 32 rows, one launch)"
 TENSOR_BOUND = {"prefill_m2048_llama3_8b_layer", "prefill_m2048_gate_up", "prefill_m2048_llama3_8b_layer_fused"}
 
 
@@ -369,7 +369,8 @@ def run_ours(args, rank, world, local_rank):
     roofline["peak_source"] = peak_kind
     # the nominal figures, for context only (HBM3e 7.7 TB/s; dense bf16 2250 TFLOP/s)
     roofline["frac_of_nominal"] = achieved / (2250.0 if tensor_bound else 7700.0)
-    roofline["kernel"] = "q8_wide_kernel" if tensor_bound else "q8_decode_kernel"
+    roofline["kernel"] = ("q8_decode_kernel_warp" if m <= 16 else "q8_stream_kernel_mid" if m <= 128
+                          else "q8_wide_kernel_pair")
     roofline["launches_timed"] = launches * args.steps
     roofline["avg_launch_us"] = kernel_ms * 1e3
     roofline["bytes_per_launch"] = step_bytes / launches
@@ -393,7 +394,8 @@ def run_ours(args, rank, world, local_rank):
         "roofline": roofline,
         "e2e": {"value": e2e_value, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": e2e_ms / args.steps, "mode": e2e_mode, "host_result_matches_device": check},
-        "gpu_launches": launches * args.steps,
+        # 17 to 128 rows of bfloat16 x are turned into binary16 by a launch of their own
+        "gpu_launches": launches * (2 if x_name == "bfloat16" and 17 <= m <= 128 else 1) * args.steps,
         "clocks": clocks,
         "device_status": status,
     }
@@ -505,9 +507,9 @@ def setup_moe(torch, ctx, world, rank, moe_fused=False, copies=2):
     hit = int((torch.bincount(ids_all.reshape(-1).long(), minlength=experts) > 0).sum())
     slice_bytes = 2 * ffn * (hidden // 32) * 34 + hidden * (ffn // 32) * 34
     step_bytes = hit * slice_bytes + tokens * hidden * 2 + tokens * hidden * 4
-    # one GPU: table, gather, gate, up, gated unit, down, sum (interleaved: one product and no
-    # gated-unit kernel less); expert parallel adds two barriers and the collection of the ids
-    launches = (5 if moe_fused else 7) if world == 1 else 10
+    # one GPU: table with sort and gather, gate and up, down, sum; expert parallel adds two barriers
+    # and the collection of the ids
+    launches = 4 if world == 1 else 7
     config = {"workload": "moe_qwen3_30b_a3b", "interleaved_gate_up": bool(moe_fused and world == 1),
               "tokens": tokens, "experts": experts, "used": used,
               "hidden": hidden, "ffn": ffn, "experts_hit": hit, "x": "float16", "y": "float32",
