@@ -394,8 +394,8 @@ def run_ours(args, rank, world, local_rank):
         "roofline": roofline,
         "e2e": {"value": e2e_value, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": e2e_ms / args.steps, "mode": e2e_mode, "host_result_matches_device": check},
-        # 17 to 128 rows of bfloat16 x are turned into binary16 by a launch of their own
-        "gpu_launches": launches * (2 if x_name == "bfloat16" and 17 <= m <= 128 else 1) * args.steps,
+        # the products; not counted: 17 to 128 rows of bfloat16 x are turned into binary16 by a launch of their own
+        "gpu_launches": launches * args.steps,
         "clocks": clocks,
         "device_status": status,
     }
