@@ -130,6 +130,18 @@ __device__ __forceinline__ uint32_t fifth_bits(uint32_t four)
     return ((four | (four << 7) | (four << 14) | (four << 21)) & 0x01010101u) << 4;
 }
 
+// Which weights of a run of 32 a lane takes does not matter to the sum, as long as x goes with them.  WIDE: 8t ..
+// 8t + 7, so that a lane's x of a run is one load of 16 bytes; else 4t .. 4t + 3 and 16 + 4t .. + 3, two loads of 8.
+// What a warp's load of x costs is its 8 rows, not its bytes; what the wide form costs is two weight words from
+// one nibble plane, and rows of words two apart.  Measured, wide against not: Q8_0 30000 x 2912, 7 rows, 30.5 us
+// against 34.0, 5003 x 2912, 40 rows, 26.7 against 28.2; Q4_K 14336 x 4096, 4 rows, 15.3 against 16.3, 30 rows
+// (two columns of eight) 49.1 against 47.9; Q4_0, 4 rows, 17.2 against 16.0.  Q6_K has a scale per step.
+template <uint32_t TYPE, uint32_t TILES>
+__host__ __device__ constexpr bool any_wide()
+{
+    return TYPE == kTypeQ8_0 || (TILES == 1u && (TYPE == kTypeQ4_K || TYPE == kTypeQ5_K));
+}
+
 // One run of 32 weights of the formats whose block is a run (run R of the piece).
 template <uint32_t TYPE, uint32_t R>
 __device__ __forceinline__ void one_run(const RowAt &row, uint32_t t, uint32_t (&codes)[4][2], float (&scale)[8], float (&off)[4])
@@ -139,8 +151,8 @@ __device__ __forceinline__ void one_run(const RowAt &row, uint32_t t, uint32_t (
     constexpr uint32_t at = R * S::block_bytes;
     scale[R] = half_bits(u16_at<at>(row));
     if constexpr (TYPE == kTypeQ8_0) {
-        codes[R][0] = word_at<W, at + 2u>(row, t);
-        codes[R][1] = word_at<W, at + 18u>(row, t);
+        codes[R][0] = word_at<W, at + 2u>(row, 2u * t);
+        codes[R][1] = word_at<W, at + 6u>(row, 2u * t);
     } else {
         constexpr bool five = TYPE == kTypeQ5_0 || TYPE == kTypeQ5_1;
         constexpr uint32_t head = S::offset ? 4u : 2u;
@@ -159,9 +171,9 @@ __device__ __forceinline__ void one_run(const RowAt &row, uint32_t t, uint32_t (
 }
 
 // The codes of four runs of 32 weights (runs 4 * HALF .. + 3 of the piece) that lane t of a
-// row's four lanes holds: codes[run][step], weights 16 step + 4t .. + 3; and the runs' scales and
+// row's four lanes holds: codes[run][step], weights 16 step + 4t .. + 3 or (WIDE) 8t + 4 step .. + 3; and the runs' scales and
 // offsets (Q6_K: scale[2 * run + step]).
-template <uint32_t TYPE, uint32_t HALF>
+template <uint32_t TYPE, uint32_t HALF, bool WIDE>
 __device__ __forceinline__ void four_runs(const RowAt &row, uint32_t t, uint32_t (&codes)[4][2], float (&scale)[8],
                                           float (&off)[4])
 {
@@ -198,7 +210,7 @@ __device__ __forceinline__ void four_runs(const RowAt &row, uint32_t t, uint32_t
         for (uint32_t c = 0; c < 2u; ++c) {
 #pragma unroll
             for (uint32_t step = 0; step < 2u; ++step) {
-                const uint32_t w = row.words[nibbles / 4u + c * 8u + step * 4u + t];
+                const uint32_t w = row.words[nibbles / 4u + c * 8u + (WIDE ? 2u * t + step : step * 4u + t)];
                 codes[2u * c][step] = w & 0x0F0F0F0Fu;
                 codes[2u * c + 1u][step] = (w >> 4) & 0x0F0F0F0Fu;
             }
@@ -206,7 +218,7 @@ __device__ __forceinline__ void four_runs(const RowAt &row, uint32_t t, uint32_t
         if constexpr (TYPE == kTypeQ5_K) {
 #pragma unroll
             for (uint32_t step = 0; step < 2u; ++step) {
-                const uint32_t w = row.words[4u + step * 4u + t] >> (4u * HALF);
+                const uint32_t w = row.words[4u + (WIDE ? 2u * t + step : step * 4u + t)] >> (4u * HALF);
 #pragma unroll
                 for (uint32_t r = 0; r < 4u; ++r) {
                     codes[r][step] |= ((w >> r) & 0x01010101u) << 4;
@@ -244,6 +256,7 @@ struct AnyArgs {
     unsigned long long row_bytes;
     uint32_t n, k, m_max;
     uint32_t y_dtype, epilogue;
+    uint32_t wide_x;               // x starts on a 16-byte boundary
 };
 
 template <uint32_t TYPE, bool BF, uint32_t TILES>
@@ -251,6 +264,7 @@ __global__ void __launch_bounds__(kAnyWarps * 32u, 2)
 q_gemv_any_kernel_warp(const AnyArgs args)
 {
     using S = AnyShape<TYPE>;
+    constexpr bool kWide = any_wide<TYPE, TILES>();
     extern __shared__ __align__(16) unsigned char any_smem_[];
     __shared__ float parts[2][kAnyWarps][8u * TILES][kAnyRows];   // partial sums of the 8 warps, two row groups in turn
     const uint32_t warp = threadIdx.x >> 5;
@@ -335,7 +349,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
     for (uint32_t j = 0; j < TILES; ++j) {
         const uint32_t token = token0 + 8u * j + g;
         x_row[j] = static_cast<const unsigned short *>(args.x) + (size_t)(token < m ? token : m - 1u) * args.k
-                 + first_piece * S::piece_runs * 32u + 4u * t;
+                 + first_piece * S::piece_runs * 32u + (kWide ? 8u : 4u) * t;
     }
     // where this lane's rows g and g + 8 start modulo 16 bytes, at the warp's first piece of a group
     const uint32_t row_shift = (uint32_t)(reinterpret_cast<uintptr_t>(args.w) + g * args.row_bytes
@@ -365,9 +379,16 @@ q_gemv_any_kernel_warp(const AnyArgs args)
                     const uint2 *from = reinterpret_cast<const uint2 *>(x_row[j] + piece * (S::piece_runs * 32u) + half * 128u);
 #pragma unroll
                     for (uint32_t r = 0; r < 4u; ++r) {
-                        if (S::super || r < live_runs) {
+                        if (!S::super && r >= live_runs) {
+                            continue;
+                        }
+                        if (kWide && args.wide_x != 0u) {
+                            const uint4 both = __ldg(reinterpret_cast<const uint4 *>(from + r * 8u));
+                            xv[j][r][0] = make_uint2(both.x, both.y);
+                            xv[j][r][1] = make_uint2(both.z, both.w);
+                        } else {
                             xv[j][r][0] = __ldg(from + r * 8u);
-                            xv[j][r][1] = __ldg(from + r * 8u + 4u);
+                            xv[j][r][1] = __ldg(from + r * 8u + (kWide ? 1u : 4u));
                         }
                     }
                 }
@@ -395,11 +416,11 @@ q_gemv_any_kernel_warp(const AnyArgs args)
                 float scale[2][8];
                 float off[2][4];
                 if (half == 0u) {
-                    four_runs<TYPE, 0>(rows[0], t, codes[0], scale[0], off[0]);
-                    four_runs<TYPE, 0>(rows[1], t, codes[1], scale[1], off[1]);
+                    four_runs<TYPE, 0, kWide>(rows[0], t, codes[0], scale[0], off[0]);
+                    four_runs<TYPE, 0, kWide>(rows[1], t, codes[1], scale[1], off[1]);
                 } else {
-                    four_runs<TYPE, 1>(rows[0], t, codes[0], scale[0], off[0]);
-                    four_runs<TYPE, 1>(rows[1], t, codes[1], scale[1], off[1]);
+                    four_runs<TYPE, 1, kWide>(rows[0], t, codes[0], scale[0], off[0]);
+                    four_runs<TYPE, 1, kWide>(rows[1], t, codes[1], scale[1], off[1]);
                 }
 #pragma unroll
                 for (uint32_t r = 0; r < 4u; ++r) {
@@ -557,6 +578,7 @@ cudaError_t launch_warp_any(cudaStream_t stream, const void *w, unsigned int typ
     args.m_max = m;
     args.y_dtype = (uint32_t)y_dtype;
     args.epilogue = epilogue;
+    args.wide_x = (reinterpret_cast<uintptr_t>(x) & 15u) == 0u ? 1u : 0u;
     const bool bf = x_bf16 != 0;
     switch (type) {
     case kTypeQ8_0: return launch_any_type<kTypeQ8_0>(stream, overlap, args, bf);

@@ -100,3 +100,17 @@ def test_dequant_exact_on_both_sides_of_the_line(ctx, rows, k):
     ctx.dequant(w, k, 0, rows, out=store[2:2 + rows * k].view(rows, k))
     assert torch.equal(store[2:2 + rows * k].view(rows, k), want)
     assert bool((store[:2] == store[-1]).all()) and bool((store[-2:] == GUARD).all())
+
+
+@pytest.mark.parametrize("kind,n,k,m", [(8, 33, 1184, 7), (8, 50, 96, 12), (12, 40, 512, 5), (13, 17, 256, 8), (2, 18, 160, 3)])
+def test_x_between_16_byte_boundaries(ctx, kind, n, k, m):
+    """The two ways to load x take the same weights into the same sums."""
+    torch = torch_mod()
+    w = dev(_blocks.random_rows(kind, n, k, np.random.Generator(np.random.PCG64(n))).reshape(-1))
+    room = torch.randn(m * k + 4, device="cuda").half()
+    shifted = room[4:].view(m, k)                 # 8 bytes past a boundary
+    ctx.set_path(1 if kind == 8 else 0)
+    a = ctx.matmul(w, n, k, shifted, type=kind)
+    b = ctx.matmul(w, n, k, shifted.clone(), type=kind)
+    ctx.set_path(0)
+    assert torch.equal(a, b)
