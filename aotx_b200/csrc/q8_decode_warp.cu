@@ -52,7 +52,10 @@ constexpr uint32_t kWarpXRow = 528;        // bytes of a row of x in a stage: 25
 template <int NTOK>
 struct WarpShape {
     static constexpr uint32_t tiles = NTOK / 8;                   // MMA columns of 8 rows of x
-    static constexpr uint32_t chains = 2;                         // sums that successive steps take in turn
+    // Sums that successive steps take in turn.  An MMA truncates the sum it adds to, so the error of a product
+    // grows with the steps that go into one sum: 4096 x 4096, one row, 3.5e-7 of the result with two sums,
+    // 2.0e-7 with four (151936 x 8192, 8 rows: 2 and 1 times 1.5e-6); the time is the same within 1.4 %.
+    static constexpr uint32_t chains = 4;
     static constexpr uint32_t stages = 2;
     static constexpr uint32_t held = tiles * 4;                   // finished sums per thread
     static constexpr uint32_t x_stage_bytes = NTOK * kWarpXRow;
@@ -401,20 +404,20 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
                     }
 #pragma unroll
                     for (uint32_t j = 0; j < S::tiles; ++j) {
-                        mma_16816(acc[0][j], a[0], xv[j].x, xv[j].y);
+                        mma_16816(acc[2u * (b & 1u)][j], a[0], xv[j].x, xv[j].y);
                     }
 #pragma unroll
                     for (uint32_t j = 0; j < S::tiles; ++j) {
-                        mma_16816(acc[1][j], a[1], xv[j].z, xv[j].w);
+                        mma_16816(acc[2u * (b & 1u) + 1u][j], a[1], xv[j].z, xv[j].w);
                     }
                 }
                 // The stage goes back when the words of every lane have arrived, not only been asked
                 // for (the next copy overwrites it): the vote needs sums that every load of the
                 // segment went into.  It is true about once in 2^32 segments, and then does nothing.
-                uint32_t seen = __float_as_uint(acc[0][0][0]) ^ __float_as_uint(acc[1][0][2]);
+                uint32_t seen = __float_as_uint(acc[2][0][0]) ^ __float_as_uint(acc[3][0][2]);
 #pragma unroll
                 for (uint32_t j = 0; j < S::tiles; ++j) {
-                    seen ^= __float_as_uint(acc[1][j][1]);
+                    seen ^= __float_as_uint(acc[3][j][1]) ^ __float_as_uint(acc[0][j][3]) ^ __float_as_uint(acc[1][j][3]);
                 }
                 if (__any_sync(0xFFFFFFFFu, seen == 0x7FB1A5C3u)) {
                     atomicOr(args.status, 0u);
@@ -429,7 +432,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__
             float v[S::held];
 #pragma unroll
             for (uint32_t i = 0; i < S::held; ++i) {
-                v[i] = acc[0][i / 4u][i % 4u] + acc[1][i / 4u][i % 4u];
+                v[i] = (acc[0][i / 4u][i % 4u] + acc[1][i / 4u][i % 4u]) + (acc[2][i / 4u][i % 4u] + acc[3][i / 4u][i % 4u]);
             }
             if (first_piece) {
                 first_piece = false;

@@ -1,0 +1,37 @@
+"""How exact the float sums of a product are, against float64.
+
+A tensor-core MMA adds sixteen products to a running sum and truncates the result: half a unit in the last
+place of the sum, towards zero, each time.  So what the error of a product grows with is the number of MMAs
+that go one after the other into one accumulator.  Over a chain of L of them the running sum of random
+products has 2/3 of its final size on average, a float is 0.72 of the next power of two, and the losses
+towards zero add up: at most 0.4 * L * 2^-24 of the result in the 2-norm, and the ordinary roundings beside
+them, 1.5 * 2^-24.
+
+`chain` is the longest chain the kernels may use at that shape: the depth of a block's run where the
+(row tile, segment) units of the tensor are dealt evenly to all places for a block, over two blocks per SM
+and four accumulators in turn (up to 16 rows), two (up to 32), one block per SM and one accumulator above."""
+import pytest
+
+from _util import torch_mod
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import aotx_b200
+    c = aotx_b200.Q8Context(0)
+    yield c
+    assert c.device_status() == 0
+    c.close()
+
+
+@pytest.mark.parametrize("n,k,m,chain", [(4096, 4096, 1, 8), (5000, 1024, 8, 4), (2048, 14336, 16, 28), (28672, 4096, 8, 40)])
+def test_error_of_the_sums(ctx, n, k, m, chain):
+    import aotx_b200
+    torch = torch_mod()
+    w = aotx_b200.synth_q8_0_device(n, k, n + m)
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)).half()
+    want = x.double() @ ctx.dequant(w, k, 0, n).double().T
+    off = ((ctx.matmul(w, n, k, x).double() - want).norm() / want.norm()).item()
+    assert off <= (1.5 + 0.4 * chain) * 2.0 ** -24
