@@ -384,10 +384,12 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     umma_commit(acc_full + 8u * buf);
                 }
             }
-            umma_commit(drain_bar);     // every MMA has finished: what the helping warps wait for
-            if (!ok) {
-                // Outstanding MMAs must finish before the tensor memory goes back.
+            if (total != 0u) {
+                // Every MMA has finished: what the helping warps wait for.  This thread waits as well, whoever
+                // else does: the arrival must not come to a shared memory that the block has left, nor may
+                // tensor memory go back under outstanding MMAs.  (A block without work issues none.)
                 uint32_t local_abort = 0;
+                umma_commit(drain_bar);
                 mbar_wait(drain_bar, 0u, &local_abort, nullptr);
             }
         }

@@ -456,9 +456,12 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     pair_commit(acc_full);
                 }
             }
-            pair_commit(drain_bar);     // every MMA has finished: what the helping warps wait for
-            if (!ok) {
+            if (total != 0u) {
+                // Every MMA has finished: what the helping warps of both blocks wait for.  This thread waits as
+                // well; a pair without work issues none, because nobody would wait for its arrivals, and they
+                // must not come to a shared memory that the blocks have left.
                 uint32_t local_abort = 0;
+                pair_commit(drain_bar);
                 mbar_wait(drain_bar, 0u, &local_abort, nullptr);
             }
         }
