@@ -17,6 +17,9 @@
 //     traffic, which at 64 rows was as many bytes as the weights.
 //   * 16 converter warps in two groups that take segments in turn (thread = row, half a segment).
 //   * The first copies of weights go out before anything else is set up.
+//   * No long chains of MMAs into one accumulator: each truncates the sum it adds to.  Two or four accumulators per
+//     value (`chains`), or, in a cluster, an accumulator that is emptied into a sum of its own every few segments
+//     (`run_segs`).  mid_accuracy says how many.
 //
 // 23 warps, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
 // status bit when it runs out.  Reference kernels replaced: as q8_stream.cu.
@@ -68,6 +71,12 @@ struct MidArgs {
     unsigned long long tile_floats;
     unsigned int x_stages, raw_stages, a_stages, acc_buffers;
     unsigned int raw_offset, raw_stride;
+    unsigned int chains;               // accumulators of a value, which parts of a segment take in turn: 1, 2 or 4
+    unsigned int run_segs;             // segments per run of a cluster's block, fewer than it has; 0: one run
+    // Columns of tensor memory: of one accumulator of a tile, of a buffer of `chains` of them (and of the sum of a
+    // cluster's runs so far, behind them); where the segments of A begin.
+    unsigned int acc_columns, buffer_columns, a_column0;
+    unsigned int read_chains;          // accumulators, and the sum of the runs, that make a finished sum
 };
 
 // A block's work: pieces of tiles, each the segments [s0, s1) of one tile.
@@ -75,6 +84,7 @@ struct MidWork {
     uint32_t tile, s0, s1;     // the piece
     uint32_t next_tile, next_seg, left, segs;
     uint32_t stride;           // from one tile of the block to the next
+    uint32_t most;             // segments per piece, at most
 
     __device__ __forceinline__ bool next()
     {
@@ -83,13 +93,62 @@ struct MidWork {
         }
         tile = next_tile;
         s0 = next_seg;
-        s1 = segs - s0 < left ? segs : s0 + left;
+        const uint32_t here = left < most ? left : most;
+        s1 = segs - s0 < here ? segs : s0 + here;
         left -= s1 - s0;
-        next_tile += stride;
-        next_seg = 0u;
+        next_seg = s1;
+        if (s1 == segs) {
+            next_tile += stride;
+            next_seg = 0u;
+        }
         return true;
     }
 };
+
+// The MMAs of one segment of A against one of x: `chains` accumulators, `stride` columns apart, which the segment's
+// four parts (64 deep) take in turn; `later`: not the first segment of its piece.
+__device__ __forceinline__ void multiply_segment(uint32_t d_tmem, uint32_t stride, uint32_t chains, uint32_t a_tmem, uint32_t x_seg,
+                                                 uint32_t x_seg_bytes, uint32_t idesc, bool later)
+{
+#pragma unroll
+    for (uint32_t j = 0; j < kSubs; ++j) {
+        const uint64_t b_desc = umma_desc_sw128(x_seg + j * (x_seg_bytes / kSubs));
+        const uint32_t d = d_tmem + (j & (chains - 1u)) * stride;
+#pragma unroll
+        for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
+            // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
+            umma_f16_ts(d, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
+                        kk != 0u || j >= chains || later ? 1u : 0u);
+        }
+    }
+}
+
+// The sums of all runs but the last (`turns` of them) of a cluster's block, added up behind the accumulators by the
+// storing warps; the readers at the end find them there.  (The MMAs of a run wait for what is done here with the
+// one before, which orders it for who waits for the MMAs.)  Out of line: few launches need it, and a short
+// launch fetches its code cold.
+__device__ __noinline__ void add_up_runs(uint32_t lane_taddr, uint32_t columns, uint32_t chains, uint32_t turns, uint32_t acc_full,
+                                         uint32_t acc_empty, volatile uint32_t *abort_flag, unsigned int *status)
+{
+    for (uint32_t turn = 0; turn < turns; ++turn) {
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(acc_full, turn & 1u, abort_flag, status))) {
+            return;
+        }
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (uint32_t c0 = 0; c0 < columns; c0 += 16u) {
+            uint32_t v[16];
+            load_sums(lane_taddr + c0, turn != 0u ? chains + 1u : chains, columns, v);
+            tmem_st_32x16(lane_taddr + chains * columns + c0, v);
+        }
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if ((threadIdx.x & 31u) == 0u) {
+            mbar_arrive(acc_empty);
+        }
+    }
+}
 
 // TWIN (grouped, pair 2): the second slab of a tile is the same rows of a second tensor, and what is stored is
 // the gated unit of the two.
@@ -147,6 +206,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     MidWork work;
     work.segs = segs;
     work.stride = 1u;
+    work.most = args.run_segs != 0u ? args.run_segs : segs;
     if (csize > 1u) {
         work.next_tile = blockIdx.x / csize;
         work.next_seg = crank * segs / csize;
@@ -237,7 +297,6 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot_ptr;
-    const uint32_t a_column0 = args.acc_buffers * pair * ntok;
 
     unsigned int m_live = args.m_max;
 
@@ -355,19 +414,11 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                             const bool wraps = xst + 1u == args.x_stages;
                             x_there = mbar_test_wait(x_full + 8u * (wraps ? 0u : xst + 1u), wraps ? xph ^ 1u : xph);
                         }
-                        const uint32_t d_tmem = tmem_base + (buf * pair + p) * ntok;
-                        const uint32_t a_tmem = tmem_base + a_column0 + ast * (kSegK / 2u);
+                        const uint32_t d_tmem = tmem_base + buf * args.buffer_columns + p * ntok;
+                        const uint32_t a_tmem = tmem_base + args.a_column0 + ast * (kSegK / 2u);
                         const uint32_t x_seg = smem0 + xst * x_seg_bytes;
-#pragma unroll
-                        for (uint32_t j = 0; j < kSubs; ++j) {
-                            const uint64_t b_desc = umma_desc_sw128(x_seg + j * (x_seg_bytes / kSubs));
-#pragma unroll
-                            for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
-                                // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
-                                umma_f16_ts(d_tmem, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
-                                            s != work.s0 || j != 0u || kk != 0u ? 1u : 0u);
-                            }
-                        }
+                        const bool later = s != work.s0;
+                        multiply_segment(d_tmem, args.acc_columns, args.chains, a_tmem, x_seg, x_seg_bytes, idesc, later);
                         umma_commit(a_empty + 8u * ast);
                         ast = anext;
                         aph = anext_ph;
@@ -404,7 +455,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         const uint32_t row = (cw & 3u) * 32u + lane;
         // rows past the slab repeat its last one (their sums are not stored)
         const uint32_t row_at = (row < args.slab_rows ? row : args.slab_rows - 1u) * kSegBytes;
-        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
+        const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + args.a_column0 + half * (kSegK / 4u);
         uint32_t full = group, fph = 0, ast = group, aph = 0;
         for (uint32_t g = group; g < total; g += kMidGroups) {
             if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
@@ -548,8 +599,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     const uint32_t c0 = piece * 16u;
                     const uint32_t slot = (p * ntok + c0) * kRows + lanes * 32u + lane;
                     uint32_t v[16];
-                    tmem_ld_32x16(lane_taddr + (buf * pair + p) * ntok + c0, v);
-                    tmem_ld_wait();
+                    load_sums(lane_taddr + buf * args.buffer_columns + p * ntok + c0, args.read_chains, args.acc_columns, v);
                     if (!owner) {
                         float *to = args.partial + (unsigned long long)blockIdx.x * args.tile_floats + slot;
 #pragma unroll
@@ -564,8 +614,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                     if (TWIN) {
                         // gate and up of the same columns lie in the two slabs' sums
                         uint32_t up[16];
-                        tmem_ld_32x16(lane_taddr + (buf * pair + 1u) * ntok + c0, up);
-                        tmem_ld_wait();
+                        load_sums(lane_taddr + buf * args.buffer_columns + ntok + c0, args.read_chains, args.acc_columns, up);
                         add_partial_sums(up, others + ntok * kRows, args.tile_floats, holders);
 #pragma unroll
                         for (uint32_t i = 0; i < 16u; ++i) {
@@ -623,9 +672,13 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // One pair of slabs per cluster.  The rows of x are dealt to its blocks in runs of `share`;
         // every block writes its part's sums into their owners' shared memory, over the rings, which are
         // idle by then: [sender][slab][run of four rows of x][row of w], 16 bytes at a time.  The owner adds the parts in block order.
+        if (args.run_segs != 0u && warp < kEpilogueWarps) {
+            add_up_runs(tmem_base + ((warp * 32u) << 16), args.acc_columns, args.chains, (work.left - 1u) / args.run_segs, acc_full,
+                        acc_empty, abort_flag, args.status);
+        }
         bool there = true;
         if (warp < kMidWeightWarp) {
-            there = mbar_wait(acc_full, 0u, abort_flag, args.status);
+            there = mbar_wait(drain_bar, 0u, abort_flag, args.status);
             tc_fence_after_sync();
         }
         const uint32_t share = ntok / csize;
@@ -641,8 +694,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 const uint32_t p = c / (ntok / 16u);
                 const uint32_t c0 = (c - p * (ntok / 16u)) * 16u;
                 uint32_t v[16];
-                tmem_ld_32x16(lane_taddr + p * ntok + c0, v);
-                tmem_ld_wait();
+                load_sums(lane_taddr + p * ntok + c0, args.read_chains, args.acc_columns, v);
 #pragma unroll
                 for (uint32_t i = 0; i < 16u; i += 4u) {
                     const uint32_t owner = (c0 + i) / share;
@@ -750,8 +802,12 @@ static cudaError_t launch_mid(cudaStream_t stream, const CUtensorMap &tw, const 
     // two segments of A.  (One piece: nothing to overlap its store with, and a third segment of A instead
     // is worth 4 %: 28672 x 4096, 64 rows, 31.9 -> 30.4 us; 4096 x 14336, 100 rows, 24.4 -> 23.5.)
     const bool one_piece = cluster > 1u || args.turns == 1u;
-    args.acc_buffers = !one_piece && 2u * args.pair * args.ntok <= 256u ? 2u : 1u;
-    const unsigned int a_stages = (512u - args.acc_buffers * args.pair * args.ntok) / (kSegK / 2u);
+    args.acc_columns = args.pair * args.ntok;
+    args.read_chains = args.chains + (args.run_segs != 0u ? 1u : 0u);
+    args.buffer_columns = args.read_chains * args.acc_columns;
+    args.acc_buffers = !one_piece && 2u * args.buffer_columns <= 256u ? 2u : 1u;
+    args.a_column0 = args.acc_buffers * args.buffer_columns;
+    const unsigned int a_stages = (512u - args.a_column0) / (kSegK / 2u);
     args.a_stages = a_stages < kMidMaxA ? a_stages : kMidMaxA;
     // Shared memory: up to four segments of x, as far as they leave about 100 KB to the weights (three
     // full slabs; 104 KB in flight per SM read memory at 6.8 TB/s), the rest to the weights.
@@ -813,6 +869,51 @@ static unsigned int clusters_of_four(unsigned int sm_count)
     return known[device];
 }
 
+// How the sums of a product are kept exact.  An MMA truncates the sum it adds to, so the error grows with the MMAs that
+// go into one accumulator one after the other.  The measure is the run of depth that a place for a block gets
+// where all (128 rows, segment) units are dealt evenly: `m` above 32 rows one place per SM, up to 32 two places
+// and two accumulators.  Blocks here get longer runs - all of a tile's depth, or a quarter or a half in a
+// cluster - and make up for it by accumulators in turn, as far as they leave two segments of A (256 columns),
+// or by runs.  4096 x 4096, 32 rows, 12.5e-7 of the result with one accumulator, 3.5e-7 so; 28672 x 4096, 32 rows,
+// 48.6e-7 and 12.6e-7; 512 x 16384, 64 rows, 48.6e-7 and 3.5e-7.  It costs a third segment of A or a second buffer
+// where those would fit, and the reads at the end: 28672 x 4096, 32 rows, 30.9 -> 31.8 us; 4096 x 14336, 100 rows,
+// 26.1 -> 27.9; in runs 300 x 16384, 128 rows, 30 -> 58.
+static void mid_accuracy(MidPlan &plan, unsigned int n, unsigned int segs, unsigned int sm_count)
+{
+    const unsigned int tiles = (n + kRows - 1u) / kRows;
+    const unsigned int acc_columns = plan.pair * plan.ntok;
+    plan.chains = 1u;
+    plan.run_segs = 0u;
+    if (plan.ntok <= 32u) {
+        // (units dealt to as many places as here, or clusters of four where there were four blocks: two)
+        plan.chains = plan.cluster == 4u && plan.pair == 2u ? 2u : 4u;
+        if (plan.cluster == 1u && plan.turns == 0u) {
+            plan.chains = 2u;
+        }
+        return;
+    }
+    if (plan.cluster > 1u) {
+        // (two slabs to a cluster: it has no more depth than an even share)
+        const unsigned int depth = (segs + plan.cluster - 1u) / plan.cluster;
+        if (plan.pair == 1u && depth > 1u && depth * sm_count > tiles * segs) {
+            if (depth * sm_count <= 2u * tiles * segs || depth == 2u) {
+                plan.chains = 2u;
+            } else {
+                plan.chains = plan.ntok <= 48u ? 4u : plan.ntok <= 80u ? 2u : 1u;
+                const unsigned int share = plan.chains * tiles * segs / sm_count;
+                plan.run_segs = share > plan.chains ? share : plan.chains;
+                const unsigned int least = segs / plan.cluster;        // 2 at least: the depth is above two
+                plan.run_segs = plan.run_segs < least ? plan.run_segs : least - 1u;
+            }
+        }
+        return;
+    }
+    // whole tiles in one or two turns: a third of them would be cut
+    if ((plan.turns == 1u || plan.turns == 2u) && 2u * acc_columns <= 256u) {
+        plan.chains = 2u;
+    }
+}
+
 MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
                  unsigned int epilogue)
 {
@@ -835,6 +936,7 @@ MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm
         const unsigned int used = (n + plan.slab_rows - 1u) / plan.slab_rows;
         plan.tiles = (used + plan.pair - 1u) / plan.pair;
         plan.grid = plan.tiles * plan.cluster;
+        mid_accuracy(plan, n, segs, sm_count);
         return plan;
     }
     plan.cluster = 1u;
@@ -853,6 +955,7 @@ MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm
         plan.tiles = (n + plan.pair * plan.slab_rows - 1u) / (plan.pair * plan.slab_rows);
         plan.grid = plan.tiles < sm_count ? plan.tiles : sm_count;
     }
+    mid_accuracy(plan, n, segs, sm_count);
     return plan;
 }
 
@@ -875,6 +978,8 @@ cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const
     args.pair = plan.pair;
     args.tiles = plan.tiles;
     args.turns = plan.turns;
+    args.chains = plan.chains;
+    args.run_segs = plan.run_segs;
     args.partial = partial;
     args.flags = flags;
     args.tile_floats = tile_floats;
@@ -903,6 +1008,7 @@ cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const
     args.ntok = ntok;
     args.slab_rows = kRows;
     args.pair = 2u;
+    args.chains = ntok <= 32u ? 2u : 1u;      // two buffers of them fit beside two segments of A
     return launch_mid(stream, tw, tw_second, tx, args, grid, 1u, overlap, y_dtype);
 }
 

@@ -7,6 +7,24 @@
 
 namespace q8 {
 
+// 16 columns of the sums at taddr: what the chains of accumulators, `stride` columns apart, hold together.
+__device__ __forceinline__ void load_sums(uint32_t taddr, uint32_t chains, uint32_t stride, uint32_t (&v)[16])
+{
+    tmem_ld_32x16(taddr, v);
+    tmem_ld_wait();
+#pragma unroll 1
+    for (uint32_t c = 1u; c < chains; ++c) {
+        uint32_t more[16];
+        taddr += stride;
+        tmem_ld_32x16(taddr, more);
+        tmem_ld_wait();
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+            v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(more[i]));
+        }
+    }
+}
+
 // Where finished sums go, and what becomes of them (the epilogue codes of q8_launch.h).
 struct RowStore {
     void *y;

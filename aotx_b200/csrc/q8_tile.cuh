@@ -648,6 +648,7 @@ cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const
 // 1: `turns` whole tiles per block, 0: units), and the launches.
 struct MidPlan {
     unsigned int ntok, slab_rows, pair, tiles, turns, cluster, grid;
+    unsigned int chains, run_segs; // see mid_accuracy in q8_mid.cu
 };
 MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
                  unsigned int epilogue);
