@@ -6,7 +6,7 @@
 //   17 .. 128     weights through tensor memory, one block per SM; also the       q8_mid.cu
 //                 grouped products of the routed experts
 //   129 ..        pairs of SMs, tiles of 256 rows of w by up to 256 of x; from    q8_pair.cu
-//                 113 rows on where w has rows for every block
+//                 65 or 113 rows on where w has rows for every block
 //
 // Where the lines lie: at 17 rows mma.sync would need a third column of eight and is bound by its
 // instructions at 32 (q8_decode_warp.cu); above 128 an accumulator of q8_mid.cu no longer fits
@@ -186,10 +186,16 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     const bool warp_kernel = ntok <= 16u && out == nullptr;
     // Above 112 rows q8_mid.cu has accumulators as wide as a pair's; with rows of w enough for every block a
     // pair of SMs, which reads half of x each, is then faster: 28672 x 4096, 128 rows, 42.0 -> 38.6 us,
-    // 151936 x 8192 359 -> 341 (100 rows: the same time; few rows of w: clusters, 24.1 against 26.1).
+    // 151936 x 8192 359 -> 341 (few rows of w: clusters, 24.1 against 26.1).  From 65 rows on where q8_mid.cu would
+    // take whole tiles in one or two turns: a pair has room for a second accumulator per value, which such tiles
+    // need (mid_accuracy), q8_mid.cu beside two slabs has not; 28672 x 4096, 100 rows, 36.8 us with one
+    // accumulator in q8_mid.cu, 37.0 with two in a pair.
+    MidPlan plan = {};
+    if (mid) {
+        plan = mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats, epilogue);
+    }
     const bool wide = ntok > 128u
-                   || (mid && m > 112u
-                       && mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats, epilogue).cluster == 1u);
+                   || (mid && plan.cluster == 1u && (m > 112u || (m > 64u && (plan.turns == 1u || plan.turns == 2u))));
     if (wide && out == nullptr && scratch.blocks >= sm_count && scratch.tile_floats >= 256ull * kRows
         && (unsigned long long)(n / (2u * kRows) + 1u) * (m / 128u + 1u) * (k / kSegK) < (1ull << 31)) {
         const unsigned int rows = pair_token_tile(m);
@@ -202,8 +208,6 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
                                   set_flags(scratch, set), scratch.tile_floats, scratch.status, overlap);
     }
     if (mid) {
-        const MidPlan plan = mid_plan(n, k, m, sm_count < scratch.blocks ? sm_count : scratch.blocks, scratch.tile_floats,
-                                      epilogue);
         CUtensorMap tw, tx;
         if (!map_weights(encode, &tw, w, n, k, plan.slab_rows) || !map_rows(encode, &tx, x, m, k, plan.ntok, false)) {
             return cudaErrorInvalidValue;

@@ -14,7 +14,7 @@
 //     into rows in shared memory (64 KB for the four warps), give the accumulator back and store
 //     from there beside the next tile.
 //   * The first tiles are dealt whole, one after the other to every pair; what is left for less than a turn of
-//     all pairs is cut into (tile, segment) units.  A cut tile is finished by the pair that holds its
+//     all pairs is cut (pair_deal in q8_schedule.cuh).  A cut tile is finished by the pair that holds its
 //     first segment, each block its own rows; that is a pair's last piece and all its warps store.
 //   * The tile's rows of x are the batch in equal parts of at most 256, rounded up to 32.
 //
@@ -26,6 +26,7 @@
 
 #include "q8_launch.h"
 #include "q8_rows.cuh"
+#include "q8_schedule.cuh"
 
 namespace q8 {
 
@@ -45,18 +46,6 @@ constexpr uint32_t kPairWarpStage = 16384;  // per storing warp: its 32 columns 
 constexpr uint32_t kPairTail = kEpilogueWarps * kPairWarpStage + kPairBars * 8 + 16;
 constexpr uint32_t kPairSmem = 227u * 1024u;
 constexpr uint32_t kPairRings = (kPairSmem - 1024u - kPairTail) / 1024u * 1024u;
-// What cutting a tile costs, in units (256 weights deep): the hand-over of the partial sums and the
-// stores at the end.
-constexpr uint32_t kPairCutUnits = 5;
-// A piece of a cut tile is worth this many units at least: every holder is a tile of sums more that the owner
-// reads back, about as long as a unit and a half takes.  Pieces of one size, whole fractions of a tile, go to as
-// many pairs as there are pieces, unless dealing the units evenly to all pairs makes the longest piece
-// kPairEvenUnits shorter.  Measured against dealing always: 19456 x 2560, 300 rows (four tiles of 10 units on 74
-// pairs: pieces of one unit) 43.5 -> 38.5 us; 2560 x 2560, 300 rows, 17.5 -> 15.0; 1000 x 2048, 200 rows,
-// 19.9 -> 14.8; 2560 x 9728, 300 rows (pieces of 10.3 units against thirds of 12.7) stays dealt: 26.2 against 26.9.
-constexpr uint32_t kPairMinPiece = 4;
-constexpr uint32_t kPairEvenUnits = 2;
-
 struct PairArgs {
     unsigned int n, k, m_max;
     const unsigned int *m_dev;
@@ -70,38 +59,9 @@ struct PairArgs {
     unsigned int x_stages, raw_stages;
 };
 
-// A pair's work: whole tiles `stride` apart, then a run of units.
-struct PairWork {
-    uint32_t tile, s0, s1;
-    uint32_t next_whole, whole_left, stride, segs;
-    uint32_t next_tile, next_seg, left;
-
-    __device__ __forceinline__ bool next()
-    {
-        if (whole_left != 0u) {
-            tile = next_whole;
-            s0 = 0u;
-            s1 = segs;
-            next_whole += stride;
-            whole_left -= 1u;
-            return true;
-        }
-        if (left == 0u) {
-            return false;
-        }
-        tile = next_tile;
-        s0 = next_seg;
-        s1 = segs - s0 < left ? segs : s0 + left;
-        left -= s1 - s0;
-        next_tile += 1u;
-        next_seg = 0u;
-        return true;
-    }
-    __device__ __forceinline__ bool last() const
-    {
-        return whole_left == 0u && left == 0u;
-    }
-};
+// Up to this many rows of x per tile a value has two accumulators, which successive pieces of x take in turn (an MMA
+// truncates the sum it adds to; q8_mid.cu says more).
+constexpr uint32_t kPairTwoChains = kPairTok / 2;
 
 // The sums of a whole tile's `rows` rows of x (accumulator columns) and this warp's 32 rows of w: into rows in the
 // warp's own shared memory, then - `release` is called in between - 16 bytes per lane to y.  Everything
@@ -110,7 +70,8 @@ struct PairWork {
 // value and the odd lane the second's.
 template <typename YT, bool GATED, typename Release>
 __device__ __forceinline__ void pair_drain(const RowStore &to, uint32_t stage, uint32_t lane_taddr, uint32_t lane,
-                                           uint32_t first_col, uint32_t first_row, uint32_t rows, Release release)
+                                           uint32_t chains, uint32_t first_col, uint32_t first_row, uint32_t rows,
+                                           Release release)
 {
     constexpr uint32_t kRowBytes = (GATED ? 16u : 32u) * sizeof(YT);
     constexpr uint32_t kRound = kPairWarpStage / kRowBytes < kPairTok ? kPairWarpStage / kRowBytes : kPairTok;
@@ -123,8 +84,7 @@ __device__ __forceinline__ void pair_drain(const RowStore &to, uint32_t stage, u
 #pragma unroll 1
         for (uint32_t c0 = 0; c0 < here; c0 += 16u) {
             uint32_t v[16];
-            tmem_ld_32x16(lane_taddr + base + c0, v);
-            tmem_ld_wait();
+            load_sums(lane_taddr + base + c0, chains, kPairTwoChains, v);
             const uint32_t at = stage + c0 * kRowBytes;
             if (GATED) {
 #pragma unroll
@@ -246,34 +206,9 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const uint32_t tok_tiles = (m + ntok - 1u) / ntok;
     const uint32_t pairs = gridDim.x / 2u;
     const uint32_t tiles = (args.n + 2u * kRows - 1u) / (2u * kRows) * tok_tiles;   // below 2^31 units: the host checks
-    uint32_t turns = tiles / pairs;
-    uint32_t cut = tiles - turns * pairs;
-    const uint32_t units = cut * segs;
     const uint32_t pair_id = blockIdx.x / 2u;
-    uint32_t sharers = units < pairs ? units : pairs;
-    if (cut != 0u && 2u * cut <= pairs) {
-        const uint32_t most = segs / kPairMinPiece > 1u ? segs / kPairMinPiece : 1u;
-        const uint32_t places = pairs / cut;
-        if (most <= places || (segs + places - 1u) / places <= units / pairs + kPairEvenUnits) {
-            sharers = cut * (most <= places ? most : places);
-        }
-    }
     PairWork work;
-    work.segs = segs;
-    work.stride = pairs;
-    work.next_whole = pair_id;
-    work.whole_left = turns;
-    work.next_tile = work.next_seg = work.left = 0u;
-    if (units != 0u && segs <= units / pairs + kPairCutUnits) {
-        work.whole_left += pair_id < cut ? 1u : 0u;               // cutting would cost more than it evens out
-    } else if (pair_id < sharers) {
-        uint32_t u_begin, u_end;
-        decode_range(pair_id, sharers, units, &u_begin, &u_end);
-        work.next_tile = turns * pairs + u_begin / segs;
-        work.next_seg = u_begin % segs;
-        work.left = u_end - u_begin;
-    }
-    const uint32_t first_cut = turns * pairs;
+    pair_deal(&work, pair_id, pairs, tiles, segs);
     const uint32_t total = work.whole_left * segs + work.left;    // segments of weights
 
     uint32_t early = 0u;
@@ -327,6 +262,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot_ptr;
     const uint32_t a_column0 = kPairTok;
+    const uint32_t chains = ntok <= kPairTwoChains ? 2u : 1u;
 
     if (warp == kPairWeightWarp) {
         // ---------------------------------------------------------------- weight copies
@@ -437,8 +373,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
                         for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
                             // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
-                            pair_mma_f16_ts(tmem_base, a_tmem + j * (kSubK / 2u) + 8u * kk, b_desc + 2u * kk, idesc,
-                                            s != work.s0 || j != 0u || kk != 0u ? 1u : 0u);
+                            pair_mma_f16_ts(tmem_base + (j & (chains - 1u)) * kPairTwoChains, a_tmem + j * (kSubK / 2u) + 8u * kk,
+                                            b_desc + 2u * kk, idesc, s != work.s0 || j >= chains || kk != 0u ? 1u : 0u);
                         }
                         pair_commit(x_empty + 8u * xst);
                         xst = xnext;
@@ -548,7 +484,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (owner && work.s1 != segs) {
                 // The other holders of this tile are the pairs right after this one; they met it at the start of
                 // their runs of units.
-                last_cc = decode_holder((work.tile - first_cut + 1u) * segs - 1u, sharers, units);
+                last_cc = pair_last_holder(work, pair_id, work.tile);
                 for (uint32_t base = pair_id + 1u; base <= last_cc; base += 32u) {
                     const uint32_t cc = base + lane;
                     if (cc <= last_cc) {
@@ -580,9 +516,9 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             };
             if (!last && owner && aligned16 && mine == 32u) {
                 if (gated) {
-                    pair_drain<YT, true>(args.to, stage, lane_taddr, lane, col, tok0, rows, release);
+                    pair_drain<YT, true>(args.to, stage, lane_taddr, lane, chains, col, tok0, rows, release);
                 } else {
-                    pair_drain<YT, false>(args.to, stage, lane_taddr, lane, col, tok0, rows, release);
+                    pair_drain<YT, false>(args.to, stage, lane_taddr, lane, chains, col, tok0, rows, release);
                 }
                 continue;
             }
@@ -592,8 +528,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             for (uint32_t c0 = helped ? helper * 16u : 0u; c0 < rows && mine != 0u; c0 += 16u * step) {
                 const uint32_t slot = c0 * kRows + lanes * 32u + lane;
                 uint32_t v[16];
-                tmem_ld_32x16(lane_taddr + c0, v);
-                tmem_ld_wait();
+                load_sums(lane_taddr + c0, chains, kPairTwoChains, v);
                 if (!owner) {
                     float *to = args.partial + (unsigned long long)blockIdx.x * args.tile_floats + slot;
 #pragma unroll

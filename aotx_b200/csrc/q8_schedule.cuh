@@ -1,0 +1,117 @@
+// The division of work between pairs of SMs (q8_pair.cu): which pieces - runs of segments of a tile - a pair works
+// on, and which others hold the rest of a tile that it finishes.  On the host as well, for the check of
+// tests/schedule_check.cu.
+#pragma once
+
+#include "q8_tile.cuh"
+
+namespace q8 {
+
+// A pair's work: whole tiles `stride` apart, then a run of units of the tiles that are cut.
+struct PairWork {
+    uint32_t tile, s0, s1;                  // the piece
+    uint32_t next_whole, whole_left, stride, segs;
+    uint32_t next_tile, next_seg, left;
+    uint32_t first_cut, units, sharers;     // the cut tiles: the first, their units, the pairs that share them
+    uint32_t pieces;                        // per cut tile; 0: the units are dealt evenly, whatever the tile
+
+    __host__ __device__ __forceinline__ bool next()
+    {
+        if (whole_left != 0u) {
+            tile = next_whole;
+            s0 = 0u;
+            s1 = segs;
+            next_whole += stride;
+            whole_left -= 1u;
+            return true;
+        }
+        if (left == 0u) {
+            return false;
+        }
+        tile = next_tile;
+        s0 = next_seg;
+        s1 = segs - s0 < left ? segs : s0 + left;
+        left -= s1 - s0;
+        next_tile += 1u;
+        next_seg = 0u;
+        return true;
+    }
+    __host__ __device__ __forceinline__ bool last() const
+    {
+        return whole_left == 0u && left == 0u;
+    }
+};
+
+// What cutting a tile costs, in units (256 weights deep): the hand-over of the partial sums and the stores at the
+// end.
+constexpr uint32_t kPairCutUnits = 5;
+// A piece of a cut tile is worth this many units at least: every holder is a tile of sums more that the owner
+// reads back, about as long as a unit and a half takes.
+constexpr uint32_t kPairMinPiece = 4;
+constexpr uint32_t kPairEvenUnits = 2;
+
+// The work of pair `id` of `pairs`.  As many turns of whole tiles as all pairs have; the tiles that are left:
+//   * Fewer than two turns: their units are dealt evenly.  Longer pieces are faster (2560 x 2560, 300 rows, 15.0 us
+//     in halves of a tile against 17.5; 1000 x 2048, 200 rows, 14.8 against 19.9), but the error of a sum grows with
+//     the depth that goes into one accumulator, and evenly dealt it is the smallest.
+//   * Behind more whole tiles, whose depth gives the error, what is faster: whole as well where cutting costs more
+//     than it evens out; else pieces of one size inside each tile, of kPairMinPiece units at least, as many as there
+//     are pairs for; else evenly dealt units, where that makes the longest piece kPairEvenUnits shorter (19456 x
+//     2560, 300 rows, four tiles of 10 units behind two turns: two pieces each 38.5 us, dealt evenly 43.5).
+__host__ __device__ __forceinline__ void pair_deal(PairWork *work, uint32_t id, uint32_t pairs, uint32_t tiles, uint32_t segs)
+{
+    const uint32_t turns = tiles / pairs;
+    const uint32_t cut = tiles - turns * pairs;
+    const uint32_t units = cut * segs;
+    work->segs = segs;
+    work->stride = pairs;
+    work->next_whole = id;
+    work->whole_left = turns;
+    work->next_tile = work->next_seg = work->left = 0u;
+    work->first_cut = turns * pairs;
+    work->units = units;
+    work->sharers = units < pairs ? units : pairs;
+    work->pieces = 0u;
+    if (cut == 0u) {
+        return;
+    }
+    if (turns > 1u) {
+        const uint32_t even = units / pairs;
+        if (segs <= even + kPairCutUnits) {
+            work->whole_left += id < cut ? 1u : 0u;
+            return;
+        }
+        const uint32_t places = pairs / cut;
+        const uint32_t most = segs / kPairMinPiece > 1u ? segs / kPairMinPiece : 1u;
+        const uint32_t pieces = most < places ? most : places;
+        if (pieces > 1u && (most <= places || (segs + pieces - 1u) / pieces <= even + kPairEvenUnits)) {
+            work->pieces = pieces;
+            work->sharers = cut * pieces;
+            if (id < work->sharers) {
+                const uint32_t i = id % pieces;
+                work->next_tile = work->first_cut + id / pieces;
+                work->next_seg = i * segs / pieces;
+                work->left = (i + 1u) * segs / pieces - work->next_seg;
+            }
+            return;
+        }
+    }
+    if (id < work->sharers) {
+        uint32_t begin, end;
+        decode_range(id, work->sharers, units, &begin, &end);
+        work->next_tile = work->first_cut + begin / segs;
+        work->next_seg = begin % segs;
+        work->left = end - begin;
+    }
+}
+
+// The last of the pairs right after `id` that hold later pieces of the cut tile whose first segment `id` holds.
+__host__ __device__ __forceinline__ uint32_t pair_last_holder(const PairWork &work, uint32_t id, uint32_t tile)
+{
+    if (work.pieces != 0u) {
+        return id + work.pieces - 1u;
+    }
+    return decode_holder((tile - work.first_cut + 1u) * work.segs - 1u, work.sharers, work.units);
+}
+
+} // namespace q8

@@ -11,7 +11,9 @@
 //      and they are the blocks directly after the owner;
 //   5. no block that takes part is without work;
 //   6. the decode kernel's own 32-bit range arithmetic (decode_range, decode_holder in
-//      q8_decode.cu) deals every unit once and names the block that holds a unit.
+//      q8_decode.cu) deals every unit once and names the block that holds a unit;
+//   7. the division between pairs of SMs (PairWork, pair_deal, pair_last_holder in q8_schedule.cuh) has the properties
+//      1 to 4, and where it cuts tiles into pieces of one size, each has kPairMinPiece segments at least.
 //
 // Prints "ok <cases>" and exits 0, or the first violated property and exits 1.
 #include <cstdio>
@@ -19,6 +21,7 @@
 #include <utility>
 #include <vector>
 
+#include "q8_schedule.cuh"
 #include "q8_tile.cuh"
 
 using namespace q8;
@@ -137,6 +140,66 @@ static int check_decode(uint32_t units, uint32_t blocks)
     return at == units ? 0 : fail("decode ranges stop short", units, 0u, blocks, 0u);
 }
 
+static int check_pairs(uint32_t tiles, uint32_t segs, uint32_t pairs)
+{
+    std::vector<unsigned int> seen((size_t)tiles * segs, 0u);
+    std::vector<std::vector<Piece>> pieces(pairs);
+    std::vector<PairWork> work(pairs);
+    for (uint32_t id = 0; id < pairs; ++id) {
+        pair_deal(&work[id], id, pairs, tiles, segs);
+        PairWork w = work[id];
+        while (w.next()) {
+            if (w.tile >= tiles || w.s0 >= w.s1 || w.s1 > segs) {
+                return fail("a pair's piece out of range", tiles, segs, pairs, id);
+            }
+            if (w.pieces != 0u && w.tile >= w.first_cut && w.s1 - w.s0 < kPairMinPiece) {
+                return fail("a piece shorter than the rule says", tiles, segs, pairs, id);
+            }
+            for (uint32_t s = w.s0; s < w.s1; ++s) {
+                seen[(size_t)w.tile * segs + s] += 1u;
+            }
+            pieces[id].push_back({w.tile, w.s0, w.s1});
+        }
+        if (!w.last()) {
+            return fail("a pair without pieces is not at its end", tiles, segs, pairs, id);
+        }
+    }
+    for (unsigned int count : seen) {
+        if (count != 1u) {
+            return fail("pairs: a unit is computed zero or several times", tiles, segs, pairs, 0u);
+        }
+    }
+    for (uint32_t id = 0; id < pairs; ++id) {
+        uint32_t published = 0u;
+        for (size_t i = 0; i < pieces[id].size(); ++i) {
+            const Piece &p = pieces[id][i];
+            if (p.s0 != 0u && ++published > 1u) {
+                return fail("a pair publishes twice", tiles, segs, pairs, id);
+            }
+            if (p.s0 == 0u && p.s1 != segs) {
+                if (i + 1u != pieces[id].size()) {
+                    return fail("a pair waits before its last piece", tiles, segs, pairs, id);
+                }
+                uint32_t at = p.s1;
+                for (uint32_t cc = id + 1u; cc <= pair_last_holder(work[id], id, p.tile); ++cc) {
+                    bool holds = false;
+                    for (const Piece &q : pieces[cc < pairs ? cc : id]) {
+                        holds = holds || (q.tile == p.tile && q.s0 == at);
+                        at = q.tile == p.tile && q.s0 == at ? q.s1 : at;
+                    }
+                    if (cc >= pairs || !holds) {
+                        return fail("a named pair does not continue the tile", tiles, segs, pairs, id);
+                    }
+                }
+                if (at != segs) {
+                    return fail("the named pairs do not finish the tile", tiles, segs, pairs, id);
+                }
+            }
+        }
+    }
+    return 0;
+}
+
 int main()
 {
     unsigned long long cases = 0;
@@ -181,6 +244,17 @@ int main()
                 return 1;
             }
             cases += 1;
+        }
+    }
+    for (uint32_t pairs : {1u, 2u, 9u, 66u, 74u}) {
+        for (uint32_t segs : {1u, 2u, 3u, 4u, 5u, 7u, 8u, 9u, 10u, 11u, 13u, 16u, 18u, 31u, 36u, 38u, 56u, 64u}) {
+            for (uint32_t tiles = 1; tiles <= 700; tiles += (tiles < 300 ? 1 : 7)) {
+                // (the launch has as many pairs as units, at most)
+                if (check_pairs(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0) {
+                    return 1;
+                }
+                cases += 1;
+            }
         }
     }
     std::printf("ok %llu\n", cases);

@@ -30,7 +30,9 @@ def ctx():
                                          # accumulators in turn: in clusters of four with one slab and with two, of two,
                                          # whole tiles in turns; runs, of one segment and of several
                                          (4096, 4096, 24, 16), (6144, 4096, 32, 32), (14336, 4096, 20, 44), (28672, 4096, 32, 77),
-                                         (4096, 4096, 48, 55), (512, 16384, 64, 28), (300, 4096, 128, 16), (2048, 14336, 100, 94)])
+                                         (4096, 4096, 48, 55), (512, 16384, 64, 28), (300, 4096, 128, 16), (2048, 14336, 100, 94),
+                                         # pairs of SMs: two accumulators; few tiles, whose units are dealt evenly
+                                         (20000, 4096, 100, 188), (5000, 1024, 160, 18), (2560, 2560, 300, 45), (1000, 2048, 200, 16)])
 def test_error_of_the_sums(ctx, n, k, m, chain):
     import aotx_b200
     torch = torch_mod()
