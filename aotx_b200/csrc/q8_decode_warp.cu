@@ -193,7 +193,7 @@ __device__ __forceinline__ void store_fragments(const UmmaArgs &args, uint32_t t
 
 template <int NTOK, bool BF, typename YT>
 __global__ void __launch_bounds__(kWarpThreads, 2)
-q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *__restrict__ x_any, const UmmaArgs args)
+q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *x_any, const UmmaArgs args)
 {
     using S = WarpShape<NTOK>;
     extern __shared__ unsigned char smem_raw_[];

@@ -73,11 +73,13 @@ unsigned int umma_token_tile(unsigned int m)
 }
 
 // x as binary16, 16 bytes a step (the conversion the kernels apply to an x tile in shared
-// memory: exact between 2^-14 and 65504, saturating above).
-__global__ void q8_x_to_f16_kernel(const uint4 *__restrict__ x, unsigned long long chunks, uint4 *__restrict__ out)
+// memory: exact between 2^-14 and 65504, saturating above).  No __restrict__ on x, here and in every kernel that
+// starts before the launch before it has ended: a read-only load wants data that does not change while
+// the kernel lives, and the wait below does not hold it back.
+__global__ void q8_x_to_f16_kernel(const uint4 *x, unsigned long long chunks, uint4 *out)
 {
-    grid_launch_dependents();
-    grid_dependency_wait();   // x, and the products that still read the copy
+    grid_launch_dependents();   // the product this is part of: nothing is written here that it reads before its own wait
+    grid_dependency_wait();     // x, and the products that still read the copy
     for (unsigned long long at = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; at < chunks;
          at += (unsigned long long)gridDim.x * blockDim.x) {
         uint4 v = x[at];

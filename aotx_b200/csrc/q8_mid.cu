@@ -640,7 +640,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         }
                         const uint32_t row_x = at.tok0 + c0 + i;
                         if (row_x < at.tok_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
-                            const uint32_t row_y = args.to.row_map != nullptr ? __ldg(args.to.row_map + row_x) : row_x;
+                            const uint32_t row_y = args.to.row_map != nullptr ? args.to.row_map[row_x] : row_x;
                             store_value<YT>(args.to, (size_t)row_y * args.to.ldy + col + (gated ? lane / 2u : lane), value);
                         }
                     }

@@ -277,13 +277,13 @@ cudaError_t launch_collect_ids(cudaStream_t stream, const unsigned int *const *i
 constexpr unsigned int kGroupAhead = 4;   // pairs per lane whose loads are issued together
 constexpr unsigned int kGroupRun = 1024;  // places of a block that are kept in shared memory as well
 
-__device__ __forceinline__ void group_load_ids(const unsigned int *__restrict__ ids, unsigned int first, unsigned int end,
+__device__ __forceinline__ void group_load_ids(const unsigned int *ids, unsigned int first, unsigned int end,
                                                unsigned int experts, unsigned int lane, unsigned int (&e)[kGroupAhead])
 {
 #pragma unroll
     for (unsigned int a = 0; a < kGroupAhead; ++a) {
         const unsigned int p = first + 32u * a + lane;
-        e[a] = p < end ? __ldg(ids + p) : 0xFFFFFFFFu;
+        e[a] = p < end ? ids[p] : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (unsigned int a = 0; a < kGroupAhead; ++a) {
@@ -313,7 +313,7 @@ __device__ __forceinline__ void group_write_tiles(GroupTile *__restrict__ tiles,
 }
 
 __global__ void __launch_bounds__(Q8_GROUP_THREADS, 1)
-q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned int *__restrict__ ids, unsigned int tokens_max,
+q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned int *ids, unsigned int tokens_max,
                        const unsigned int *tokens_dev, unsigned int used, unsigned int experts, unsigned int feed,
                        unsigned int hidden, unsigned int *sorted_pair, GroupTile *__restrict__ tiles_feed,
                        GroupTile *__restrict__ tiles_down, unsigned int *__restrict__ counts, unsigned int tile_tokens,
@@ -338,8 +338,8 @@ q8_group_build_kernel_many(const __grid_constant__ RowParts x, const unsigned in
         edge[1] = 0u;
     }
     __syncwarp();
-    grid_launch_dependents();
     grid_dependency_wait();
+    grid_launch_dependents();
     unsigned int tokens = tokens_max;
     if (tokens_dev != nullptr) {
         const unsigned int live = *tokens_dev;

@@ -142,7 +142,7 @@ __device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t s
         const uint32_t row_x = first_row + step * kRowsPerStep + lane / kLanesPerRow;
         at[step] = nullptr;
         if (row_x < row_limit && part * 4u < columns) {
-            const uint32_t row_y = to.row_map != nullptr ? __ldg(to.row_map + row_x) : row_x;
+            const uint32_t row_y = to.row_map != nullptr ? to.row_map[row_x] : row_x;
             at[step] = static_cast<YT *>(to.y) + (size_t)row_y * to.ldy + first_col + part * 4u;
         }
     }

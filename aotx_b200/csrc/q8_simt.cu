@@ -28,13 +28,15 @@ namespace q8 {
 // their way: a thread asks for four pieces before it turns the first.
 // ---------------------------------------------------------------------------------------
 template <unsigned int TOGETHER>
-__device__ __forceinline__ void dequant_body(const unsigned char *__restrict__ w, unsigned long long blocks,
+__device__ __forceinline__ void dequant_body(const unsigned char *w, unsigned long long blocks,
                                              __half *__restrict__ out, int wide_store)
 {
     const unsigned long long total = blocks * 4ull;
     const unsigned int step = blockDim.x;    // neighbouring threads, neighbouring pieces
-    grid_launch_dependents();
+    // The next launch starts after the wait: it may read its weights at once, and what was written two launches
+    // before it is there by then.
     grid_dependency_wait();
+    grid_launch_dependents();
     for (unsigned long long first = (unsigned long long)blockIdx.x * blockDim.x * TOGETHER + threadIdx.x;
          first < total; first += (unsigned long long)gridDim.x * blockDim.x * TOGETHER) {
         unsigned short scale[TOGETHER];
@@ -77,13 +79,13 @@ __device__ __forceinline__ void dequant_body(const unsigned char *__restrict__ w
 }
 
 #define Q8_DEQUANT_TOGETHER 4u
-__global__ void q8_dequant_kernel(const unsigned char *__restrict__ w, unsigned long long blocks,
+__global__ void q8_dequant_kernel(const unsigned char *w, unsigned long long blocks,
                                   __half *__restrict__ out, int wide_store)
 {
     dequant_body<1u>(w, blocks, out, wide_store);
 }
 
-__global__ void q8_dequant_kernel_many(const unsigned char *__restrict__ w, unsigned long long blocks,
+__global__ void q8_dequant_kernel_many(const unsigned char *w, unsigned long long blocks,
                                        __half *__restrict__ out, int wide_store)
 {
     dequant_body<Q8_DEQUANT_TOGETHER>(w, blocks, out, wide_store);
@@ -178,7 +180,7 @@ __device__ __forceinline__ void route_arrive()
 }
 
 template <unsigned int TOKENS, unsigned int EXPERTS, unsigned int AHEAD>
-__device__ __forceinline__ void route_body(const __half *__restrict__ x, const float *__restrict__ router,
+__device__ __forceinline__ void route_body(const __half *x, const float *router,
                                            unsigned int tokens_max, const unsigned int *tokens_dev,
                                            unsigned int hidden, unsigned int experts, unsigned int used,
                                            float *__restrict__ prob, unsigned int *__restrict__ ids, float *route_x,
@@ -410,14 +412,14 @@ __device__ __forceinline__ void route_body(const __half *__restrict__ x, const f
 
 #define Q8_ROUTE_KERNEL(NAME, TOKENS, EXPERTS, AHEAD)                                                               \
     __global__ void __launch_bounds__(Q8_ROUTE_GPU_THREADS, 2)                                                      \
-    NAME(const __half *__restrict__ x, const float *__restrict__ router, unsigned int tokens_max,                   \
+    NAME(const __half *x, const float *router, unsigned int tokens_max,                                             \
          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts, unsigned int used,              \
          float *__restrict__ prob, unsigned int *__restrict__ ids)                                                  \
     {                                                                                                               \
         Q8_ROUTE_DYNAMIC                                                                                            \
         __shared__ float probability[TOKENS][Q8_ROUTE_EXPERTS];                                                     \
-        grid_launch_dependents();                                                                                   \
         grid_dependency_wait();                                                                                     \
+        grid_launch_dependents();                                                                                   \
         route_body<TOKENS, EXPERTS, AHEAD>(x, router, tokens_max, tokens_dev, hidden, experts, used, prob, ids,     \
                                            route_x, probability);                                                   \
     }
@@ -519,14 +521,14 @@ q8_expert_down_kernel(const unsigned char *__restrict__ w_down, unsigned int hid
 // GPUs as shard_rows deals rows: the first `extra` of them one expert more), at the row of
 // the pair among all GPUs' pairs (first_pair + t * used + r).
 template <typename YT, unsigned int WIDTH>
-__global__ void q8_expert_sum_kernel(const __grid_constant__ ProjParts from, const float *__restrict__ prob,
-                                     const unsigned int *__restrict__ ids, unsigned int tokens_max,
+__global__ void q8_expert_sum_kernel(const __grid_constant__ ProjParts from, const float *prob,
+                                     const unsigned int *ids, unsigned int tokens_max,
                                      const unsigned int *tokens_dev, unsigned int hidden,
                                      unsigned int experts, unsigned int used, YT *__restrict__ out)
 {
     constexpr unsigned int kTogether = 8u;
-    grid_launch_dependents();
     grid_dependency_wait();
+    grid_launch_dependents();
     unsigned int tokens = tokens_max;
     if (tokens_dev != nullptr) {
         unsigned int live = *tokens_dev;

@@ -52,6 +52,12 @@ __device__ __forceinline__ void copy_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+// Ask for a line into L2.  It is a hint that reads nothing: a later write to the line is seen by later reads.
+__device__ __forceinline__ void prefetch_l2(const void *at)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(at) : "memory");
+}
+
 // An approximate reciprocal (within an ulp).
 __device__ __forceinline__ float rcp_approx(float v)
 {

@@ -62,3 +62,55 @@ def test_routed_steps_with_fewer_tiles_than_blocks(ctx):
         calls.append(lambda ids=ids, out=out, work=work: ctx.moe_ffn(wg, wu, wd, experts, hidden, ffn, x, prob, ids, out=out,
                                                                      workspace=work))
     in_turn_and_alone(ctx, calls)
+
+
+def test_results_that_the_next_launch_reads(ctx):
+    """Launches start before the one before them has ended and read its results: y of one product is x of the next, two
+    buffers in turn, through the kernels of every regime and of the other block types, the conversion of bfloat16 x,
+    the router and the routed step.  The same as with every launch by itself."""
+    import aotx_b200
+    import numpy as np
+    import _blocks
+    from _util import dev
+    torch = torch_mod()
+    k = 1024
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    q8 = [aotx_b200.synth_q8_0_device(k, k, s) for s in range(3)]
+    other = {t: dev(_blocks.random_rows(t, k, k, np.random.Generator(np.random.PCG64(t))).reshape(-1)) for t in (2, 12, 14)}
+    experts, used, ffn = 16, 2, 256
+    wg, wu = (aotx_b200.synth_q8_0_device(experts * ffn, k, s) for s in (4, 5))
+    wd = aotx_b200.synth_q8_0_device(experts * k, ffn, 6)
+    router = torch.randn(experts, k, device="cuda", generator=gen) / k ** 0.5
+    results = []
+    for m in (3, 12, 40, 200):
+        for kind in (torch.float16, torch.bfloat16):
+            start = torch.randn(m, k, device="cuda", generator=gen).to(kind)
+            a, b = torch.empty_like(start), torch.empty_like(start)
+            out = torch.empty(m, k, device="cuda")
+            work = ctx.moe_workspace(m, used, k, ffn)
+
+            def chain():
+                a.copy_(start)
+                ctx.matmul(q8[0], k, k, a, y=b)
+                ctx.matmul(other[2], k, k, b, y=a, type=2)
+                ctx.matmul(other[12], k, k, a, y=b, type=12)
+                ctx.matmul(q8[1], k, k, b, y=a)
+                ctx.set_path(1)
+                ctx.matmul(q8[2], k, k, a, y=b)
+                ctx.set_path(0)
+                ctx.matmul(other[14], k, k, b, y=a, type=14)
+                if kind == torch.float16:
+                    prob, ids = ctx.moe_route(a, router, used)
+                    ctx.moe_ffn(wg, wu, wd, experts, k, ffn, a, prob, ids, out=out, workspace=work)
+                    return a.clone(), out.clone()
+                return (a.clone(),)
+
+            ctx.set_overlap(False)
+            alone = chain()
+            torch.cuda.synchronize()
+            ctx.set_overlap(True)
+            for _ in range(10):
+                for got, want in zip(chain(), alone):
+                    assert torch.equal(got, want)
+            results.append(alone[0].float().abs().max().item())
+    assert all(0.0 < r < 60000.0 for r in results)      # nothing died away or left the range of binary16
