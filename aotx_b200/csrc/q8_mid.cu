@@ -636,7 +636,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         float value = __uint_as_float(v[i]);
                         if (gated) {
                             const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-                            value = value / (1.0f + expf(-value)) * other;
+                            value = gated_unit(value, other);
                         }
                         const uint32_t row_x = at.tok0 + c0 + i;
                         if (row_x < at.tok_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
@@ -738,7 +738,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 float sum = sums[i];
                 if (gated) {
                     const float up = __shfl_xor_sync(0xFFFFFFFFu, sum, 1u);
-                    sum = sum / (1.0f + expf(-sum)) * up;
+                    sum = gated_unit(sum, up);
                 }
                 if (token + i < m_live && row < args.slab_rows && j < args.n && (!gated || (row & 1u) == 0u)) {
                     store_value<YT>(args.to, (size_t)(token + i) * args.to.ldy + (gated ? j / 2u : j), sum);

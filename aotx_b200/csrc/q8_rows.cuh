@@ -50,15 +50,16 @@ __device__ __forceinline__ void row_words_present(const uint32_t (&raw)[36], uns
 // silu(gate) * up (cuda/model/norm.cu:92-105).  The quotient gate / (1 + e^-gate) by a reciprocal and one
 // correction of the quotient by its remainder (Markstein's division step) in place of the division
 // operator, whose branches kept a storing warp from working on several values at a time: 1300 cycles per
-// 8 values a lane, 16 x 32 sums, against 280 for a plain store.  The divisor is at least 1; where e^-gate
-// would overflow (gate below -88) it stays finite and its reciprocal is zero or tiny: the value is
-// then zero to within 1e-36.
+// 8 values a lane, 16 x 32 sums, against 280 for a plain store.  Where the step has no meaning - an infinite gate, a
+// divisor that overflows (gate below -88.7) - the remainder is NaN and the quotient stands as it is: infinite, or
+// zero, as the operator gives it.
 __device__ __forceinline__ float gated_unit(float gate, float up)
 {
-    const float divisor = 1.0f + expf(-fmaxf(gate, -88.0f));
+    const float divisor = 1.0f + expf(-gate);
     const float r = rcp_approx(divisor);
     const float quotient = gate * r;
-    return fmaf(fmaf(-quotient, divisor, gate), r, quotient) * up;
+    const float closer = fmaf(fmaf(-quotient, divisor, gate), r, quotient);
+    return (closer == closer ? closer : quotient) * up;
 }
 
 // The partial sums of one piece (16 rows of x by 32 rows of w) that other blocks have left in `slots` (one slot
