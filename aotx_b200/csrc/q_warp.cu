@@ -259,6 +259,31 @@ struct AnyArgs {
     uint32_t wide_x;               // x starts on a 16-byte boundary
 };
 
+// One product weight by weight by a warp, as the kernels on the ordinary cores form it (lanes take runs 32 apart, their
+// parts are added in a tree): what a sum in whole-number form is replaced by when it is not finite.  There s * q and
+// o of one weight meet x apart, so an infinite x can give NaN where the weight times x is infinite, and q * x can
+// leave the float range where s * q * x does not.
+template <uint32_t TYPE, bool BF>
+__device__ __noinline__ float sum_by_weights(const unsigned char *row, const unsigned short *x, uint32_t runs)
+{
+    float sum = 0.0f;
+#pragma unroll 1
+    for (uint32_t run = threadIdx.x & 31u; run < runs; run += 32u) {
+        float values[32];
+        decode_run(TYPE, row, run, values);
+#pragma unroll
+        for (uint32_t i = 0; i < 32u; ++i) {
+            const uint32_t bits = x[run * 32u + i];
+            sum = fmaf(values[i], BF ? __uint_as_float(bits << 16) : half_bits(bits), sum);
+        }
+    }
+#pragma unroll
+    for (uint32_t step = 16u; step != 0u; step >>= 1) {
+        sum += __shfl_down_sync(0xFFFFFFFFu, sum, step);
+    }
+    return __shfl_sync(0xFFFFFFFFu, sum, 0);
+}
+
 template <uint32_t TYPE, bool BF, uint32_t TILES>
 __global__ void __launch_bounds__(kAnyWarps * 32u, 2)
 q_gemv_any_kernel_warp(const AnyArgs args)
@@ -501,6 +526,16 @@ q_gemv_any_kernel_warp(const AnyArgs args)
                 sum += mine[v][at / kAnyRows][row];
             }
             const uint32_t j = group * kAnyRows + row;
+            uint32_t open = __ballot_sync(0xFFFFFFFFu, !(fabsf(sum) <= 3.402823466e38f) && token < m && j < args.n);
+            while (open != 0u) {
+                const uint32_t who = __ffs(open) - 1u;
+                open &= open - 1u;
+                const uint32_t its_row = __shfl_sync(0xFFFFFFFFu, j, who);
+                const uint32_t its_token = __shfl_sync(0xFFFFFFFFu, token, who);
+                const float again = sum_by_weights<TYPE, BF>(args.w + its_row * args.row_bytes,
+                                                             static_cast<const unsigned short *>(args.x) + (size_t)its_token * args.k, runs);
+                sum = lane == who ? again : sum;
+            }
             uint32_t columns = args.n;
             uint32_t column = j;
             bool writes = token < m && j < args.n;

@@ -1,7 +1,10 @@
-"""What becomes of values at the ends of the number range: gates far below and above zero, infinities."""
+"""What becomes of values at the ends of the number range: gates far below and above zero, infinities, sums that
+are finite though the sums of their whole-number form are not."""
+import numpy as np
 import pytest
 
-from _util import torch_mod
+import _blocks
+from _util import dev, torch_mod
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +61,34 @@ def test_gates_at_the_limits(ctx, n, m, path, kind):
         assert same_kind(got, want)
         fine = want.isfinite()
         assert bool(((got - want).abs() <= 2.0 ** -20 * want.abs() + 2.0 ** -120)[fine].all())
+
+
+@pytest.fixture(scope="module")
+def decoder(tmp_path_factory):
+    return _blocks.HostDecoder(tmp_path_factory.mktemp("decoder"))
+
+
+@pytest.mark.parametrize("type", [8, 2, 3, 6, 7, 12, 13, 14])
+@pytest.mark.parametrize("m", [4, 20])
+@pytest.mark.parametrize("kind", ["float16", "bfloat16"])
+def test_infinities_and_large_x(ctx, decoder, type, m, kind):
+    """A finite weight times an infinite x is infinite with the sign of the product (or, for a weight of zero, not a
+    number), and a sum that fits a float is finite, whatever the scales and offsets of the format."""
+    torch = torch_mod()
+    kind = getattr(torch, kind)
+    n, k = 70, 1024
+    w = _blocks.random_rows(type, n, k, np.random.Generator(np.random.PCG64(type)))
+    weights = torch.from_numpy(decoder.rows(type, w, n, k)).double().cuda()
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)).to(kind)
+    x[0, 5], x[1, 40], x[2, 300] = float("inf"), float("-inf"), float("nan")
+    if kind == torch.bfloat16:
+        x[3] = 0.0
+        x[3, 64:128] = 3e36       # whole numbers times it leave the float range
+    want = x.double() @ weights.T
+    ctx.set_path(1 if type == 8 else 0)
+    got = ctx.matmul(dev(w), n, k, x, type=type)
+    ctx.set_path(0)
+    assert same_kind(got, want.float())
+    fine = want.isfinite()
+    bound = (k + 8) * 2.0 ** -23 * 4.0 * (x.double().abs() @ weights.abs().amax(dim=1, keepdim=True).expand(n, k).T)
+    assert bool(((got.double() - want).abs() <= bound)[fine].all())
