@@ -26,7 +26,6 @@ namespace q8 {
 
 constexpr uint32_t kAnyWarps = 8;
 constexpr uint32_t kAnyRows = 16;
-constexpr uint32_t kAnyDepth = 4;      // pieces of a warp in flight or in use
 
 template <uint32_t TYPE>
 struct AnyShape {
@@ -48,8 +47,19 @@ struct AnyShape {
     static constexpr uint32_t units = (piece_bytes + 14 + 15) / 16;   // 16-byte units that can touch a piece
     static constexpr uint32_t slot = 16 * (units | 1u);          // 8 rows of a slot start 4 * odd words apart
     static constexpr uint32_t stage = kAnyRows * slot;
-    static constexpr uint32_t warp_bytes = kAnyDepth * stage;
+};
+
+// A warp's ring: four pieces in flight or in use, three where four would leave room for one block on an SM only (Q6_K,
+// and Q5_K at 16 rows of x: the grid below has two blocks per SM, which then ran one behind the other; Q6_K 14336 x
+// 4096, 4 rows, 25.8 us against 18.2, 16 rows, 36.4 against 30.0).
+template <uint32_t TYPE, uint32_t TILES>
+struct AnyRing {
+    static constexpr uint32_t sums_bytes = 2u * kAnyWarps * 8u * TILES * kAnyRows * 4u;
+    static constexpr uint32_t most_bytes = (228u * 1024u) / 2u - 1024u;      // two blocks' shared memory on one SM
+    static constexpr uint32_t depth = kAnyWarps * 4u * AnyShape<TYPE>::stage + sums_bytes <= most_bytes ? 4u : 3u;
+    static constexpr uint32_t warp_bytes = depth * AnyShape<TYPE>::stage;
     static constexpr uint32_t smem_bytes = kAnyWarps * warp_bytes;
+    static_assert(smem_bytes + sums_bytes <= most_bytes, "two blocks' shared memory on one SM");
 };
 
 // Four codes of 8 bits as the two operand words of an MMA step.  Codes are whole numbers below 64
@@ -289,6 +299,8 @@ __global__ void __launch_bounds__(kAnyWarps * 32u, 2)
 q_gemv_any_kernel_warp(const AnyArgs args)
 {
     using S = AnyShape<TYPE>;
+    using R = AnyRing<TYPE, TILES>;
+    constexpr uint32_t kAnyDepth = R::depth;
     constexpr bool kWide = any_wide<TYPE, TILES>();
     extern __shared__ __align__(16) unsigned char any_smem_[];
     __shared__ float parts[2][kAnyWarps][8u * TILES][kAnyRows];   // partial sums of the 8 warps, two row groups in turn
@@ -303,7 +315,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
     const uint32_t groups = (args.n + kAnyRows - 1u) / kAnyRows;
     const uint32_t my_groups = (groups - blockIdx.y + gridDim.y - 1u) / gridDim.y;
     const uint32_t items = my_groups * my_pieces;   // the host keeps this below 2^32
-    const uint32_t ring_at = smem_u32(any_smem_) + warp * S::warp_bytes;
+    const uint32_t ring_at = smem_u32(any_smem_) + warp * R::warp_bytes;
 
     // Item i of this warp: piece first_piece + i % my_pieces of the rows of group i / my_pieces.
     // Neighbouring lanes copy neighbouring 16-byte units of a row, then those of the next row.  (Two
@@ -437,7 +449,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
 #pragma unroll
             for (uint32_t r = 0; r < 2u; ++r) {
                 const uint32_t shift = (group_shift + r * eight_rows + piece * S::piece_bytes) & 15u;
-                const uint32_t at = warp * S::warp_bytes + (item % kAnyDepth) * S::stage + (g + 8u * r) * S::slot + shift;
+                const uint32_t at = warp * R::warp_bytes + (item % kAnyDepth) * S::stage + (g + 8u * r) * S::slot + shift;
                 rows[r].bytes = any_smem_ + at;
                 rows[r].words = reinterpret_cast<const uint32_t *>(any_smem_ + (at & ~3u));
                 rows[r].even = (at & 2u) != 0u ? 0x5432u : 0x3210u;
@@ -568,7 +580,7 @@ q_gemv_any_kernel_warp(const AnyArgs args)
 template <uint32_t TYPE, bool BF, uint32_t TILES>
 static cudaError_t launch_any_tiles(cudaStream_t stream, bool overlap, const AnyArgs &args)
 {
-    using S = AnyShape<TYPE>;
+    using S = AnyRing<TYPE, TILES>;
     static unsigned long long configured = 0ull;
     cudaError_t err = allow_shared_memory(q_gemv_any_kernel_warp<TYPE, BF, TILES>, S::smem_bytes, &configured, true);
     if (err != cudaSuccess) {
