@@ -699,10 +699,15 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     // row longer than 4096 no longer leave room for two blocks on an SM.  Latency bounds all three, so a
     // block has 16 warps of one or two experts each (measured against 8 warps of two or four; 128
     // experts, 2048 wide: 8 tokens 9.5 -> 7.2 us, 128 tokens 20.8 -> 13.0, 512 tokens 25.0 -> 22.6).
+    // Few experts leave most warps of such a cluster without work, and every block of it reads the group's
+    // activations: then a block takes all experts of four tokens by itself.  (Clusters, and one block for all: 8
+    // experts, 2048 wide, 512 tokens 15.4 us and 9.0, 4096 wide, 2048 tokens 160 and 24; 64 experts, 2048 wide, 512
+    // tokens 17.2 and 29.3, 2048 tokens 64.1 and 57.2, 8192 wide, 300 tokens 74.3 and 53.2.)
     const bool few = tokens <= 36u;
-    const bool many = !few && tokens > 148u && hidden <= 4096u;
+    const bool alone = tokens > 148u && experts <= 64u && (experts <= 16u || hidden > 4096u || tokens > 1024u);
+    const bool many = !few && !alone && tokens > 148u && hidden <= 4096u;
     const unsigned int group = few ? 2u : (many ? 8u : 4u);
-    const unsigned int cluster = many ? 4u : 8u;
+    const unsigned int cluster = alone ? 1u : (many ? 4u : 8u);
     const unsigned int stride = few ? RouteShape<2u>::stride : (many ? RouteShape<8u>::stride : RouteShape<4u>::stride);
     const size_t smem = (size_t)stride * hidden * sizeof(float);
     if (smem > 200u * 1024u) {

@@ -177,3 +177,24 @@ def test_grouped_path_equals_per_pair_path_at_full_size(ctx, oracle):
     counts = np.bincount(ids.cpu().numpy().reshape(-1), minlength=experts)
     assert counts.sum() == tokens * used and counts.max() > 32
     assert ctx.device_status() == 0
+
+
+# a block for all experts of four tokens: few experts, long rows, many tokens; beside each the clusters that share them
+@pytest.mark.parametrize("tokens,experts,hidden", [(149, 8, 512), (148, 8, 512), (301, 16, 2048), (150, 33, 4128), (1025, 64, 512),
+                                                   (1024, 64, 512), (2500, 3, 96)])
+def test_router_on_both_sides_of_the_line(tokens, experts, hidden):
+    import aotx_b200
+    torch = torch_mod()
+    ctx = aotx_b200.Q8Context(0)
+    used = min(experts, 3)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).half()
+    router = torch.randn(experts, hidden, device="cuda", generator=gen) / hidden ** 0.5
+    prob, ids = ctx.moe_route(x, router, used)
+    want = torch.softmax(x.double() @ router.double().T, dim=1)
+    # the logits' float sums, and a softmax of at most `experts` terms
+    slack = hidden * 2.0 ** -23 * (x.double().abs() @ router.double().abs().T).amax(dim=1, keepdim=True) * 2.0 + experts * 2.0 ** -23
+    assert bool(((prob.double() - want).abs() <= slack * want + 1e-30).all())
+    order = torch.sort(prob, dim=1, descending=True, stable=True)[1][:, :used]
+    assert torch.equal(ids.long(), order)
+    ctx.close()
