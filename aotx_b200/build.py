@@ -70,33 +70,6 @@ def resource_usage():
     return usage
 
 
-TRACE_LIB = os.path.join(HERE, "libaotx_q8_b200_trace.so")
-
-
-def build_trace():
-    """The library with -DQ8_TRACE: the decode kernel writes time stamps (block start, first x
-    segment landed, conversion done, accumulator ready, the two cluster barriers, end) that
-    aotx_b200/timeline.py reads back.  Never the product build; loaded instead of it when
-    AOTX_Q8_LIBRARY=trace (aotx_b200/library.py)."""
-    out = os.path.join(OBJ, "trace")
-    os.makedirs(out, exist_ok=True)
-    flags = [f for f in NVCC_FLAGS if f not in ("-Xptxas", "-v")] + ["-DQ8_TRACE"]
-
-    def one(src):
-        obj = os.path.join(out, os.path.splitext(src)[0] + ".o")
-        done = subprocess.run(["nvcc", *flags, "-c", os.path.join(CSRC, src), "-o", obj], capture_output=True,
-                              text=True)
-        if done.returncode != 0:
-            raise RuntimeError("nvcc failed for %s:\n%s" % (src, done.stderr))
-        return obj
-
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
-        objs = list(pool.map(one, SOURCES))
-    subprocess.run(["nvcc", "-shared", "-o", TRACE_LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a"],
-                   check=True)
-    return TRACE_LIB
-
-
 def build(verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
@@ -115,7 +88,4 @@ def build(verbose=False):
 
 
 if __name__ == "__main__":
-    if "--trace" in sys.argv:
-        print(build_trace())
-    else:
-        print(build(verbose="-v" in sys.argv))
+    print(build(verbose="-v" in sys.argv))

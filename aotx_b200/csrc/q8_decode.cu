@@ -92,17 +92,6 @@ struct DecodeShape {
                   "two accumulators, then the A pieces, in half of the tensor memory");
 };
 
-#ifdef Q8_TRACE
-#define Q8_STAMP(slot, cond)                                                         \
-    if (args.trace != nullptr && (cond)) {                                           \
-        unsigned long long t_;                                                       \
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));                       \
-        args.trace[blockIdx.x * 8u + (slot)] = t_;                                   \
-    }
-#else
-#define Q8_STAMP(slot, cond)
-#endif
-
 // The store with every option, once per kernel instance (see store_chunk in q8_tile.cuh).
 template <typename YT>
 static __device__ __noinline__ void store_eight_any(const UmmaArgs &args, const TilePlace &place, uint32_t lane_row,
@@ -321,7 +310,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
-    Q8_STAMP(0u, threadIdx.x == 0u)
 
     // The next kernel on the stream may start its blocks beside this one's.  Work that only
     // reads the weights runs ahead of the kernels before this one; everything that reads x or
@@ -428,7 +416,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         uint32_t issued = 0;
         if (elect_one()) {
             grid_dependency_wait();
-            Q8_STAMP(2u, true)                     // the launches before this one have finished
             for (; issued < total; ++issued) {
                 const uint32_t st = issued % S::x_depth;
                 const uint32_t ph = (issued / S::x_depth) & 1u;
@@ -478,7 +465,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                                    args.status)) {
                         ok = false;
                     }
-                    Q8_STAMP(1u, g == 0u)                   // the first x segment is ready
                     if (ok && s == s0 && !mbar_wait(r.acc_empty, aph ^ 1u, abort_flag, args.status)) {
                         ok = false;
                     }
@@ -541,7 +527,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 break;
             }
         }
-        Q8_STAMP(3u, cw == 0u && lane == 0u)       // conversion of the block's units done
     } else {
         // ---------------------------------------------------------------- read sums, store
         const uint32_t wq = warp;
@@ -672,7 +657,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             // the block's one piece: wait for its MMAs, the exchange below reads the accumulator
             mbar_wait(r.acc_full, 0u, abort_flag, args.status);
             tc_fence_after_sync();
-            Q8_STAMP(5u, wq == 0u && lane == 0u)
         }
     }
 
@@ -683,7 +667,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             tc_fence_after_sync();
             tmem_dealloc(tmem_base, S::tmem_columns);
         }
-        Q8_STAMP(7u, threadIdx.x == 0u)
         return;
     }
 
@@ -699,7 +682,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncwarp();
     cluster_arrive_release();
     cluster_wait_acquire();
-    Q8_STAMP(4u, threadIdx.x == 0u)
     const uint32_t lane_row = warp * 32u + lane;
     if (warp < kEpilogueWarps) {
         const uint32_t lane_taddr = tmem_base + ((warp * 32u) << 16);
@@ -730,7 +712,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncwarp();
     cluster_arrive_release();
     cluster_wait_acquire();
-    Q8_STAMP(6u, threadIdx.x == 0u)
     if (warp == kDecMmaWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, S::tmem_columns);
@@ -783,7 +764,6 @@ q8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             store_four<YT>(args, run, lane_row, j, first, 1u, sums);
         }
     }
-    Q8_STAMP(7u, threadIdx.x == 0u)
 }
 
 template <int NTOK, typename YT>
@@ -830,11 +810,6 @@ unsigned int decode_grid(unsigned int row_tiles, unsigned int segs, unsigned int
         // half as many blocks convert.)
         unsigned int pieces = 2u * sm_count / row_tiles;
         unsigned int most = kDecMaxCluster;
-#ifdef Q8_TRACE
-        if (getenv("Q8_ONE_PER_SM") != nullptr) {
-            pieces = sm_count / row_tiles;   // development builds: the other placement, for comparison
-        }
-#endif
         pieces = pieces > most ? most : pieces;
         pieces = pieces > segs ? segs : pieces;
         // a power of two: clusters of 6 took three times as long to be placed as clusters of 4 or 8

@@ -19,17 +19,11 @@
 // regime switch of cuda/model/graph_host.cu:20-40 and cuda/model/product.cu:24-49, which this
 // replaces with one launch per product.
 #include <cuda.h>
-#include <stdlib.h>
 
 #include "q8_launch.h"
 #include "q8_tile.cuh"
 
 namespace q8 {
-
-#ifdef Q8_TRACE
-static unsigned long long *g_trace_base = nullptr;
-static unsigned int g_trace_launches = 0;
-#endif
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
@@ -263,23 +257,7 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     args.status = scratch.status;
     args.tile_floats = scratch.tile_floats;
     args.b_bf16 = x_bf16 ? 1u : 0u;
-#ifdef Q8_TRACE
-    if (getenv("Q8_TRACE") != nullptr) {
-        // time stamps of the decode kernel: 8 words per block, 320 blocks, the last 256 launches
-        if (g_trace_base == nullptr) {
-            cudaMalloc((void **)&g_trace_base, 256ull * 320ull * 8ull * 8ull);
-            cudaMemset(g_trace_base, 0, 256ull * 320ull * 8ull * 8ull);
-        }
-        args.trace = g_trace_base + (unsigned long long)(g_trace_launches % 256u) * 320ull * 8ull;
-        g_trace_launches += 1;
-    }
-#endif
-#ifdef Q8_TRACE
-    const bool decode_kernel = getenv("Q8_DECODE") == nullptr || atoi(getenv("Q8_DECODE")) != 0;
-#else
-    const bool decode_kernel = true;
-#endif
-    if (ntok <= 32u && decode_kernel) {
+    if (ntok <= 32u) {
         // one token tile: the decode kernel, two blocks per SM (q8_decode.cu); its unit
         // arithmetic is 32-bit
         if (units >= (1ull << 31)) {
@@ -368,15 +346,3 @@ cudaError_t launch_umma_grouped(cudaStream_t stream, const UmmaScratch &scratch,
 }
 
 } // namespace q8
-
-#ifdef Q8_TRACE
-// The time stamps of the last 256 launches of the decode kernel ([launch][block][8] words) and the
-// number of launches so far (development builds only, see aotx_b200/timeline.py).
-extern "C" unsigned int q8_trace_read(unsigned long long *host)
-{
-    if (q8::g_trace_base != nullptr) {
-        cudaMemcpy(host, q8::g_trace_base, 256ull * 320ull * 8ull * 8ull, cudaMemcpyDeviceToHost);
-    }
-    return q8::g_trace_launches;
-}
-#endif

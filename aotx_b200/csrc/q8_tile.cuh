@@ -76,10 +76,6 @@ struct UmmaArgs {
     // Decode kernel (q8_decode.cu): nonzero when the launch is one cluster of blocks per weight
     // row tile, each block taking one run of the tile's segments; zero for the unit schedule.
     unsigned int split;
-#ifdef Q8_TRACE
-    // development builds (-DQ8_TRACE): time stamps of the decode kernel, 8 words per block, or null
-    unsigned long long *trace;
-#endif
 };
 
 // The units [begin, end) of block `b` out of `blocks`, of `units` in all.
