@@ -27,6 +27,7 @@
 
 #include "q8_launch.h"
 #include "q8_rows.cuh"
+#include "q8_schedule.cuh"
 
 namespace q8 {
 
@@ -77,32 +78,6 @@ struct MidArgs {
     // cluster's runs so far, behind them); where the segments of A begin.
     unsigned int acc_columns, buffer_columns, a_column0;
     unsigned int read_chains;          // accumulators, and the sum of the runs, that make a finished sum
-};
-
-// A block's work: pieces of tiles, each the segments [s0, s1) of one tile.
-struct MidWork {
-    uint32_t tile, s0, s1;     // the piece
-    uint32_t next_tile, next_seg, left, segs;
-    uint32_t stride;           // from one tile of the block to the next
-    uint32_t most;             // segments per piece, at most
-
-    __device__ __forceinline__ bool next()
-    {
-        if (left == 0u) {
-            return false;
-        }
-        tile = next_tile;
-        s0 = next_seg;
-        const uint32_t here = left < most ? left : most;
-        s1 = segs - s0 < here ? segs : s0 + here;
-        left -= s1 - s0;
-        next_seg = s1;
-        if (s1 == segs) {
-            next_tile += stride;
-            next_seg = 0u;
-        }
-        return true;
-    }
 };
 
 // The MMAs of one segment of A against one of x: `chains` accumulators, `stride` columns apart, which the segment's
@@ -203,39 +178,15 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t tiles = grouped ? *reinterpret_cast<const volatile unsigned int *>(args.group_count) / entries : args.tiles;
     const uint32_t units = tiles * segs;      // the host refuses products with 2^31 units or more
     const uint32_t blocks = units < gridDim.x ? units : gridDim.x;
-    MidWork work;
-    work.segs = segs;
-    work.stride = 1u;
-    work.most = args.run_segs != 0u ? args.run_segs : segs;
-    if (csize > 1u) {
-        work.next_tile = blockIdx.x / csize;
-        work.next_seg = crank * segs / csize;
-        work.left = (crank + 1u) * segs / csize - work.next_seg;
-    } else {
-        uint32_t turns = args.turns;
-        if (grouped) {
-            turns = (tiles + gridDim.x - 1u) / gridDim.x;
-            if (turns * segs > units / gridDim.x + kMidCutUnits) {
-                turns = 0u;
-            }
-        }
-        if (turns != 0u) {
-            // neighbouring blocks take neighbouring tiles, and where the last turn is not full its
-            // blocks have memory to themselves
-            work.next_tile = blockIdx.x;
-            work.next_seg = 0u;
-            work.stride = gridDim.x;
-            work.left = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * segs : 0u;
-        } else {
-            uint32_t u_begin = 0u, u_end = 0u;
-            if (blockIdx.x < blocks) {
-                decode_range(blockIdx.x, blocks, units, &u_begin, &u_end);
-            }
-            work.next_tile = u_begin / segs;
-            work.next_seg = u_begin - work.next_tile * segs;
-            work.left = u_end - u_begin;
+    uint32_t turns = args.turns;
+    if (grouped) {
+        turns = (tiles + gridDim.x - 1u) / gridDim.x;
+        if (turns * segs > units / gridDim.x + kMidCutUnits) {
+            turns = 0u;
         }
     }
+    MidWork work;
+    mid_deal(&work, blockIdx.x, gridDim.x, csize, crank, tiles, segs, turns, args.run_segs);
     const uint32_t total = work.left * pair;   // segments of weights
 
     grid_launch_dependents();

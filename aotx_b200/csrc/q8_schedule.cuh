@@ -1,11 +1,72 @@
-// The division of work between pairs of SMs (q8_pair.cu): which pieces - runs of segments of a tile - a pair works
-// on, and which others hold the rest of a tile that it finishes.  On the host as well, for the check of
-// tests/schedule_check.cu.
+// The division of work of the kernels on tensor memory (q8_mid.cu, q8_pair.cu): which pieces - runs of segments of
+// a tile - a block, or a pair of blocks, works on, and which others hold the rest of a tile that it finishes.
+// On the host as well, for the check of tests/schedule_check.cu.
 #pragma once
 
 #include "q8_tile.cuh"
 
 namespace q8 {
+
+// A block's work: pieces of tiles, each the segments [s0, s1) of one tile.
+struct MidWork {
+    uint32_t tile, s0, s1;     // the piece
+    uint32_t next_tile, next_seg, left, segs;
+    uint32_t stride;           // from one tile of the block to the next
+    uint32_t most;             // segments per piece, at most
+
+    __host__ __device__ __forceinline__ bool next()
+    {
+        if (left == 0u) {
+            return false;
+        }
+        tile = next_tile;
+        s0 = next_seg;
+        const uint32_t here = left < most ? left : most;
+        s1 = segs - s0 < here ? segs : s0 + here;
+        left -= s1 - s0;
+        next_seg = s1;
+        if (s1 == segs) {
+            next_tile += stride;
+            next_seg = 0u;
+        }
+        return true;
+    }
+};
+
+// The work of block `block` of `grid`.  Clusters (csize above one): one tile each, a run of its segments per block, in
+// pieces of at most run_segs (0: one piece).  Else whole tiles in `turns`, or (0) (tile, segment) units dealt evenly,
+// the same arithmetic as the decode kernel's; decode_holder names the block that holds a unit.
+__host__ __device__ __forceinline__ void mid_deal(MidWork *work, uint32_t block, uint32_t grid, uint32_t csize, uint32_t crank,
+                                                  uint32_t tiles, uint32_t segs, uint32_t turns, uint32_t run_segs)
+{
+    work->segs = segs;
+    work->stride = 1u;
+    work->most = run_segs != 0u ? run_segs : segs;
+    if (csize > 1u) {
+        work->next_tile = block / csize;
+        work->next_seg = crank * segs / csize;
+        work->left = (crank + 1u) * segs / csize - work->next_seg;
+        return;
+    }
+    if (turns != 0u) {
+        // neighbouring blocks take neighbouring tiles, and where the last turn is not full its
+        // blocks have memory to themselves
+        work->next_tile = block;
+        work->next_seg = 0u;
+        work->stride = grid;
+        work->left = block < tiles ? (tiles - block + grid - 1u) / grid * segs : 0u;
+        return;
+    }
+    const uint32_t units = tiles * segs;
+    const uint32_t blocks = units < grid ? units : grid;
+    uint32_t begin = 0u, end = 0u;
+    if (block < blocks) {
+        decode_range(block, blocks, units, &begin, &end);
+    }
+    work->next_tile = begin / segs;
+    work->next_seg = begin - work->next_tile * segs;
+    work->left = end - begin;
+}
 
 // A pair's work: whole tiles `stride` apart, then a run of units of the tiles that are cut.
 struct PairWork {

@@ -13,7 +13,9 @@
 //   6. the decode kernel's own 32-bit range arithmetic (decode_range, decode_holder in
 //      q8_decode.cu) deals every unit once and names the block that holds a unit;
 //   7. the division between pairs of SMs (PairWork, pair_deal, pair_last_holder in q8_schedule.cuh) has the properties
-//      1 to 4, and where it cuts tiles into pieces of one size, each has kPairMinPiece segments at least.
+//      1 to 4, and where it cuts tiles into pieces of one size, each has kPairMinPiece segments at least;
+//   8. the division between blocks and clusters (MidWork, mid_deal): every unit once, by the block that decode_holder
+//      names where units are dealt, the pieces of a cluster's block within run_segs and in one tile.
 //
 // Prints "ok <cases>" and exits 0, or the first violated property and exits 1.
 #include <cstdio>
@@ -200,6 +202,51 @@ static int check_pairs(uint32_t tiles, uint32_t segs, uint32_t pairs)
     return 0;
 }
 
+// `way`: 0 units, 1 whole tiles in turns, 2 and 4 clusters of that size.
+static int check_mid(uint32_t tiles, uint32_t segs, uint32_t grid, uint32_t way, uint32_t run_segs)
+{
+    const uint32_t csize = way >= 2u ? way : 1u;
+    if (csize > 1u) {
+        if (segs < csize) {
+            return 0;
+        }
+        grid = tiles * csize;
+    }
+    const uint32_t units = tiles * segs;
+    const uint32_t blocks = units < grid ? units : grid;
+    std::vector<unsigned int> seen((size_t)units, 0u);
+    for (uint32_t b = 0; b < grid; ++b) {
+        MidWork w;
+        mid_deal(&w, b, grid, csize, b % csize, tiles, segs, way == 1u ? (tiles + grid - 1u) / grid : 0u, csize > 1u ? run_segs : 0u);
+        while (w.next()) {
+            if (w.tile >= tiles || w.s0 >= w.s1 || w.s1 > segs) {
+                return fail("a block's piece out of range", tiles, segs, grid, b);
+            }
+            if (csize > 1u && (w.tile != b / csize || (run_segs != 0u && w.s1 - w.s0 > run_segs))) {
+                return fail("a cluster's piece in another tile or too long", tiles, segs, grid, b);
+            }
+            if (way == 1u && (w.s0 != 0u || w.s1 != segs)) {
+                return fail("a cut tile in turns", tiles, segs, grid, b);
+            }
+            for (uint32_t s = w.s0; s < w.s1; ++s) {
+                seen[(size_t)w.tile * segs + s] += 1u;
+                if (way == 0u && decode_holder(w.tile * segs + s, blocks, units) != b) {
+                    return fail("decode_holder names another block of the units", tiles, segs, grid, b);
+                }
+            }
+        }
+        if (w.left != 0u) {
+            return fail("a block's work has no end", tiles, segs, grid, b);
+        }
+    }
+    for (unsigned int count : seen) {
+        if (count != 1u) {
+            return fail("blocks: a unit is computed zero or several times", tiles, segs, grid, way);
+        }
+    }
+    return 0;
+}
+
 int main()
 {
     unsigned long long cases = 0;
@@ -244,6 +291,18 @@ int main()
                 return 1;
             }
             cases += 1;
+        }
+    }
+    for (uint32_t way : {0u, 1u, 2u, 4u}) {
+        for (uint32_t run_segs : {0u, 1u, 3u}) {
+            for (uint32_t segs : {1u, 2u, 3u, 5u, 8u, 11u, 16u, 56u, 64u}) {
+                for (uint32_t tiles = 1; tiles <= 600; tiles += (tiles < 40 ? 1 : 17)) {
+                    if (check_mid(tiles, segs, 148u, way, run_segs) != 0 || check_mid(tiles, segs, 7u, way, run_segs) != 0) {
+                        return 1;
+                    }
+                    cases += 2;
+                }
+            }
         }
     }
     for (uint32_t pairs : {1u, 2u, 9u, 66u, 74u}) {
