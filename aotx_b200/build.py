@@ -43,29 +43,32 @@ def _compile(src):
 
 
 def resource_usage():
-    """{kernel name (mangled): {"registers": r, "spill_stores": s, "spill_loads": l, "stack": b}}
-    from the ptxas reports kept beside the objects (build() first)."""
+    """{kernel or out-of-line function (mangled): {"registers": r (kernels only), "spill_stores": s,
+    "spill_loads": l, "stack": b}} from the ptxas reports kept beside the objects (build() first)."""
     import re
     usage = {}
     for src in SOURCES:
         log = os.path.join(OBJ, os.path.splitext(src)[0] + ".o.ptxas.log")
         if not os.path.exists(log):
             continue
-        name = None
+        name = None      # the kernel that is being compiled
+        about = None     # the function that the next frame and spills belong to
         for line in open(log):
             found = re.search(r"Compiling entry function '([^']+)'", line)
             if found:
                 name = found.group(1)
                 usage[name] = {}
                 continue
-            if name is None:
+            found = re.search(r"Function properties for (\S+)", line)
+            if found:
+                about = found.group(1)
                 continue
             found = re.search(r"(\d+) bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads", line)
-            if found:
-                usage[name].update(stack=int(found.group(1)), spill_stores=int(found.group(2)),
-                                   spill_loads=int(found.group(3)))
+            if found and about is not None:
+                usage.setdefault(about, {}).update(stack=int(found.group(1)), spill_stores=int(found.group(2)),
+                                                   spill_loads=int(found.group(3)))
             found = re.search(r"Used (\d+) registers", line)
-            if found:
+            if found and name is not None:
                 usage[name]["registers"] = int(found.group(1))
     return usage
 
