@@ -10,6 +10,10 @@
 
 namespace q8 {
 
+// SMs of the GPU this library is built for (B200), where a grid or a line between two kernels is chosen without a
+// context at hand; a count that is off costs time, not results.
+constexpr unsigned int kSmCount = 148u;
+
 // Every kernel of the library is launched through this one function (or, for the tensor-core
 // kernels with their launch attributes, through launch_tile_kernel in q8_tile.cuh).  In the
 // tests' host emulation (-DQ8_HOST_EMULATION: the kernels compiled as host code) the same call

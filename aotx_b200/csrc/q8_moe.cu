@@ -18,7 +18,6 @@ namespace q8 {
 
 #define Q8_GROUP_THREADS 1024u
 #define Q8_GROUP_MAX_EXPERTS 256u
-#define Q8_GROUP_TOKENS_MAX 64u /* largest token tile of the grouped products */
 
 #ifndef Q8_GROUP_TOKENS
 #define Q8_GROUP_TOKENS 64u /* token tile of the grouped products */

@@ -21,7 +21,7 @@
 // 23 warps per block, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 of the
 // first block issues the MMAs.  Every wait is bounded and raises a status bit when it runs out.
 // Measured against q8_wide.cu: gate+up 28672 x 4096, 2048 rows, bfloat16, 489 -> 350 us (1377 TFLOP/s); the
-// fused layer of 2560 by 9728, 300 rows, 365 -> 116 us.  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
+// fused layer of 2560 by 9728, 300 rows, 365 -> 120 us.  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
 #include <cuda.h>
 
 #include "q8_launch.h"

@@ -2,9 +2,9 @@
 // any-shape product (depth any multiple of 32, any alignment the block layout allows), the
 // expert router, the per-pair expert products and the ordered expert sum.
 //
-// The streaming tensor-core kernel in q8_umma.cu takes the shapes it supports (depth a
-// multiple of 256, 16-byte aligned rows); the product here serves every other shape, so
-// that the library covers the whole contract of the reference's kernels:
+// The kernels behind q8_dispatch.cu take products with a depth of a multiple of 256 and 16-byte
+// aligned rows, q_warp.cu the others with x on an 8-byte boundary; the product here serves what is
+// left, so that the library covers the whole contract of the reference's kernels:
 //   cuda/model/dequant.cu:9-70      -> q8_dequant_kernel
 //   cuda/model/gemv.cuh:33-145      -> q8_gemv_simt_kernel
 //   cuda/model/experts.cu:10-75     -> q8_route_kernel
@@ -619,7 +619,7 @@ cudaError_t launch_dequant(cudaStream_t stream, const void *w, unsigned int k, u
     // 14336 x 4096 38.1 -> 32.9 us (5.5 TB/s), 20000 x 8192 104 -> 86.  (Blocks that come back for more, the
     // grid's width further on, keep as much in flight and take 39 us.)
     const unsigned long long many = (pieces + 256ull * Q8_DEQUANT_TOGETHER - 1ull) / (256ull * Q8_DEQUANT_TOGETHER);
-    if (many >= 4ull * 148ull) {
+    if (many >= 4ull * (unsigned long long)kSmCount) {
         const unsigned int grid = (unsigned int)(many < (1ull << 30) ? many : (1ull << 30));
         return launch_kernel_early(overlap, q8_dequant_kernel_many, grid, 256, 0, stream, base, blocks,
                                    static_cast<__half *>(out), wide);
@@ -634,7 +634,7 @@ static cudaError_t launch_gemv_simt_typed(cudaStream_t stream, const void *w, un
                                           const unsigned int *m_dev, void *y, unsigned int epilogue)
 {
     unsigned int want = (n + Q8_SIMT_WARPS - 1u) / Q8_SIMT_WARPS;
-    unsigned int grid = want < 148u * 8u ? want : 148u * 8u;
+    unsigned int grid = want < kSmCount * 8u ? want : kSmCount * 8u;
     if (epilogue == kEpilogueStore) {
         return launch_kernel(q8_gemv_simt_kernel<XT, YT>, grid, Q8_SIMT_WARPS * 32u, 0, stream,
                              static_cast<const unsigned char *>(w), n, k, static_cast<const XT *>(x), m, m_dev,
@@ -704,8 +704,8 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     // experts, 2048 wide, 512 tokens 15.4 us and 9.0, 4096 wide, 2048 tokens 160 and 24; 64 experts, 2048 wide, 512
     // tokens 17.2 and 29.3, 2048 tokens 64.1 and 57.2, 8192 wide, 300 tokens 74.3 and 53.2.)
     const bool few = tokens <= 36u;
-    const bool alone = tokens > 148u && experts <= 64u && (experts <= 16u || hidden > 4096u || tokens > 1024u);
-    const bool many = !few && !alone && tokens > 148u && hidden <= 4096u;
+    const bool alone = tokens > kSmCount && experts <= 64u && (experts <= 16u || hidden > 4096u || tokens > 1024u);
+    const bool many = !few && !alone && tokens > kSmCount && hidden <= 4096u;
     const unsigned int group = few ? 2u : (many ? 8u : 4u);
     const unsigned int cluster = alone ? 1u : (many ? 4u : 8u);
     const unsigned int stride = few ? RouteShape<2u>::stride : (many ? RouteShape<8u>::stride : RouteShape<4u>::stride);
@@ -714,7 +714,7 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
         return cudaErrorInvalidValue;
     }
     unsigned int clusters = (tokens + group - 1u) / group;
-    const unsigned int most = 148u * 4u / cluster;
+    const unsigned int most = kSmCount * 4u / cluster;
     clusters = clusters < most ? clusters : most;
     static unsigned long long configured[3] = {0ull, 0ull, 0ull};
     void (*const kernels[3])(const __half *, const float *, unsigned int, const unsigned int *, unsigned int, unsigned int,
@@ -779,7 +779,7 @@ static cudaError_t expert_sum_launch(bool overlap, bool wide, cudaStream_t strea
     // a block per part of a token's row (see the kernel), eight blocks per SM at most
     const unsigned int step = 256u * (wide ? 4u : 1u);
     const unsigned long long items = (unsigned long long)tokens * ((hidden + step - 1u) / step);
-    const unsigned int grid = items < 148u * 8u ? (unsigned int)items : 148u * 8u;
+    const unsigned int grid = items < kSmCount * 8u ? (unsigned int)items : kSmCount * 8u;
     if (wide) {
         return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 4u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
                              hidden, experts, used, static_cast<YT *>(out));

@@ -591,7 +591,7 @@ static cudaError_t launch_any_tiles(cudaStream_t stream, bool overlap, const Any
     // Two blocks per SM where the rows are enough for it, some with a group more than others.  (As few blocks as
     // give all the same number of groups leave half of the SMs with one block: 14336 rows, 896 groups: 224
     // blocks of four against 296 of three or four.)
-    const uint32_t wave = (2u * 148u + passes - 1u) / passes;
+    const uint32_t wave = (2u * kSmCount + passes - 1u) / passes;
     const uint32_t blocks = groups < wave ? groups : wave;
     return launch_kernel_early(overlap, q_gemv_any_kernel_warp<TYPE, BF, TILES>, dim3(passes, blocks), kAnyWarps * 32u, S::smem_bytes,
                          stream, args);

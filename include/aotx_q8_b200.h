@@ -12,9 +12,9 @@
  * 8 (Q8_0) is the path this library is built for: every entry point takes it, on the
  * tensor-core kernels where the shape allows.  aotx_q8_dequant and aotx_q8_matmul also take the
  * other types the reference's kernels read - F32 0, F16 1, Q4_0 2, Q4_1 3, Q5_0 6, Q5_1 7,
- * Q2_K 10, Q3_K 11, Q4_K 12, Q5_K 13, Q6_K 14 - through one decoder on the ordinary cores (rows
- * of whole blocks: k a multiple of 32, of 256 for the K types); any other id is
- * AOTX_Q8_ERR_TYPE.
+ * Q2_K 10, Q3_K 11, Q4_K 12, Q5_K 13, Q6_K 14 - rows of whole blocks: k a multiple of 32, of 256
+ * for the K types; products of Q4_0, Q4_1, Q5_0, Q5_1, Q4_K, Q5_K and Q6_K on the warp-level tensor
+ * path, the others and dequantisation on the ordinary cores; any other id is AOTX_Q8_ERR_TYPE.
  *
  * Return value: 0 on success, one of the AOTX_Q8_ERR_* codes otherwise.  On an error nothing
  * is enqueued and no output is written (the reference's kernels likewise write nothing for a
@@ -55,7 +55,7 @@ extern "C" {
 
 /* kernel family, for aotx_q8_set_path */
 #define AOTX_Q8_PATH_AUTO 0    /* tensor-core streaming kernel where it applies, else general */
-#define AOTX_Q8_PATH_GENERAL 1 /* the any-shape kernel on the ordinary cores */
+#define AOTX_Q8_PATH_GENERAL 1 /* the any-shape kernels, no k % 256, no alignment asked for */
 #define AOTX_Q8_PATH_TENSOR 2  /* the tcgen05 streaming kernel; ERR_UNSUPPORTED if it cannot run */
 
 /* what a product does with a finished sum, for aotx_q8_matmul_fused */
@@ -84,7 +84,10 @@ int aotx_q8_set_path(aotx_q8_ctx *ctx, int path);
  * bytes, while the work before it on the stream is still finishing; they wait for that work
  * before they read x or the live batch or write y.  The weight tensor itself must therefore
  * not be written by the operation just before the product on the same stream; switch the
- * overlap off around such a sequence.  No counterpart in the reference. */
+ * overlap off around such a sequence.  This holds for the Q8_0 products with k a multiple of
+ * 256 and the routed experts; the any-shape products, the other block types and dequantisation
+ * start early too, but read nothing before the work before them has finished.
+ * No counterpart in the reference. */
 int aotx_q8_set_overlap(aotx_q8_ctx *ctx, int enabled);
 
 /* The last CUDA error code an entry point of this context saw (cudaError_t as int). */
