@@ -192,7 +192,7 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     }
     const bool wide = ntok > 128u
                    || (mid && plan.cluster == 1u && (m > 112u || (m > 64u && (plan.turns == 1u || plan.turns == 2u))));
-    if (wide && out == nullptr && scratch.blocks >= sm_count && scratch.tile_floats >= 256ull * kRows
+    if (wide && out == nullptr && scratch.blocks >= 2u * sm_count && scratch.tile_floats >= 256ull * kRows
         && (unsigned long long)(n / (2u * kRows) + 1u) * (m / 128u + 1u) * (k / kSegK) < (1ull << 31)) {
         const unsigned int rows = pair_token_tile(m);
         CUtensorMap tw, tx;

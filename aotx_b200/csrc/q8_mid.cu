@@ -582,19 +582,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         }
                         continue;
                     }
-#pragma unroll
-                    for (uint32_t i = 0; i < 16u; ++i) {
-                        float value = __uint_as_float(v[i]);
-                        if (gated) {
-                            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-                            value = gated_unit(value, other);
-                        }
-                        const uint32_t row_x = at.tok0 + c0 + i;
-                        if (row_x < at.tok_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
-                            const uint32_t row_y = args.to.row_map != nullptr ? args.to.row_map[row_x] : row_x;
-                            store_value<YT>(args.to, (size_t)row_y * args.to.ldy + col + (gated ? lane / 2u : lane), value);
-                        }
-                    }
+                    store_rows_direct<YT>(args.to, gated, lane, mine, col, at.tok0 + c0, at.tok_limit, v);
                 }
                 piece -= live;
             }

@@ -14,14 +14,17 @@
 //     into rows in shared memory (64 KB for the four warps), give the accumulator back and store
 //     from there beside the next tile.
 //   * The first tiles are dealt whole, one after the other to every pair; what is left for less than a turn of
-//     all pairs is cut (pair_deal in q8_schedule.cuh).  A cut tile is finished by the pair that holds its
-//     first segment, each block its own rows; that is a pair's last piece and all its warps store.
+//     all pairs is cut (pair_split in q8_schedule.cuh).  A cut tile is finished by the pair that holds its
+//     first segment, each block its own rows (that is a pair's last piece and all its warps store), or by all of its
+//     holders, each a run of its rows of x (kPairShareMore says when).
+//   * The first weights are on their way before the live batch is known; the accumulator goes back before a part of a
+//     cut tile is published.
 //   * The tile's rows of x are the batch in equal parts of at most 256, rounded up to 32.
 //
 // 23 warps per block, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 of the
 // first block issues the MMAs.  Every wait is bounded and raises a status bit when it runs out.
 // Measured against q8_wide.cu: gate+up 28672 x 4096, 2048 rows, bfloat16, 489 -> 350 us (1377 TFLOP/s); the
-// fused layer of 2560 by 9728, 300 rows, 365 -> 120 us.  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
+// fused layer of 2560 by 9728, 300 rows, 365 -> 112 us (120 before the two points above).  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
 #include <cuda.h>
 
 #include "q8_launch.h"
@@ -41,9 +44,10 @@ constexpr uint32_t kPairMaxRaw = 4;
 constexpr uint32_t kPairMaxX = 8;
 constexpr uint32_t kPairAStages = 2;
 constexpr uint32_t kPairAColumns = kSegK / 2;
-constexpr uint32_t kPairBars = 3 * kPairMaxRaw + 2 * kPairMaxX + 2 * kPairAStages + 2 + 1;
+constexpr uint32_t kPairBars = 3 * kPairMaxRaw + 2 * kPairMaxX + 2 * kPairAStages + 2 + 1 + 1;
 constexpr uint32_t kPairWarpStage = 16384;  // per storing warp: its 32 columns of the tile's rows of x
-constexpr uint32_t kPairTail = kEpilogueWarps * kPairWarpStage + kPairBars * 8 + 16;
+constexpr uint32_t kPairPlanBytes = 128;
+constexpr uint32_t kPairTail = kEpilogueWarps * kPairWarpStage + kPairBars * 8 + 16 + kPairPlanBytes;
 constexpr uint32_t kPairSmem = 227u * 1024u;
 constexpr uint32_t kPairRings = (kPairSmem - 1024u - kPairTail) / 1024u * 1024u;
 struct PairArgs {
@@ -57,6 +61,7 @@ struct PairArgs {
     unsigned int *flags;
     unsigned long long tile_floats;
     unsigned int x_stages, raw_stages;
+    PairSplit split;                   // of the whole batch's tiles
 };
 
 // Up to this many rows of x per tile a value has two accumulators, which successive pieces of x take in turn (an MMA
@@ -150,6 +155,171 @@ __device__ __forceinline__ void pair_drain(const RowStore &to, uint32_t stage, u
     }
 }
 
+// A cut tile that a pair holds a piece of: the tile and its holders, `holders` pairs from `first` on.
+struct PairCut {
+    uint32_t tile, first, holders;
+};
+
+__device__ __forceinline__ PairCut pair_cut(const PairWork &work, uint32_t id)
+{
+    PairCut cut;
+    cut.tile = work.tile;
+    cut.first = pair_first_holder(work, id, work.tile);
+    cut.holders = pair_last_holder(work, cut.first, work.tile) + 1u - cut.first;
+    return cut;
+}
+
+// A cut tile is finished by the pair that began it, or, where it has more holders than a pair has units by so many, by
+// all its holders.  The one that began it reads as many tiles of sums as there are others, 0.8 us a round trip, but most
+// of it before its own sums are there: the longer the runs, the more.  All together read one tile's worth each, and
+// everybody waits for the last to publish.  (Beginner against all: 1000 x 2048, 200 rows, 1 unit and 8 holders, 19.8 and
+// 11.3 us; 1024 x 4096, 300 rows, 24.1 and 16.4; 2560 x 2560, 300 rows, 2.7 units and 4 or 5 holders, 15.7 and 16.1, with
+// the line between 4 and 5 14.7; 2560 x 9728, 10.3 units, 4 or 5 holders, 25.9 and 27.3.)
+constexpr uint32_t kPairShareMore = 3;
+
+// What a block works on.  One thread works it out and the roles read it from shared memory: the divisions take a
+// microsecond, and kept in registers across the roles it costs the converters theirs.
+struct PairPlan {
+    uint32_t m;                 // live rows of x
+    PairWork work;
+    uint32_t share_from;        // from this many holders on a cut tile is finished by all of them
+    PairCut begun, begins;      // the cut tiles that the pair has pieces of: begun by another pair, and by itself
+};
+static_assert(sizeof(PairPlan) <= kPairPlanBytes, "room for the plan");
+
+__device__ __forceinline__ void pair_plan_cuts(PairPlan *plan, uint32_t id)
+{
+    plan->begun.holders = plan->begins.holders = 0u;
+    plan->share_from = (plan->work.pieces != 0u ? plan->work.segs / plan->work.pieces : plan->work.each) + kPairShareMore;
+    PairWork ahead = plan->work;
+    ahead.whole_left = 0u;
+    while (ahead.next()) {
+        if (ahead.s0 != 0u) {
+            plan->begun = pair_cut(ahead, id);
+        } else if (ahead.s1 != ahead.segs) {
+            plan->begins = pair_cut(ahead, id);
+        }
+    }
+}
+
+// Where a block's part of a cut tile lies: a block has two slots (the context's scratch is sized for two blocks per
+// SM), for the tile that it begins and for the one that others began.
+__device__ __forceinline__ uint32_t pair_slot(uint32_t block, bool begins)
+{
+    return begins ? gridDim.x + block : block;
+}
+
+__device__ __forceinline__ uint32_t pair_cut_slot(const PairCut &cut, uint32_t holder, uint32_t rank)
+{
+    return pair_slot(2u * (cut.first + holder) + rank, holder == 0u);
+}
+
+// A partial sum that another block has left, past the first-level cache.  Volatile, so that the loads of a piece are
+// issued one after the other before the first is used: a round trip is 0.7 us.
+__device__ __forceinline__ float ld_partial(const float *from)
+{
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(from) : "memory");
+    return v;
+}
+
+// The parts of one run of rows that the holders after the first have left (a slot every `stride` floats, `count` of
+// them), added to v in order; two of them are on their way at a time.
+__device__ __forceinline__ void add_parts(uint32_t (&v)[16], const float *slots, unsigned long long stride, uint32_t count)
+{
+#pragma unroll 1
+    for (uint32_t c = 0; c < count; c += 2u) {
+        const bool two = c + 1u < count;
+        float a[16], b[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+            a[i] = ld_partial(slots + i * kRows);
+        }
+        slots += two ? stride : 0ull;
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+            b[i] = ld_partial(slots + i * kRows);
+        }
+        slots += stride;
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+            v[i] = __float_as_uint(__uint_as_float(v[i]) + a[i] + (two ? b[i] : 0.0f));
+        }
+    }
+}
+
+// Add to v the 16 columns of sums at taddr (load_sums in q8_rows.cuh).
+__device__ __forceinline__ void add_sums(uint32_t taddr, uint32_t chains, uint32_t stride, uint32_t (&v)[16])
+{
+#pragma unroll 1
+    for (uint32_t c = 0; c < chains; ++c, taddr += stride) {
+        uint32_t more[16];
+        tmem_ld_32x16(taddr, more);
+        tmem_ld_wait();
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+            v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(more[i]));
+        }
+    }
+}
+
+// Wait until the holders from `from` on have published their part of this quarter of the tile.
+__device__ __forceinline__ void wait_for_parts(const PairArgs &args, const PairCut &at, uint32_t from, uint32_t rank, uint32_t lanes,
+                                               uint32_t lane, volatile uint32_t *abort_flag)
+{
+    for (uint32_t h = from + lane; h < at.holders; h += 32u) {
+        const unsigned int *flag = args.flags + kFlagWords * pair_cut_slot(at, h, rank) + lanes;
+        const long long begin = clock64();
+        while (ld_acquire_gpu(flag) < kPublishers) {
+            if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
+                atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
+                break;
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// Rows of x that a warp finishes of a cut tile at a time.
+constexpr uint32_t kPairShareRows = 8;
+
+// The parts of a cut tile's holders, `partial` being this lane's place in slot 0, added in order; the loads of three
+// holders are on their way at a time.
+__device__ __forceinline__ void sum_of_parts(uint32_t (&v)[kPairShareRows], const float *partial, unsigned long long tile_floats,
+                                             const PairCut &cut, uint32_t rank)
+{
+    constexpr uint32_t kTogether = 4u;
+    float sum[kPairShareRows];
+#pragma unroll
+    for (uint32_t i = 0; i < kPairShareRows; ++i) {
+        sum[i] = 0.0f;
+    }
+#pragma unroll 1
+    for (uint32_t h0 = 0; h0 < cut.holders; h0 += kTogether) {
+        float part[kTogether][kPairShareRows];
+#pragma unroll
+        for (uint32_t h = 0; h < kTogether; ++h) {
+            const bool there = h0 + h < cut.holders;
+            const float *from = partial + pair_cut_slot(cut, there ? h0 + h : h0, rank) * tile_floats;
+#pragma unroll
+            for (uint32_t i = 0; i < kPairShareRows; ++i) {
+                part[h][i] = ld_partial(from + i * kRows);
+            }
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < kTogether; ++h) {
+#pragma unroll
+            for (uint32_t i = 0; i < kPairShareRows; ++i) {
+                sum[i] += h0 + h < cut.holders ? part[h][i] : 0.0f;
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kPairShareRows; ++i) {
+        v[i] = __float_as_uint(sum[i]);
+    }
+}
+
 template <bool BF>
 __device__ __forceinline__ void pair_convert(uint32_t half, const uint32_t (&raw)[36], uint32_t taddr)
 {
@@ -183,7 +353,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const uint32_t acc_full = a_empty + 8u * kPairAStages;
     const uint32_t acc_empty = acc_full + 8u;                     // the first block's: both blocks' sums are out
     const uint32_t drain_bar = acc_empty + 8u;
-    const uint32_t tmem_slot = drain_bar + 8u;
+    const uint32_t cuts_bar = drain_bar + 8u;                     // plan->begun and plan->begins are there
+    const uint32_t tmem_slot = cuts_bar + 8u;
     volatile uint32_t *tmem_slot_ptr = reinterpret_cast<volatile uint32_t *>(smem + (tmem_slot - smem0));
     volatile uint32_t *abort_flag = tmem_slot_ptr + 1;
 
@@ -192,24 +363,11 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const uint32_t rank = cluster_ctarank();
 
     grid_launch_dependents();
-    unsigned int m = args.m_max;
-    if (args.m_dev != nullptr) {
-        // the live batch decides how many tiles there are
-        grid_dependency_wait();
-        const unsigned int live = *args.m_dev;
-        m = live < m ? live : m;
-    }
-    if (m == 0u) {
-        return;
-    }
     const uint32_t segs = args.k / kSegK;
-    const uint32_t tok_tiles = (m + ntok - 1u) / ntok;
     const uint32_t pairs = gridDim.x / 2u;
-    const uint32_t tiles = (args.n + 2u * kRows - 1u) / (2u * kRows) * tok_tiles;   // below 2^31 units: the host checks
+    const uint32_t row_tiles = (args.n + 2u * kRows - 1u) / (2u * kRows);   // below 2^31 units: the host checks
     const uint32_t pair_id = blockIdx.x / 2u;
-    PairWork work;
-    pair_deal(&work, pair_id, pairs, tiles, segs);
-    const uint32_t total = work.whole_left * segs + work.left;    // segments of weights
+    PairPlan *plan = reinterpret_cast<PairPlan *>(smem + (tmem_slot + 16u - smem0));
 
     uint32_t early = 0u;
     if (warp == kPairWeightWarp && elect_one()) {
@@ -231,11 +389,15 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         mbar_init(acc_full, 1u);
         mbar_init(acc_empty, 2u * kEpilogueWarps);
         mbar_init(drain_bar, 1u);
+        mbar_init(cuts_bar, 1u);
         *abort_flag = 0u;
         mbar_init_fence();
         fence_proxy_async_smem();
         // the first weights: only this block's own barriers have to be there
-        PairWork ahead = work;
+        PairWork ahead;
+        const uint32_t tok_tiles = (args.m_max + ntok - 1u) / ntok;
+        pair_work(&ahead, args.split, pair_id, pairs, segs);
+        const uint32_t total = ahead.whole_left * segs + ahead.left;
         uint32_t s = 0u;
         ahead.s1 = 0u;
         for (; early < args.raw_stages && early < total; ++early, ++s) {
@@ -247,6 +409,41 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             tma_load_2d(raw_base + early * kRawStageBytes, &tmap_w, raw_full + 8u * early, (int)(s * kSegWords),
                         (int)((ahead.tile / tok_tiles * 2u + rank) * kRows));
         }
+        // The live batch decides how many tiles there are, and is known when the launch before this one has ended.
+        // The first weights are on their way by then, as the whole batch wants them; where it has more tiles than
+        // the live one, they land first and their barriers are made anew.
+        if (args.m_dev != nullptr) {
+            grid_dependency_wait();
+            const unsigned int live = *args.m_dev;
+            if (live < args.m_max && (live + ntok - 1u) / ntok != tok_tiles) {
+                uint32_t local_abort = 0;
+                for (uint32_t i = 0; i < early; ++i) {
+                    mbar_wait(raw_full + 8u * i, 0u, &local_abort, nullptr);
+                    mbar_inval(raw_full + 8u * i);
+                    mbar_init(raw_full + 8u * i, 1u);
+                }
+                mbar_init_fence();
+                fence_proxy_async_smem();
+                early = 0u;
+            }
+        }
+    }
+    if (threadIdx.x == 0u) {
+        PairWork work;
+        uint32_t m = args.m_max;
+        if (args.m_dev != nullptr) {
+            prefetch_l2(args.m_dev);
+            grid_dependency_wait();
+            const unsigned int live = *args.m_dev;
+            m = live < m ? live : m;
+        }
+        if ((m + ntok - 1u) / ntok == (args.m_max + ntok - 1u) / ntok) {
+            pair_work(&work, args.split, pair_id, pairs, segs);
+        } else {
+            pair_deal(&work, pair_id, pairs, row_tiles * ((m + ntok - 1u) / ntok), segs);
+        }
+        plan->m = m;
+        plan->work = work;
     }
     if (warp == kPairMmaWarp) {
         pair_tmem_alloc(tmem_slot, 512u);
@@ -261,6 +458,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot_ptr;
+    const uint32_t m = plan->m;
+    const uint32_t tok_tiles = (m + ntok - 1u) / ntok;
     const uint32_t a_column0 = kPairTok;
     const uint32_t chains = ntok <= kPairTwoChains ? 2u : 1u;
 
@@ -270,6 +469,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             uint32_t g = 0;
             bool ok = true;
             uint32_t full = 0u;
+            PairWork work = plan->work;
             uint32_t st = 0u, ph = 1u;
             while (ok && work.next()) {
                 const uint32_t w_row = (work.tile / tok_tiles * 2u + rank) * kRows;
@@ -307,6 +507,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             bool ok = true;
             uint32_t st = 0u, ph = 1u;
             const uint32_t signal = mapa_shared(x_full, 0u);
+            PairWork work = plan->work;
             while (ok && work.next()) {
                 const uint32_t row = work.tile % tok_tiles * ntok + rank * (ntok / 2u);
                 for (uint32_t sub = work.s0 * kSubs; sub < work.s1 * kSubs; ++sub, ++q) {
@@ -341,6 +542,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             uint32_t ast = 0u, aph = 0u;
             uint32_t x_there = 0u, a_there = 0u;   // the next piece of x, the next segment of A, are known to be there
             bool ok = true;
+            PairWork work = plan->work;
+            const bool works = !work.last();
             for (uint32_t turn = 0; ok && work.next(); ++turn) {
                 if (!mbar_wait_hot(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
                     ok = false;
@@ -392,7 +595,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     pair_commit(acc_full);
                 }
             }
-            if (total != 0u) {
+            if (works) {
                 // Every MMA has finished: what the helping warps of both blocks wait for.  This thread waits as
                 // well; a pair without work issues none, because nobody would wait for its arrivals, and they
                 // must not come to a shared memory that the blocks have left.
@@ -409,6 +612,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const uint32_t row_at = ((cw & 3u) * 32u + lane) * kSegBytes;
         const uint32_t lane_base = tmem_base + (((cw & 3u) * 32u) << 16) + a_column0 + half * (kSegK / 4u);
         const uint32_t signal = mapa_shared(a_full, 0u);
+        const PairWork work = plan->work;
+        const uint32_t total = work.whole_left * segs + work.left;    // segments of weights
         uint32_t full = group, fph = 0, ast = group, aph = 0;
         for (uint32_t g = group; g < total; g += kPairGroups) {
             if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(raw_full + 8u * full, fph, abort_flag, args.status))) {
@@ -452,13 +657,18 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
     }
 
-    uint32_t last_cc = pair_id;         // the last pair whose partial sums this one takes
-    if (warp < kPairWeightWarp && total != 0u) {
+    if (warp < kPairWeightWarp) {
         // ---------------------------------------------------------------- read sums, store
         const uint32_t lanes = warp & 3u;
         const uint32_t helper = warp >> 2;                       // 0: the storing warps
         const uint32_t lane_taddr = tmem_base + ((lanes * 32u) << 16);
         const bool gated = args.to.epilogue == kEpilogueSwiglu;
+        PairWork work = plan->work;
+        if (threadIdx.x == 0u) {
+            pair_plan_cuts(plan, pair_id);
+            mbar_arrive(cuts_bar);
+        }
+        __syncwarp();
         const uint32_t stage = helper == 0u ? stage_base + warp * kPairWarpStage : smem0 + (warp - kEpilogueWarps) * 4096u;
         const uint32_t release_bar = mapa_shared(acc_empty, 0u);
         uint32_t flip = 0u;      // the two turns of a helper's staging buffer
@@ -470,6 +680,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const bool last = work.last();
             const bool owner = work.s0 == 0u;
             const bool helped = last;
+            const bool cut = !owner || work.s1 != segs;
             if (helper != 0u && !helped) {
                 continue;
             }
@@ -481,24 +692,28 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t mine = inside < 32u ? inside : 32u;
             const uint32_t columns = gated ? mine / 2u : mine;
             const uint32_t col = gated ? j / 2u : j;
-            if (owner && work.s1 != segs) {
-                // The other holders of this tile are the pairs right after this one; they met it at the start of
-                // their runs of units.
-                last_cc = pair_last_holder(work, pair_id, work.tile);
-                for (uint32_t base = pair_id + 1u; base <= last_cc; base += 32u) {
-                    const uint32_t cc = base + lane;
-                    if (cc <= last_cc) {
-                        const unsigned int *flag = args.flags + kFlagWords * (2u * cc + rank) + lanes;
-                        const long long begin = clock64();
-                        while (ld_acquire_gpu(flag) < kPublishers) {
-                            if (clock64() - begin > Q8_WAIT_CYCLES || *abort_flag != 0u) {
-                                atomicOr(args.status, Q8_DEV_FLAG_TIMEOUT);
-                                break;
-                            }
-                        }
-                    }
+            uint32_t others = 0u;          // holders whose parts this pair adds to its own
+            bool publish = false;
+            if (cut) {
+                mbar_wait_hot(cuts_bar, 0u, abort_flag, args.status);
+                const PairCut at = owner ? plan->begins : plan->begun;
+                publish = !owner || at.holders >= plan->share_from;
+                if (!publish) {
+                    // The pairs right after this one; they met the tile at the start of their runs of units.
+                    others = at.holders - 1u;
+                    wait_for_parts(args, at, 1u, rank, lanes, lane, abort_flag);
                 }
-                __syncwarp();
+            }
+            auto add_others = [&](uint32_t (&v)[16], uint32_t first_row) {
+                add_parts(v, args.partial + (2ull * pair_id + 2u + rank) * args.tile_floats + first_row * kRows + lanes * 32u + lane,
+                                 2u * args.tile_floats, others);
+            };
+            const uint32_t step = helped ? kPairWeightWarp / 4u : 1u;
+            uint32_t c0 = helped ? helper * 16u : 0u;
+            uint32_t v[16] = {};
+            if (others != 0u && c0 < rows && mine != 0u) {
+                // the others' parts of this warp's first run of rows, before its own sums are there
+                add_others(v, c0);
             }
             // (a helper has seen none of the pieces before, so it does not ask for a parity of their barrier)
             if (!__all_sync(0xFFFFFFFFu, helper == 0u ? mbar_wait_hot(acc_full, turn & 1u, abort_flag, args.status)
@@ -523,24 +738,101 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 continue;
             }
             const bool staged = aligned4 && (columns % 4u) == 0u;
-            const uint32_t step = helped ? kPairWeightWarp / 4u : 1u;
 #pragma unroll 1
-            for (uint32_t c0 = helped ? helper * 16u : 0u; c0 < rows && mine != 0u; c0 += 16u * step) {
-                const uint32_t slot = c0 * kRows + lanes * 32u + lane;
-                uint32_t v[16];
-                load_sums(lane_taddr + c0, chains, kPairTwoChains, v);
-                if (!owner) {
-                    float *to = args.partial + (unsigned long long)blockIdx.x * args.tile_floats + slot;
+            for (; c0 < rows && mine != 0u; c0 += 16u * step) {
+                add_sums(lane_taddr + c0, chains, kPairTwoChains, v);
+                if (publish) {
+                    float *to = args.partial + (unsigned long long)pair_slot(blockIdx.x, owner) * args.tile_floats + c0 * kRows
+                              + lanes * 32u + lane;
 #pragma unroll
                     for (uint32_t i = 0; i < 16u; ++i) {
                         __stcg(to + i * kRows, __uint_as_float(v[i]));
                     }
-                    continue;
+                } else if (staged) {
+                    const uint32_t buffer = stage + flip;
+                    flip ^= 2048u;
+                    if (gated) {
+                        store_rows_staged<YT, true>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                    } else {
+                        // in two halves: the old values of an add take as many registers as the sums
+                        uint32_t half[8];
+#pragma unroll
+                        for (uint32_t h = 0; h < 16u; h += 8u) {
+#pragma unroll
+                            for (uint32_t i = 0; i < 8u; ++i) {
+                                half[i] = v[h + i];
+                            }
+                            store_rows_staged<YT, false>(args.to, buffer + h * 32u * sizeof(YT), lane, col, columns, tok0 + c0 + h,
+                                                         tok0 + rows, half);
+                        }
+                    }
+                } else {
+                    store_rows_direct<YT>(args.to, gated, lane, mine, col, tok0 + c0, tok0 + rows, v);
                 }
-                if (last_cc != pair_id) {
-                    add_partial_sums(v, args.partial + (2ull * pair_id + 2u + rank) * args.tile_floats + slot, 2u * args.tile_floats,
-                                     last_cc - pair_id);
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; ++i) {
+                    v[i] = 0u;
                 }
+                if (others != 0u && c0 + 16u * step < rows) {
+                    add_others(v, c0 + 16u * step);
+                }
+            }
+            if (!last) {
+                release();
+            }
+            if (publish) {
+                // Publish this warp's quarter; every lane makes its own stores visible first.
+                __threadfence();
+                __syncwarp();
+                if (lane == 0u) {
+                    red_release_gpu_add(args.flags + kFlagWords * pair_slot(blockIdx.x, owner) + lanes, helped ? 1u : kPublishers);
+                }
+            }
+        }
+        // ------------------------------------------------------------ tiles of many holders
+        // Every holder finishes a share of the tile's rows of x: the parts of all holders, its own among them, added
+        // in the order of the depth.  A pair has published all it has before it waits here, so that whoever waits,
+        // waits for pairs that need nothing from it.
+        mbar_wait_hot(cuts_bar, 0u, abort_flag, args.status);
+#pragma unroll 1
+        for (uint32_t which = 0; which < 2u; ++which) {
+            const PairCut at = which == 0u ? plan->begun : plan->begins;
+            if (at.holders < plan->share_from) {
+                continue;
+            }
+            const uint32_t row_tile = at.tile / tok_tiles;
+            const uint32_t tok0 = (at.tile - row_tile * tok_tiles) * ntok;
+            const uint32_t rows = m - tok0 < ntok ? m - tok0 : ntok;
+            const uint32_t j = (row_tile * 2u + rank) * kRows + lanes * 32u;
+            const uint32_t inside = args.n > j ? args.n - j : 0u;
+            const uint32_t mine = inside < 32u ? inside : 32u;
+            const uint32_t columns = gated ? mine / 2u : mine;
+            const uint32_t col = gated ? j / 2u : j;
+            const bool staged = aligned4 && (columns % 4u) == 0u;
+            const uint32_t runs = (rows + kPairShareRows - 1u) / kPairShareRows;
+            const uint32_t index = pair_id - at.first;
+            const uint32_t end = (index + 1u) * runs / at.holders;
+            uint32_t run = index * runs / at.holders + helper;
+            if (mine == 0u) {
+                run = end;
+            }
+            if (run < end) {
+                wait_for_parts(args, at, 0u, rank, lanes, lane, abort_flag);
+            }
+            // This warp has published and has seen what it needs.  The last warp of the holders to say so clears the
+            // flag, and the count of those that have.
+            unsigned int *flag = args.flags + kFlagWords * pair_cut_slot(at, lane < at.holders ? lane : 0u, rank) + lanes;
+            const uint32_t all = at.holders * kPublishers;
+            uint32_t came = 0u;
+            if (lane < at.holders) {
+                came = atomicAdd(flag + kEpilogueWarps, 1u) + 1u;
+            }
+#pragma unroll 1
+            for (; run < end; run += kPairWeightWarp / 4u) {
+                const uint32_t c0 = run * kPairShareRows;
+                const uint32_t slot = c0 * kRows + lanes * 32u + lane;
+                uint32_t v[kPairShareRows];
+                sum_of_parts(v, args.partial + slot, args.tile_floats, at, rank);
                 if (staged) {
                     const uint32_t buffer = stage + flip;
                     flip ^= 2048u;
@@ -551,28 +843,19 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     }
                     continue;
                 }
-#pragma unroll
-                for (uint32_t i = 0; i < 16u; ++i) {
-                    float value = __uint_as_float(v[i]);
-                    if (gated) {
-                        const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
-                        value = gated_unit(value, other);
-                    }
-                    if (c0 + i < rows && lane < mine && (!gated || (lane & 1u) == 0u)) {
-                        store_value<YT>(args.to, (size_t)(tok0 + c0 + i) * args.to.ldy + col + (gated ? lane / 2u : lane), value);
-                    }
-                }
+                store_rows_direct<YT>(args.to, gated, lane, mine, col, tok0 + c0, tok0 + rows, v);
             }
-            if (!owner) {
-                // Publish this warp's quarter; every lane makes its own stores visible first.
-                __threadfence();
-                __syncwarp();
-                if (lane == 0u) {
-                    red_release_gpu_add(args.flags + kFlagWords * blockIdx.x + lanes, helped ? 1u : kPublishers);
+            for (uint32_t h = lane;;) {
+                if (came == all) {
+                    *reinterpret_cast<volatile unsigned int *>(flag) = 0u;
+                    *reinterpret_cast<volatile unsigned int *>(flag + kEpilogueWarps) = 0u;
                 }
-            }
-            if (!last) {
-                release();
+                h += 32u;
+                if (h >= at.holders) {
+                    break;
+                }
+                flag = args.flags + kFlagWords * pair_cut_slot(at, h, rank) + lanes;
+                came = atomicAdd(flag + kEpilogueWarps, 1u) + 1u;
             }
         }
     }
@@ -584,9 +867,11 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     cluster_arrive_relaxed();
     cluster_wait_acquire();
     if (warp < kEpilogueWarps) {
-        // Hand the consumed slots back for the next launch that uses this set (ordered by the end of the kernel).
-        for (uint32_t cc = pair_id + 1u + lane; cc <= last_cc; cc += 32u) {
-            *reinterpret_cast<volatile unsigned int *>(args.flags + kFlagWords * (2u * cc + rank) + warp) = 0u;
+        // The slots that an owner alone has read go back for the next launch that uses this set (every warp has passed
+        // its waits; ordered by the end of the kernel).
+        const PairCut at = plan->begins;
+        for (uint32_t h = 1u + lane; at.holders < plan->share_from && h < at.holders; h += 32u) {
+            *reinterpret_cast<volatile unsigned int *>(args.flags + kFlagWords * pair_cut_slot(at, h, rank) + warp) = 0u;
         }
     }
     if (warp == kPairMmaWarp) {
@@ -661,6 +946,7 @@ cudaError_t launch_pair_kernel(cudaStream_t stream, const CUtensorMap &tw, const
     args.x_stages = x_stages < kPairMaxX ? x_stages : kPairMaxX;
     const unsigned long long units = (unsigned long long)((n + 2u * kRows - 1u) / (2u * kRows)) * ((m + ntok - 1u) / ntok) * (k / kSegK);
     const unsigned int pairs = units < sm_count / 2u ? (unsigned int)units : sm_count / 2u;
+    args.split = pair_split(pairs, (n + 2u * kRows - 1u) / (2u * kRows) * ((m + ntok - 1u) / ntok), k / kSegK);
     switch (y_dtype) {
     case 0:
         return launch_pair_typed<float>(stream, tw, tx, args, 2u * pairs, overlap);

@@ -103,24 +103,45 @@ __device__ __forceinline__ void store_value(const RowStore &to, size_t at, float
     }
 }
 
-// 16 rows of x by this warp's 32 columns of y, every lane one column: turned round in shared memory of
+// The same values without the detour of store_rows_staged, for columns that are no multiple of four: each lane its
+// column (`gated`: each pair of lanes) of ROWS rows of x; `mine` of the warp's 32 rows of w are inside the tensor.
+template <typename YT, int ROWS>
+__device__ __forceinline__ void store_rows_direct(const RowStore &to, bool gated, uint32_t lane, uint32_t mine, uint32_t first_col,
+                                                  uint32_t first_row, uint32_t row_limit, const uint32_t (&v)[ROWS])
+{
+#pragma unroll
+    for (uint32_t i = 0; i < (uint32_t)ROWS; ++i) {
+        float value = __uint_as_float(v[i]);
+        if (gated) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);
+            value = gated_unit(value, other);
+        }
+        const uint32_t row_x = first_row + i;
+        if (row_x < row_limit && lane < mine && (!gated || (lane & 1u) == 0u)) {
+            const uint32_t row_y = to.row_map != nullptr ? to.row_map[row_x] : row_x;
+            store_value<YT>(to, (size_t)row_y * to.ldy + first_col + (gated ? lane / 2u : lane), value);
+        }
+    }
+}
+
+// ROWS (16 or 8) rows of x by this warp's 32 columns of y, every lane one column: turned round in shared memory of
 // the warp's own and written four values per lane, 2 to 4 store instructions instead of 16 (the
 // number of store instructions is what a store costs here, see q8_tile.cuh).  GATED: neighbouring
 // lanes hold gate and up of one column (cuda/model/norm.cu:92-105); 16 columns then.
 // `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.
-template <typename YT, bool GATED>
+template <typename YT, bool GATED, int ROWS>
 __device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t stage, uint32_t lane, uint32_t first_col,
                                                  uint32_t columns, uint32_t first_row, uint32_t row_limit,
-                                                 const uint32_t (&v)[16])
+                                                 const uint32_t (&v)[ROWS])
 {
     constexpr uint32_t kColumns = GATED ? 16u : 32u;
     constexpr uint32_t kRowBytes = kColumns * sizeof(YT);
     constexpr uint32_t kLanesPerRow = kColumns / 4u;
     constexpr uint32_t kRowsPerStep = 32u / kLanesPerRow;      // 4 or 8
-    constexpr uint32_t kSteps = 16u / kRowsPerStep;
+    constexpr uint32_t kSteps = (uint32_t)ROWS / kRowsPerStep;
     const uint32_t column = GATED ? lane / 2u : lane;
 #pragma unroll
-    for (uint32_t i = 0; i < 16u; ++i) {
+    for (uint32_t i = 0; i < (uint32_t)ROWS; ++i) {
         float value = __uint_as_float(v[i]);
         if (GATED) {
             const float other = __shfl_xor_sync(0xFFFFFFFFu, value, 1u);

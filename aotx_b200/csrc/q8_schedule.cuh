@@ -75,6 +75,7 @@ struct PairWork {
     uint32_t next_tile, next_seg, left;
     uint32_t first_cut, units, sharers;     // the cut tiles: the first, their units, the pairs that share them
     uint32_t pieces;                        // per cut tile; 0: the units are dealt evenly, whatever the tile
+    uint32_t each, more;                    // ... `each` units to every sharer and one more to the first `more`
 
     __host__ __device__ __forceinline__ bool next()
     {
@@ -111,7 +112,12 @@ constexpr uint32_t kPairCutUnits = 5;
 constexpr uint32_t kPairMinPiece = 4;
 constexpr uint32_t kPairEvenUnits = 2;
 
-// The work of pair `id` of `pairs`.  As many turns of whole tiles as all pairs have; the tiles that are left:
+// How the tiles are divided between all pairs; the divisions that need no pair's number, so that the host can do them.
+struct PairSplit {
+    uint32_t turns, first_cut, cut, units, sharers, pieces, each, more;
+};
+
+// As many turns of whole tiles as all pairs have; the tiles that are left:
 //   * Fewer than two turns: their units are dealt evenly.  Longer pieces are faster (2560 x 2560, 300 rows, 15.0 us
 //     in halves of a tile against 17.5; 1000 x 2048, 200 rows, 14.8 against 19.9), but the error of a sum grows with
 //     the depth that goes into one accumulator, and evenly dealt it is the smallest.
@@ -119,51 +125,89 @@ constexpr uint32_t kPairEvenUnits = 2;
 //     than it evens out; else pieces of one size inside each tile, of kPairMinPiece units at least, as many as there
 //     are pairs for; else evenly dealt units, where that makes the longest piece kPairEvenUnits shorter (19456 x
 //     2560, 300 rows, four tiles of 10 units behind two turns: two pieces each 38.5 us, dealt evenly 43.5).
-__host__ __device__ __forceinline__ void pair_deal(PairWork *work, uint32_t id, uint32_t pairs, uint32_t tiles, uint32_t segs)
+__host__ __device__ __forceinline__ PairSplit pair_split(uint32_t pairs, uint32_t tiles, uint32_t segs)
 {
-    const uint32_t turns = tiles / pairs;
-    const uint32_t cut = tiles - turns * pairs;
-    const uint32_t units = cut * segs;
-    work->segs = segs;
-    work->stride = pairs;
-    work->next_whole = id;
-    work->whole_left = turns;
-    work->next_tile = work->next_seg = work->left = 0u;
-    work->first_cut = turns * pairs;
-    work->units = units;
-    work->sharers = units < pairs ? units : pairs;
-    work->pieces = 0u;
-    if (cut == 0u) {
-        return;
+    PairSplit split;
+    split.turns = tiles / pairs;
+    split.first_cut = split.turns * pairs;
+    split.cut = tiles - split.first_cut;
+    split.units = split.cut * segs;
+    split.sharers = split.units < pairs ? split.units : pairs;
+    split.pieces = split.each = split.more = 0u;
+    if (split.cut == 0u) {
+        return split;
     }
-    if (turns > 1u) {
-        const uint32_t even = units / pairs;
+    if (split.turns > 1u) {
+        const uint32_t even = split.units / pairs;
         if (segs <= even + kPairCutUnits) {
-            work->whole_left += id < cut ? 1u : 0u;
-            return;
+            split.sharers = 0u;      // whole tiles as well
+            return split;
         }
-        const uint32_t places = pairs / cut;
+        const uint32_t places = pairs / split.cut;
         const uint32_t most = segs / kPairMinPiece > 1u ? segs / kPairMinPiece : 1u;
         const uint32_t pieces = most < places ? most : places;
         if (pieces > 1u && (most <= places || (segs + pieces - 1u) / pieces <= even + kPairEvenUnits)) {
-            work->pieces = pieces;
-            work->sharers = cut * pieces;
-            if (id < work->sharers) {
-                const uint32_t i = id % pieces;
-                work->next_tile = work->first_cut + id / pieces;
-                work->next_seg = i * segs / pieces;
-                work->left = (i + 1u) * segs / pieces - work->next_seg;
-            }
-            return;
+            split.pieces = pieces;
+            split.sharers = split.cut * pieces;
+            return split;
         }
     }
-    if (id < work->sharers) {
-        uint32_t begin, end;
-        decode_range(id, work->sharers, units, &begin, &end);
-        work->next_tile = work->first_cut + begin / segs;
-        work->next_seg = begin % segs;
-        work->left = end - begin;
+    split.each = split.units / split.sharers;
+    split.more = split.units - split.each * split.sharers;
+    return split;
+}
+
+// The work of pair `id`.
+__host__ __device__ __forceinline__ void pair_work(PairWork *work, const PairSplit &split, uint32_t id, uint32_t pairs, uint32_t segs)
+{
+    work->segs = segs;
+    work->stride = pairs;
+    work->next_whole = id;
+    work->whole_left = split.turns + (split.sharers == 0u && id < split.cut ? 1u : 0u);
+    work->next_tile = work->next_seg = work->left = 0u;
+    work->first_cut = split.first_cut;
+    work->units = split.units;
+    work->sharers = split.sharers;
+    work->pieces = split.pieces;
+    work->each = split.each;
+    work->more = split.more;
+    if (id >= split.sharers) {
+        return;
     }
+    if (split.pieces != 0u) {
+        const uint32_t tile = id / split.pieces;
+        const uint32_t i = id - tile * split.pieces;
+        work->next_tile = split.first_cut + tile;
+        work->next_seg = i * segs / split.pieces;
+        work->left = (i + 1u) * segs / split.pieces - work->next_seg;
+        return;
+    }
+    const uint32_t begin = id * split.each + (id < split.more ? id : split.more);
+    const uint32_t tile = begin / segs;
+    work->next_tile = split.first_cut + tile;
+    work->next_seg = begin - tile * segs;
+    work->left = split.each + (id < split.more ? 1u : 0u);
+}
+
+__host__ __device__ __forceinline__ void pair_deal(PairWork *work, uint32_t id, uint32_t pairs, uint32_t tiles, uint32_t segs)
+{
+    pair_work(work, pair_split(pairs, tiles, segs), id, pairs, segs);
+}
+
+// The pair that holds a unit of the evenly dealt ones.
+__host__ __device__ __forceinline__ uint32_t pair_holder(const PairWork &work, uint32_t unit)
+{
+    const uint32_t cut = work.more * (work.each + 1u);
+    return unit < cut ? unit / (work.each + 1u) : work.more + (unit - cut) / work.each;
+}
+
+// The first of the pairs that hold pieces of the cut tile that `id` holds a piece of.
+__host__ __device__ __forceinline__ uint32_t pair_first_holder(const PairWork &work, uint32_t id, uint32_t tile)
+{
+    if (work.pieces != 0u) {
+        return id - id % work.pieces;
+    }
+    return pair_holder(work, (tile - work.first_cut) * work.segs);
 }
 
 // The last of the pairs right after `id` that hold later pieces of the cut tile whose first segment `id` holds.
@@ -172,7 +216,7 @@ __host__ __device__ __forceinline__ uint32_t pair_last_holder(const PairWork &wo
     if (work.pieces != 0u) {
         return id + work.pieces - 1u;
     }
-    return decode_holder((tile - work.first_cut + 1u) * work.segs - 1u, work.sharers, work.units);
+    return pair_holder(work, (tile - work.first_cut + 1u) * work.segs - 1u);
 }
 
 } // namespace q8

@@ -52,6 +52,12 @@ __device__ __forceinline__ void copy_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+// A barrier's memory may be used for something else, another barrier for instance.
+__device__ __forceinline__ void mbar_inval(uint32_t bar)
+{
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // Ask for a line into L2.  It is a hint that reads nothing: a later write to the line is seen by later reads.
 __device__ __forceinline__ void prefetch_l2(const void *at)
 {

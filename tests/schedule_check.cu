@@ -202,6 +202,25 @@ static int check_pairs(uint32_t tiles, uint32_t segs, uint32_t pairs)
     return 0;
 }
 
+// Every holder of a cut tile names the same first pair, the one that has the tile's first segment.
+static int check_first_holder(uint32_t tiles, uint32_t segs, uint32_t pairs)
+{
+    std::vector<uint32_t> first(tiles, pairs);
+    for (uint32_t id = 0; id < pairs; ++id) {
+        PairWork w;
+        pair_deal(&w, id, pairs, tiles, segs);
+        while (w.next()) {
+            if (w.s0 == 0u) {
+                first[w.tile] = id;
+            }
+            if ((w.s0 != 0u || w.s1 != segs) && pair_first_holder(w, id, w.tile) != first[w.tile]) {
+                return fail("a holder names another pair as the tile's first", tiles, segs, pairs, id);
+            }
+        }
+    }
+    return 0;
+}
+
 // `way`: 0 units, 1 whole tiles in turns, 2 and 4 clusters of that size.
 static int check_mid(uint32_t tiles, uint32_t segs, uint32_t grid, uint32_t way, uint32_t run_segs)
 {
@@ -309,7 +328,8 @@ int main()
         for (uint32_t segs : {1u, 2u, 3u, 4u, 5u, 7u, 8u, 9u, 10u, 11u, 13u, 16u, 18u, 31u, 36u, 38u, 56u, 64u}) {
             for (uint32_t tiles = 1; tiles <= 700; tiles += (tiles < 300 ? 1 : 7)) {
                 // (the launch has as many pairs as units, at most)
-                if (check_pairs(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0) {
+                if (check_pairs(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0
+                    || check_first_holder(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0) {
                     return 1;
                 }
                 cases += 1;
