@@ -150,32 +150,19 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
         return cudaErrorNotSupported;
     }
     const unsigned int ntok = umma_token_tile(m);
-    // bfloat16 activations at 33 to 128 rows: the one-block-per-SM kernel would turn every x
-    // tile into binary16 in shared memory, in every block and for every weight row tile, as many
-    // bytes again as the weights; one pass over x into the context's copy does it once
+    // bfloat16 activations at 17 to 128 rows become binary16: in the kernel as x comes (mid_converts_x), or by one pass
+    // over x into the context's copy, 2.7 us between the launch before and the product.
     const bool copy_fits = scratch.x16 != nullptr && (unsigned long long)m * k * 2ull <= scratch.x16_bytes;
 #ifdef Q8_HOST_EMULATION
     const bool mid = false;
 #else
-    // the kernel for 17 to 128 rows takes binary16 x
+    // the kernel for 17 to 128 rows multiplies binary16 x
     const bool mid = ntok > 16u && ntok <= 128u && out == nullptr && (!x_bf16 || copy_fits)
                   && (unsigned long long)(n / kRows + 1u) * (k / kSegK) < (1ull << 31);
 #endif
-    if (x_bf16 && (mid || ntok >= 64u) && ntok <= 128u && copy_fits) {
-        const unsigned long long chunks = (unsigned long long)m * k / 8ull;
-        const unsigned int blocks = (unsigned int)((chunks + 255ull) / 256ull < 4ull * sm_count
-                                                       ? (chunks + 255ull) / 256ull : 4ull * sm_count);
-        cudaError_t turned = launch_kernel_early(overlap, q8_x_to_f16_kernel, blocks, 256, 0, stream,
-                                           static_cast<const uint4 *>(x), chunks, static_cast<uint4 *>(scratch.x16));
-        if (turned != cudaSuccess) {
-            return turned;
-        }
-        x = scratch.x16;
-        x_bf16 = 0;
-    }
-
 #ifdef Q8_HOST_EMULATION
     const bool warp_kernel = false; // cluster launches and warp-level MMA are not modelled
+    const bool as_it_is = false;
 #else
     // Up to 16 rows, one copy of y: the register-fed kernel; up to 128: q8_mid.cu.  Stores into the
     // peers' copies stay with the kernels they were measured on.
@@ -192,6 +179,21 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     }
     const bool wide = ntok > 128u
                    || (mid && plan.cluster == 1u && (m > 112u || (m > 64u && (plan.turns == 1u || plan.turns == 2u))));
+    const bool as_it_is = mid && !wide && mid_converts_x(plan);
+#endif
+    if (x_bf16 && !as_it_is && (mid || ntok >= 64u) && ntok <= 128u && copy_fits) {
+        const unsigned long long chunks = (unsigned long long)m * k / 8ull;
+        const unsigned int blocks = (unsigned int)((chunks + 255ull) / 256ull < 4ull * sm_count
+                                                       ? (chunks + 255ull) / 256ull : 4ull * sm_count);
+        cudaError_t turned = launch_kernel_early(overlap, q8_x_to_f16_kernel, blocks, 256, 0, stream,
+                                           static_cast<const uint4 *>(x), chunks, static_cast<uint4 *>(scratch.x16));
+        if (turned != cudaSuccess) {
+            return turned;
+        }
+        x = scratch.x16;
+        x_bf16 = 0;
+    }
+#ifndef Q8_HOST_EMULATION
     if (wide && out == nullptr && scratch.blocks >= 2u * sm_count && scratch.tile_floats >= 256ull * kRows
         && (unsigned long long)(n / (2u * kRows) + 1u) * (m / 128u + 1u) * (k / kSegK) < (1ull << 31)) {
         const unsigned int rows = pair_token_tile(m);
@@ -205,12 +207,12 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
     }
     if (mid) {
         CUtensorMap tw, tx;
-        if (!map_weights(encode, &tw, w, n, k, plan.slab_rows) || !map_rows(encode, &tx, x, m, k, plan.ntok, false)) {
+        if (!map_weights(encode, &tw, w, n, k, plan.slab_rows) || !map_rows(encode, &tx, x, m, k, plan.ntok, x_bf16 != 0)) {
             return cudaErrorInvalidValue;
         }
         return launch_mid_product(stream, tw, tx, plan, n, k, m, m_dev, y, y_dtype, epilogue == kEpilogueSwiglu ? n / 2u : n,
                                   epilogue, set_partial(scratch, set), set_flags(scratch, set), scratch.tile_floats,
-                                  scratch.status, overlap);
+                                  scratch.status, overlap, x_bf16 != 0);
     }
 #endif
 

@@ -40,9 +40,10 @@ constexpr uint32_t kMidMmaWarp = 22;
 constexpr uint32_t kMidMaxRaw = 12;        // stages of the rings, at most
 constexpr uint32_t kMidMaxX = 8;
 constexpr uint32_t kMidMaxA = 3;
-constexpr uint32_t kMidBars = 3 * kMidMaxRaw + 2 * kMidMaxX + 2 * kMidMaxA + 4 + 1;
+constexpr uint32_t kMidBars = 3 * kMidMaxRaw + 3 * kMidMaxX + 2 * kMidMaxA + 4 + 1;
 constexpr uint32_t kMidStageBytes = 4 * 2 * 2048;   // per storing warp: two turns of 16 rows of x by 32 columns, floats
 constexpr uint32_t kMidTail = kMidStageBytes + kMidBars * 8 + 16;
+constexpr uint32_t kMidConvertStep = kEpilogueWarps * 32u * 16u;      // bytes of x that the storing warps convert at a time
 constexpr uint32_t kMidSmem = 227u * 1024u;
 constexpr uint32_t kMidRings = (kMidSmem - 1024u - kMidTail) / 1024u * 1024u;   // both rings' shared memory
 
@@ -77,6 +78,7 @@ struct MidArgs {
     // Columns of tensor memory: of one accumulator of a tile, of a buffer of `chains` of them (and of the sum of a
     // cluster's runs so far, behind them); where the segments of A begin.
     unsigned int acc_columns, buffer_columns, a_column0;
+    unsigned int x_bf16;               // x is bfloat16 and becomes binary16 in shared memory (one piece per block only)
     unsigned int read_chains;          // accumulators, and the sum of the runs, that make a finished sum
 };
 
@@ -151,7 +153,8 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const uint32_t acc_full = a_empty + 8u * kMidMaxA;
     const uint32_t acc_empty = acc_full + 16u;
     const uint32_t drain_bar = acc_empty + 16u;
-    const uint32_t tmem_slot = drain_bar + 8u;
+    const uint32_t x_ready = drain_bar + 8u;      // x is binary16
+    const uint32_t tmem_slot = x_ready + 8u * kMidMaxX;
     volatile uint32_t *tmem_slot_ptr = reinterpret_cast<volatile uint32_t *>(smem + (tmem_slot - smem0));
     volatile uint32_t *abort_flag = tmem_slot_ptr + 1;
 
@@ -206,6 +209,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         for (uint32_t i = 0; i < args.x_stages; ++i) {
             mbar_init(x_full + 8u * i, 1u);
             mbar_init(x_empty + 8u * i, 1u);
+            mbar_init(x_ready + 8u * i, kEpilogueWarps);
         }
         for (uint32_t i = 0; i < args.a_stages; ++i) {
             mbar_init(a_full + 8u * i, kMidGroupWarps);
@@ -331,6 +335,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         // ---------------------------------------------------------------- MMA issue
         if (elect_one()) {
             const uint32_t idesc = umma_idesc(kRows, ntok, 0u, 0u);
+            const uint32_t x_bar = args.x_bf16 != 0u ? x_ready : x_full;
             // (counted up, not divided: a division by a number that only the launch knows takes longer
             // than the MMAs of a segment)
             uint32_t xst = 0u, xph = 0u;
@@ -346,7 +351,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                 }
                 tc_fence_after_sync();
                 for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
-                    if (!x_there && !mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
+                    if (!x_there && !mbar_wait_hot(x_bar + 8u * xst, xph, abort_flag, args.status)) {
                         ok = false;
                         break;
                     }
@@ -363,7 +368,7 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                         a_there = mbar_test_wait(a_full + 8u * anext, anext_ph);
                         if (p + 1u == pair) {
                             const bool wraps = xst + 1u == args.x_stages;
-                            x_there = mbar_test_wait(x_full + 8u * (wraps ? 0u : xst + 1u), wraps ? xph ^ 1u : xph);
+                            x_there = mbar_test_wait(x_bar + 8u * (wraps ? 0u : xst + 1u), wraps ? xph ^ 1u : xph);
                         }
                         const uint32_t d_tmem = tmem_base + buf * args.buffer_columns + p * ntok;
                         const uint32_t a_tmem = tmem_base + args.a_column0 + ast * (kSegK / 2u);
@@ -451,6 +456,38 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             if (ast >= args.a_stages) {
                 ast -= args.a_stages;
                 aph ^= 1u;
+            }
+        }
+    } else if (args.x_bf16 != 0u) {
+        // ---------------------------------------------------------------- x to binary16
+        // The storing warps have nothing to store before the block's one piece is done.
+        uint32_t st = 0u, ph = 0u;
+        for (uint32_t g = 0; g < work.left; ++g) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_hot(x_full + 8u * st, ph, abort_flag, args.status))) {
+                break;
+            }
+            const uint32_t mine = smem0 + st * x_seg_bytes + threadIdx.x * 16u;
+#pragma unroll 1
+            for (uint32_t at = mine; at < mine + x_seg_bytes; at += 4u * kMidConvertStep) {
+                uint32_t v[4][4];
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; ++i) {
+                    ld_shared_v4(at + i * kMidConvertStep, v[i][0], v[i][1], v[i][2], v[i][3]);
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; ++i) {
+                    st_shared_v4(at + i * kMidConvertStep, bf16x2_to_f16x2(v[i][0]), bf16x2_to_f16x2(v[i][1]),
+                                 bf16x2_to_f16x2(v[i][2]), bf16x2_to_f16x2(v[i][3]));
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0u) {
+                mbar_arrive(x_ready + 8u * st);
+            }
+            if (++st == args.x_stages) {
+                st = 0u;
+                ph ^= 1u;
             }
         }
     }
@@ -853,6 +890,15 @@ static void mid_accuracy(MidPlan &plan, unsigned int n, unsigned int segs, unsig
     }
 }
 
+// Where the storing warps are free until the block's last sums are there they turn bfloat16 x into binary16 as it comes,
+// and no launch has to do it before this one.  Four warps do 32 rows beside everything else (6144 x 4096 14.6 -> 13.6 us,
+// 28672 x 4096 32.2 -> 30.0; 13.2 with binary16 x); 64 rows where a segment of x meets two whole slabs (28672 x 4096
+// 34.8 -> 33.4), not in a cluster (4096 x 14336 22.0 -> 23.3); 100 rows take longer than the launch did (27.8 -> 32.3).
+bool mid_converts_x(const MidPlan &plan)
+{
+    return (plan.cluster > 1u ? plan.ntok <= 32u : plan.turns == 1u && plan.ntok <= 64u) && plan.run_segs == 0u;
+}
+
 MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
                  unsigned int epilogue)
 {
@@ -901,9 +947,10 @@ MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm
 cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
                                unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
                                unsigned int ldy, unsigned int epilogue, float *partial, unsigned int *flags,
-                               unsigned long long tile_floats, unsigned int *status, bool overlap)
+                               unsigned long long tile_floats, unsigned int *status, bool overlap, bool x_bf16)
 {
     MidArgs args = {};
+    args.x_bf16 = x_bf16 ? 1u : 0u;
     args.n = n;
     args.k = k;
     args.m_max = m;

@@ -648,10 +648,12 @@ struct MidPlan {
 };
 MidPlan mid_plan(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned long long tile_floats,
                  unsigned int epilogue);
+// Whether the kernel takes bfloat16 x as it is under this plan (else it wants binary16).
+bool mid_converts_x(const MidPlan &plan);
 cudaError_t launch_mid_product(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap &tx, const MidPlan &plan,
                                unsigned int n, unsigned int k, unsigned int m, const unsigned int *m_dev, void *y, int y_dtype,
                                unsigned int ldy, unsigned int epilogue, float *partial, unsigned int *flags,
-                               unsigned long long tile_floats, unsigned int *status, bool overlap);
+                               unsigned long long tile_floats, unsigned int *status, bool overlap, bool x_bf16);
 cudaError_t launch_mid_grouped(cudaStream_t stream, const CUtensorMap &tw, const CUtensorMap *tw_second,
                                const CUtensorMap &tx, bool table_late, unsigned int grid, unsigned int k, unsigned int ntok, const GroupTile *tiles, const unsigned int *count_dev,
                                const unsigned int *row_map, void *y, unsigned int ldy, int y_dtype, unsigned int epilogue,
