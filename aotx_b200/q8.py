@@ -8,7 +8,7 @@ import ctypes as C
 
 import numpy as np
 
-from .library import load_library
+from .library import load_library, native_call
 
 Q8_0 = 8  # cuda/model/model.cuh:31
 F32, F16, BF16 = 0, 1, 2
@@ -126,6 +126,10 @@ class Q8Context:
         handle = C.c_void_p()
         self._check(self.lib.aotx_q8_init(C.byref(handle), device))
         self.handle = handle
+        self._address = handle.value     # None once closed, which every entry point refuses
+        self._matmul = native_call(self.lib, "aotx_q8_matmul")
+        self._matmul_fused = native_call(self.lib, "aotx_q8_matmul_fused")
+        self._dequant = native_call(self.lib, "aotx_q8_dequant")
         # The current stream as a number.  (Through the Stream object it took 2.4 us of the 8.2 us
         # that the smallest product keeps the host; this takes 0.1.)
         self._device_index = self.device.index
@@ -133,6 +137,7 @@ class Q8Context:
 
     def close(self):
         if getattr(self, "handle", None) is not None:
+            self._address = None
             self.lib.aotx_q8_destroy(self.handle)
             self.handle = None
 
@@ -172,8 +177,7 @@ class Q8Context:
         torch = _torch()
         if out is None:
             out = torch.empty((rows, k), dtype=torch.float16, device=self.device)
-        self._check(self.lib.aotx_q8_dequant(self.handle, self._stream(), w.data_ptr(), type, k,
-                                             first_row, rows, out.data_ptr()))
+        self._check(self._dequant(self._address, self._stream(), w.data_ptr(), type, k, first_row, rows, out.data_ptr()))
         return out
 
     # -- aotx_model_matrix --------------------------------------------------------------
@@ -185,8 +189,8 @@ class Q8Context:
         if y is None:
             torch = _torch()
             y = torch.empty((m, n), dtype=y_dtype or torch.float32, device=self.device)
-        code = self.lib.aotx_q8_matmul(
-            self.handle, self._stream(), w.data_ptr(), type, n, k, x.data_ptr(),
+        code = self._matmul(
+            self._address, self._stream(), w.data_ptr(), type, n, k, x.data_ptr(),
             _dtype_code(x.dtype), m, m_dev.data_ptr() if m_dev is not None else None,
             y.data_ptr(), _dtype_code(y.dtype))
         if code != 0:
@@ -205,8 +209,8 @@ class Q8Context:
             torch = _torch()
             width = n // 2 if epilogue == EPILOGUE_SWIGLU else n
             y = torch.empty((m, width), dtype=y_dtype or torch.float32, device=self.device)
-        self._check(self.lib.aotx_q8_matmul_fused(
-            self.handle, self._stream(), w.data_ptr(), type, n, k, x.data_ptr(),
+        self._check(self._matmul_fused(
+            self._address, self._stream(), w.data_ptr(), type, n, k, x.data_ptr(),
             _dtype_code(x.dtype), m, m_dev.data_ptr() if m_dev is not None else None,
             y.data_ptr(), _dtype_code(y.dtype), epilogue))
         return y
