@@ -1,0 +1,34 @@
+"""The package's own way of calling the library (csrc/host_calls.c) passes what ctypes passes, and refuses what is no call."""
+import ctypes as C
+
+import pytest
+
+from aotx_b200.library import load_library, native_call
+
+ARGUMENTS = {"aotx_q8_matmul": (None, 0, 0, 8, 1, 32, 0, 0, 1, None, 0, 0),
+             "aotx_q8_matmul_fused": (None, 0, 0, 8, 1, 32, 0, 0, 1, None, 0, 0, 0),
+             "aotx_q8_dequant": (None, 0, 0, 8, 32, 0, 1, 0)}
+
+
+@pytest.mark.parametrize("name", sorted(ARGUMENTS))
+def test_same_answer_as_through_ctypes(name):
+    lib = load_library()
+    call = native_call(lib, name)
+    assert call(*ARGUMENTS[name]) == getattr(lib, name)(*ARGUMENTS[name]) != 0      # no context
+    for wrong in (ARGUMENTS[name][:-1], ARGUMENTS[name] + (0,), (1.5,) + ARGUMENTS[name][1:], ("x",) + ARGUMENTS[name][1:]):
+        with pytest.raises(TypeError):
+            call(*wrong)
+
+
+def test_every_argument_arrives_in_its_place():
+    seen = []
+    kind = C.CFUNCTYPE(C.c_int, *[C.c_void_p] * 3, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p, C.c_int, C.c_uint32, C.c_void_p,
+                       C.c_void_p, C.c_int, C.c_int)
+
+    class Library:
+        aotx_q8_matmul_fused = kind(lambda *args: seen.append(args) or 7)
+
+    big = 0x7F1234567890
+    sent = (big, big + 1, big + 2, 8, 2 ** 32 - 1, 2 ** 32 + 5, big + 3, 1, 9, None, big + 4, 2, -1)
+    assert native_call(Library, "aotx_q8_matmul_fused")(*sent) == 7
+    assert seen == [(big, big + 1, big + 2, 8, 2 ** 32 - 1, 5, big + 3, 1, 9, None, big + 4, 2, -1)]
