@@ -38,6 +38,7 @@
 // cuda/model/graph_host.cu:31-39 for these batches).
 #include <cuda.h>
 
+#include "q8_decode_operands.cuh"
 #include "q8_launch.h"
 #include "q8_tile.cuh"
 #include "q8_warp_ptx.cuh"
@@ -47,7 +48,6 @@ namespace q8 {
 constexpr uint32_t kWarpThreads = 384;
 constexpr uint32_t kWarpCompute = 8;       // multiplying warps
 constexpr uint32_t kWarpLoaders = 4;       // warps that bring x in
-constexpr uint32_t kWarpXRow = 528;        // bytes of a row of x in a stage: 256 halves and a shift of 16 bytes
 
 template <int NTOK>
 struct WarpShape {
@@ -70,45 +70,6 @@ struct WarpShape {
     static constexpr uint32_t smem_bytes = bar_offset + bar_count * 8 + 16 + 1024;
     static_assert(2u * (smem_bytes + 1024u) <= 228u * 1024u, "two blocks' shared memory on one SM");
 };
-
-// Bring a row piece of x into the order of the weights and store it: `v` holds halves 8 lane ..
-// 8 lane + 7 of the segment.  Blocks of 32 weights are 4 lanes; even blocks are turned by two
-// halves (one word), so a lane needs its neighbour's first word.
-template <bool BF>
-__device__ __forceinline__ void stage_x_row(uint4 v, uint32_t row_at, uint32_t lane)
-{
-    if (BF) {
-        v.x = bf16x2_to_f16x2(v.x);
-        v.y = bf16x2_to_f16x2(v.y);
-        v.z = bf16x2_to_f16x2(v.z);
-        v.w = bf16x2_to_f16x2(v.w);
-    }
-    const uint32_t next = __shfl_sync(0xFFFFFFFFu, v.x, (int)((lane & ~3u) | ((lane + 1u) & 3u)));
-    if ((lane & 4u) == 0u) {
-        v = make_uint4(v.y, v.z, v.w, next);
-    }
-    // step = two per block, lane t of the MMA: halves 4t .. 4t+3 of the step's sixteen
-    const uint32_t step = ((lane >> 2) & 1u) * 2u + ((lane >> 1) & 1u);
-    const uint32_t at = row_at + (lane >> 3) * 128u + (lane & 1u) * 64u + step * 8u;
-    st_shared_v2(at, v.x, v.y);
-    st_shared_v2(at + 32u, v.z, v.w);
-}
-
-// The halves of one 32-weight block of rows g and g + 8 as the two steps' A operands.
-__device__ __forceinline__ void block_operands(const uint32_t (&first)[2], const uint32_t (&second)[2],
-                                               const uint32_t (&d_bits)[2], uint32_t (&a)[2][4])
-{
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const __half2 d2 = *reinterpret_cast<const __half2 *>(&d_bits[r]);
-        const uint32_t f0 = first[r] ^ 0x80808080u;
-        const uint32_t f1 = second[r] ^ 0x80808080u;
-        a[0][r] = dequant_pair<0>(f0, d2);
-        a[0][r + 2] = dequant_pair<1>(f0, d2);
-        a[1][r] = dequant_pair<0>(f1, d2);
-        a[1][r + 2] = dequant_pair<1>(f1, d2);
-    }
-}
 
 // Finished sums: value `i` of a thread belongs to row row_of(i) of the tile and row token_of(i) of x.
 static __device__ __forceinline__ uint32_t row_of(uint32_t i, uint32_t warp, uint32_t g)
@@ -377,24 +338,8 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *x_
                 const unsigned char *x_at = x_lane + st * S::x_stage_bytes;
 #pragma unroll
                 for (uint32_t b = 0; b < kSegK / 32u; ++b) {
-                    // block b: its scale in word 0 (low half) or 8 (high half) of the pair
-                    const uint32_t word0 = (b / 2u) * 68u + (b & 1u) * 32u;
                     uint32_t a[2][4];
-                    uint32_t first[2], second[2], d_bits[2];
-#pragma unroll
-                    for (uint32_t r = 0; r < 2u; ++r) {
-                        const unsigned char *row = w_at + r * 8u * kSegBytes + word0;
-                        const uint32_t scale = *reinterpret_cast<const uint32_t *>(row - 4u * t);
-                        first[r] = *reinterpret_cast<const uint32_t *>(row + 4u);
-                        second[r] = *reinterpret_cast<const uint32_t *>(row + 20u);
-                        if ((b & 1u) == 0u) {
-                            second[r] = prmt(second[r], scale, turn);
-                            d_bits[r] = prmt(scale, scale, 0x1010u);
-                        } else {
-                            d_bits[r] = prmt(scale, scale, 0x3232u);
-                        }
-                    }
-                    block_operands(first, second, d_bits, a);
+                    block_of_rows(w_at, w_at + 8u * kSegBytes, t, turn, b, a);
                     // one step of all columns before the next: an MMA that adds to the sums of the one
                     // before it waits for them, about four MMAs' time
                     uint4 xv[S::tiles];

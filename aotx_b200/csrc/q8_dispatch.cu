@@ -2,6 +2,7 @@
 // grid and its scratch.
 //
 //   rows of x     kernel                                                          file
+//   1 .. 4        whole rows of w per block, where w has 3000 to 4736 of them      q8_decode_rows.cu
 //   1 .. 16       weights through registers into mma.sync, two blocks per SM      q8_decode_warp.cu
 //   17 .. 128     weights through tensor memory, one block per SM; also the       q8_mid.cu
 //                 grouped products of the routed experts
@@ -217,7 +218,13 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
 #endif
 
     CUtensorMap tw, tx;
-    if (!map_weights(encode, &tw, w, n, k, kRows) || (!warp_kernel && !map_rows(encode, &tx, x, m, k, ntok, x_bf16 != 0))) {
+#ifndef Q8_HOST_EMULATION
+    const unsigned int height = warp_kernel ? rows_height(n, k, m, sm_count, epilogue) : 0u;
+    const unsigned int box_rows = height != 0u ? height : kRows;
+#else
+    const unsigned int box_rows = kRows;
+#endif
+    if (!map_weights(encode, &tw, w, n, k, box_rows) || (!warp_kernel && !map_rows(encode, &tx, x, m, k, ntok, x_bf16 != 0))) {
         return cudaErrorInvalidValue;
     }
 
@@ -270,6 +277,9 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
                                                        scratch.blocks, &cluster);
         args.split = cluster;
 #ifndef Q8_HOST_EMULATION
+        if (height != 0u) {
+            return launch_decode_rows(stream, tw, x, x_bf16 != 0, height, args, y_dtype);
+        }
         if (warp_kernel) {
             return launch_decode_warp(stream, tw, x, args, decode_blocks, cluster, y_dtype);
         }

@@ -639,6 +639,12 @@ cudaError_t launch_decode_kernel(cudaStream_t stream, const CUtensorMap &tw, con
 cudaError_t launch_decode_warp(cudaStream_t stream, const CUtensorMap &tw, const void *x, const UmmaArgs &args,
                                unsigned int grid, unsigned int cluster, int y_dtype);
 
+// The product for one to four rows of x in tiles of whole rows of w (q8_decode_rows.cu): the tiles' height, which is the
+// tensor map's box's (0: not by this kernel), and the launch.
+unsigned int rows_height(unsigned int n, unsigned int k, unsigned int m, unsigned int sm_count, unsigned int epilogue);
+cudaError_t launch_decode_rows(cudaStream_t stream, const CUtensorMap &tw, const void *x, bool x_bf16, unsigned int height,
+                               const UmmaArgs &from, int y_dtype);
+
 // The product for 17 to 128 rows and the grouped products (q8_mid.cu): how a product's rows of w are
 // dealt (tiles of `pair` slabs of slab_rows rows; `cluster` blocks share a tile's depth, or
 // 1: `turns` whole tiles per block, 0: units), and the launches.
