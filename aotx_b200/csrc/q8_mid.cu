@@ -666,18 +666,23 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const uint32_t quarter_lanes = warp & 3u;
             const uint32_t lane_taddr = tmem_base + ((quarter_lanes * 32u) << 16);
             const uint32_t row = quarter_lanes * 32u + lane;
-            for (uint32_t c = warp >> 2; c < pair * ntok / 16u; c += kMidWeightWarp / 4u) {
+            const uint32_t chunks = quarter_lanes * 32u < args.slab_rows ? pair * ntok / 16u : 0u;     // (rows of w past the slab)
+            for (uint32_t c = warp >> 2; c < chunks; c += kMidWeightWarp / 4u) {
                 const uint32_t p = c / (ntok / 16u);
                 const uint32_t c0 = (c - p * (ntok / 16u)) * 16u;
                 uint32_t v[16];
                 load_sums(lane_taddr + p * ntok + c0, args.read_chains, args.acc_columns, v);
+                uint32_t owner = c0 / share;
+                uint32_t run = (c0 - owner * share) / 4u;
 #pragma unroll
                 for (uint32_t i = 0; i < 16u; i += 4u) {
-                    const uint32_t owner = (c0 + i) / share;
-                    const uint32_t run = (c0 + i - owner * share) / 4u;
                     const uint32_t at = smem0 + (((crank * pair + p) * (share / 4u) + run) * kRows + row) * 16u;
                     st_shared_cluster_v4_f32(mapa_shared(at, owner), __uint_as_float(v[i]), __uint_as_float(v[i + 1u]),
                                              __uint_as_float(v[i + 2u]), __uint_as_float(v[i + 3u]));
+                    if (++run == share / 4u) {
+                        run = 0u;
+                        ++owner;
+                    }
                 }
             }
             tc_fence_before_sync();
@@ -700,6 +705,9 @@ q8_stream_kernel_mid(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         for (uint32_t at = warp; at < runs * (kRows / 32u); at += kMidThreads / 32u) {
             const uint32_t local = at / (kRows / 32u);                  // slab * (share / 4) + run within the share
             const uint32_t row = (at % (kRows / 32u)) * 32u + lane;
+            if (row - lane >= args.slab_rows) {
+                continue;
+            }
             const uint32_t p = local / (share / 4u);
             const uint32_t token = crank * share + (local - p * (share / 4u)) * 4u;
             float4 four = recv[local * kRows + row];
