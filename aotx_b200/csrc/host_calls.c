@@ -1,5 +1,5 @@
 /* The entry points that a decode step calls most, from Python without ctypes: converting twelve arguments there takes
- * 1.6 us, a third of what the host spends on a product; here 0.3.  The caller gives the function's address (the
+ * 1.6 us, a third of what the host spends on a product; here 0.2.  The caller gives the function's address (the
  * library's, of whichever library is loaded) and its arguments as integers, None for a null pointer; integers are taken
  * modulo their width, as ctypes takes them.  The interpreter's lock is released during the call. */
 #define PY_SSIZE_T_CLEAN

@@ -21,7 +21,7 @@
 //     value (`chains`), or, in a cluster, an accumulator that is emptied into a sum of its own every few segments
 //     (`run_segs`).  mid_accuracy says how many.
 //
-// 23 warps, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
+// 23 warps, one block per SM: 0-3 store (and before that turn bfloat16 x into binary16, mid_converts_x), 4-19 convert, 20 copies weights, 21 copies x, 22 issues the MMAs.  Every wait is bounded and raises a
 // status bit when it runs out.  Reference kernels replaced: as q8_stream.cu.
 #include <cuda.h>
 

@@ -67,7 +67,7 @@ def load_library():
 
 def native_call(lib, name):
     """An entry point as a callable that takes its arguments as integers and None, converted by this package's own
-    module (csrc/host_calls.c) and not by ctypes: 0.3 us of a call in place of 1.6."""
+    module (csrc/host_calls.c) and not by ctypes: 0.2 us of a call in place of 1.6."""
     try:
         from . import _host_calls
     except ImportError as error:
