@@ -171,7 +171,8 @@ cudaError_t launch_expert_sum_parts(cudaStream_t stream, const ProjParts &proj, 
 // The streaming tensor-core product.  Scratch, in two sets that alternate between launches:
 // `partial` holds one float tile of 128 x token_tile per block of the grid, `flags` kFlagWords
 // words per block (zero between launches); `status` is one word that kernels only ever OR bits into.
-constexpr unsigned int kFlagWords = 8u; // hand-over flags per block: one per warp that publishes
+// Words per block: the flags of the quarters of its part, then, where several finish a tile (q8_pair.cu), what they count.
+constexpr unsigned int kFlagWords = 8u;
 
 struct UmmaScratch {
     float *partial;

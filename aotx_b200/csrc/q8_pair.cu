@@ -819,14 +819,17 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (run < end) {
                 wait_for_parts(args, at, 0u, rank, lanes, lane, abort_flag);
             }
-            // This warp has published and has seen what it needs.  The last warp of the holders to say so clears the
-            // flag, and the count of those that have.
-            unsigned int *flag = args.flags + kFlagWords * pair_cut_slot(at, lane < at.holders ? lane : 0u, rank) + lanes;
-            const uint32_t all = at.holders * kPublishers;
+            // This warp has published, and has seen what it needs of the others: lane 0, which has published for the warp, says
+            // so, and the last warp of the holders to say so clears their flags and this count.  Release here and
+            // acquire there, so that every publication lies before the clearing, those of warps that had nothing to
+            // wait for among them (no rows of w or of x left for them).
+            unsigned int *count = args.flags + kFlagWords * pair_cut_slot(at, 0u, rank) + kEpilogueWarps + lanes;
             uint32_t came = 0u;
-            if (lane < at.holders) {
-                came = atomicAdd(flag + kEpilogueWarps, 1u) + 1u;
+            if (lane == 0u) {
+                __threadfence();
+                came = atomicAdd(count, 1u) + 1u;
             }
+            __syncwarp();
 #pragma unroll 1
             for (; run < end; run += kPairWeightWarp / 4u) {
                 const uint32_t c0 = run * kPairShareRows;
@@ -845,17 +848,14 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
                 store_rows_direct<YT>(args.to, gated, lane, mine, col, tok0 + c0, tok0 + rows, v);
             }
-            for (uint32_t h = lane;;) {
-                if (came == all) {
-                    *reinterpret_cast<volatile unsigned int *>(flag) = 0u;
-                    *reinterpret_cast<volatile unsigned int *>(flag + kEpilogueWarps) = 0u;
+            if (__shfl_sync(0xFFFFFFFFu, came, 0) == at.holders * kPublishers) {
+                __threadfence();
+                for (uint32_t h = lane; h < at.holders; h += 32u) {
+                    *reinterpret_cast<volatile unsigned int *>(args.flags + kFlagWords * pair_cut_slot(at, h, rank) + lanes) = 0u;
                 }
-                h += 32u;
-                if (h >= at.holders) {
-                    break;
+                if (lane == 0u) {
+                    *reinterpret_cast<volatile unsigned int *>(count) = 0u;
                 }
-                flag = args.flags + kFlagWords * pair_cut_slot(at, h, rank) + lanes;
-                came = atomicAdd(flag + kEpilogueWarps, 1u) + 1u;
             }
         }
     }
