@@ -169,20 +169,12 @@ __device__ __forceinline__ PairCut pair_cut(const PairWork &work, uint32_t id)
     return cut;
 }
 
-// A cut tile is finished by the pair that began it, or, where it has more holders than a pair has units by so many, by
-// all its holders.  The one that began it reads as many tiles of sums as there are others, 0.8 us a round trip, but most
-// of it before its own sums are there: the longer the runs, the more.  All together read one tile's worth each, and
-// everybody waits for the last to publish.  (Beginner against all: 1000 x 2048, 200 rows, 1 unit and 8 holders, 19.8 and
-// 11.3 us; 1024 x 4096, 300 rows, 24.1 and 16.4; 2560 x 2560, 300 rows, 2.7 units and 4 or 5 holders, 15.7 and 16.1, with
-// the line between 4 and 5 14.7; 2560 x 9728, 10.3 units, 4 or 5 holders, 25.9 and 27.3.)
-constexpr uint32_t kPairShareMore = 3;
-
 // What a block works on.  One thread works it out and the roles read it from shared memory: the divisions take a
 // microsecond, and kept in registers across the roles it costs the converters theirs.
 struct PairPlan {
     uint32_t m;                 // live rows of x
     PairWork work;
-    uint32_t share_from;        // from this many holders on a cut tile is finished by all of them
+    uint32_t share_from;        // from this many holders on a cut tile may be finished by all of them
     PairCut begun, begins;      // the cut tiles that the pair has pieces of: begun by another pair, and by itself
 };
 static_assert(sizeof(PairPlan) <= kPairPlanBytes, "room for the plan");
@@ -190,7 +182,7 @@ static_assert(sizeof(PairPlan) <= kPairPlanBytes, "room for the plan");
 __device__ __forceinline__ void pair_plan_cuts(PairPlan *plan, uint32_t id)
 {
     plan->begun.holders = plan->begins.holders = 0u;
-    plan->share_from = (plan->work.pieces != 0u ? plan->work.segs / plan->work.pieces : plan->work.each) + kPairShareMore;
+    plan->share_from = pair_share_from(plan->work);
     PairWork ahead = plan->work;
     ahead.whole_left = 0u;
     while (ahead.next()) {
@@ -212,6 +204,50 @@ __device__ __forceinline__ uint32_t pair_slot(uint32_t block, bool begins)
 __device__ __forceinline__ uint32_t pair_cut_slot(const PairCut &cut, uint32_t holder, uint32_t rank)
 {
     return pair_slot(2u * (cut.first + holder) + rank, holder == 0u);
+}
+
+// Words of a quarter of a cut tile that its holders may finish together, behind the flags of the first two holders'
+// parts: how many warps have published and seen what they need, and which holders have begun (kPairAlone).
+__device__ __forceinline__ unsigned int *pair_count(unsigned int *flags, const PairCut &cut, uint32_t rank, uint32_t lanes)
+{
+    return flags + kFlagWords * pair_cut_slot(cut, 0u, rank) + kEpilogueWarps + lanes;
+}
+
+__device__ __forceinline__ unsigned int *pair_begun(unsigned int *flags, const PairCut &cut, uint32_t rank, uint32_t lanes)
+{
+    return flags + kFlagWords * pair_cut_slot(cut, 1u, rank) + kEpilogueWarps + lanes;
+}
+
+// This block runs: for the tiles that it may have to finish together with others.  (By a thread that counts itself in
+// pair_count later on, so that nothing is added to a word after it has been cleared.)
+__device__ __forceinline__ void pair_say_begun(unsigned int *flags, const PairPlan &plan, uint32_t rank, uint32_t lanes)
+{
+    if (plan.begun.holders >= plan.share_from) {
+        atomicAdd(pair_begun(flags, plan.begun, rank, lanes), 1u);
+    }
+    if (plan.begins.holders >= plan.share_from) {
+        atomicAdd(pair_begun(flags, plan.begins, rank, lanes), 1u);
+    }
+}
+
+// Of which of a pair's cut tiles all holders have begun by now: bit 0 the tile that others began, bit 1 its own.
+__device__ __forceinline__ uint32_t pair_all_begun(unsigned int *flags, const PairPlan &plan, uint32_t rank, uint32_t lanes)
+{
+    const uint32_t first = plan.begun.holders >= plan.share_from ? ld_relaxed_gpu(pair_begun(flags, plan.begun, rank, lanes)) : 0u;
+    const uint32_t second = plan.begins.holders >= plan.share_from ? ld_relaxed_gpu(pair_begun(flags, plan.begins, rank, lanes)) : 0u;
+    return (__all_sync(0xFFFFFFFFu, first == plan.begun.holders) ? 1u : 0u)
+         | (__all_sync(0xFFFFFFFFu, second == plan.begins.holders) ? 2u : 0u);
+}
+
+// Whether all holders finish a quarter of a cut tile; else the one that began the tile does.
+__device__ __forceinline__ bool pair_together(unsigned int *word, uint32_t holders)
+{
+    uint32_t seen = ld_relaxed_gpu(word);
+    while (pair_undecided(seen, holders)) {
+        const uint32_t now = atomicCAS(word, seen, seen | kPairAlone);
+        seen = now == seen ? seen | kPairAlone : now;
+    }
+    return seen == holders;
 }
 
 // A partial sum that another block has left, past the first-level cache.  Volatile, so that the loads of a piece are
@@ -673,6 +709,14 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const uint32_t release_bar = mapa_shared(acc_empty, 0u);
         uint32_t flip = 0u;      // the two turns of a helper's staging buffer
         grid_dependency_wait();
+        if (helper == 0u) {
+            mbar_wait_hot(cuts_bar, 0u, abort_flag, args.status);
+            if (lane == 0u) {
+                pair_say_begun(args.flags, *plan, rank, lanes);
+            }
+            __syncwarp();
+        }
+        uint32_t all_begun = 0u;      // bits: of which of the pair's two cut tiles all holders are known to have begun
         // rows of y on a boundary of 16 bytes (the drain of a whole tile) or of four values (the others)
         const bool aligned16 = ((size_t)args.to.ldy * sizeof(YT)) % 16u == 0u && (reinterpret_cast<uintptr_t>(args.to.y) % 16u) == 0u;
         const bool aligned4 = (args.to.ldy % 4u) == 0u && (reinterpret_cast<uintptr_t>(args.to.y) % (4u * sizeof(YT))) == 0u;
@@ -714,6 +758,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (others != 0u && c0 < rows && mine != 0u) {
                 // the others' parts of this warp's first run of rows, before its own sums are there
                 add_others(v, c0);
+            }
+            if (last && cut) {
+                // asked before the last sums are there, so that the answer is
+                all_begun = pair_all_begun(args.flags, *plan, rank, lanes);
             }
             // (a helper has seen none of the pieces before, so it does not ask for a parity of their barrier)
             if (!__all_sync(0xFFFFFFFFu, helper == 0u ? mbar_wait_hot(acc_full, turn & 1u, abort_flag, args.status)
@@ -791,8 +839,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         // ------------------------------------------------------------ tiles of many holders
         // Every holder finishes a share of the tile's rows of x: the parts of all holders, its own among them, added
-        // in the order of the depth.  A pair has published all it has before it waits here, so that whoever waits,
-        // waits for pairs that need nothing from it.
+        // in the order of the depth.  A pair has published all it has before it waits here, and waits only where all
+        // holders have begun: it holds its SMs while it waits, and a launch of another stream may hold those that a
+        // holder yet needs.  Where not all have begun when the first comes here, the pair that began the tile
+        // finishes it and the others go, as with few holders.  (tests/schedule_check.cu, point 9)
         mbar_wait_hot(cuts_bar, 0u, abort_flag, args.status);
 #pragma unroll 1
         for (uint32_t which = 0; which < 2u; ++which) {
@@ -810,9 +860,13 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint32_t col = gated ? j / 2u : j;
             const bool staged = aligned4 && (columns % 4u) == 0u;
             const uint32_t runs = (rows + kPairShareRows - 1u) / kPairShareRows;
-            const uint32_t index = pair_id - at.first;
-            const uint32_t end = (index + 1u) * runs / at.holders;
-            uint32_t run = index * runs / at.holders + helper;
+            if (((all_begun >> which) & 1u) == 0u) {
+                const bool together = lane == 0u && pair_together(pair_begun(args.flags, at, rank, lanes), at.holders);
+                all_begun |= (__any_sync(0xFFFFFFFFu, together) ? 1u : 0u) << which;
+            }
+            uint32_t run, end;
+            pair_share(((all_begun >> which) & 1u) != 0u, pair_id - at.first, at.holders, runs, &run, &end);
+            run += helper;
             if (mine == 0u) {
                 run = end;
             }
@@ -820,10 +874,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 wait_for_parts(args, at, 0u, rank, lanes, lane, abort_flag);
             }
             // This warp has published, and has seen what it needs of the others: lane 0, which has published for the warp, says
-            // so, and the last warp of the holders to say so clears their flags and this count.  Release here and
+            // so, and the last warp of the holders to say so clears their flags and both counts.  Release here and
             // acquire there, so that every publication lies before the clearing, those of warps that had nothing to
             // wait for among them (no rows of w or of x left for them).
-            unsigned int *count = args.flags + kFlagWords * pair_cut_slot(at, 0u, rank) + kEpilogueWarps + lanes;
+            unsigned int *count = pair_count(args.flags, at, rank, lanes);
             uint32_t came = 0u;
             if (lane == 0u) {
                 __threadfence();
@@ -855,6 +909,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
                 if (lane == 0u) {
                     *reinterpret_cast<volatile unsigned int *>(count) = 0u;
+                    *reinterpret_cast<volatile unsigned int *>(pair_begun(args.flags, at, rank, lanes)) = 0u;
                 }
             }
         }

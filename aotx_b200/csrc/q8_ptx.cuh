@@ -271,7 +271,15 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const unsigned int *p)
     return v;
 }
 
-// The same at system scope: a word that another GPU of the box writes or reads through a
+// A word that others add to, as it is at some time.
+__device__ __forceinline__ uint32_t ld_relaxed_gpu(const unsigned int *p)
+{
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// ld_acquire_gpu at system scope: a word that another GPU of the box writes or reads through a
 // peer-mapped address.
 __device__ __forceinline__ uint32_t ld_acquire_sys(const unsigned int *p)
 {

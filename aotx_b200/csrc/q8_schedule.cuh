@@ -219,4 +219,34 @@ __host__ __device__ __forceinline__ uint32_t pair_last_holder(const PairWork &wo
     return pair_holder(work, (tile - work.first_cut + 1u) * work.segs - 1u);
 }
 
+// A cut tile is finished by the pair that began it, or, where it has more holders than a pair has units by so many and
+// all of them run (pair_undecided), by all its holders.  The one that began it reads as many tiles of sums as there are
+// others, 0.8 us a round trip, but most of it before its own sums are there: the longer the runs, the more.  All together read one tile's worth each, and
+// everybody waits for the last to publish.  (Beginner against all: 1000 x 2048, 200 rows, 1 unit and 8 holders, 19.8 and
+// 11.3 us; 1024 x 4096, 300 rows, 24.1 and 16.4; 2560 x 2560, 300 rows, 2.7 units and 4 or 5 holders, 15.7 and 16.1, with
+// the line between 4 and 5 14.7; 2560 x 9728, 10.3 units, 4 or 5 holders, 25.9 and 27.3.)
+constexpr uint32_t kPairShareMore = 3;
+
+__host__ __device__ __forceinline__ uint32_t pair_share_from(const PairWork &work)
+{
+    return (work.pieces != 0u ? work.segs / work.pieces : work.each) + kPairShareMore;
+}
+
+// What such a tile's holders go by: a word that counts those that have begun, with kPairAlone set by the first that came
+// to wait before all had.  Once all have begun, or the bit is set, it says the same for good.
+constexpr uint32_t kPairAlone = 1u << 31;
+
+__host__ __device__ __forceinline__ bool pair_undecided(uint32_t word, uint32_t holders)
+{
+    return word != holders && (word & kPairAlone) == 0u;
+}
+
+// The runs of rows [run, end) that holder `index` finishes.
+__host__ __device__ __forceinline__ void pair_share(bool together, uint32_t index, uint32_t holders, uint32_t runs, uint32_t *run,
+                                                    uint32_t *end)
+{
+    *run = together ? index * runs / holders : 0u;
+    *end = together ? (index + 1u) * runs / holders : index == 0u ? runs : 0u;
+}
+
 } // namespace q8

@@ -1,6 +1,6 @@
 // Hand-over words of the kernel on pairs of SMs (q8_pair.cu), from a program that has the scratch itself: whatever way
-// cut tiles are finished, every word is zero after the launch, no status bit is set, and a launch that follows right
-// behind gives the same bits.
+// cut tiles are finished, every word is zero after the launch, no status bit is set, and launches that follow right
+// behind, or run beside those of another stream, give the same bits.
 //
 // Prints "pass" at the end; exits 1 on the first failure.
 #include <cuda_fp16.h>
@@ -12,6 +12,8 @@
 #include <vector>
 
 #include "q8_launch.h"
+#include "q8_schedule.cuh"
+#include "q8_tile.cuh"
 
 #define CHECK_CUDA(call)                                                                       \
     do {                                                                                       \
@@ -120,6 +122,34 @@ struct Product {
     void forget() { CHECK_CUDA(cudaMemset(y, 0xFF, (size_t)m * n * sizeof(float))); }
 };
 
+// Say of every cut tile of a launch on set 0 that may be finished by all its holders that one of them came to wait before
+// all had begun: the one that began it finishes it then.  Returns how many tiles that are.
+static unsigned int leave_to_the_first(const Scratch &scratch, const Product &p, unsigned int sm_count)
+{
+    const unsigned int ntok = q8::pair_token_tile(p.m);
+    const unsigned int tiles = (p.n + 255u) / 256u * ((p.m + ntok - 1u) / ntok), segs = p.k / 256u;
+    const unsigned int pairs = tiles * segs < sm_count / 2u ? tiles * segs : sm_count / 2u;
+    unsigned int found = 0;
+    for (unsigned int id = 0; id < pairs; ++id) {
+        q8::PairWork work;
+        q8::pair_deal(&work, id, pairs, tiles, segs);
+        const unsigned int from = q8::pair_share_from(work);
+        while (work.next()) {
+            if (work.s0 != 0u || work.s1 == segs || q8::pair_last_holder(work, id, work.tile) + 1u - id < from) {
+                continue;
+            }
+            found += 1u;
+            for (unsigned int rank = 0; rank < 2u; ++rank) {
+                // the second holder's slot, behind its four flags
+                std::vector<unsigned int> alone(4u, q8::kPairAlone);
+                CHECK_CUDA(cudaMemcpy(scratch.use.flags + q8::kFlagWords * (2u * (id + 1u) + rank) + 4u, alone.data(), 16u,
+                                      cudaMemcpyHostToDevice));
+            }
+        }
+    }
+    return found;
+}
+
 static int fail(const char *what, const Product &p, unsigned int live)
 {
     std::printf("%s: %u x %u, %u rows, %u live\n", what, p.n, p.k, p.m, live);
@@ -138,6 +168,7 @@ int main()
     // block has warps to finish them, and none
     const unsigned int shapes[][3] = {{1000, 2048, 200}, {256, 16384, 150}, {130, 16384, 257}, {130, 4096, 129},
                                       {2560, 2560, 300}, {300, 16384, 140}, {300, 256, 700},   {5000, 1024, 161}};
+    unsigned int shared = 0;
     for (const auto &shape : shapes) {
         for (unsigned int live : {shape[2], 129u, 9u, 1u, 0u}) {
             Product p(shape[0], shape[1], shape[2], live);
@@ -158,7 +189,54 @@ int main()
             if (std::memcmp(first.data(), p.result().data(), first.size() * sizeof(float)) != 0) {
                 return fail("another result", p, live);
             }
+            if (live == shape[2]) {
+                p.forget();
+                shared += leave_to_the_first(scratch, p, sm_count);
+                p.launch(stream, scratch, sm_count, 0u);
+                CHECK_CUDA(cudaStreamSynchronize(stream));
+                if (!scratch.all_zero()) {
+                    return fail("words left by the first holder", p, live);
+                }
+                if (std::memcmp(first.data(), p.result().data(), first.size() * sizeof(float)) != 0) {
+                    return fail("another result by the first holder", p, live);
+                }
+            }
         }
+    }
+    if (shared < 20u) {
+        std::printf("only %u tiles of many holders\n", shared);
+        return 1;
+    }
+    // two streams, one of them of a higher priority, a scratch each
+    int low = 0, high = 0;
+    CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&low, &high));
+    cudaStream_t other;
+    CHECK_CUDA(cudaStreamCreateWithPriority(&other, cudaStreamNonBlocking, high));
+    Scratch scratch2(sm_count);
+    Product deep(256u, 16384u, 150u, 150u), many(1000u, 2048u, 200u, 200u);
+    deep.launch(stream, scratch, sm_count, 0u);
+    CHECK_CUDA(cudaDeviceSynchronize());
+    many.launch(other, scratch2, sm_count, 0u);
+    CHECK_CUDA(cudaDeviceSynchronize());
+    const std::vector<float> want_deep = deep.result(), want_many = many.result();
+    for (unsigned int repeat = 0; repeat < 200u; ++repeat) {
+        deep.launch(stream, scratch, sm_count, repeat);
+        many.launch(other, scratch2, sm_count, 2u * repeat);
+        many.launch(other, scratch2, sm_count, 2u * repeat + 1u);
+        if (repeat % 20u != 19u) {
+            continue;
+        }
+        CHECK_CUDA(cudaDeviceSynchronize());
+        if (!scratch.all_zero() || !scratch2.all_zero()) {
+            return fail("words left beside another stream", deep, deep.m);
+        }
+        if (std::memcmp(want_deep.data(), deep.result().data(), want_deep.size() * sizeof(float)) != 0
+            || std::memcmp(want_many.data(), many.result().data(), want_many.size() * sizeof(float)) != 0) {
+            return fail("another result beside another stream", deep, deep.m);
+        }
+        deep.forget();
+        many.forget();
+        CHECK_CUDA(cudaDeviceSynchronize());
     }
     std::printf("pass\n");
     return 0;

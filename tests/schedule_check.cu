@@ -15,7 +15,10 @@
 //   7. the division between pairs of SMs (PairWork, pair_deal, pair_last_holder in q8_schedule.cuh) has the properties
 //      1 to 4, and where it cuts tiles into pieces of one size, each has kPairMinPiece segments at least;
 //   8. the division between blocks and clusters (MidWork, mid_deal): every unit once, by the block that decode_holder
-//      names where units are dealt, the pieces of a cluster's block within run_segs and in one tile.
+//      names where units are dealt, the pieces of a cluster's block within run_segs and in one tile;
+//   9. launches of pairs that share the SMs (streams of one's own, in any order of steps) come to their end with as few
+//      as one place more than there are launches, and every run of rows of a cut tile is finished once: pair_undecided,
+//      pair_share.  With holders that wait whether or not all others run, some of the same orders have no end.
 //
 // Prints "ok <cases>" and exits 0, or the first violated property and exits 1.
 #include <cstdio>
@@ -266,9 +269,189 @@ static int check_mid(uint32_t tiles, uint32_t segs, uint32_t grid, uint32_t way,
     return 0;
 }
 
+// A launch of pairs, step by step as a pair goes through q8_pair.cu; a quarter of its blocks stands for all.
+struct Launch {
+    struct Cut {
+        uint32_t first = 0, holders = 0, word = 0, published = 0;
+        std::vector<unsigned int> finished;      // per run of rows
+    };
+    struct Pair {
+        int at = -1;                             // -1: has no place yet
+        std::vector<Piece> pieces;               // the cut ones, in order
+        std::vector<int> together;               // per piece; -1: not decided
+    };
+    uint32_t runs, share_from, placed = 0, left = 0;
+    std::vector<Cut> cuts;
+    std::vector<Pair> pairs;
+    bool always;
+
+    Launch(uint32_t tiles, uint32_t segs, uint32_t count, uint32_t runs_, bool always_)
+        : runs(runs_), cuts(tiles), pairs(tiles * segs < count ? tiles * segs : count), always(always_)
+    {
+        count = (uint32_t)pairs.size();
+        for (uint32_t id = 0; id < count; ++id) {
+            PairWork w;
+            pair_deal(&w, id, count, tiles, segs);
+            share_from = pair_share_from(w);
+            while (w.next()) {
+                if (w.s0 == 0u && w.s1 == w.segs) {
+                    continue;
+                }
+                pairs[id].pieces.push_back({w.tile, w.s0, w.s1});
+                pairs[id].together.push_back(-1);
+                Cut &cut = cuts[w.tile];
+                cut.first = cut.holders == 0u ? id : cut.first;
+                cut.holders += 1u;
+                cut.finished.assign(runs, 0u);
+            }
+        }
+    }
+    bool shared(const Cut &cut) const { return cut.holders >= share_from; }
+    bool done() const { return left == pairs.size(); }
+    bool place()
+    {
+        if (placed == pairs.size()) {
+            return false;
+        }
+        pairs[placed++].at = 0;
+        return true;
+    }
+    void finish(Cut &cut, uint32_t begin, uint32_t end)
+    {
+        for (uint32_t r = begin; r < end; ++r) {
+            cut.finished[r] += 1u;
+        }
+    }
+    // One step of a pair: false if it has to wait.  `gone` is set when it gives its place back.
+    bool step(uint32_t id, bool *gone)
+    {
+        Pair &pair = pairs[id];
+        const int pieces = (int)pair.pieces.size();
+        if (pair.at == 0) {
+            for (const Piece &p : pair.pieces) {
+                cuts[p.tile].word += shared(cuts[p.tile]) ? 1u : 0u;
+            }
+        } else if (pair.at <= pieces) {
+            const Piece &p = pair.pieces[pair.at - 1];
+            Cut &cut = cuts[p.tile];
+            if (p.s0 == 0u && !shared(cut)) {
+                if (cut.published + 1u != cut.holders) {
+                    return false;
+                }
+                finish(cut, 0u, runs);
+            } else {
+                cut.published += 1u;
+            }
+        } else if (pair.at <= 2 * pieces) {
+            const int i = pair.at - 1 - pieces;
+            Cut &cut = cuts[pair.pieces[i].tile];
+            if (shared(cut)) {
+                if (pair.together[i] < 0) {
+                    if (!always && pair_undecided(cut.word, cut.holders)) {
+                        cut.word |= kPairAlone;
+                    }
+                    pair.together[i] = always || cut.word == cut.holders ? 1 : 0;
+                }
+                uint32_t run, end;
+                pair_share(pair.together[i] == 1, id - cut.first, cut.holders, runs, &run, &end);
+                if (run < end && cut.published != cut.holders) {
+                    return false;
+                }
+                finish(cut, run, end);
+            }
+        } else {
+            left += 1u;
+            *gone = true;
+            pair.at = -2;
+            return true;
+        }
+        pair.at += 1;
+        return true;
+    }
+};
+
+// 0: both launches ended and were right; 1: no step is left that anybody could take; 2: wrong
+static int run_together(Launch &a, Launch &b, uint32_t places, uint32_t &state)
+{
+    Launch *launches[2] = {&a, &b};
+    uint32_t taken = 0u;
+    while (!a.done() || !b.done()) {
+        bool moved = false;
+        for (uint32_t tries = 0; tries < 400u && !moved; ++tries) {
+            state = state * 1664525u + 1013904223u;
+            Launch &l = *launches[(state >> 9) & 1u];
+            if ((state >> 12) % 3u == 0u) {
+                moved = taken < places && l.place();
+                taken += moved ? 1u : 0u;
+            } else if (l.placed != 0u) {
+                const uint32_t id = (state >> 14) % l.placed;
+                bool gone = false;
+                moved = l.pairs[id].at >= 0 && l.step(id, &gone);
+                taken -= gone ? 1u : 0u;
+            }
+        }
+        for (int i = 0; i < 2 && !moved; ++i) {       // nothing by chance: anything at all?
+            moved = taken < places && launches[i]->place();
+            taken += moved ? 1u : 0u;
+            for (uint32_t id = 0; id < launches[i]->placed && !moved; ++id) {
+                bool gone = false;
+                moved = launches[i]->pairs[id].at >= 0 && launches[i]->step(id, &gone);
+                taken -= gone ? 1u : 0u;
+            }
+        }
+        if (!moved) {
+            return 1;
+        }
+    }
+    for (Launch *l : launches) {
+        for (const Launch::Cut &cut : l->cuts) {
+            for (unsigned int times : cut.finished) {
+                if (times != 1u) {
+                    return 2;
+                }
+            }
+        }
+    }
+    return 0;
+}
+
+// *stuck: how many orders had no end with holders that always wait for all
+static int check_shared_places(uint32_t *stuck, unsigned long long *cases)
+{
+    // one tile of many segments, a few of few, units dealt evenly with one or two tiles to a pair, equal pieces
+    const uint32_t shapes[][2] = {{1u, 64u}, {8u, 8u}, {20u, 4u}, {20u, 10u}, {4u, 64u}, {158u, 10u}, {39u, 16u}};
+    uint32_t state = 1u;
+    for (const auto &one : shapes) {
+        for (const auto &other : shapes) {
+            for (uint32_t places : {3u, 9u, 74u}) {
+                for (uint32_t runs : {1u, 7u, 32u}) {
+                    Launch a(one[0], one[1], 74u, runs, false), b(other[0], other[1], 74u, runs, false);
+                    const int ended = run_together(a, b, places, state);
+                    if (ended != 0) {
+                        return fail(ended == 1 ? "launches of pairs that wait for each other" : "a run of rows not finished once",
+                                    one[0], one[1], other[0], places);
+                    }
+                    *cases += 1u;
+                    Launch c(one[0], one[1], 74u, runs, true), d(other[0], other[1], 74u, runs, true);
+                    *stuck += run_together(c, d, places, state) == 1 ? 1u : 0u;
+                }
+            }
+        }
+    }
+    return 0;
+}
+
 int main()
 {
     unsigned long long cases = 0;
+    uint32_t stuck = 0;
+    if (check_shared_places(&stuck, &cases) != 0) {
+        return 1;
+    }
+    if (stuck == 0u) {
+        std::printf("violated: holders that always wait came to an end in every order\n");
+        return 1;
+    }
     const unsigned int grids[] = {1u, 2u, 3u, 7u, 16u, 37u, 64u, 132u, 147u, 148u, 160u};
     const uint32_t seg_counts[] = {1u, 2u, 3u, 4u, 8u, 16u, 32u, 56u};
     for (unsigned int grid : grids) {
