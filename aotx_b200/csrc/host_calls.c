@@ -1,21 +1,24 @@
 /* The entry points that a decode step calls most, from Python without ctypes: converting twelve arguments there takes
  * 1.6 us, a third of what the host spends on a product; here 0.2.  The caller gives the function's address (the
- * library's, of whichever library is loaded) and its arguments as integers, None for a null pointer; integers are taken
- * modulo their width, as ctypes takes them.  The interpreter's lock is released during the call. */
+ * library's, of whichever library is loaded) and its arguments as integers, None for a null pointer and for nothing else;
+ * integers are taken modulo their width, as ctypes takes them.  The interpreter's lock is released during the call. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "../../include/aotx_q8_b200.h"
 
-static int take(PyObject *const *args, Py_ssize_t count, Py_ssize_t want, uint64_t *values)
+/* `kinds`: a letter per argument, p a pointer, n a number. */
+static int take(PyObject *const *args, Py_ssize_t count, const char *kinds, uint64_t *values)
 {
+    const Py_ssize_t want = (Py_ssize_t)strlen(kinds);
     if (count != want) {
         PyErr_Format(PyExc_TypeError, "%zd arguments, not %zd", want, count);
         return 0;
     }
     for (Py_ssize_t i = 0; i < count; ++i) {
-        if (args[i] == Py_None) {
+        if (args[i] == Py_None && kinds[i] == 'p') {
             values[i] = 0;
             continue;
         }
@@ -38,7 +41,7 @@ static PyObject *call_matmul(PyObject *self, PyObject *const *args, Py_ssize_t c
     uint64_t v[13];
     int code;
     (void)self;
-    if (!take(args, count, 13, v)) {
+    if (!take(args, count, "ppppnnnpnnppn", v)) {
         return NULL;
     }
     Py_BEGIN_ALLOW_THREADS
@@ -53,7 +56,7 @@ static PyObject *call_matmul_fused(PyObject *self, PyObject *const *args, Py_ssi
     uint64_t v[14];
     int code;
     (void)self;
-    if (!take(args, count, 14, v)) {
+    if (!take(args, count, "ppppnnnpnnppnn", v)) {
         return NULL;
     }
     Py_BEGIN_ALLOW_THREADS
@@ -68,7 +71,7 @@ static PyObject *call_dequant(PyObject *self, PyObject *const *args, Py_ssize_t 
     uint64_t v[9];
     int code;
     (void)self;
-    if (!take(args, count, 9, v)) {
+    if (!take(args, count, "ppppnnnnp", v)) {
         return NULL;
     }
     Py_BEGIN_ALLOW_THREADS

@@ -20,6 +20,21 @@ def test_same_answer_as_through_ctypes(name):
             call(*wrong)
 
 
+@pytest.mark.parametrize("name", sorted(ARGUMENTS))
+def test_none_is_a_null_pointer_and_no_number(name):
+    lib = load_library()
+    call = native_call(lib, name)
+    good = ARGUMENTS[name]
+    for i, kind in enumerate(getattr(lib, name).argtypes):
+        one = good[:i] + (None,) + good[i + 1:]
+        if kind is C.c_void_p:
+            assert call(*one) == getattr(lib, name)(*one) != 0
+            continue
+        for way, error in ((call, TypeError), (getattr(lib, name), C.ArgumentError)):
+            with pytest.raises(error):
+                way(*one)
+
+
 def test_every_argument_arrives_in_its_place():
     seen = []
     kind = C.CFUNCTYPE(C.c_int, *[C.c_void_p] * 3, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p, C.c_int, C.c_uint32, C.c_void_p,
