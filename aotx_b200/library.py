@@ -71,7 +71,7 @@ def native_call(lib, name):
     try:
         from . import _host_calls
     except ImportError as error:
-        raise LibraryMissing("aotx_b200/_host_calls.so is not built; run `python -m aotx_b200.build`") from error
+        raise LibraryMissing("the module aotx_b200/_host_calls is not built for this Python; run `python -m aotx_b200.build`") from error
     return functools.partial(getattr(_host_calls, name), C.cast(getattr(lib, name), C.c_void_p).value)
 
 

@@ -1,5 +1,7 @@
 """The package's own way of calling the library (csrc/host_calls.c) passes what ctypes passes, and refuses what is no call."""
 import ctypes as C
+import os
+import sysconfig
 
 import pytest
 
@@ -47,3 +49,11 @@ def test_every_argument_arrives_in_its_place():
     sent = (big, big + 1, big + 2, 8, 2 ** 32 - 1, 2 ** 32 + 5, big + 3, 1, 9, None, big + 4, 2, -1)
     assert native_call(Library, "aotx_q8_matmul_fused")(*sent) == 7
     assert seen == [(big, big + 1, big + 2, 8, 2 ** 32 - 1, 5, big + 3, 1, 9, None, big + 4, 2, -1)]
+
+
+def test_another_interpreter_does_not_find_the_module():
+    from aotx_b200 import _host_calls, build
+    build.build()
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert suffix != ".so" and _host_calls.__file__ == build.CALLS and build.CALLS.endswith(suffix)
+    assert not os.path.exists(os.path.join(build.HERE, "_host_calls.so"))
