@@ -4,6 +4,7 @@ The library is built in-tree with nvcc; nothing is compiled at import time.  `bu
 rebuilds only the objects whose sources changed.
 """
 import os
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -76,6 +77,17 @@ def resource_usage():
     return usage
 
 
+def _build_calls(include=sysconfig.get_paths()["include"]):
+    """The module of csrc/host_calls.c.  Only Python programs are faster with it, and without it they call through
+    ctypes: where there are no Python headers or no gcc, the library is all that is built."""
+    calls = os.path.join(CSRC, "host_calls.c")
+    if not os.path.exists(os.path.join(include, "Python.h")) or shutil.which("gcc") is None:
+        print("no Python headers or no gcc: " + os.path.basename(CALLS) + " is not built", file=sys.stderr)
+        return
+    if _stale(CALLS, [calls, os.path.join(CSRC, "..", "..", "include", "aotx_q8_b200.h")]):
+        subprocess.run(["gcc", "-O2", "-Wall", "-Werror", "-shared", "-fPIC", "-I" + include, "-o", CALLS, calls], check=True)
+
+
 def build(verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
@@ -88,10 +100,7 @@ def build(verbose=False):
     if _stale(LIB, objs):
         subprocess.run(["nvcc", "-shared", "-o", LIB, *objs, "-gencode",
                         "arch=compute_100a,code=sm_100a"], check=True)
-    calls = os.path.join(CSRC, "host_calls.c")
-    if _stale(CALLS, [calls, os.path.join(CSRC, "..", "..", "include", "aotx_q8_b200.h")]):
-        subprocess.run(["gcc", "-O2", "-Wall", "-Werror", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
-                        "-o", CALLS, calls], check=True)
+    _build_calls()
     untagged = os.path.join(HERE, "_host_calls.so")     # of a build before the name said so; any interpreter would load it
     if os.path.exists(untagged):
         os.remove(untagged)

@@ -57,3 +57,17 @@ def test_another_interpreter_does_not_find_the_module():
     suffix = sysconfig.get_config_var("EXT_SUFFIX")
     assert suffix != ".so" and _host_calls.__file__ == build.CALLS and build.CALLS.endswith(suffix)
     assert not os.path.exists(os.path.join(build.HERE, "_host_calls.so"))
+
+
+def test_library_needs_neither_the_module_nor_python_headers(monkeypatch, tmp_path, capsys):
+    import sys
+    import aotx_b200
+    from aotx_b200 import build
+    monkeypatch.setattr(build, "CALLS", str(tmp_path / "module.so"))
+    build._build_calls(str(tmp_path))
+    assert "not built" in capsys.readouterr().err and not os.path.exists(build.CALLS)
+    monkeypatch.delattr(aotx_b200, "_host_calls", raising=False)
+    monkeypatch.setitem(sys.modules, "aotx_b200._host_calls", None)      # an import of it fails
+    lib = load_library()
+    for name, arguments in ARGUMENTS.items():
+        assert native_call(lib, name)(*arguments) == getattr(lib, name)(*arguments) != 0
