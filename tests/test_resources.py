@@ -22,10 +22,11 @@ SMALL_SPILLS = {"q8_stream_kernel_mid": 16, "q8_wide_kernel_pair": 16, "q8_decod
                 "add_up_runs": 0, "sum_by_weights": 0,
                 "q8_gemv_simt_kernel": 32, "q8_gemv_simt_fused_kernel": 64, "q_gemv_any_kernel": 16,
                 "q8_expert_feed_kernel": 64, "q8_expert_down_kernel": 64,
-                "q8_stream_kernel": 696, "q8_wide_kernel": 720, "q8_decode_kernel": 576,
+                "q8_stream_kernel_rows": 0, "q8_stream_kernel": 696, "q8_wide_kernel": 720, "q8_decode_kernel": 576,
                 "store_eight_any": 64, "store_four_any": 64, "store_eight_peers": 64,
                 "mbar_wait": 0, "q8_peer_barrier_kernel": 0}
-FRAMES = {"q8_stream_kernel_mid": 32, "q8_wide_kernel_pair": 32, "q8_decode_kernel_warp": 8, "q_gemv_any_kernel_warp": 16}
+FRAMES = {"q8_stream_kernel_mid": 32, "q8_wide_kernel_pair": 32, "q8_decode_kernel_warp": 8, "q_gemv_any_kernel_warp": 16,
+          "q8_stream_kernel_rows": 8}
 
 
 @pytest.fixture(scope="module")
@@ -33,6 +34,9 @@ def usage():
     builder.build()
     found = builder.resource_usage()
     assert found, "no ptxas reports beside the objects"
+    # every kernel that is listed by name is there under it
+    for listed in list(SMALL_SPILLS) + list(FRAMES):
+        assert any(listed in name for name in found), listed
     return found
 
 
