@@ -26,7 +26,8 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("n,k,m,chain", [(4096, 4096, 1, 8), (5000, 1024, 8, 4), (2048, 14336, 16, 28), (28672, 4096, 8, 40),
+@pytest.mark.parametrize("n,k,m,chain", [(4096, 4096, 1, 8), (3072, 4096, 4, 8), (4600, 14336, 1, 28),
+                                         (4736, 16384, 4, 32), (5000, 1024, 8, 4), (2048, 14336, 16, 28), (28672, 4096, 8, 40),
                                          # accumulators in turn: in clusters of four with one slab and with two, of two,
                                          # whole tiles in turns; runs, of one segment and of several
                                          (4096, 4096, 24, 16), (6144, 4096, 32, 32), (14336, 4096, 20, 44), (28672, 4096, 32, 77),

@@ -114,3 +114,35 @@ def test_results_that_the_next_launch_reads(ctx):
                     assert torch.equal(got, want)
             results.append(alone[0].float().abs().max().item())
     assert all(0.0 < r < 60000.0 for r in results)      # nothing died away or left the range of binary16
+
+
+# whole rows of w per block, both its depths; bfloat16 x that becomes binary16 in the kernel, in clusters and whole tiles;
+# the pairs' cut tiles of many holders and of few
+@pytest.mark.parametrize("n,k,m", [(3072, 3072, 1), (4096, 2048, 4), (4700, 9216, 3), (1024, 1024, 24), (28672, 1024, 24),
+                                   (28672, 1024, 60), (1000, 2048, 200), (2560, 2560, 300)])
+@pytest.mark.parametrize("kind", ["float16", "bfloat16"])
+def test_results_that_the_same_kernel_reads(ctx, n, k, m, kind):
+    """Back and forth between two buffers, k to n and n to k: each product reads what the launch before it wrote."""
+    import aotx_b200
+    torch = torch_mod()
+    kind = getattr(torch, kind)
+    n = n // 256 * 256
+    there, back = aotx_b200.synth_q8_0_device(n, k, 1), aotx_b200.synth_q8_0_device(k, n, 2)
+    start = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)).to(kind)
+    a, b = torch.empty_like(start), torch.empty(m, n, device="cuda", dtype=kind)
+
+    def chain():
+        a.copy_(start)
+        for _ in range(3):
+            ctx.matmul(there, n, k, a, y=b)
+            ctx.matmul(back, k, n, b, y=a)
+        return a.clone(), b.clone()
+
+    ctx.set_overlap(False)
+    alone = chain()
+    torch.cuda.synchronize()
+    ctx.set_overlap(True)
+    for _ in range(10):
+        for got, want in zip(chain(), alone):
+            assert torch.equal(got, want)
+    assert all(0.0 < t.float().abs().max().item() < 60000.0 for t in alone)

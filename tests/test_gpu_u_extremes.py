@@ -29,18 +29,19 @@ GATES = [0.0, 1.0, -1.0, 20.0, -50.0, -87.0, -88.0, -88.5, -89.0, -90.0, -100.0,
          float("inf"), float("-inf"), float("nan"), -1e10, 1e10, -1e30, 1e30]
 
 
-# the general path; up to 16 rows; clusters, units and turns of the kernel for 17 to 128 rows, a width that is no
-# multiple of four; pairs of SMs
-@pytest.mark.parametrize("n,m,path", [(256, 24, 1), (5000, 8, 1), (256, 8, 0), (40000, 16, 0), (256, 24, 0), (9000, 100, 0),
-                                      (12006, 32, 0), (40000, 64, 0), (60002, 100, 0), (512, 200, 0), (20002, 300, 0)])
+# the general path; up to 16 rows; whole rows of w per block; clusters, units and turns of the kernel for 17 to 128 rows, a
+# width that is no multiple of four; pairs of SMs: cut tiles of few holders and of many
+@pytest.mark.parametrize("n,m,path,k", [(256, 24, 1, 256), (5000, 8, 1, 256), (256, 8, 0, 256), (40000, 16, 0, 256), (4000, 4, 0, 2048),
+                                        (4600, 3, 0, 5120), (256, 24, 0, 256), (9000, 100, 0, 256), (12006, 32, 0, 256),
+                                        (40000, 64, 0, 256), (60002, 100, 0, 256), (512, 200, 0, 256), (20002, 300, 0, 256),
+                                        (512, 200, 0, 4096)])
 @pytest.mark.parametrize("kind", ["float16", "bfloat16"])
-def test_gates_at_the_limits(ctx, n, m, path, kind):
+def test_gates_at_the_limits(ctx, n, m, path, k, kind):
     """Rows of weights that are 1 in the first place: gate and up are the x in that place.  The unit is the float
     expression g / (1 + exp(-g)) * g within four roundings; what lies below the smallest normal float may be zero."""
     import aotx_b200
     torch = torch_mod()
     kind = getattr(torch, kind)
-    k = 256
     raw = torch.zeros(n, k // 32, 34, dtype=torch.uint8, device="cuda")
     raw[:, :, :2] = torch.tensor([1.0], dtype=torch.float16).view(torch.uint8).cuda()
     raw[:, 0, 2] = 1
