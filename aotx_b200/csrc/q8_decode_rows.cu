@@ -14,8 +14,8 @@
 // Every block reads all of x, and every warp turns its part round by itself, so it pays for few rows of x only, and a
 // warp's own copies and hand-overs cost instructions, so it pays where a launch is short (rows_height has both sides).
 // 4096 x 4096, one row, 7.3 -> 5.6 us (weights in L2, from call to call 6.7 -> 4.6); four rows 7.3 -> 6.2.  At 28672 x 4096,
-// slabs of several such tiles took 29 us against 26, and eight rows of x 31 against 25.  Every wait is bounded and raises a status bit when it runs out.  Reference
-// kernels replaced: as q8_decode_warp.cu.
+// several such tiles to a block took 29 us against 26, and eight rows of x 31 against 25.  Every wait is bounded and raises a
+// status bit when it runs out.  Reference kernels replaced: as q8_decode_warp.cu.
 #include <cuda.h>
 
 #include "q8_decode_operands.cuh"
@@ -35,10 +35,24 @@ constexpr uint32_t kRowsLeast = 77u * 1024u;
 // The sums of a warp in shared memory: [row of x][row of w], the rows 4 words longer than they are so that the MMA's
 // fragments are stored without bank conflicts.
 constexpr uint32_t kRowsPitch = 20;
-// Tiles of fewer rows multiply repeats (2048 x 8192, 8 rows a tile, 8.1 -> 10.6 us; 3072 x 3072, 11, 5.6 -> 4.4), and with
-// more depth it is memory that counts (4096 x 7936, 4 rows of x, 9.9 -> 10.5; 4096 x 14336, one, 14.4 both ways).  Above 32
-// tiles of 128 rows the clusters of eight of q8_decode_warp.cu do not all run at once, and any depth is faster here
-// (4600 x 14336, one row, 22.7 -> 13.9 us; 4600 x 8192, four, 15.5 -> 9.9).
+// Where the lines lie, between this kernel and q8_decode_warp.cu: tiles of fewer rows multiply repeats, and with more depth
+// it is memory that counts.  Above 32 tiles of 128 rows the clusters of eight of q8_decode_warp.cu do not all run at once,
+// and any depth is faster here.  That kernel's us and this one's, launches in a graph, weights from memory:
+//   rows a tile       8            10           11           13           14           15           16
+//   one row of x
+//     2048 deep   3.9   3.1    4.2   3.2    4.4   3.2    4.9   3.3    5.5   3.3    7.1   3.4    7.4   3.5
+//     4096 deep   5.3   4.8    5.7   5.2    5.9   5.4    6.4   5.8    6.9   5.6    9.4   6.2   10.5   6.4
+//     5120 deep   6.3   6.4    6.9   7.0    7.1   7.3    7.8   7.8    8.1   7.6   12.1   8.3   12.3   8.5
+//     8192 deep   8.0   8.6    8.5   9.6    8.8  10.1    9.7   9.8   10.0   9.8   15.0  10.8   15.5  11.2
+//    14336 deep  13.1  12.6   13.5  13.5   13.7  14.1   14.3  13.9   14.6  14.1   22.4  14.8   23.2  15.5
+//   four
+//     2048 deep   4.0   3.4    4.3   3.5    4.4   3.6    4.9   3.8    5.4   3.8    7.2   3.9    7.6   3.9
+//     4096 deep   5.4   5.4    5.8   5.7    6.1   5.9    6.5   6.1    6.9   6.2    9.6   6.4   10.8   6.6
+//     5120 deep   6.5   7.0    7.0   7.6    7.3   7.8    8.0   8.3    8.3   8.3   12.2   7.9   12.4   8.0
+//     8192 deep   8.2   9.6    8.6  10.6    8.9  10.3    9.8  11.0   10.1  11.0   15.0  10.3   15.5  10.5
+//    14336 deep  13.0  14.3   13.7  15.1   13.9  14.8   14.5  15.7   14.8  15.7   22.4  15.2   23.4  15.4
+// (In the column of 14 rows the tensor has 4096.)  The lines are on the safe side: this kernel is no slower from 8 rows a tile
+// on up to 4096 deep, nor at 1024 deep (8 rows a tile, one row of x, 3.1 and 2.4; 16, 3.6 and 2.6).
 constexpr uint32_t kRowsHeight = 11;
 constexpr uint32_t kRowsDepth = 4096;
 constexpr uint32_t kRowsChains = 4;            // accumulators of a value (q8_decode_warp.cu says why)
@@ -52,7 +66,7 @@ struct RowsArgs {
     unsigned int ldy, epilogue;
     unsigned int height;               // rows of w per tile, up to 16
     unsigned int stages, stage_bytes;  // of a warp's ring
-    unsigned int x_bytes;              // of a warp's x, and of its sums at the slab's end
+    unsigned int x_bytes;              // of a warp's x, and of its sums at the tile's end
 };
 
 template <bool BF, typename YT>

@@ -2,7 +2,9 @@
 // grid and its scratch.
 //
 //   rows of x     kernel                                                          file
-//   1 .. 4        whole rows of w per block, where w has 3000 to 4736 of them      q8_decode_rows.cu
+//   1 .. 4        whole rows of w per block, where w has 11 to 16 rows to a block  q8_decode_rows.cu
+//                 (148 SMs: 2961 to 4736) and is 2048 to 4096 deep, to 16384
+//                 above 4096 rows
 //   1 .. 16       weights through registers into mma.sync, two blocks per SM      q8_decode_warp.cu
 //   17 .. 128     weights through tensor memory, one block per SM; also the       q8_mid.cu
 //                 grouped products of the routed experts

@@ -16,7 +16,7 @@
 //   * The first tiles are dealt whole, one after the other to every pair; what is left for less than a turn of
 //     all pairs is cut (pair_split in q8_schedule.cuh).  A cut tile is finished by the pair that holds its
 //     first segment, each block its own rows (that is a pair's last piece and all its warps store), or by all of its
-//     holders, each a run of its rows of x (kPairShareMore says when).
+//     holders, each a run of its rows of x (kPairShareMore and pair_undecided say when).
 //   * The first weights are on their way before the live batch is known; the accumulator goes back before a part of a
 //     cut tile is published.
 //   * The tile's rows of x are the batch in equal parts of at most 256, rounded up to 32.
@@ -24,7 +24,8 @@
 // 23 warps per block, one block per SM: 0-3 store, 4-19 convert, 20 copies weights, 21 copies x, 22 of the
 // first block issues the MMAs.  Every wait is bounded and raises a status bit when it runs out.
 // Measured against q8_wide.cu: gate+up 28672 x 4096, 2048 rows, bfloat16, 489 -> 350 us (1377 TFLOP/s); the
-// fused layer of 2560 by 9728, 300 rows, 365 -> 112 us (120 before the two points above).  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
+// fused layer of 2560 by 9728, 300 rows, 365 -> 112 us (120 before the shares, and the first weights and the accumulator's
+// return as above).  Reference kernel replaced: cuda/model/gemm.cuh:55-189.
 #include <cuda.h>
 
 #include "q8_launch.h"
@@ -319,7 +320,7 @@ __device__ __forceinline__ void wait_for_parts(const PairArgs &args, const PairC
 // Rows of x that a warp finishes of a cut tile at a time.
 constexpr uint32_t kPairShareRows = 8;
 
-// The parts of a cut tile's holders, `partial` being this lane's place in slot 0, added in order; the loads of three
+// The parts of a cut tile's holders, `partial` being this lane's place in slot 0, added in order; the loads of four
 // holders are on their way at a time.
 __device__ __forceinline__ void sum_of_parts(uint32_t (&v)[kPairShareRows], const float *partial, unsigned long long tile_floats,
                                              const PairCut &cut, uint32_t rank)

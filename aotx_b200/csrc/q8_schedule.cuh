@@ -105,11 +105,14 @@ struct PairWork {
 };
 
 // What cutting a tile costs, in units (256 weights deep): the hand-over of the partial sums and the stores at the
-// end.
+// end.  (21248 x 1024, 300 rows, tiles of 4 units: whole behind two turns 23.5 us, cut 28.5.  A line at 8 units is no
+// different at the sizes of pair_split's last point.)
 constexpr uint32_t kPairCutUnits = 5;
-// A piece of a cut tile is worth this many units at least: every holder is a tile of sums more that the owner
-// reads back, about as long as a unit and a half takes.
+// A piece of a cut tile is worth this many units at least: every holder is a tile of sums more that is written and read
+// back.  (20480 x 4096, 300 rows: 6 units 56.6 us, 4 units 54.4, 2 the same.)
 constexpr uint32_t kPairMinPiece = 4;
+// What pieces may be longer than evenly dealt units.  (21504 x 8192, 300 rows, 20 tiles of 32 units, three pieces of 11 or
+// dealt in runs of 8 or 9: 106 us both.)
 constexpr uint32_t kPairEvenUnits = 2;
 
 // How the tiles are divided between all pairs; the divisions that need no pair's number, so that the host can do them.
@@ -118,13 +121,16 @@ struct PairSplit {
 };
 
 // As many turns of whole tiles as all pairs have; the tiles that are left:
-//   * Fewer than two turns: their units are dealt evenly.  Longer pieces are faster (2560 x 2560, 300 rows, 15.0 us
-//     in halves of a tile against 17.5; 1000 x 2048, 200 rows, 14.8 against 19.9), but the error of a sum grows with
-//     the depth that goes into one accumulator, and evenly dealt it is the smallest.
+//   * Fewer than two turns: their units are dealt evenly, because the error of a sum grows with the depth that goes into
+//     one accumulator, and evenly dealt it is the smallest.  Pieces of at least four units are faster where the evenly
+//     dealt ones are short and have many holders (256 x 16384, 150 rows, 13.5 us against 19.0; 5000 x 1024, 160 rows, 8.1
+//     against 12.6; 300 x 16384, 700 rows, 19.6 against 27.4; 2560 x 2560, 300 rows, 14.1 against 14.6), not always (1000 x
+//     2048, 200 rows, 14.8 against 11.6; 1024 x 4096, 300 rows, 14.4 against 13.8).
 //   * Behind more whole tiles, whose depth gives the error, what is faster: whole as well where cutting costs more
 //     than it evens out; else pieces of one size inside each tile, of kPairMinPiece units at least, as many as there
-//     are pairs for; else evenly dealt units, where that makes the longest piece kPairEvenUnits shorter (19456 x
-//     2560, 300 rows, four tiles of 10 units behind two turns: two pieces each 38.5 us, dealt evenly 43.5).
+//     are pairs for; else evenly dealt units, where that makes the longest piece more than kPairEvenUnits
+//     shorter (20480 x 4096, 300 rows, twelve tiles of 16 units behind two turns: four pieces each 55.4 us, dealt evenly
+//     59.2; 19456 x 2560, four of 10: two pieces each 37.3, dealt evenly 36.2).
 __host__ __device__ __forceinline__ PairSplit pair_split(uint32_t pairs, uint32_t tiles, uint32_t segs)
 {
     PairSplit split;
@@ -221,10 +227,12 @@ __host__ __device__ __forceinline__ uint32_t pair_last_holder(const PairWork &wo
 
 // A cut tile is finished by the pair that began it, or, where it has more holders than a pair has units by so many and
 // all of them run (pair_undecided), by all its holders.  The one that began it reads as many tiles of sums as there are
-// others, 0.8 us a round trip, but most of it before its own sums are there: the longer the runs, the more.  All together read one tile's worth each, and
-// everybody waits for the last to publish.  (Beginner against all: 1000 x 2048, 200 rows, 1 unit and 8 holders, 19.8 and
-// 11.3 us; 1024 x 4096, 300 rows, 24.1 and 16.4; 2560 x 2560, 300 rows, 2.7 units and 4 or 5 holders, 15.7 and 16.1, with
-// the line between 4 and 5 14.7; 2560 x 9728, 10.3 units, 4 or 5 holders, 25.9 and 27.3.)
+// others, 0.8 us a round trip, but most of it before its own sums are there: the longer the runs, the more.  All together
+// read one tile's worth each, and everybody waits for the last to publish.  (Units per pair, holders: beginner and all, us.  1, 8, 1000 x 2048, 200 rows:
+// 19.1 and 11.7; 1, 64, 256 x 16384, 150 rows: 54.0 and 19.0; 1.7, 10, 1024 x 4096, 300 rows: 21.2 and 13.8; 2.7, 4 or 5,
+// 2560 x 2560, 300 rows: 15.4 and 18.1, with the line between 4 and 5 14.6; 3.5, 10, 1024 x 8192, 300 rows: 20.8 and 18.7;
+// 4.3, 15, 1280 x 16384, 150 rows: 26.1 and 22.2; 5.2, 13, 300 x 16384, 700 rows: 34.4 and 27.4; 6.9, 10, 2048 x 16384, 150
+// rows: 25.5 and 25.1; 8.6, 8, 2560 x 16384, 150 rows: 27.1 and 27.7; 10.3, 4 or 5, 2560 x 9728, 300 rows: 23.4 and 27.1.)
 constexpr uint32_t kPairShareMore = 3;
 
 __host__ __device__ __forceinline__ uint32_t pair_share_from(const PairWork &work)

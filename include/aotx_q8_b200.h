@@ -70,7 +70,7 @@ extern "C" {
 typedef struct aotx_q8_ctx aotx_q8_ctx;
 
 /* Make / release the per-device context: SM count, the scratch tiles and flags of the
- * streaming kernel (about 40 MB) and a device status word.  Call outside stream capture.
+ * tensor-core kernels (about 86 MB) and a device status word.  Call outside stream capture.
  * No counterpart in the reference, whose kernels need no scratch; it takes the place of the
  * buffers that cuda/model/model_host.cu:95-153 makes before its capture starts. */
 int aotx_q8_init(aotx_q8_ctx **ctx, int device);
