@@ -62,7 +62,7 @@ EPILOGUE_OF = {"o": 1, "down": 1, "gate_up": 2}  # AOTX_Q8_EPILOGUE_ADD / _SWIGL
 
 # DRAM bytes (read + write) per algorithmic byte of the dominant kernel: one ncu capture of the
 # gate+up projection at 32 rows, scaled to the average launch by bytes (source named in the line).
-TRAFFIC_RATIO = {"decode_m32_llama3_8b_layer": 0.9973, "decode_m32_gate_up": 0.9973}
+TRAFFIC_RATIO = {"decode_m32_llama3_8b_layer": 0.9978, "decode_m32_gate_up": 0.9978}
 TRAFFIC_SOURCE = "profiles/q8_products_by_regime.md (28672 x 4096, 32 rows, one launch)"
 TENSOR_BOUND = {"prefill_m2048_llama3_8b_layer", "prefill_m2048_gate_up", "prefill_m2048_llama3_8b_layer_fused"}
 
