@@ -801,7 +801,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     const uint32_t buffer = stage + flip;
                     flip ^= 2048u;
                     if (gated) {
-                        store_rows_staged<YT, true>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                        store_rows_staged<YT, true, false>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
                     } else {
                         // in two halves: the old values of an add take as many registers as the sums
                         uint32_t half[8];
@@ -811,7 +811,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                             for (uint32_t i = 0; i < 8u; ++i) {
                                 half[i] = v[h + i];
                             }
-                            store_rows_staged<YT, false>(args.to, buffer + h * 32u * sizeof(YT), lane, col, columns, tok0 + c0 + h,
+                            store_rows_staged<YT, false, false>(args.to, buffer + h * 32u * sizeof(YT), lane, col, columns, tok0 + c0 + h,
                                                          tok0 + rows, half);
                         }
                     }
@@ -895,9 +895,9 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     const uint32_t buffer = stage + flip;
                     flip ^= 2048u;
                     if (gated) {
-                        store_rows_staged<YT, true>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                        store_rows_staged<YT, true, false>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
                     } else {
-                        store_rows_staged<YT, false>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
+                        store_rows_staged<YT, false, false>(args.to, buffer, lane, col, columns, tok0 + c0, tok0 + rows, v);
                     }
                     continue;
                 }

@@ -128,11 +128,13 @@ __device__ __forceinline__ void store_rows_direct(const RowStore &to, bool gated
 // the warp's own and written four values per lane, 2 to 4 store instructions instead of 16 (the
 // number of store instructions is what a store costs here, see q8_tile.cuh).  GATED: neighbouring
 // lanes hold gate and up of one column (cuda/model/norm.cu:92-105); 16 columns then.
-// `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.
-template <typename YT, bool GATED, int ROWS>
+// `columns`: how many of the 32 (16) are inside the tensor, a multiple of four.  MAPPED: row i of x goes to row
+// `mapped` of lane i of y, which the caller has from before the sums were there (fetched here, the row map's latency
+// came to every 16 rows: q8_mid.cu); else to the row of the same number.
+template <typename YT, bool GATED, bool MAPPED, int ROWS>
 __device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t stage, uint32_t lane, uint32_t first_col,
                                                  uint32_t columns, uint32_t first_row, uint32_t row_limit,
-                                                 const uint32_t (&v)[ROWS])
+                                                 const uint32_t (&v)[ROWS], uint32_t mapped = 0u)
 {
     constexpr uint32_t kColumns = GATED ? 16u : 32u;
     constexpr uint32_t kRowBytes = kColumns * sizeof(YT);
@@ -161,10 +163,11 @@ __device__ __forceinline__ void store_rows_staged(const RowStore &to, uint32_t s
     YT *at[kSteps];
 #pragma unroll
     for (uint32_t step = 0; step < kSteps; ++step) {
-        const uint32_t row_x = first_row + step * kRowsPerStep + lane / kLanesPerRow;
+        const uint32_t local = step * kRowsPerStep + lane / kLanesPerRow;
+        const uint32_t row_x = first_row + local;
+        const uint32_t row_y = MAPPED ? __shfl_sync(0xFFFFFFFFu, mapped, local) : row_x;
         at[step] = nullptr;
         if (row_x < row_limit && part * 4u < columns) {
-            const uint32_t row_y = to.row_map != nullptr ? to.row_map[row_x] : row_x;
             at[step] = static_cast<YT *>(to.y) + (size_t)row_y * to.ldy + first_col + part * 4u;
         }
     }
