@@ -16,9 +16,9 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libaotx_q8_b200.so")
 # The Python module of csrc/host_calls.c, under the name that only the interpreter it is built for looks for.
 CALLS = os.path.join(HERE, "_host_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
-SOURCES = ["q8_api.cu", "q8_simt.cu", "q8_dispatch.cu", "q8_stream.cu", "q8_decode.cu", "q8_decode_warp.cu", "q8_decode_rows.cu", "q8_mid.cu", "q8_pair.cu", "q8_wide.cu", "q8_static.cu", "q8_moe.cu", "q8_peers.cu",
+SOURCES = ["q8_api.cu", "q8_simt.cu", "q8_dispatch.cu", "q8_stream.cu", "q8_decode.cu", "q8_decode_warp.cu", "q8_decode_rows.cu", "q8_mid.cu", "q8_pair.cu", "q8_wide.cu", "q8_static.cu", "q8_moe.cu", "q8_route.cu", "q8_peers.cu",
            "q_generic.cu", "q_warp.cu", "gguf_table.cpp", "gguf_upload.cu"]
-HEADERS = ["q8_common.cuh", "q8_ptx.cuh", "q8_warp_ptx.cuh", "q8_rows.cuh", "q8_schedule.cuh", "q8_decode_operands.cuh", "q8_store.cuh", "q8_simt_gemv.cuh", "q8_launch.h", "q8_tile.cuh", "q_blocks.cuh", os.path.join("..", "..", "include", "aotx_q8_b200.h"),
+HEADERS = ["q8_common.cuh", "q8_ptx.cuh", "q8_warp_ptx.cuh", "q8_rows.cuh", "q8_schedule.cuh", "q8_decode_operands.cuh", "q8_store.cuh", "q8_simt_gemv.cuh", "q8_route.cuh", "q8_launch.h", "q8_tile.cuh", "q_blocks.cuh", os.path.join("..", "..", "include", "aotx_q8_b200.h"),
            os.path.join("..", "..", "include", "aotx_gguf_b200.h")]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

@@ -319,7 +319,7 @@ extern "C" int aotx_q8_moe_route(aotx_q8_ctx *ctx, void *stream, const void *x_f
         return AOTX_Q8_ERR_UNSUPPORTED; /* four rows of x as floats must fit in shared memory */
     }
     cudaError_t err = q8::launch_route((cudaStream_t)stream, x_f16, router, tokens, tokens_dev, hidden,
-                                       experts, used, prob, ids, ctx->overlap != 0);
+                                       experts, used, prob, ids, ctx->scratch.status, ctx->overlap != 0);
     return err == cudaSuccess ? AOTX_Q8_OK : cuda_fail(ctx, err);
 }
 

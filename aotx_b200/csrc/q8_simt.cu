@@ -12,12 +12,11 @@
 //   cuda/model/experts.cu:77-98     -> q8_expert_sum_kernel
 #include "q8_common.cuh"
 #include "q8_launch.h"
+#include "q8_route.cuh"
 #include "q8_simt_gemv.cuh"
 #ifndef Q8_HOST_EMULATION
 #include "q8_warp_ptx.cuh"
 #endif
-
-#include <math_constants.h>
 
 namespace q8 {
 
@@ -109,7 +108,6 @@ __global__ void q8_dequant_kernel_many(const unsigned char *w, unsigned long lon
 // ---------------------------------------------------------------------------------------
 #define Q8_ROUTE_THREADS 256u     // of the emulated launch
 #define Q8_ROUTE_GPU_THREADS 512u
-#define Q8_ROUTE_EXPERTS 256u
 
 // Activations of a group in shared memory, [position along the row][token], rows padded so that
 // 16-byte reads of 8 neighbouring lanes meet 32 different banks.
@@ -149,27 +147,6 @@ __device__ __forceinline__ void route_step(const float *at, const float (&r)[EXP
     }
 }
 
-// The largest value over the warp and the lowest index that has it.  Every value is a probability or -1, so
-// their bits order them as signed integers do: two reductions in place of ten shuffles.
-__device__ __forceinline__ void largest_first(float *best, float *best_at)
-{
-#ifdef Q8_HOST_EMULATION
-    for (unsigned int step = 16u; step != 0u; step >>= 1) {
-        const float other = __shfl_xor_sync(0xFFFFFFFFu, *best, step);
-        const float other_at = __shfl_xor_sync(0xFFFFFFFFu, *best_at, step);
-        if (other > *best || (other == *best && other_at < *best_at)) {
-            *best = other;
-            *best_at = other_at;
-        }
-    }
-#else
-    const int most = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(*best));
-    const unsigned int mine = __float_as_int(*best) == most ? (unsigned int)*best_at : 0xFFFFFFFFu;
-    *best_at = (float)__reduce_min_sync(0xFFFFFFFFu, mine);
-    *best = __int_as_float(most);
-#endif
-}
-
 __device__ __forceinline__ void route_arrive()
 {
 #ifdef Q8_HOST_EMULATION
@@ -187,7 +164,6 @@ __device__ __forceinline__ void route_body(const __half *x, const float *router,
                                            float (&probability)[TOKENS][Q8_ROUTE_EXPERTS])
 {
     constexpr unsigned int kStride = RouteShape<TOKENS>::stride;
-    constexpr unsigned int kPerLane = Q8_ROUTE_EXPERTS / 32u;
     unsigned int tokens = tokens_max;
     if (tokens_dev != nullptr) {
         unsigned int live = *tokens_dev;
@@ -324,74 +300,7 @@ __device__ __forceinline__ void route_body(const __half *x, const float *router,
             cluster_wait_acquire();
         }
         for (unsigned int g = crank + csize * warp; g < group; g += csize * warps) {
-            // one warp per token, lane holds experts lane, lane + 32, ..
-            const unsigned int t = t0 + g;
-            float value[kPerLane];
-            float sum[kPerLane];
-            float top = -CUDART_INF_F;
-#pragma unroll
-            for (unsigned int j = 0; j < kPerLane; ++j) {
-                const unsigned int e = lane + 32u * j;
-                value[j] = e < experts ? probability[g][e] : -CUDART_INF_F;
-                top = fmaxf(top, value[j]);
-            }
-            for (unsigned int step = 16u; step != 0u; step >>= 1) {
-                top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, step));
-            }
-#pragma unroll
-            for (unsigned int j = 0; j < kPerLane; ++j) {
-                value[j] = lane + 32u * j < experts ? expf(value[j] - top) : 0.0f;
-                sum[j] = value[j];
-            }
-            // the reference's tree over 256 places: halves 128 apart, 64, 32, then within the warp
-#pragma unroll
-            for (unsigned int half = kPerLane / 2u; half != 0u; half >>= 1) {
-#pragma unroll
-                for (unsigned int j = 0; j < half; ++j) {
-                    sum[j] += sum[j + half];
-                }
-            }
-            for (unsigned int step = 16u; step != 0u; step >>= 1) {
-                sum[0] += __shfl_down_sync(0xFFFFFFFFu, sum[0], step);
-            }
-            // lane 0 holds the whole sum: hand it round (every other lane puts in a zero)
-            float total = lane == 0u ? sum[0] : 0.0f;
-            for (unsigned int step = 16u; step != 0u; step >>= 1) {
-                total += __shfl_xor_sync(0xFFFFFFFFu, total, step);
-            }
-#pragma unroll
-            for (unsigned int j = 0; j < kPerLane; ++j) {
-                const unsigned int e = lane + 32u * j;
-                value[j] /= total;
-                if (e < experts) {
-                    prob[(size_t)t * experts + e] = value[j];
-                } else {
-                    value[j] = -1.0f; // below every probability
-                }
-            }
-            // the largest that is left, ties to the lower index, `used` times over
-            for (unsigned int rank = 0; rank < used; ++rank) {
-                float best = -1.0f;
-                float best_at = (float)rank;   // an index as a float: exact, at most 255
-#pragma unroll
-                for (unsigned int j = 0; j < kPerLane; ++j) {
-                    if (value[j] > best) {
-                        best = value[j];
-                        best_at = (float)(lane + 32u * j);
-                    }
-                }
-                largest_first(&best, &best_at);
-                const unsigned int chosen = (unsigned int)best_at;
-#pragma unroll
-                for (unsigned int j = 0; j < kPerLane; ++j) {
-                    if (lane + 32u * j == chosen) {
-                        value[j] = -1.0f;
-                    }
-                }
-                if (lane == 0u) {
-                    ids[(size_t)t * used + rank] = chosen;
-                }
-            }
+            route_choose(probability[g], t0 + g, experts, used, prob, ids);
         }
         // the next group's activations and logits come after everyone has read this one's
         if (t0 + gridDim.x / csize * TOKENS >= tokens) {
@@ -681,11 +590,18 @@ cudaError_t launch_gemv_simt(cudaStream_t stream, const void *w, unsigned int n,
 
 cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
-                         unsigned int used, float *prob, unsigned int *ids, bool overlap)
+                         unsigned int used, float *prob, unsigned int *ids, unsigned int *status, bool overlap)
 {
     if (tokens == 0u) {
         return cudaSuccess;
     }
+#ifndef Q8_HOST_EMULATION
+    if (route_tiles_fits(x, router, tokens, hidden, experts)) {
+        return launch_route_tiles(stream, x, router, tokens, tokens_dev, hidden, experts, used, prob, ids, status, overlap);
+    }
+#else
+    (void)status;
+#endif
 #ifdef Q8_HOST_EMULATION
     // a cluster of one block: it takes all experts
     const size_t emulated = (size_t)RouteShape<4u>::stride * hidden * sizeof(float);
@@ -700,7 +616,8 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     // block has 16 warps of one or two experts each (measured against 8 warps of two or four; 128
     // experts, 2048 wide: 8 tokens 9.5 -> 7.2 us, 128 tokens 20.8 -> 13.0, 512 tokens 25.0 -> 22.6).
     // Few experts leave most warps of such a cluster without work, and every block of it reads the group's
-    // activations: then a block takes all experts of four tokens by itself.  (Clusters, and one block for all: 8
+    // activations: then a block takes all experts of four tokens by itself.  (Above 148 tokens all this is left to rows of
+    // other widths or off a 16-byte boundary, and to at most 16 experts: q8_route.cu.)  (Clusters, and one block for all: 8
     // experts, 2048 wide, 512 tokens 15.4 us and 9.0, 4096 wide, 2048 tokens 160 and 24; 64 experts, 2048 wide, 512
     // tokens 17.2 and 29.3, 2048 tokens 64.1 and 57.2, 8192 wide, 300 tokens 74.3 and 53.2.)
     const bool few = tokens <= 36u;

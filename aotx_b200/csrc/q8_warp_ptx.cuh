@@ -160,4 +160,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// A float into the shared memory of a block of the cluster, counted on that block's barrier `bar`
+// (addresses of mapa_shared).
+__device__ __forceinline__ void store_counted(uint32_t addr, float v, uint32_t bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)),
+                 "r"(bar)
+                 : "memory");
+}
+
 } // namespace q8

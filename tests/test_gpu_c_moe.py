@@ -66,6 +66,34 @@ def test_route(ctx, oracle, tokens, experts, used, precision):
         assert (mass < 0.999).all()
 
 
+@pytest.mark.parametrize("tokens,experts,used,hidden,live", [
+    (149, 17, 3, 32, 149),        # a chunk that is one step; the fewest tokens and experts of the tiles
+    (153, 33, 4, 160, 150),       # two blocks of which one has one expert; a last group cut by the live count
+    (300, 128, 8, 2048, 297),     # eight tokens to a group, a ring that goes round
+    (593, 16, 2, 1120, 592),      # a block for all experts
+    (601, 5, 5, 288, 1),          # fewer experts than a block's, one live token
+    (1203, 250, 9, 1056, 1203)])  # the largest cluster, groups one behind the other
+def test_route_of_many_tokens(ctx, oracle, tokens, experts, used, hidden, live):
+    torch = torch_mod()
+    rng = np.random.Generator(np.random.PCG64(tokens + experts))
+    router = rng.standard_normal((experts, hidden)).astype(np.float32) / np.float32(np.sqrt(hidden))
+    router[experts - 1] = router[0]           # the same sums: the lower index first
+    x = rng.standard_normal((tokens, hidden)).astype(np.float16)
+    prob = torch.full((tokens, experts), GUARD, dtype=torch.float32, device="cuda")
+    ids = torch.full((tokens, used), -1, dtype=torch.int32, device="cuda")
+    ctx.moe_route(dev(x), dev(router), used, tokens=tokens, tokens_dev=dev(np.array([live], np.int32)), prob=prob, ids=ids)
+    torch.cuda.synchronize()
+    got_p = prob.cpu().numpy()
+    got_i = ids.cpu().numpy().view(np.uint32)
+    want_p, want_i = oracle.route(x[:live].view(np.uint16), router, used)
+    assert np.abs(got_p[:live] - want_p).max() < 2e-6
+    assert np.array_equal(got_i[:live], oracle.rank(got_p[:live], used))
+    assert np.array_equal(got_i[:live], want_i)
+    assert np.array_equal(got_p[:live, experts - 1], got_p[:live, 0])
+    assert (got_p[live:] == GUARD).all() and (got_i[live:] == 0xFFFFFFFF).all()
+    assert ctx.device_status() == 0
+
+
 def _moe_case(oracle, tokens, experts, used, hidden, ffn, seed):
     import aotx_b200
     wg = aotx_b200.synth_q8_0(experts * ffn, hidden, seed)
