@@ -62,6 +62,7 @@ struct PairArgs {
     unsigned int *flags;
     unsigned long long tile_floats;
     unsigned int x_stages, raw_stages;
+    unsigned int x_pieces;             // of x, 64 deep, per stage of its ring: 1 or 2
     PairSplit split;                   // of the whole batch's tiles
 };
 
@@ -369,6 +370,63 @@ __device__ __forceinline__ void pair_convert(uint32_t half, const uint32_t (&raw
     }
 }
 
+// What the thread that issues a pair's MMAs knows.
+struct PairIssue {
+    uint32_t x_full, x_empty, a_full, a_empty, acc_full, acc_empty;     // barriers
+    uint32_t tmem_base, a_column0, smem0, x_piece_bytes, x_stages, idesc, chains;
+    unsigned int *status;
+};
+
+// All of a pair's MMAs.  PIECES: of x per stage of its ring (launch_pair_kernel).  Every wait stands where it is needed:
+// asking for the next stage before the MMAs of this one cost more than it hid, because the answer is waited for where it
+// is asked for (2048 rows, layer 782 -> 773 us without).
+template <uint32_t PIECES>
+__device__ __forceinline__ void pair_issue(PairWork &work, const PairIssue &at, volatile uint32_t *abort_flag)
+{
+    uint32_t xst = 0u, xph = 0u;
+    uint32_t ast = 0u, aph = 0u;
+    for (uint32_t turn = 0; work.next(); ++turn) {
+        if (!mbar_wait_hot(at.acc_empty, (turn & 1u) ^ 1u, abort_flag, at.status)) {
+            return;
+        }
+        tc_fence_after_sync();
+        for (uint32_t s = work.s0; s < work.s1; ++s) {
+            if (!mbar_wait_hot(at.a_full + 8u * ast, aph, abort_flag, at.status)) {
+                return;
+            }
+            const uint32_t a_tmem = at.tmem_base + at.a_column0 + ast * kPairAColumns;
+#pragma unroll 1
+            for (uint32_t j0 = 0; j0 < kSubs; j0 += PIECES) {
+                if (!mbar_wait_hot(at.x_full + 8u * xst, xph, abort_flag, at.status)) {
+                    return;
+                }
+                tc_fence_after_sync();
+                const uint32_t x_stage = at.smem0 + xst * (PIECES * at.x_piece_bytes);
+#pragma unroll
+                for (uint32_t i = 0; i < PIECES; ++i) {
+                    const uint32_t j = j0 + i;
+                    const uint64_t b_desc = umma_desc_sw128(x_stage + i * at.x_piece_bytes);
+#pragma unroll
+                    for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
+                        // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
+                        pair_mma_f16_ts(at.tmem_base + (j & (at.chains - 1u)) * kPairTwoChains, a_tmem + j * (kSubK / 2u) + 8u * kk,
+                                        b_desc + 2u * kk, at.idesc, s != work.s0 || j >= at.chains || kk != 0u ? 1u : 0u);
+                    }
+                }
+                pair_commit(at.x_empty + 8u * xst);
+                xst = xst + 1u == at.x_stages ? 0u : xst + 1u;
+                xph ^= xst == 0u ? 1u : 0u;
+            }
+            pair_commit(at.a_empty + 8u * ast);
+            if (++ast == kPairAStages) {
+                ast = 0u;
+                aph ^= 1u;
+            }
+        }
+        pair_commit(at.acc_full);
+    }
+}
+
 template <typename YT>
 __global__ void __launch_bounds__(kPairThreads, 1)
 q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const PairArgs args)
@@ -377,7 +435,8 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const uint32_t smem0 = (smem_u32(smem_raw_) + 1023u) & ~1023u;
     unsigned char *const smem = smem_raw_ + (smem0 - smem_u32(smem_raw_));
     const uint32_t ntok = args.ntok;
-    const uint32_t x_stage_bytes = ntok * (kSubK * 2u) / 2u;      // this block's half of the rows, 64 deep
+    const uint32_t x_piece_bytes = ntok * (kSubK * 2u) / 2u;      // this block's half of the rows, 64 deep
+    const uint32_t x_stage_bytes = x_piece_bytes * args.x_pieces;
     const uint32_t raw_base = smem0 + args.x_stages * x_stage_bytes;
     const uint32_t stage_base = smem0 + kPairRings;
     const uint32_t raw_full = stage_base + kEpilogueWarps * kPairWarpStage;
@@ -547,7 +606,7 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             PairWork work = plan->work;
             while (ok && work.next()) {
                 const uint32_t row = work.tile % tok_tiles * ntok + rank * (ntok / 2u);
-                for (uint32_t sub = work.s0 * kSubs; sub < work.s1 * kSubs; ++sub, ++q) {
+                for (uint32_t sub = work.s0 * kSubs; sub < work.s1 * kSubs; sub += args.x_pieces, ++q) {
                     if (!mbar_wait_hot(x_empty + 8u * st, ph, abort_flag, args.status)) {
                         ok = false;
                         break;
@@ -555,7 +614,10 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     if (rank == 0u) {
                         mbar_expect_tx(x_full + 8u * st, 2u * x_stage_bytes);
                     }
-                    pair_tma_load_2d(smem0 + st * x_stage_bytes, &tmap_x, signal + 8u * st, (int)(sub * kSubK), (int)row);
+                    for (uint32_t i = 0; i < args.x_pieces; ++i) {
+                        pair_tma_load_2d(smem0 + st * x_stage_bytes + i * x_piece_bytes, &tmap_x, signal + 8u * st,
+                                         (int)((sub + i) * kSubK), (int)row);
+                    }
                     if (++st == args.x_stages) {
                         st = 0u;
                         ph ^= 1u;
@@ -575,62 +637,14 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         // ---------------------------------------------------------------- MMA issue, for both blocks
         if (rank == 0u && elect_one()) {
             const uint32_t idesc = umma_idesc(2u * kRows, ntok, args.b_bf16, args.b_bf16);
-            uint32_t xst = 0u, xph = 0u;
-            uint32_t ast = 0u, aph = 0u;
-            uint32_t x_there = 0u, a_there = 0u;   // the next piece of x, the next segment of A, are known to be there
-            bool ok = true;
             PairWork work = plan->work;
             const bool works = !work.last();
-            for (uint32_t turn = 0; ok && work.next(); ++turn) {
-                if (!mbar_wait_hot(acc_empty, (turn & 1u) ^ 1u, abort_flag, args.status)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                for (uint32_t s = work.s0; ok && s < work.s1; ++s) {
-                    if (!a_there && !mbar_wait_hot(a_full + 8u * ast, aph, abort_flag, args.status)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t a_tmem = tmem_base + a_column0 + ast * kPairAColumns;
-#pragma unroll 1
-                    for (uint32_t j = 0; j < kSubs; ++j) {
-                        if (!x_there && !mbar_wait_hot(x_full + 8u * xst, xph, abort_flag, args.status)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after_sync();
-                        // ask for the next piece (and segment) before the MMAs of this one are issued: an answer
-                        // takes as long as two MMAs, and with every wait in the way of the issue a piece took 350
-                        // cycles whatever its width
-                        const uint32_t xnext = xst + 1u == args.x_stages ? 0u : xst + 1u;
-                        const uint32_t xnext_ph = xst + 1u == args.x_stages ? xph ^ 1u : xph;
-                        x_there = mbar_test_wait(x_full + 8u * xnext, xnext_ph);
-                        if (j + 1u == kSubs) {
-                            a_there = mbar_test_wait(a_full + 8u * (ast ^ 1u), ast == 0u ? aph : aph ^ 1u);
-                        }
-                        const uint64_t b_desc = umma_desc_sw128(smem0 + xst * x_stage_bytes);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < kSubK / 16u; ++kk) {
-                            // 16 halves: 8 columns of A, 32 bytes along the swizzled row of x
-                            pair_mma_f16_ts(tmem_base + (j & (chains - 1u)) * kPairTwoChains, a_tmem + j * (kSubK / 2u) + 8u * kk,
-                                            b_desc + 2u * kk, idesc, s != work.s0 || j >= chains || kk != 0u ? 1u : 0u);
-                        }
-                        pair_commit(x_empty + 8u * xst);
-                        xst = xnext;
-                        xph = xnext_ph;
-                    }
-                    if (ok) {
-                        pair_commit(a_empty + 8u * ast);
-                        if (++ast == kPairAStages) {
-                            ast = 0u;
-                            aph ^= 1u;
-                        }
-                    }
-                }
-                if (ok) {
-                    pair_commit(acc_full);
-                }
+            const PairIssue at = {x_full, x_empty, a_full, a_empty, acc_full, acc_empty, tmem_base, a_column0, smem0, x_piece_bytes,
+                                  args.x_stages, idesc, chains, args.status};
+            if (args.x_pieces == 1u) {
+                pair_issue<1u>(work, at, abort_flag);
+            } else {
+                pair_issue<2u>(work, at, abort_flag);
             }
             if (works) {
                 // Every MMA has finished: what the helping warps of both blocks wait for.  This thread waits as
@@ -995,9 +1009,15 @@ cudaError_t launch_pair_kernel(cudaStream_t stream, const CUtensorMap &tw, const
     args.partial = partial;
     args.flags = flags;
     args.tile_floats = tile_floats;
-    // Shared memory: two raw segments and as many pieces of x as fit, three where that leaves five pieces.
-    const unsigned int x_stage = ntok * kSubK;                    // bytes: half of the rows, 64 halves each
-    args.raw_stages = 3u * kRawStageBytes + 5u * x_stage <= kPairRings ? 3u : 2u;
+    // Shared memory: two raw segments and as many stages of x as fit, three where that leaves five of one piece.
+    // A wait, even for what is there, and a commit take the thread that issues the MMAs as long as four MMAs of 160
+    // columns, one piece: so few columns have two pieces to a stage, and a raw segment less to make room for them
+    // (layer of 300 rows, 160 columns, 112.1 -> 109.8 us; with the third raw segment and half the stages 120.7).  256
+    // columns: 773 us a layer of 2048 rows with one piece, 793 with two in a loop.  Four pieces below 128 columns: the
+    // same as two.
+    args.x_pieces = ntok <= 192u ? 2u : 1u;
+    const unsigned int x_stage = ntok * kSubK * args.x_pieces;
+    args.raw_stages = args.x_pieces == 1u && 3u * kRawStageBytes + 5u * x_stage <= kPairRings ? 3u : 2u;
     const unsigned int x_stages = (kPairRings - args.raw_stages * kRawStageBytes) / x_stage;
     args.x_stages = x_stages < kPairMaxX ? x_stages : kPairMaxX;
     const unsigned long long units = (unsigned long long)((n + 2u * kRows - 1u) / (2u * kRows)) * ((m + ntok - 1u) / ntok) * (k / kSegK);
