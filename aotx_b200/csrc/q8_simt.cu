@@ -687,21 +687,25 @@ cudaError_t launch_expert_pairs_simt(cudaStream_t stream, const void *w_gate, co
                          ids, experts, tokens, tokens_dev, used, proj);
 }
 
+constexpr unsigned int kSumThreads = 64;
+
 template <typename YT>
 static cudaError_t expert_sum_launch(bool overlap, bool wide, cudaStream_t stream, const ProjParts &proj,
                                      const float *prob, const unsigned int *ids, unsigned int tokens,
                                      const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
                                      unsigned int used, void *out)
 {
-    // a block per part of a token's row (see the kernel), eight blocks per SM at most
-    const unsigned int step = 256u * (wide ? 4u : 1u);
+    // A block per part of a token's row (see the kernel), sixteen blocks per SM at most.  Blocks of 64 threads, because the
+    // down product before this leaves 6656 registers of an SM: the first blocks are there when it ends (routed experts, 512
+    // tokens, 200.9 -> 199.6 us, 8 tokens 75.0 -> 73.7 against blocks of 256).
+    const unsigned int step = kSumThreads * (wide ? 4u : 1u);
     const unsigned long long items = (unsigned long long)tokens * ((hidden + step - 1u) / step);
-    const unsigned int grid = items < kSmCount * 8u ? (unsigned int)items : kSmCount * 8u;
+    const unsigned int grid = items < kSmCount * 16u ? (unsigned int)items : kSmCount * 16u;
     if (wide) {
-        return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 4u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
+        return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 4u>, grid, kSumThreads, 0, stream, proj, prob, ids, tokens, tokens_dev,
                              hidden, experts, used, static_cast<YT *>(out));
     }
-    return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 1u>, grid, 256, 0, stream, proj, prob, ids, tokens, tokens_dev,
+    return launch_kernel_early(overlap, q8_expert_sum_kernel<YT, 1u>, grid, kSumThreads, 0, stream, proj, prob, ids, tokens, tokens_dev,
                          hidden, experts, used, static_cast<YT *>(out));
 }
 
