@@ -283,6 +283,9 @@ cudaError_t launch_umma(cudaStream_t stream, const UmmaScratch &scratch, unsigne
             return launch_decode_rows(stream, tw, x, x_bf16 != 0, height, args, y_dtype);
         }
         if (warp_kernel) {
+            // (One piece per tile, rows of one segment: no cluster is launched, and whole tiles are units as any others.  The
+            // counted stores of a cluster's exchange are an illegal instruction in a launch without clusters.)
+            args.split = cluster > 1u ? cluster : 0u;
             return launch_decode_warp(stream, tw, x, args, decode_blocks, cluster, y_dtype);
         }
 #endif
