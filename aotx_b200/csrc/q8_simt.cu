@@ -7,7 +7,7 @@
 // left, so that the library covers the whole contract of the reference's kernels:
 //   cuda/model/dequant.cu:9-70      -> q8_dequant_kernel
 //   cuda/model/gemv.cuh:33-145      -> q8_gemv_simt_kernel
-//   cuda/model/experts.cu:10-75     -> q8_route_kernel
+//   cuda/model/experts.cu:10-75     -> q8_route_kernel (many tokens: q8_route.cu)
 //   cuda/model/expert_matrix.cu:8-27, cuda/model/norm.cu:92-105 -> q8_expert_feed_kernel / q8_expert_down_kernel
 //   cuda/model/experts.cu:77-98     -> q8_expert_sum_kernel
 #include "q8_common.cuh"
@@ -104,7 +104,8 @@ __global__ void q8_dequant_kernel_many(const unsigned char *w, unsigned long lon
 // batch, many tokens per row value for a long one.  One block for all experts of four tokens,
 // one row of eight loads per warp at a time, took 78 us at any number of tokens up to
 // 512 (140 us with the router cold in L2); this takes 7 us for 8 tokens and
-// 23 us for 512 (128 experts, hidden 2048).
+// 22 us for 512 (128 experts, hidden 2048), for which q8_route.cu takes 17: above 148 tokens these kernels
+// are left with rows off a 16-byte boundary or of no multiple of 32 values, and with few experts.
 // ---------------------------------------------------------------------------------------
 #define Q8_ROUTE_THREADS 256u     // of the emulated launch
 #define Q8_ROUTE_GPU_THREADS 512u

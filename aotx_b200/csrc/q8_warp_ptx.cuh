@@ -52,6 +52,12 @@ __device__ __forceinline__ void copy_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+// All of this thread's copies, committed or not.
+__device__ __forceinline__ void copy_async_wait_all()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // A barrier's memory may be used for something else, another barrier for instance.
 __device__ __forceinline__ void mbar_inval(uint32_t bar)
 {
