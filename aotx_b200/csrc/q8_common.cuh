@@ -167,6 +167,14 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
     return mbar_wait(bar, parity, abort_flag, status);
 }
 
+// The wait for what other blocks of the cluster store here with stores that count themselves on the barrier
+// (store_counted): their arrivals release at cluster scope, so it takes an acquire at that scope before the values are read.
+__device__ __forceinline__ bool mbar_wait_counted(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
+                                                  unsigned int *status)
+{
+    return mbar_wait(bar, parity, abort_flag, status) && mbar_test_cluster(bar, parity) != 0u;
+}
+
 // ---------------------------------------------------------------------------------------
 // Bulk tensor copies (TMA), global -> shared, no multicast.
 // ---------------------------------------------------------------------------------------

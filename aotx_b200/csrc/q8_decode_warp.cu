@@ -487,7 +487,7 @@ q8_decode_kernel_warp(const __grid_constant__ CUtensorMap tmap_w, const void *x_
         // The stores count themselves on their owner's barrier, which is all it waits for.  (A barrier of the cluster with
         // release and acquire in its place: 4096 x 4096, 8 rows, 6.95 us against 6.62, 4096 x 14336 14.9 and 14.4, 2560 x
         // 9728, 12 rows, 11.9 and 11.3.)
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(received, 0u, abort_flag, args.status))) {
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait_counted(received, 0u, abort_flag, args.status))) {
             // Pieces are missing, and may still be on their way into this block's shared memory: it stays until every
             // other thread of the cluster has ended or come here.
             cluster_arrive_relaxed();

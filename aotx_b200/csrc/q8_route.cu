@@ -265,7 +265,7 @@ q8_route_kernel_tiles(const RouteArgs args)
     if (warp >= chosen_here) {
         return;
     }
-    if (!__all_sync(0xFFFFFFFFu, mbar_wait(gathered, 0u, abort_flag, args.status))) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait_counted(gathered, 0u, abort_flag, args.status))) {
         // Logits are missing, and may still be on their way into this block's shared memory: it stays until every
         // other thread of the cluster has ended (or come here).
         cluster_arrive_relaxed();

@@ -333,7 +333,7 @@ inline uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
     return done ? 1u : 0u;
 }
 
-inline uint32_t mbar_test_wait(uint32_t bar, uint32_t parity)
+inline uint32_t mbar_test_cluster(uint32_t bar, uint32_t parity)
 {
     return mbar_try_wait(bar, parity);
 }
