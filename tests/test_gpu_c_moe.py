@@ -94,6 +94,53 @@ def test_route_of_many_tokens(ctx, oracle, tokens, experts, used, hidden, live):
     assert ctx.device_status() == 0
 
 
+def _off_boundary(t, values):
+    """A copy that starts `values` elements after a 16-byte boundary, which the router's tiles do not take."""
+    flat = torch_mod().empty(t.numel() + values, dtype=t.dtype, device="cuda")
+    return flat[values:].view(t.shape).copy_(t)
+
+
+# Every form of the tiles (tokens to a group, experts to a block) and every size of cluster, with a last group and a last
+# block that are not full; beside them the kernels that take rows off a boundary, for more than 148 tokens clusters of
+# four blocks, and one block for all experts where rows are long or tokens many and experts at most 64.
+@pytest.mark.parametrize("tokens,experts,used,hidden", [
+    (149, 17, 3, 32), (153, 33, 4, 160), (220, 136, 8, 512), (200, 192, 7, 1056),      # groups of 4, clusters of 1, 2, 5, 6
+    (257, 100, 8, 2048), (592, 64, 6, 288), (1000, 17, 2, 544), (180, 72, 5, 4096),    # groups of 8, clusters of 4, 2, 1, 3
+    (593, 64, 6, 288), (297, 128, 8, 2048), (300, 96, 8, 640), (149, 200, 8, 1024),    # groups of 16, clusters of 2, 4, 3, 7
+    (256, 224, 8, 4096), (256, 256, 8, 2048), (1203, 250, 9, 1056),                    # clusters of 7 and 8, groups one behind the other
+    (150, 48, 3, 4128), (1201, 20, 4, 96),                                             # beside one block for all experts
+    (593, 16, 2, 1120), (1300, 14, 2, 288)])                                           # a block for all of few experts, 8 and 16 tokens
+def test_router_tiles_give_the_floats_of_the_other_kernels(ctx, tokens, experts, used, hidden):
+    torch = torch_mod()
+    gen = torch.Generator(device="cuda").manual_seed(tokens * 7 + experts)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).half()
+    router = torch.randn(experts, hidden, device="cuda", generator=gen) / hidden ** 0.5
+    router[experts - 1] = router[0]
+    prob = torch.full((tokens + 1, experts), GUARD, dtype=torch.float32, device="cuda")
+    ids = torch.full((tokens + 1, used), -1, dtype=torch.int32, device="cuda")
+    ctx.moe_route(x, router, used, tokens=tokens, prob=prob, ids=ids)
+    for x_other, router_other in ((_off_boundary(x, 4), router), (x, _off_boundary(router, 1))):
+        want_p, want_i = ctx.moe_route(x_other, router_other, used)
+        assert torch.equal(prob[:tokens].view(torch.int32), want_p.view(torch.int32))
+        assert torch.equal(ids[:tokens], want_i)
+    assert bool((prob[tokens:] == GUARD).all()) and bool((ids[tokens:] == -1).all())
+    assert ctx.device_status() == 0
+
+
+# more than 148 tokens, rows of no multiple of 32 values: clusters of four, and one block for all experts
+@pytest.mark.parametrize("tokens,experts,hidden", [(149, 33, 1000), (300, 128, 2040), (160, 20, 4100), (1100, 64, 500)])
+def test_router_of_other_widths(ctx, oracle, tokens, experts, hidden):
+    torch = torch_mod()
+    rng = np.random.Generator(np.random.PCG64(tokens + hidden))
+    router = rng.standard_normal((experts, hidden)).astype(np.float32) / np.float32(np.sqrt(hidden))
+    x = rng.standard_normal((tokens, hidden)).astype(np.float16)
+    prob, ids = ctx.moe_route(dev(x), dev(router), 4)
+    torch.cuda.synchronize()
+    want_p, want_i = oracle.route(x.view(np.uint16), router, 4)
+    assert np.abs(prob.cpu().numpy() - want_p).max() < 2e-6
+    assert np.array_equal(ids.cpu().numpy().view(np.uint32), want_i)
+
+
 def _moe_case(oracle, tokens, experts, used, hidden, ffn, seed):
     import aotx_b200
     wg = aotx_b200.synth_q8_0(experts * ffn, hidden, seed)
