@@ -134,12 +134,13 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
                          const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts,
                          unsigned int used, float *prob, unsigned int *ids, unsigned int *status, bool overlap = false);
 
-// The router on tiles of shared memory (q8_route.cu), for many tokens: rows of a multiple of 32 values, x and router on
-// 16-byte boundaries.
-bool route_tiles_fits(const void *x, const float *router, unsigned int tokens, unsigned int hidden, unsigned int experts);
+// The router on tiles of shared memory (q8_route.cu), for many tokens whose number the host knows: rows of a multiple of 32
+// values, x and router on 16-byte boundaries.
+bool route_tiles_fits(const void *x, const float *router, unsigned int tokens, const unsigned int *tokens_dev,
+                      unsigned int hidden, unsigned int experts);
 cudaError_t launch_route_tiles(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
-                               const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts, unsigned int used,
-                               float *prob, unsigned int *ids, unsigned int *status, bool overlap);
+                               unsigned int hidden, unsigned int experts, unsigned int used, float *prob, unsigned int *ids,
+                               unsigned int *status, bool overlap);
 
 // Expert parallel (several GPUs, each holding a run of the experts; q8_api.cu aotx_q8_moe_ep).
 // Where the rows of x of all GPUs' tokens lie: rows_per_part rows in each of `parts` arrays

@@ -39,11 +39,10 @@ constexpr uint32_t kRouteMostBytes = 200u * 1024u; // of shared memory
 struct RouteArgs {
     const __half *x;
     const float *router;
-    const unsigned int *tokens_dev;
     float *prob;
     unsigned int *ids;
     unsigned int *status;
-    uint32_t tokens_max, hidden, experts, used;
+    uint32_t tokens, hidden, experts, used;
     uint32_t stages;
 };
 
@@ -138,16 +137,8 @@ q8_route_kernel_tiles(const RouteArgs args)
 
     grid_dependency_wait();
     grid_launch_dependents();
-    uint32_t tokens = args.tokens_max;
-    if (args.tokens_dev != nullptr) {
-        const uint32_t live = *args.tokens_dev;
-        tokens = live < tokens ? live : tokens;
-    }
     const uint32_t t0 = blockIdx.x / csize * S::tokens;
-    if (t0 >= tokens) {
-        return;     // the whole cluster
-    }
-    const uint32_t group = tokens - t0 < S::tokens ? tokens - t0 : S::tokens;
+    const uint32_t group = args.tokens - t0 < S::tokens ? args.tokens - t0 : S::tokens;
     const uint32_t chosen_here = group > crank ? (group - crank + csize - 1u) / csize : 0u;   // tokens crank, crank + csize, ..
     if (threadIdx.x == 0u) {
         for (uint32_t i = 0; i < args.stages; ++i) {
@@ -287,7 +278,7 @@ static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool
         return err;
     }
     const uint32_t cluster = (args.experts + SET - 1u) / SET;
-    const uint32_t groups = (args.tokens_max + S::tokens - 1u) / S::tokens;
+    const uint32_t groups = (args.tokens + S::tokens - 1u) / S::tokens;
     const uint32_t chunks = (args.hidden + kRouteChunk - 1u) / kRouteChunk;
     const uint32_t logits = (S::tokens + cluster - 1u) / cluster * args.experts * 4u;
     // a block per SM: as deep a ring as fits; more: half of it, so that two are on an SM
@@ -317,24 +308,27 @@ static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool
 // 12.2, 256 18.2 and 12.2, 512 22.0 and 16.8, 700 35.4 and 26.8, 2048 82.2 and 53.8; 64 x 2048, 128 tokens 9.6 and 11.2,
 // 149 14.0 and 11.2, 512 16.2 and 12.2; 32 x 1024, 128 tokens 6.6 and 7.2, 149 10.2 and 7.2, 700 21.0 and 7.9; 16 x
 // 2048, 300 tokens 7.9 and 8.2, 512 8.0 and 8.2, 700 11.1 and 10.0, 2048 21.2 and 13.6; 8 x 2048, 512 tokens 6.8 and 8.3.
-bool route_tiles_fits(const void *x, const float *router, unsigned int tokens, unsigned int hidden, unsigned int experts)
+// Only where the host knows the number of tokens: the tile of a group costs the same for one token as for all of them, and a
+// launch for a maximum of which few are live was slower (maximum, live, experts x 2048: 512, 1, 128 14.5 and 16.6; 2048, 64, 8
+// 7.4 and 15.0; 65536, 64, 256 23.8 and 56.4).
+bool route_tiles_fits(const void *x, const float *router, unsigned int tokens, const unsigned int *tokens_dev,
+                      unsigned int hidden, unsigned int experts)
 {
-    return tokens > (experts > kRouteFewExperts ? kSmCount : 4u * kSmCount) && (hidden % kRouteStep) == 0u
+    return tokens_dev == nullptr && tokens > (experts > kRouteFewExperts ? kSmCount : 4u * kSmCount) && (hidden % kRouteStep) == 0u
         && (reinterpret_cast<uintptr_t>(x) & 15u) == 0u && (reinterpret_cast<uintptr_t>(router) & 15u) == 0u;
 }
 
 cudaError_t launch_route_tiles(cudaStream_t stream, const void *x, const float *router, unsigned int tokens,
-                               const unsigned int *tokens_dev, unsigned int hidden, unsigned int experts, unsigned int used,
-                               float *prob, unsigned int *ids, unsigned int *status, bool overlap)
+                               unsigned int hidden, unsigned int experts, unsigned int used, float *prob, unsigned int *ids,
+                               unsigned int *status, bool overlap)
 {
     RouteArgs args = {};
     args.x = static_cast<const __half *>(x);
     args.router = router;
-    args.tokens_dev = tokens_dev;
     args.prob = prob;
     args.ids = ids;
     args.status = status;
-    args.tokens_max = tokens;
+    args.tokens = tokens;
     args.hidden = hidden;
     args.experts = experts;
     args.used = used;

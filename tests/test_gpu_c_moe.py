@@ -141,6 +141,45 @@ def test_router_of_other_widths(ctx, oracle, tokens, experts, hidden):
     assert np.array_equal(ids.cpu().numpy().view(np.uint32), want_i)
 
 
+def _route_us(ctx, x, router, used, live):
+    torch = torch_mod()
+    tokens, experts = x.shape[0], router.shape[0]
+    prob = torch.empty(tokens, experts, device="cuda")
+    ids = torch.empty(tokens, used, dtype=torch.int32, device="cuda")
+    count = None if live is None else torch.tensor([live], dtype=torch.int32, device="cuda")
+    ctx.moe_route(x, router, used, tokens_dev=count, prob=prob, ids=ids)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(10):
+            ctx.moe_route(x, router, used, tokens_dev=count, prob=prob, ids=ids)
+    graph.replay()
+    times = []
+    for _ in range(7):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        for _ in range(4):
+            graph.replay()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end) * 1000.0 / 40.0)
+    return min(times)
+
+
+# The rule between the router's kernels: rows on a boundary may take another kernel than rows off it, not a slower one.  A
+# fifth is more than two runs of one kernel differ by.
+@pytest.mark.parametrize("tokens,experts,hidden,live", [
+    (2048, 8, 2048, 64), (2048, 32, 2048, 8)])     # few of the most are live: 2.0 and 1.5 of the others' time on tiles
+def test_router_on_a_boundary_is_not_slower(ctx, tokens, experts, hidden, live):
+    torch = torch_mod()
+    gen = torch.Generator(device="cuda").manual_seed(tokens + experts)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).half()
+    router = torch.randn(experts, hidden, device="cuda", generator=gen) / hidden ** 0.5
+    on = _route_us(ctx, x, router, min(8, experts), live)
+    off = _route_us(ctx, _off_boundary(x, 4), router, min(8, experts), live)
+    assert on <= 1.2 * off, (on, off)
+
+
 def _moe_case(oracle, tokens, experts, used, hidden, ffn, seed):
     import aotx_b200
     wg = aotx_b200.synth_q8_0(experts * ffn, hidden, seed)
