@@ -22,6 +22,8 @@
 #include "q8_route.cuh"
 #include "q8_warp_ptx.cuh"
 
+#include <atomic>
+
 namespace q8 {
 
 constexpr uint32_t kRouteWarps = 8;
@@ -34,7 +36,8 @@ constexpr uint32_t kRouteXBytes = kRouteChunk * 2u + 64u;
 constexpr uint32_t kRouteMaxStages = 32;
 constexpr uint32_t kRouteBarBytes = 8u * kRouteMaxStages + 16u;
 constexpr uint32_t kRouteFewExperts = 16;          // one set of them to a block, no cluster
-constexpr uint32_t kRouteMostBytes = 200u * 1024u; // of shared memory
+constexpr uint32_t kRouteMostBytes = 200u * 1024u; // of shared memory, one block per SM
+constexpr uint32_t kRouteHalfBytes = (228u * 1024u) / 2u - 1536u;    // two blocks
 
 struct RouteArgs {
     const __half *x;
@@ -269,7 +272,7 @@ q8_route_kernel_tiles(const RouteArgs args)
 }
 
 template <uint32_t TT, uint32_t ET, uint32_t SET>
-static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool overlap)
+static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool deep, bool overlap)
 {
     using S = RouteTile<TT, ET, SET>;
     static unsigned long long configured = 0ull;
@@ -281,8 +284,7 @@ static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool
     const uint32_t groups = (args.tokens + S::tokens - 1u) / S::tokens;
     const uint32_t chunks = (args.hidden + kRouteChunk - 1u) / kRouteChunk;
     const uint32_t logits = (S::tokens + cluster - 1u) / cluster * args.experts * 4u;
-    // a block per SM: as deep a ring as fits; more: half of it, so that two are on an SM
-    const uint32_t most = groups * cluster <= kSmCount ? kRouteMostBytes : (228u * 1024u) / 2u - 1536u;
+    const uint32_t most = deep ? kRouteMostBytes : kRouteHalfBytes;
     const uint32_t fits = (most - kRouteBarBytes - logits) / S::stage_bytes;
     args.stages = chunks < fits ? chunks : fits;
     args.stages = args.stages < kRouteMaxStages ? args.stages : kRouteMaxStages;
@@ -301,6 +303,44 @@ static cudaError_t launch_route_sized(cudaStream_t stream, RouteArgs &args, bool
     config.attrs = attribute;
     config.numAttrs = overlap ? 2u : 1u;
     return cudaLaunchKernelEx(&config, q8_route_kernel_tiles<TT, ET, SET>, args);
+}
+
+// How many clusters of `cluster` blocks run at the same time: low half a block per SM, high half two.  What a chip's
+// parts have room for differs from one to the next, so it is asked for, once per device and size.
+static uint32_t route_clusters(uint32_t cluster)
+{
+    static std::atomic<uint32_t> known[64][Q8_ROUTE_EXPERTS / 32u + 1u];
+    static unsigned long long configured = 0ull;
+    auto kernel = q8_route_kernel_tiles<4u, 8u, 32u>;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || allow_shared_memory(kernel, kRouteMostBytes, &configured) != cudaSuccess) {
+        return 0u;
+    }
+    uint32_t at_once = known[device & 63][cluster].load(std::memory_order_relaxed);
+    if (at_once == 0u) {
+        cudaLaunchAttribute attribute[1];
+        attribute[0].id = cudaLaunchAttributeClusterDimension;
+        attribute[0].val.clusterDim.x = cluster;
+        attribute[0].val.clusterDim.y = 1;
+        attribute[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(cluster, 1, 1);
+        config.blockDim = dim3(kRouteThreads, 1, 1);
+        config.attrs = attribute;
+        config.numAttrs = 1u;
+        int alone = 0, paired = 0;
+        config.dynamicSmemBytes = kRouteMostBytes;
+        cudaError_t err = cudaOccupancyMaxActiveClusters(&alone, kernel, &config);
+        config.dynamicSmemBytes = kRouteHalfBytes;
+        err = err == cudaSuccess ? cudaOccupancyMaxActiveClusters(&paired, kernel, &config) : err;
+        if (err != cudaSuccess) {
+            (void)cudaGetLastError();     // the launch does without
+            return 0u;
+        }
+        at_once = (uint32_t)alone | ((uint32_t)paired << 16);
+        known[device & 63][cluster].store(at_once, std::memory_order_relaxed);
+    }
+    return at_once;
 }
 
 // More tokens than SMs, and where one block of q8_route_kernel takes all of few experts, more than one turn of them (four
@@ -332,20 +372,16 @@ cudaError_t launch_route_tiles(cudaStream_t stream, const void *x, const float *
     args.hidden = hidden;
     args.experts = experts;
     args.used = used;
-    // The fewest tokens to a group with which every block still has an SM.
     const bool wide = experts > kRouteFewExperts;
-    const uint32_t cluster = wide ? (experts + 31u) / 32u : 1u;
-    uint32_t group = wide ? 4u : 8u;
-    while (group < 16u && (tokens + group - 1u) / group * cluster > kSmCount) {
-        group *= 2u;
-    }
+    const uint32_t at_once = route_clusters(wide ? (experts + 31u) / 32u : 1u);
+    const RoutePlan plan = route_plan(tokens, wide ? 4u : 8u, at_once & 0xFFFFu, at_once >> 16);
     if (wide) {
-        return group == 4u   ? launch_route_sized<1u, 8u, 32u>(stream, args, overlap)
-               : group == 8u ? launch_route_sized<2u, 8u, 32u>(stream, args, overlap)
-                             : launch_route_sized<4u, 8u, 32u>(stream, args, overlap);
+        return plan.group == 4u   ? launch_route_sized<1u, 8u, 32u>(stream, args, plan.deep, overlap)
+               : plan.group == 8u ? launch_route_sized<2u, 8u, 32u>(stream, args, plan.deep, overlap)
+                                  : launch_route_sized<4u, 8u, 32u>(stream, args, plan.deep, overlap);
     }
-    return group == 8u ? launch_route_sized<1u, 8u, 16u>(stream, args, overlap)
-                       : launch_route_sized<2u, 8u, 16u>(stream, args, overlap);
+    return plan.group == 8u ? launch_route_sized<1u, 8u, 16u>(stream, args, plan.deep, overlap)
+                            : launch_route_sized<2u, 8u, 16u>(stream, args, plan.deep, overlap);
 }
 
 } // namespace q8

@@ -5,10 +5,34 @@
 #include "q8_common.cuh"
 
 #include <math_constants.h>
+#include <stdint.h>
 
 namespace q8 {
 
 #define Q8_ROUTE_EXPERTS 256u
+
+// How q8_route_kernel_tiles divides the tokens: rows of x to a group, and whether its rings are as deep as one block of an SM
+// has room for, or half of that, for two.
+struct RoutePlan {
+    uint32_t group;
+    bool deep;
+};
+
+// The fewest tokens to a group (`smallest`, doubled up to 16) with which all clusters run at the same time, a block per SM:
+// `alone` is how many do, `paired` how many with two blocks to an SM.  Where not even groups of 16 do, groups of 8 if they
+// run at the same time in pairs, else groups of 16.  (Clusters of five blocks and more leave SMs of each part of the chip
+// over - 15 clusters of seven or eight, not 21 or 18 - and one cluster behind the others takes as long as all of them: 256 experts
+// x 4096, 256 tokens, 16 clusters of groups of 16, 59 us alone, 49 in pairs, which share SMs while others have none; 32 clusters
+// of groups of 8 in pairs 32.)
+__host__ __device__ inline RoutePlan route_plan(uint32_t tokens, uint32_t smallest, uint32_t alone, uint32_t paired)
+{
+    for (uint32_t group = smallest; group <= 16u; group *= 2u) {
+        if ((tokens + group - 1u) / group <= alone) {
+            return {group, true};
+        }
+    }
+    return {(tokens + 7u) / 8u <= paired ? 8u : 16u, false};
+}
 
 // The largest value over the warp and the lowest index that has it.  Every value is a probability or -1, so
 // their bits order them as signed integers do: two reductions in place of ten shuffles.

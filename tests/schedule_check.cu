@@ -18,7 +18,10 @@
 //      names where units are dealt, the pieces of a cluster's block within run_segs and in one tile;
 //   9. launches of pairs that share the SMs (streams of one's own, in any order of steps) come to their end with as few
 //      as one place more than there are launches, and every run of rows of a cut tile is finished once: pair_undecided,
-//      pair_share.  With holders that wait whether or not all others run, some of the same orders have no end.
+//      pair_share.  With holders that wait whether or not all others run, some of the same orders have no end;
+//  10. the router's tiles (route_plan in q8_route.cuh) take a ring as deep as one block of an SM has room for only where all
+//      clusters run at the same time that way, with the fewest tokens to a group, and else groups of 8 where those run at the
+//      same time in pairs.
 //
 // Prints "ok <cases>" and exits 0, or the first violated property and exits 1.
 #include <cstdio>
@@ -26,6 +29,7 @@
 #include <utility>
 #include <vector>
 
+#include "q8_route.cuh"
 #include "q8_schedule.cuh"
 #include "q8_tile.cuh"
 
@@ -441,6 +445,20 @@ static int check_shared_places(uint32_t *stuck, unsigned long long *cases)
     return 0;
 }
 
+// `alone`, `paired`: clusters that run at the same time with one block, with two, to an SM.
+static int check_route(uint32_t tokens, uint32_t smallest, uint32_t alone, uint32_t paired)
+{
+    const RoutePlan plan = route_plan(tokens, smallest, alone, paired);
+    auto groups = [&](uint32_t group) { return (tokens + group - 1u) / group; };
+    bool right = plan.group >= smallest && plan.group <= 16u && (plan.group & (plan.group - 1u)) == 0u;
+    if (plan.deep) {
+        right = right && groups(plan.group) <= alone && (plan.group == smallest || groups(plan.group / 2u) > alone);
+    } else {
+        right = right && groups(16u) > alone && plan.group == (groups(8u) <= paired ? 8u : 16u);
+    }
+    return right ? 0 : fail("the router's groups", tokens, alone, paired, plan.group);
+}
+
 int main()
 {
     unsigned long long cases = 0;
@@ -513,6 +531,19 @@ int main()
                 // (the launch has as many pairs as units, at most)
                 if (check_pairs(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0
                     || check_first_holder(tiles, segs, tiles * segs < pairs ? tiles * segs : pairs) != 0) {
+                    return 1;
+                }
+                cases += 1;
+            }
+        }
+    }
+    // a B200's clusters of one to eight blocks, and none known
+    const uint32_t at_once[][2] = {{148u, 296u}, {74u, 148u}, {45u, 93u}, {33u, 71u}, {26u, 56u}, {22u, 45u}, {15u, 37u},
+                                   {15u, 33u},   {0u, 0u}};
+    for (const auto &clusters : at_once) {
+        for (uint32_t smallest : {4u, 8u}) {
+            for (uint32_t tokens = 1; tokens <= 5000u; ++tokens) {
+                if (check_route(tokens, smallest, clusters[0], clusters[1]) != 0) {
                     return 1;
                 }
                 cases += 1;

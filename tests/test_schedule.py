@@ -1,8 +1,8 @@
 """The division of work of the kernels on tensor memory, checked on the host.
 
 `schedule_check.cu` drives the kernels' own scheduling helpers (`unit_range`, `WorkIter`,
-`last_holder` in aotx_b200/csrc/q8_tile.cuh, `mid_deal` and `pair_deal` in q8_schedule.cuh) over a sweep
-of shapes and grid sizes and checks that every unit is computed once, that a block publishes
+`last_holder` in aotx_b200/csrc/q8_tile.cuh, `mid_deal` and `pair_deal` in q8_schedule.cuh, `route_plan` in
+q8_route.cuh) over a sweep of shapes and grid sizes and checks that every unit is computed once, that a block publishes
 before it waits, that the owner of a cut tile waits for exactly the blocks that hold the rest of it, and
 that pieces are as long as their rules say.  The reference has no
 counterpart: its product kernel launches one block for each tile of y (cuda/model/gemm.cu:2-3)."""
