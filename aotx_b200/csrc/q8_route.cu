@@ -343,18 +343,13 @@ static uint32_t route_clusters(uint32_t cluster)
     return at_once;
 }
 
-// More tokens than SMs, and where one block of q8_route_kernel takes all of few experts, more than one turn of them (four
-// tokens to a block).  Us, those kernels and this one, experts x width: 128 x 2048, 128 tokens 12.9 and 11.3, 149 15.0 and
-// 12.2, 256 18.2 and 12.2, 512 22.0 and 16.8, 700 35.4 and 26.8, 2048 82.2 and 53.8; 64 x 2048, 128 tokens 9.6 and 11.2,
-// 149 14.0 and 11.2, 512 16.2 and 12.2; 32 x 1024, 128 tokens 6.6 and 7.2, 149 10.2 and 7.2, 700 21.0 and 7.9; 16 x
-// 2048, 300 tokens 7.9 and 8.2, 512 8.0 and 8.2, 700 11.1 and 10.0, 2048 21.2 and 13.6; 8 x 2048, 512 tokens 6.8 and 8.3.
 // Only where the host knows the number of tokens: the tile of a group costs the same for one token as for all of them, and a
-// launch for a maximum of which few are live was slower (maximum, live, experts x 2048: 512, 1, 128 14.5 and 16.6; 2048, 64, 8
-// 7.4 and 15.0; 65536, 64, 256 23.8 and 56.4).
+// launch for a maximum of which few are live was slower (us, other kernels and this one; maximum, live, experts x 2048: 512, 1,
+// 128 14.5 and 16.6; 2048, 64, 8 7.4 and 15.0; 65536, 64, 256 23.8 and 56.4).
 bool route_tiles_fits(const void *x, const float *router, unsigned int tokens, const unsigned int *tokens_dev,
                       unsigned int hidden, unsigned int experts)
 {
-    return tokens_dev == nullptr && tokens > (experts > kRouteFewExperts ? kSmCount : 4u * kSmCount) && (hidden % kRouteStep) == 0u
+    return tokens_dev == nullptr && route_tiles_pay(tokens, hidden, experts) && (hidden % kRouteStep) == 0u
         && (reinterpret_cast<uintptr_t>(x) & 15u) == 0u && (reinterpret_cast<uintptr_t>(router) & 15u) == 0u;
 }
 

@@ -170,7 +170,8 @@ def _route_us(ctx, x, router, used, live):
 # fifth is more than two runs of one kernel differ by.
 @pytest.mark.parametrize("tokens,experts,hidden,live", [
     (2048, 8, 2048, 64), (2048, 32, 2048, 8),      # few of the most are live: 2.0 and 1.5 of the others' time on tiles
-    (256, 224, 4096, None)])                       # 16 clusters, of which 15 run at the same time alone on their SMs: 1.6
+    (256, 224, 4096, None),                        # 16 clusters, of which 15 run at the same time alone on their SMs: 1.6
+    (1024, 8, 4096, None), (593, 2, 6144, None), (200, 17, 8192, None), (592, 24, 5120, None)])   # one block for all experts: 1.3 to 2.2
 def test_router_on_a_boundary_is_not_slower(ctx, tokens, experts, hidden, live):
     torch = torch_mod()
     gen = torch.Generator(device="cuda").manual_seed(tokens + experts)
