@@ -614,9 +614,11 @@ q8_wide_kernel_pair(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     if (rank == 0u) {
                         mbar_expect_tx(x_full + 8u * st, 2u * x_stage_bytes);
                     }
-                    for (uint32_t i = 0; i < args.x_pieces; ++i) {
-                        pair_tma_load_2d(smem0 + st * x_stage_bytes + i * x_piece_bytes, &tmap_x, signal + 8u * st,
-                                         (int)((sub + i) * kSubK), (int)row);
+                    // (a loop over the pieces in place of the two: 0.6 % slower over 110 shapes of 96 to 540 rows)
+                    pair_tma_load_2d(smem0 + st * x_stage_bytes, &tmap_x, signal + 8u * st, (int)(sub * kSubK), (int)row);
+                    if (args.x_pieces > 1u) {
+                        pair_tma_load_2d(smem0 + st * x_stage_bytes + x_piece_bytes, &tmap_x, signal + 8u * st,
+                                         (int)((sub + 1u) * kSubK), (int)row);
                     }
                     if (++st == args.x_stages) {
                         st = 0u;
@@ -1011,11 +1013,14 @@ cudaError_t launch_pair_kernel(cudaStream_t stream, const CUtensorMap &tw, const
     args.tile_floats = tile_floats;
     // Shared memory: two raw segments and as many stages of x as fit, three where that leaves five of one piece.
     // A wait, even for what is there, and a commit take the thread that issues the MMAs as long as four MMAs of 160
-    // columns, one piece: so few columns have two pieces to a stage, and a raw segment less to make room for them
-    // (layer of 300 rows, 160 columns, 112.1 -> 109.8 us; with the third raw segment and half the stages 120.7).  256
-    // columns: 773 us a layer of 2048 rows with one piece, 793 with two in a loop.  Four pieces below 128 columns: the
-    // same as two.
-    args.x_pieces = ntok <= 192u ? 2u : 1u;
+    // columns, one piece: so few columns have two pieces to a stage, and a raw segment less to make room for them.  Us with
+    // one piece and with two: 28672 x 4096, 96 rows, 38.5 and 35.9, 128 rows 39.7 and 37.6 (three raw segments beside two
+    // pieces: the same), 150 rows 42.0 and 40.3, 300 rows (160 columns) 71.0 and 69.1; four pieces below 128 columns: the same
+    // as two.  192 columns: three stages of two hold less than seven of one, which one token tile feels (20480 x 4096, 192 rows,
+    // 35.5 and 36.3, 28672 x 4096 44.7 and 45.1, 14336 x 4096 26.5 and 26.3) and several do not (28672 x 4096, 370 rows, 78.0
+    // and 77.4, 540 rows 110.4 and 109.3, 24000 x 4096, 540 rows, 90.5 and 89.2).  224 columns: 28672 x 4096, 224 rows, 47.3
+    // and 48.2; 256: 250 rows 55.0 and 60.7.
+    args.x_pieces = ntok <= (m > ntok ? 192u : 160u) ? 2u : 1u;
     const unsigned int x_stage = ntok * kSubK * args.x_pieces;
     args.raw_stages = args.x_pieces == 1u && 3u * kRawStageBytes + 5u * x_stage <= kPairRings ? 3u : 2u;
     const unsigned int x_stages = (kPairRings - args.raw_stages * kRawStageBytes) / x_stage;

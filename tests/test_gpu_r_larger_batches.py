@@ -32,7 +32,8 @@ def sums(ctx, w, n, k, x, extra=0.0):
 # rows of w: a partial tile; one tile; a cluster of four's, of two's; two turns; cut into units; and deep
 # enough that one tile has several holders
 SHAPES = [(20004, 512, 113), (1, 256, 17), (130, 1024, 33), (1023, 2048, 128), (9990, 512, 40), (20004, 768, 64), (60001, 256, 100),
-          (77, 1536, 129), (300, 5120, 257), (2049, 1024, 300), (19456, 512, 512), (40962, 256, 700)]
+          (77, 1536, 129), (300, 5120, 257), (2049, 1024, 300), (19456, 512, 512), (40962, 256, 700),
+          (20004, 512, 192), (20004, 512, 325), (1500, 2048, 370), (2049, 1024, 576)]
 
 
 @pytest.mark.parametrize("n,k,m", SHAPES)
