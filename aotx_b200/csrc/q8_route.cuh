@@ -1,5 +1,5 @@
-// The end of the expert router for one token: the softmax over its logits and the experts in order of probability.
-// Shared by the router kernels (q8_simt.cu, q8_route.cu).
+// What the router kernels share (q8_simt.cu, q8_route.cu): the host's rules between and for them, and the end of the router for
+// one token, the softmax over its logits and the experts in order of probability.
 #pragma once
 
 #include "q8_common.cuh"
@@ -14,8 +14,9 @@ namespace q8 {
 // Whether the router runs on q8_route_kernel_tiles, for the number of tokens that it has.  Where the lines lie (us, the other
 // kernels and this one, experts x width):
 //   * Up to 148 tokens the others have an SM or more per token: 64 x 2048, 128 tokens 9.6 and 11.2; 149 14.0 and 11.2; 512 16.2
-//     and 12.2; 128 x 2048, 128 tokens 12.9 and 11.3, 149 15.1 and 12.4, 256 18.3 and 12.4, 512 22.0 and 17.0, 2048 82 and 54;
-//     256 x 4096, 400 tokens 74 and 49.  (33 to 72 experts fill little more than half of their blocks: 65 to 72 of 1536 to 2048,
+//     and 12.2; 32 x 1024, 128 tokens 6.6 and 7.2, 149 10.2 and 7.2; 256 x 4096, 400 tokens 74 and 49.  One line for all
+//     numbers of experts, although 128 x 2048 have theirs below it: 128 tokens 12.9 and 11.3, 149 15.1 and 12.4, 256 18.3 and 12.4,
+//     512 22.0 and 17.0, 2048 82 and 54.  (33 to 72 experts fill little more than half of their blocks: 65 to 72 of 1536 to 2048,
 //     365 to 592 tokens, are a tenth slower at most, the same of 2560 or 4096 half the time of the others.)
 //   * Few experts leave the tiles, 16 of them, without work, and one block of the others takes all of four tokens (two such
 //     blocks to an SM: 1184 tokens at once).  16 x 2048, 300 tokens 7.9 and 8.2, 700 11.9 and 10.7, 2048 22 and 15; 16 x

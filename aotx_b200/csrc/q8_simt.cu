@@ -105,7 +105,8 @@ __global__ void q8_dequant_kernel_many(const unsigned char *w, unsigned long lon
 // one row of eight loads per warp at a time, took 78 us at any number of tokens up to
 // 512 (140 us with the router cold in L2); this takes 7 us for 8 tokens and
 // 22 us for 512 (128 experts, hidden 2048), for which q8_route.cu takes 17: above 148 tokens these kernels
-// are left with a live count on the device, rows off a 16-byte boundary or of no multiple of 32 values, and few experts.
+// are left with a live count on the device, rows off a 16-byte boundary or of no multiple of 32 values, and the numbers of
+// experts and widths for which they are the faster ones (route_tiles_pay in q8_route.cuh).
 // ---------------------------------------------------------------------------------------
 #define Q8_ROUTE_THREADS 256u     // of the emulated launch
 #define Q8_ROUTE_GPU_THREADS 512u
@@ -617,8 +618,8 @@ cudaError_t launch_route(cudaStream_t stream, const void *x, const float *router
     // block has 16 warps of one or two experts each (measured against 8 warps of two or four; 128
     // experts, 2048 wide: 8 tokens 9.5 -> 7.2 us, 128 tokens 20.8 -> 13.0, 512 tokens 25.0 -> 22.6).
     // Few experts leave most warps of such a cluster without work, and every block of it reads the group's
-    // activations: then a block takes all experts of four tokens by itself.  (Above 148 tokens all this is left to live
-    // counts on the device, rows of other widths or off a 16-byte boundary, and to at most 16 experts: q8_route.cu.)  (Clusters, and one block for all: 8
+    // activations: then a block takes all experts of four tokens by itself.  (Above 148 tokens q8_route.cu takes
+    // most calls before they come here.)  (Clusters, and one block for all: 8
     // experts, 2048 wide, 512 tokens 15.4 us and 9.0, 4096 wide, 2048 tokens 160 and 24; 64 experts, 2048 wide, 512
     // tokens 17.2 and 29.3, 2048 tokens 64.1 and 57.2, 8192 wide, 300 tokens 74.3 and 53.2.)
     const bool few = tokens <= 36u;

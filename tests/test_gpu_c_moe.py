@@ -66,13 +66,14 @@ def test_route(ctx, oracle, tokens, experts, used, precision):
         assert (mass < 0.999).all()
 
 
+# (a live count on the device: the kernels with tiles take only what the host has counted)
 @pytest.mark.parametrize("tokens,experts,used,hidden,live", [
-    (149, 17, 3, 32, 149),        # a chunk that is one step; the fewest tokens and experts of the tiles
-    (153, 33, 4, 160, 150),       # two blocks of which one has one expert; a last group cut by the live count
-    (300, 128, 8, 2048, 297),     # eight tokens to a group, a ring that goes round
+    (149, 17, 3, 32, 149),        # rows of one step
+    (153, 33, 4, 160, 150),       # eight tokens to a cluster of four blocks; a last group cut by the live count
+    (300, 128, 8, 2048, 297),     # the same, full rounds of a row
     (593, 16, 2, 1120, 592),      # a block for all experts
-    (601, 5, 5, 288, 1),          # fewer experts than a block's, one live token
-    (1203, 250, 9, 1056, 1203)])  # the largest cluster, groups one behind the other
+    (601, 5, 5, 288, 1),          # the same, one live token
+    (1203, 250, 9, 1056, 1203)])  # groups one behind the other
 def test_route_of_many_tokens(ctx, oracle, tokens, experts, used, hidden, live):
     torch = torch_mod()
     rng = np.random.Generator(np.random.PCG64(tokens + experts))
@@ -100,14 +101,19 @@ def _off_boundary(t, values):
     return flat[values:].view(t.shape).copy_(t)
 
 
-# Every form of the tiles (tokens to a group, experts to a block) and every size of cluster, with a last group and a last
-# block that are not full; beside them the kernels that take rows off a boundary, for more than 148 tokens clusters of
-# four blocks, and one block for all experts where rows are long or tokens many and experts at most 64.
+# Every form of the tiles (tokens to a group, experts to a block, one block of an SM or two) and every size of cluster, with a
+# last group and a last block that are not full, and the sizes next to a line; beside them the kernels that take rows off a
+# boundary, for more than 148 tokens clusters of four blocks, and one block for all experts where rows are long or tokens
+# many and experts at most 64.  (Which form it is follows from how many clusters run at the same time, here as on a B200 with 15
+# clusters of seven.)
 @pytest.mark.parametrize("tokens,experts,used,hidden", [
-    (149, 17, 3, 32), (153, 33, 4, 160), (220, 136, 8, 512), (200, 192, 7, 1056),      # groups of 4, clusters of 1, 2, 5, 6
-    (257, 100, 8, 2048), (592, 64, 6, 288), (1000, 17, 2, 544), (180, 72, 5, 4096),    # groups of 8, clusters of 4, 2, 1, 3
-    (593, 64, 6, 288), (297, 128, 8, 2048), (300, 96, 8, 640), (149, 200, 8, 1024),    # groups of 16, clusters of 2, 4, 3, 7
-    (256, 224, 8, 4096), (256, 256, 8, 2048), (1203, 250, 9, 1056),                    # clusters of 7 and 8, groups one behind the other
+    (149, 17, 3, 32), (153, 33, 4, 160), (180, 72, 5, 4096),                           # groups of 4, clusters of 1, 2, 3
+    (1000, 17, 2, 544), (592, 64, 6, 288), (300, 96, 8, 640), (257, 100, 8, 2048),     # groups of 8, clusters of 1, 2, 3, 4
+    (200, 136, 8, 512), (161, 192, 7, 1056),                                           # clusters of 5, 6
+    (593, 64, 6, 288), (361, 96, 8, 640), (297, 128, 8, 2048), (220, 136, 8, 512),     # groups of 16, clusters of 2, 3, 4, 5
+    (200, 192, 7, 1056), (149, 200, 8, 1024), (150, 256, 3, 992),          # clusters of 6, 7, 8
+    (256, 224, 8, 4096), (256, 256, 8, 2048),                                          # two blocks to an SM, groups of 8
+    (1203, 250, 9, 1056), (1185, 48, 4, 256),                                          # groups of 16
     (150, 48, 3, 4128), (1201, 20, 4, 96),                                             # beside one block for all experts
     (593, 16, 2, 1120), (1300, 14, 2, 288)])                                           # a block for all of few experts, 8 and 16 tokens
 def test_router_tiles_give_the_floats_of_the_other_kernels(ctx, tokens, experts, used, hidden):
@@ -295,7 +301,8 @@ def test_grouped_path_equals_per_pair_path_at_full_size(ctx, oracle):
     assert ctx.device_status() == 0
 
 
-# a block for all experts of four tokens: few experts, long rows, many tokens; beside each the clusters that share them
+# A block for all experts of four tokens: few experts (149, 301, 2500 tokens), long rows of up to 47 (150); clusters that share
+# them (148); tiles (1024, 1025).
 @pytest.mark.parametrize("tokens,experts,hidden", [(149, 8, 512), (148, 8, 512), (301, 16, 2048), (150, 33, 4128), (1025, 64, 512),
                                                    (1024, 64, 512), (2500, 3, 96)])
 def test_router_on_both_sides_of_the_line(tokens, experts, hidden):
